@@ -42,154 +42,225 @@ __global__ void __launch_bounds__(DN_THREADS) pb_deltanet_kernel(const PbDeltaPa
     pb_stamp(p.stamps, 5, st_first); pb_stamp(p.stamps, 7, st_last);
 }
 
-// A run of T consecutive tokens of ONE sequence (a prefill chunk): the recurrence is sequential in the tokens, so the
-// CTA of (V head, 32 state columns) keeps its slice of S in registers for the whole run instead of one launch, one
-// read and one write of the state per token (the reference loops the tokens inside k_delta_m the same way,
-// src/model/qn_cube.rs:2839-2913).  Token j reads row j of proj (row stride ldp) and writes row j of out (stride ldo);
-// p.pos[0] is the position of token 0.  The conv history of in-window tokens comes from the earlier rows of proj, that
-// of the tokens before the window from the ring; the arithmetic per token is that of pb_deltanet_unit.
-template <int RPW>
-__global__ void __launch_bounds__(DN_THREADS) pb_deltanet_seq_kernel(const PbDeltaParams p, int T, const PbDeltaCk ck) {
+// ---- T consecutive tokens of ONE sequence (a prefill chunk, a verify window), in two kernels ----
+//
+// Only the state recurrence is sequential in the tokens.  Everything that feeds it -- conv + SiLU, L2 norms, gates -- is made for all
+// tokens at once by pb_deltanet_inputs_kernel; pb_deltanet_run_kernel then walks the tokens with its slice of S in registers.
+// What bounds the walk is the latency of one token: two dot products over dk, their reduction, the update.  A column of S is held by four
+// lanes (dk / 4 rows each, so the reduction is two shuffles), both dots run over the state as the previous token left it
+// (S'^T q = g (S^T q) + delta (k.q), with k.q made beforehand), the multiply-adds are packed pairs, and no barrier is taken per token:
+// the inputs of PB_DR_TB tokens at a time are brought into shared memory behind the computation.  256 tokens of 32 heads of 128 x 128:
+// 535 us as one kernel with six barriers per token, see the launcher for the present figure.
+// The reference loops the tokens inside k_delta_m (src/model/qn_cube.rs:2839-2913).
+#define PB_DR_TB 8       // tokens per block of inputs
+
+// scratch rows of the run: normalized q | k per K head, conv'd v, {decay, beta} per V head, k.q per K head
+struct PbDeltaRun { float* qk; float* v; float2* gb; float* kq; };
+
+// TB tokens per CTA: 8 for a chunk (the taps of neighbouring tokens are loaded once), 1 for a window, whose few tokens then spread over the GPU.
+// grid (token blocks, nk + nv), dk (q / k heads) or dv (v heads) threads at most 256 -- one channel (or one of q and one of k) per thread
+template <int TB>
+__global__ void __launch_bounds__(256) pb_deltanet_inputs_kernel(const PbDeltaParams p, int T, const PbDeltaRun r) {
     constexpr int K = 4;                                    // conv taps (checked by the launcher)
-    const int nk = p.nk, nv = p.nv, dk = p.dk, dv = p.dv;
-    const int splits = dv / DN_COLS;
-    const int h = blockIdx.x / splits, j0 = (blockIdx.x % splits) * DN_COLS;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ch = 2 * nk * dk + nv * dv, kh = h % nk;
-    extern __shared__ float sm[];
-    __shared__ float nrm[2];
-    float* qs = sm; float* ks = sm + dk; float* vs = sm + 2 * dk; float* red = sm + 2 * dk + DN_COLS;
+    const int nk = p.nk, nv = p.nv, dk = p.dk, dv = p.dv, ch = 2 * nk * dk + nv * dv;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    const int t0 = blockIdx.x * TB, t1 = min(T, t0 + TB);
+    const bool isv = (int)blockIdx.y >= nk;
+    const int head = isv ? (int)blockIdx.y - nk : (int)blockIdx.y;
+    __shared__ float red[2][3][8];
+    const int n = isv ? dv : dk;
+    const bool live = tid < n;
+    const int c0 = isv ? 2 * nk * dk + head * dv + tid : head * dk + tid, c1 = nk * dk + head * dk + tid;   // q and k channel, or the v channel
+    float w0[K], w1[K];
+    if (live) {
+#pragma unroll
+        for (int k = 0; k < K; k++) { w0[k] = p.conv_w[(size_t)c0 * K + k]; w1[k] = isv ? 0.f : p.conv_w[(size_t)c1 * K + k]; }
+    }
     pb_pdl_wait();
     pb_pdl_trigger();
     const int64_t pos0 = p.pos[0];
-    float* S = p.ssm + ((size_t)h * dk) * dv + j0 + lane;
-    float s[RPW];
+    // inputs of tokens t0 - 3 .. t1 - 1: rows of proj, before token 0 the ring slots of their positions
+    float x0[TB + K - 1], x1[TB + K - 1];
 #pragma unroll
-    for (int r = 0; r < RPW; r++) s[r] = S[(size_t)(warp * RPW + r) * dv];
-    // this thread's channels (at most two), their conv weights and the history before the window (oldest first)
-    const int nel = 2 * dk + DN_COLS;
-    float cw[2][K], hist[2][K - 1];
-    int cidx[2]; bool own[2];
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-        const int i = tid + e * DN_THREADS;
-        int c = 0;
-        if (i < nel) {
-            if (i < dk) c = kh * dk + i;
-            else if (i < 2 * dk) c = nk * dk + kh * dk + (i - dk);
-            else c = 2 * nk * dk + h * dv + j0 + (i - 2 * dk);
-#pragma unroll
-            for (int k = 0; k < K; k++) cw[e][k] = p.conv_w[c * K + k];
-#pragma unroll
-            for (int k = 0; k < K - 1; k++) hist[e][k] = p.conv[(size_t)((int)(pos0 % K) + 1 + k) % K * ch + c];
+    for (int i = 0; i < TB + K - 1; i++) {
+        const int j = t0 + i - (K - 1);
+        x0[i] = x1[i] = 0.f;
+        if (live && j < t1) {
+            const float* src = j >= 0 ? p.proj + (size_t)j * p.ldp : p.conv + (size_t)((pos0 + j + K) % K) * ch;
+            x0[i] = src[c0];
+            if (!isv) x1[i] = src[c1];
         }
-        cidx[e] = c;
-        own[e] = i < nel && (i >= 2 * dk || (h == kh && j0 == 0));
     }
-    const float dt_h = p.dt[h], a_h = p.a[h];
-    // inputs of token 0; those of token j + 1 are requested while token j is computed
-    float cur[2] = {0.f, 0.f}, alpha, beta;
 #pragma unroll
-    for (int e = 0; e < 2; e++) if (tid + e * DN_THREADS < nel) cur[e] = __ldcg(p.proj + cidx[e]);
-    alpha = __ldcg(p.proj + ch + nv * dv + nv + h); beta = __ldcg(p.proj + ch + nv * dv + h);
-    for (int j = 0; j < T; j++) {
-        float ncur[2] = {0.f, 0.f}, nalpha = 0.f, nbeta = 0.f;
-        if (j + 1 < T) {
-            const float* pn = p.proj + (size_t)(j + 1) * p.ldp;
+    for (int i = 0; i < TB; i++) {
+        const int j = t0 + i;
+        if (j >= t1) break;
+        // o = w[K-1] * cur + sum_{k < K-1} w[k] * hist[k], then SiLU   (:1645)
+        float a = 0.f, b = 0.f;
+        if (live) {
+            a = w0[K - 1] * x0[i + K - 1];
 #pragma unroll
-            for (int e = 0; e < 2; e++) if (tid + e * DN_THREADS < nel) ncur[e] = __ldcg(pn + cidx[e]);
-            nalpha = __ldcg(pn + ch + nv * dv + nv + h); nbeta = __ldcg(pn + ch + nv * dv + h);
-        }
-        // 1) conv + SiLU (:1645), history shifted by one
+            for (int k = 0; k < K - 1; k++) a = fmaf(w0[k], x0[i + k], a);
+            a = pb_silu(a);
+            if (!isv) {
+                b = w1[K - 1] * x1[i + K - 1];
 #pragma unroll
-        for (int e = 0; e < 2; e++) {
-            const int i = tid + e * DN_THREADS;
-            if (i < nel) {
-                float o = cw[e][K - 1] * cur[e];
-#pragma unroll
-                for (int k = 0; k < K - 1; k++) o = fmaf(cw[e][k], hist[e][k], o);
-                const float co = pb_silu(o);
-                if (i < dk) qs[i] = co; else if (i < 2 * dk) ks[i - dk] = co; else vs[i - 2 * dk] = co;
-#pragma unroll
-                for (int k = 0; k + 1 < K - 1; k++) hist[e][k] = hist[e][k + 1];
-                hist[e][K - 2] = cur[e];
-                if (own[e] && j + K > T) p.conv[(size_t)((pos0 + j) % K) * ch + cidx[e]] = cur[e];   // the ring keeps the last K inputs
+                for (int k = 0; k < K - 1; k++) b = fmaf(w1[k], x1[i + k], b);
+                b = pb_silu(b);
             }
         }
-        __syncthreads();
-        // 2) L2 norms (:1650-1651)
-        if (warp < 2) {
-            const float* src = warp == 0 ? qs : ks;
-            float ss = 0.f;
-            for (int i = lane; i < dk; i += 32) ss = fmaf(src[i], src[i], ss);
-            ss = pb_warp_sum(ss);
-            if (lane == 0) nrm[warp] = 1.0f / sqrtf(ss + 1e-6f) * (warp == 0 ? 1.0f / sqrtf((float)dk) : 1.0f);
+        if (isv) {
+            if (live) r.v[(size_t)j * nv * dv + head * dv + tid] = a;
+            if (tid == 0) {   // gates (:1660)
+                const float* pr = p.proj + (size_t)j * p.ldp + ch + nv * dv;
+                r.gb[(size_t)j * nv + head] = make_float2(expf(pb_softplus(pr[nv + head] + p.dt[head]) * p.a[head]), pb_sigm(pr[head]));
+            }
+        } else {
+            // x * (1/sqrt(sum x^2 + 1e-6)), q also times 1/sqrt(dk)  (:1650-1651); and k.q of the normalized vectors
+            const float sq = pb_warp_sum(a * a), sk = pb_warp_sum(b * b), sd = pb_warp_sum(a * b);
+            float (&rd)[3][8] = red[i & 1];
+            if (lane == 0) { rd[0][warp] = sq; rd[1][warp] = sk; rd[2][warp] = sd; }
+            __syncthreads();
+            float tq = 0.f, tk = 0.f, td = 0.f;
+            for (int w = 0; w < nw; w++) { tq += rd[0][w]; tk += rd[1][w]; td += rd[2][w]; }
+            const float fq = 1.0f / sqrtf(tq + 1e-6f) * (1.0f / sqrtf((float)dk)), fk = 1.0f / sqrtf(tk + 1e-6f);
+            float* dst = r.qk + ((size_t)j * nk + head) * 2 * dk;
+            if (live) { dst[tid] = a * fq; dst[dk + tid] = b * fk; }
+            if (tid == 0) r.kq[(size_t)j * nk + head] = td * fq * fk;
         }
-        __syncthreads();
-        for (int i = tid; i < 2 * dk; i += DN_THREADS) sm[i] *= nrm[i < dk ? 0 : 1];
-        __syncthreads();
-        // 3) gates (:1660), 4) state update and readout (:1663)
-        const float g = expf(pb_softplus(alpha + dt_h) * a_h);
-        const float bt = pb_sigm(beta);
-        float mem = 0.f;
-#pragma unroll
-        for (int r = 0; r < RPW; r++) {
-            const int i = warp * RPW + r;
-            s[r] *= g;
-            mem = fmaf(s[r], ks[i], mem);
-        }
-        red[warp * DN_COLS + lane] = mem;
-        __syncthreads();
-        mem = 0.f;
-#pragma unroll
-        for (int w = 0; w < 8; w++) mem += red[w * DN_COLS + lane];
-        const float delta = (vs[lane] - mem) * bt;
-        __syncthreads();
-        float o = 0.f;
-#pragma unroll
-        for (int r = 0; r < RPW; r++) {
-            const int i = warp * RPW + r;
-            s[r] = fmaf(ks[i], delta, s[r]);
-            o = fmaf(s[r], qs[i], o);
-        }
-        red[warp * DN_COLS + lane] = o;
-        __syncthreads();
-        if (warp == 0) {
-            o = 0.f;
-#pragma unroll
-            for (int w = 0; w < 8; w++) o += red[w * DN_COLS + lane];
-            p.out[(size_t)j * p.ldo + h * dv + j0 + lane] = o;
-        }
-        __syncthreads();   // red and the q / k / v vectors are rewritten by the next token
-        // rollback checkpoint after token j (k_delta_m writes them from registers too, src/model/qn_cube.rs:2839-2913): the
-        // state slice, and the K - 1 inputs the next token's conv reads, at their ring slots
-        if (j < 8 && j + 1 < T && ck.ssm[j]) {
-            float* C = ck.ssm[j] + ((size_t)h * dk) * dv + j0 + lane;
-#pragma unroll
-            for (int r = 0; r < RPW; r++) C[(size_t)(warp * RPW + r) * dv] = s[r];
-#pragma unroll
-            for (int e = 0; e < 2; e++)
-                if (own[e])
-#pragma unroll
-                    for (int k = 0; k < K - 1; k++) ck.conv[j][(size_t)((pos0 + j - (K - 2) + k + K) % K) * ch + cidx[e]] = hist[e][k];
-        }
-        cur[0] = ncur[0]; cur[1] = ncur[1]; alpha = nalpha; beta = nbeta;
     }
-#pragma unroll
-    for (int r = 0; r < RPW; r++) S[(size_t)(warp * RPW + r) * dv] = s[r];
 }
 
-// T consecutive tokens of sequence 0 in one launch; false when the shape is outside what the kernel is built for
-bool pb_deltanet_seq_supported(const PbDeltaParams& p) { return p.conv_k == 4 && p.dv % DN_COLS == 0 && (p.dk == 128 || p.dk == 64 || p.dk == 32) && 2 * p.dk + DN_COLS <= 2 * DN_THREADS; }
-int pb_launch_deltanet_seq(pb_ctx* ctx, const PbDeltaParams& p, int T, const PbDeltaCk* ckp) {
+__device__ __forceinline__ unsigned long long pb_f2(float a, float b) { unsigned long long v; asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); return v; }
+__device__ __forceinline__ float2 pb_f2_get(unsigned long long v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ unsigned long long pb_fma2(unsigned long long a, unsigned long long b, unsigned long long c) { unsigned long long d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ unsigned long long pb_add2(unsigned long long a, unsigned long long b) { unsigned long long d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ unsigned long long pb_mul2(unsigned long long a, unsigned long long b) { unsigned long long d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+
+// grid nv * dv / DN_COLS, 128 threads: lane = 4 * column + part; part r holds rows 16 m + 4 r + {0..3} of its column
+template <int DK, bool CK>
+__global__ void __launch_bounds__(128) pb_deltanet_run_kernel(const PbDeltaParams p, int T, const PbDeltaRun r, const PbDeltaCk ck) {
+    constexpr int K = 4, NM = DK / 16, ROW = 2 * DK + DN_COLS + 4;   // floats of one token's inputs: q | k | v | decay, beta, k.q
+    const int nk = p.nk, nv = p.nv, dv = p.dv;
+    const int splits = dv / DN_COLS, h = blockIdx.x / splits, j0 = (blockIdx.x % splits) * DN_COLS, kh = h % nk;
+    const int tid = threadIdx.x, lane = tid & 31, part = lane & 3, col = (tid >> 5) * 8 + (lane >> 2);
+    const int ch = 2 * nk * DK + nv * dv;
+    __shared__ __align__(16) float in[2][PB_DR_TB][ROW];
+    pb_pdl_wait();
+    pb_pdl_trigger();
+    auto fetch = [&](int t0, int buf) {
+        const int n = min(PB_DR_TB, T - t0);
+        constexpr int PQ = 2 * DK / 4, PV = DN_COLS / 4;
+        for (int i = tid; i < n * (PQ + PV); i += 128) {
+            const int t = i / (PQ + PV), c = i - t * (PQ + PV);
+            const float* src = c < PQ ? r.qk + ((size_t)(t0 + t) * nk + kh) * 2 * DK + 4 * c : r.v + (size_t)(t0 + t) * nv * dv + h * dv + j0 + 4 * (c - PQ);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(pb_smem_u32(&in[buf][t][4 * c])), "l"(src) : "memory");
+        }
+        if (tid < 3 * n) {
+            const int t = tid / 3, c = tid - 3 * t;
+            const float* src = c < 2 ? reinterpret_cast<const float*>(r.gb + (size_t)(t0 + t) * nv + h) + c : r.kq + (size_t)(t0 + t) * nk + kh;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(pb_smem_u32(&in[buf][t][2 * DK + DN_COLS + c])), "l"(src) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0, 0);
+    float* S = p.ssm + ((size_t)h * DK) * dv + j0 + col;
+    unsigned long long s[2 * NM];
+#pragma unroll
+    for (int m = 0; m < NM; m++) {
+        const float* c = S + (size_t)(16 * m + 4 * part) * dv;
+        s[2 * m] = pb_f2(c[0], c[dv]); s[2 * m + 1] = pb_f2(c[2 * (size_t)dv], c[3 * (size_t)dv]);
+    }
+    auto store = [&](float* base) {
+#pragma unroll
+        for (int m = 0; m < NM; m++) {
+            float* c = base + (size_t)(16 * m + 4 * part) * dv;
+            const float2 a = pb_f2_get(s[2 * m]), b = pb_f2_get(s[2 * m + 1]);
+            c[0] = a.x; c[dv] = a.y; c[2 * (size_t)dv] = b.x; c[3 * (size_t)dv] = b.y;
+        }
+    };
+    int buf = 0;
+    for (int t0 = 0; t0 < T; t0 += PB_DR_TB, buf ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                    // this block's inputs have landed; the other buffer is free
+        if (t0 + PB_DR_TB < T) fetch(t0 + PB_DR_TB, buf ^ 1);
+        const int n = min(PB_DR_TB, T - t0);
+        // k and q of a token are read from shared memory while the token before it is computed
+        unsigned long long k2[2 * NM], q2[2 * NM];
+        auto load = [&](int t, unsigned long long (&kk)[2 * NM], unsigned long long (&qq)[2 * NM]) {
+            const float* x = in[buf][t] + 4 * part;
+#pragma unroll
+            for (int m = 0; m < NM; m++) {
+                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(x + 16 * m), b = *reinterpret_cast<const ulonglong2*>(x + DK + 16 * m);
+                qq[2 * m] = a.x; qq[2 * m + 1] = a.y; kk[2 * m] = b.x; kk[2 * m + 1] = b.y;
+            }
+        };
+        load(0, k2, q2);
+#pragma unroll 2
+        for (int t = 0; t < n; t++) {
+            const float* x = in[buf][t];
+            const float g = x[2 * DK + DN_COLS], bt = x[2 * DK + DN_COLS + 1], kq = x[2 * DK + DN_COLS + 2], v = x[2 * DK + col];
+            unsigned long long a[4] = {0, 0, 0, 0}, b[4] = {0, 0, 0, 0}, kn[2 * NM], qn[2 * NM];   // zeros: pairs of f32 0
+#pragma unroll
+            for (int i = 0; i < 2 * NM; i++) { a[i & 3] = pb_fma2(s[i], k2[i], a[i & 3]); b[i & 3] = pb_fma2(s[i], q2[i], b[i & 3]); }
+            load(t + 1 < n ? t + 1 : t, kn, qn);
+            const float2 ax = pb_f2_get(pb_add2(pb_add2(a[0], a[1]), pb_add2(a[2], a[3]))), bx = pb_f2_get(pb_add2(pb_add2(b[0], b[1]), pb_add2(b[2], b[3])));
+            float mem = ax.x + ax.y, oq = bx.x + bx.y;
+            mem += __shfl_xor_sync(0xffffffffu, mem, 1); oq += __shfl_xor_sync(0xffffffffu, oq, 1);
+            mem += __shfl_xor_sync(0xffffffffu, mem, 2); oq += __shfl_xor_sync(0xffffffffu, oq, 2);
+            const unsigned long long g2 = pb_f2(g, g);
+#pragma unroll
+            for (int i = 0; i < 2 * NM; i++) s[i] = pb_mul2(s[i], g2);
+            const float delta = (v - g * mem) * bt;         // mem_j = sum_i (g S[i][j]) k_i   (:1663)
+            const unsigned long long d2 = pb_f2(delta, delta);
+#pragma unroll
+            for (int i = 0; i < 2 * NM; i++) s[i] = pb_fma2(k2[i], d2, s[i]);
+            const int j = t0 + t;
+            if (part == 0) p.out[(size_t)j * p.ldo + h * dv + j0 + col] = fmaf(delta, kq, g * oq);   // readout before the gated norm
+            if (CK && j < 8 && j + 1 < T && ck.ssm[j]) store(ck.ssm[j] + ((size_t)h * DK) * dv + j0 + col);   // rollback checkpoint after token j
+#pragma unroll
+            for (int i = 0; i < 2 * NM; i++) { k2[i] = kn[i]; q2[i] = qn[i]; }
+        }
+    }
+    store(S);
+    // the conv ring keeps the last K inputs, a checkpoint the K - 1 inputs the next token's conv reads, at their ring slots.  Channels:
+    // this slice's v columns; q and k of a K head by the first slice of the first V head that reads it
+    const int64_t pos0 = p.pos[0];
+    const int nel = DN_COLS + (h == kh && j0 == 0 ? 2 * DK : 0);
+    for (int i = tid; i < nel; i += 128) {
+        const int c = i < DN_COLS ? 2 * nk * DK + h * dv + j0 + i : (i - DN_COLS < DK ? kh * DK + i - DN_COLS : nk * DK + kh * DK + i - DN_COLS - DK);
+        float before[K - 1];                                // inputs at positions pos0 - 3 .. pos0 - 1
+#pragma unroll
+        for (int k = 0; k < K - 1; k++) before[k] = p.conv[(size_t)((pos0 + 1 + k) % K) * ch + c];
+        for (int j = 0; CK && j < 8 && j + 1 < T; j++)
+            if (ck.conv[j])
+#pragma unroll
+                for (int k = 0; k < K - 1; k++) {
+                    const int jj = j - (K - 2) + k;
+                    ck.conv[j][(size_t)((pos0 + jj + K) % K) * ch + c] = jj >= 0 ? p.proj[(size_t)jj * p.ldp + c] : before[jj + K - 1];
+                }
+        for (int j = max(0, T - K); j < T; j++) p.conv[(size_t)((pos0 + j) % K) * ch + c] = p.proj[(size_t)j * p.ldp + c];
+    }
+}
+
+// T consecutive tokens of sequence 0; false when the shape is outside what the kernels are built for
+bool pb_deltanet_seq_supported(const PbDeltaParams& p) { return p.conv_k == 4 && p.dv % DN_COLS == 0 && p.dv <= 256 && (p.dk == 128 || p.dk == 64 || p.dk == 32); }
+size_t pb_deltanet_seq_scratch(const PbDeltaParams& p, int T) { return (size_t)T * (2 * p.nk * p.dk + p.nv * p.dv + 2 * p.nv + p.nk) + 16; }   // floats
+int pb_launch_deltanet_seq(pb_ctx* ctx, const PbDeltaParams& p, int T, float* scratch, const PbDeltaCk* ckp) {
     if (!pb_deltanet_seq_supported(p)) PB_FAIL(ctx, PB_UNSUPPORTED, "deltanet run: dk=%d dv=%d conv_k=%d not supported", p.dk, p.dv, p.conv_k);
     PbDeltaCk ck; memset(&ck, 0, sizeof ck);
     if (ckp) ck = *ckp;
+    PbDeltaRun r;
+    r.qk = scratch; r.v = r.qk + (size_t)T * 2 * p.nk * p.dk; r.gb = reinterpret_cast<float2*>(r.v + (size_t)T * p.nv * p.dv); r.kq = reinterpret_cast<float*>(r.gb + (size_t)T * p.nv);
+    const int wide = p.dk > p.dv ? p.dk : p.dv;
+    if (T >= 32) pb_launch_k(ctx, pb_deltanet_inputs_kernel<8>, dim3((T + 7) / 8, p.nk + p.nv), dim3((wide + 31) & ~31), (size_t)0, p, T, r);
+    else pb_launch_k(ctx, pb_deltanet_inputs_kernel<1>, dim3(T, p.nk + p.nv), dim3((wide + 31) & ~31), (size_t)0, p, T, r);
+    ctx->kernels_launched++;
+    PB_CUDA(ctx, cudaGetLastError());
     const dim3 grid(p.nv * (p.dv / DN_COLS));
-    const size_t smem = (size_t)(2 * p.dk + DN_COLS + 8 * DN_COLS) * 4;
-    if (p.dk == 128) pb_launch_k(ctx, pb_deltanet_seq_kernel<16>, grid, dim3(DN_THREADS), smem, p, T, ck);
-    else if (p.dk == 64) pb_launch_k(ctx, pb_deltanet_seq_kernel<8>, grid, dim3(DN_THREADS), smem, p, T, ck);
-    else pb_launch_k(ctx, pb_deltanet_seq_kernel<4>, grid, dim3(DN_THREADS), smem, p, T, ck);
+#define GO(DK) { if (ckp) pb_launch_k(ctx, pb_deltanet_run_kernel<DK, true>, grid, dim3(128), (size_t)0, p, T, r, ck); else pb_launch_k(ctx, pb_deltanet_run_kernel<DK, false>, grid, dim3(128), (size_t)0, p, T, r, ck); }
+    if (p.dk == 128) GO(128) else if (p.dk == 64) GO(64) else GO(32)
+#undef GO
     ctx->kernels_launched++;
     PB_CUDA(ctx, cudaGetLastError());
     return PB_OK;

@@ -71,7 +71,7 @@ struct pb_state {
     float *x = nullptr, *xin = nullptr, *proj = nullptr, *olin = nullptr, *att = nullptr, *rlogits = nullptr, *yout = nullptr;
     uint32_t* xq = nullptr;
     int *sel_e = nullptr, *n_used = nullptr, *used_e = nullptr, *used_off = nullptr, *ent_tok = nullptr, *ent_slot = nullptr;
-    uint32_t* hq = nullptr;
+    uint32_t* hq = nullptr; float* dn_run = nullptr;   // dn_run: inputs of a DeltaNet run, all tokens of a window or chunk
     float *sel_w = nullptr, *ent_w = nullptr, *h = nullptr, *h_sh = nullptr, *part = nullptr, *part_sh = nullptr, *logits = nullptr;
     float *part_ml = nullptr, *part_acc = nullptr;
     int nsplit = 1, nsplit_packed = 0;
@@ -488,6 +488,11 @@ static int state_create(pb_model* m, int batch, bool sharded, pb_state** out) {
         for (int i = 0; i < m->n_ple; i++) { if (rc == PB_OK) rc = dalloc(s, &s->ple_ring[(size_t)i], (size_t)B * s->ple_R * w); }
     }
     if (c.hc > 0) { A(hxn, (size_t)Ba * c.hc * c.d); A(hgate, (size_t)Ba * c.hc * c.d); A(hlo, (size_t)Ba * c.hc_lr); A(hinj, (size_t)Ba * c.hc); A(hmix, (size_t)Ba * c.d); }
+    if (solo && m->n_lin > 0) {
+        PbDeltaParams dp; memset(&dp, 0, sizeof dp);
+        dp.nk = c.lin_nk; dp.nv = c.lin_nv; dp.dk = c.lin_dk; dp.dv = c.lin_dv;
+        A(dn_run, pb_deltanet_seq_scratch(dp, PB_PREFILL_CHUNK));
+    }
     A(xin, (size_t)Ba * (wide > c.d ? wide : c.d)); A(yout, (size_t)Ba * c.d);
     A(proj, (size_t)Ba * s->ldproj); A(olin, (size_t)Ba * wide); A(att, (size_t)Ba * wide);
     A(rlogits, (size_t)Bm * (c.n_exp + 1));
@@ -701,7 +706,7 @@ static int run_lin(pb_state* s, int il, const float* x_in, const float* norm_w, 
         d.pos = s->wpos; d.batch = 1;
         PbDeltaCk ck; memset(&ck, 0, sizeof ck);
         if (s->win_ckpt) for (int j = 0; j + 1 < s->win_t; j++) { ck.conv[j] = s->ck_conv[(size_t)li * PB_MAX_WINDOW + j]; ck.ssm[j] = s->ck_ssm[(size_t)li * PB_MAX_WINDOW + j]; }
-        PB_TRY(pb_launch_deltanet_seq(ctx, d, s->win_t, s->win_ckpt ? &ck : nullptr));
+        PB_TRY(pb_launch_deltanet_seq(ctx, d, s->win_t, s->dn_run, s->win_ckpt ? &ck : nullptr));
     } else if (s->win_t > 0) {
         // the recurrence is sequential: one launch per token, with a rollback checkpoint after each but the last
         for (int j = 0; j < s->win_t; j++) {
