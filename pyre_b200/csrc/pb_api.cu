@@ -8,6 +8,9 @@
 #include <string.h>
 #include <new>
 #include <pthread.h>
+#include <map>
+#include <mutex>
+#include <utility>
 
 static const char* kNoCtx = "pyre_b200: null context";
 
@@ -25,6 +28,36 @@ unsigned long long* pb_stamp_slot(pb_ctx* ctx, int kernel_id) {
     if (!ctx->stamps || ctx->stamp_next >= ctx->stamp_slots) return nullptr;
     ctx->stamp_ids[ctx->stamp_next] = kernel_id;
     return ctx->stamps + (size_t)PB_STAMP_WORDS * ctx->stamp_next++;
+}
+
+int pb_ensure_smem_fn(pb_ctx* ctx, const void* kern, size_t smem) {
+    static std::mutex mu;
+    static std::map<std::pair<int, const void*>, size_t> limit;   // (device, function) -> limit set so far
+    std::lock_guard<std::mutex> lock(mu);
+    size_t& have = limit[{ctx->device, kern}];
+    if (have >= smem) return PB_OK;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) PB_FAIL(ctx, PB_ERR_CUDA, "cudaFuncSetAttribute(%zu bytes of shared memory): %s", smem, cudaGetErrorString(e));
+    have = smem;
+    return PB_OK;
+}
+
+int pb_max_clusters(pb_ctx* ctx, const void* kern, int threads, size_t smem, int cluster) {
+    if (cluster <= 1) return ctx->sm_count;
+    static std::mutex mu;
+    static std::map<std::pair<std::pair<int, const void*>, std::pair<size_t, int>>, int> known;
+    std::lock_guard<std::mutex> lock(mu);
+    int& n = known[{{ctx->device, kern}, {smem, cluster * 1024 + threads}}];
+    if (n == 0) {
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof cfg);
+        cfg.gridDim = dim3((unsigned)(ctx->sm_count / cluster * cluster)); cfg.blockDim = dim3((unsigned)threads); cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = (unsigned)cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        cfg.attrs = at; cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = ctx->sm_count / cluster; }
+    }
+    return n;
 }
 
 int pb_scratch(pb_ctx* ctx, size_t bytes, void** out) {
@@ -211,13 +244,13 @@ static int qmat_alloc(pb_ctx* ctx, int type, int64_t rows, int64_t cols, pb_qmat
 static int qmat_recode(pb_ctx* ctx, pb_qmat* m) {
     static const bool on = !(getenv("PYRE_B200_REPACK") && atoi(getenv("PYRE_B200_REPACK")) == 0);
     const int64_t bpr = m->cols / 256;
-    if (!on || m->type != PB_T_IQ3_S || m->cols % 256 || (bpr & 1)) return PB_OK;   // rows of the copy must stay 16-byte aligned
+    if (!on || m->type != PB_T_IQ3_S || m->cols % 256) return PB_OK;
     m->r_row_bytes = bpr * 136;
-    const size_t nb = (size_t)m->rows * (size_t)m->r_row_bytes;
+    const size_t nb = (size_t)((m->rows + 7) / 8 * 8) * (size_t)m->r_row_bytes;   // whole groups of eight rows
     cudaError_t e = cudaMalloc(&m->rdata, nb + 256);
     if (e != cudaSuccess) { m->rdata = nullptr; PB_FAIL(ctx, PB_ERR_OOM, "cudaMalloc(%zu) for the re-coded copy: %s", nb + 256, cudaGetErrorString(e)); }
     cudaMemsetAsync(m->rdata + nb, 0, 256, ctx->stream);
-    return pb_launch_repack_iq3s(ctx, m->data, m->rdata, m->rows * bpr);
+    return pb_launch_repack_iq3s(ctx, m->data, m->rdata, m->rows, (int)bpr);
 }
 
 int pb_qmat_upload(pb_ctx* ctx, int type, int64_t rows, int64_t cols, const void* bytes, size_t nbytes, pb_qmat** out) {

@@ -70,6 +70,7 @@ struct pb_state {
     int64_t* pos = nullptr; uint32_t* ids = nullptr; uint32_t* next = nullptr; unsigned long long* amax = nullptr; unsigned int* ticket = nullptr;
     float *x = nullptr, *xin = nullptr, *proj = nullptr, *olin = nullptr, *att = nullptr, *rlogits = nullptr, *yout = nullptr;
     uint32_t* xq = nullptr;
+    int4* virt = nullptr; float* tok_scale = nullptr;   // groups of entries and token scales for the tensor-core expert kernels
     int *sel_e = nullptr, *n_used = nullptr, *used_e = nullptr, *used_off = nullptr, *ent_tok = nullptr, *ent_slot = nullptr;
     uint32_t* hq = nullptr; float* dn_run = nullptr;   // dn_run: inputs of a DeltaNet run, all tokens of a window or chunk
     float *sel_w = nullptr, *ent_w = nullptr, *h = nullptr, *h_sh = nullptr, *part = nullptr, *part_sh = nullptr, *logits = nullptr;
@@ -487,18 +488,19 @@ static int state_create(pb_model* m, int batch, bool sharded, pb_state** out) {
         s->ple_ring.assign((size_t)m->n_ple, nullptr);
         for (int i = 0; i < m->n_ple; i++) { if (rc == PB_OK) rc = dalloc(s, &s->ple_ring[(size_t)i], (size_t)B * s->ple_R * w); }
     }
-    if (c.hc > 0) { A(hxn, (size_t)Ba * c.hc * c.d); A(hgate, (size_t)Ba * c.hc * c.d); A(hlo, (size_t)Ba * c.hc_lr); A(hinj, (size_t)Ba * c.hc); A(hmix, (size_t)Ba * c.d); }
     if (solo && m->n_lin > 0) {
         PbDeltaParams dp; memset(&dp, 0, sizeof dp);
         dp.nk = c.lin_nk; dp.nv = c.lin_nv; dp.dk = c.lin_dk; dp.dv = c.lin_dv;
         A(dn_run, pb_deltanet_seq_scratch(dp, PB_PREFILL_CHUNK));
     }
+    if (c.hc > 0) { A(hxn, (size_t)Ba * c.hc * c.d); A(hgate, (size_t)Ba * c.hc * c.d); A(hlo, (size_t)Ba * c.hc_lr); A(hinj, (size_t)Ba * c.hc); A(hmix, (size_t)Ba * c.d); }
     A(xin, (size_t)Ba * (wide > c.d ? wide : c.d)); A(yout, (size_t)Ba * c.d);
     A(proj, (size_t)Ba * s->ldproj); A(olin, (size_t)Ba * wide); A(att, (size_t)Ba * wide);
     A(rlogits, (size_t)Bm * (c.n_exp + 1));
     A(xq, (size_t)Bm * pb_xq_words(c.d));
     A(sel_e, (size_t)Bm * c.top_k); A(sel_w, (size_t)Bm * c.top_k); A(n_used, 4); A(used_e, c.n_exp + 1); A(used_off, c.n_exp + 2);
     A(ent_tok, (size_t)Bm * c.top_k); A(ent_slot, (size_t)Bm * c.top_k); A(ent_w, (size_t)Bm * c.top_k);
+    A(virt, (size_t)c.n_exp + (size_t)Bm * c.top_k / PB_VGROUP + 1); A(tok_scale, Bm);
     A(h, (size_t)Bm * c.top_k * c.ff_exp); A(h_sh, (size_t)Bm * c.ff_sh);
     A(hq, (size_t)Bm * (c.top_k + 1) * pb_xq_words(c.ff_exp > c.ff_sh ? c.ff_exp : c.ff_sh));
     A(part, (size_t)Bm * c.top_k * c.d); A(part_sh, (size_t)Bm * c.d);
@@ -673,9 +675,9 @@ static void seg(PbGemvQArgs& a, int i, pb_qmat* q, int64_t yoff) { a.seg[i].w = 
 static int gemv_cols(pb_ctx* ctx, PbGemvQArgs a, int B, bool prefill = false) {
     const float* x = a.x; float* y = a.y; const float* z = a.z; const uint32_t* xq = a.xq_in;
     a.exact = prefill ? 0 : 1;   // decode steps and verify windows keep exact weights; prefill chunks may take the tcgen05 GEMM
-    // the tensor-core path takes all columns at once (one staging pass for all its launches)
+    // the tensor-core paths take all columns at once
     static const bool use_mma = !(getenv("PYRE_B200_MMA") && atoi(getenv("PYRE_B200_MMA")) == 0);
-    if (use_mma && a.mode != PB_ACT_PREQ && pb_gemmh_supported(a.type, a.cols, B) && (size_t)B * a.cols * 4 + 256 * (size_t)((B + 7) / 8) <= PB_XH_BYTES) { a.t = B; return pb_launch_gemvq(ctx, a); }
+    if (use_mma && a.mode != PB_ACT_PREQ && pb_gemmh_supported(a.type, a.cols, B)) { a.t = B; return pb_launch_gemvq(ctx, a); }
     for (int b0 = 0; b0 < B; b0 += 16) {
         a.t = B - b0 < 16 ? B - b0 : 16;
         a.x = x ? x + (int64_t)b0 * a.ldx : nullptr; a.y = y + (int64_t)b0 * a.ldy; a.z = z ? z + (int64_t)b0 * a.ldz : nullptr;
@@ -805,6 +807,16 @@ static int run_attn(pb_state* s, int il, const float* x_in, const float* norm_w,
     return gemv_cols(ctx, o, ncol, prefill);
 }
 
+// whether the expert kernels of layer il run on the tensor cores for t tokens (the type the kernels stream: re-coded copies where all have one)
+static bool expert_mma(pb_model* m, int il, int t) {
+    const pb_cfg& c = m->cfg;
+    const int roles[6] = {PB_R_EXP_GATE, PB_R_EXP_UP, PB_R_SH_GATE, PB_R_SH_UP, PB_R_EXP_DOWN, PB_R_SH_DOWN};
+    int type = M(m, il, PB_R_EXP_GATE)->type;
+    for (int r : roles) if (M(m, il, r)->type != type) return false;
+    if (type == PB_T_IQ3_S) { for (int r : roles) if (!M(m, il, r)->rdata) return false; type = PB_T_IQ3S_N4; }
+    return c.ff_exp == c.ff_sh && pb_moeh_supported(type, c.d, c.ff_exp, t);
+}
+
 // MoE block on t tokens: x_in [t][d] (normalized when norm_w == null) -> y (stored or added)
 static int run_moe(pb_state* s, int il, const float* x_in, const float* norm_w, int t, float* y, int64_t ldy, int accumulate) {
     pb_model* m = s->m; pb_ctx* ctx = m->ctx; const pb_cfg& c = m->cfg;
@@ -815,11 +827,13 @@ static int run_moe(pb_state* s, int il, const float* x_in, const float* norm_w, 
     PbRouterParams r; memset(&r, 0, sizeof r);
     r.cols = c.d; r.norm_w = norm_w; r.eps = c.eps;
     r.router = reinterpret_cast<const float*>(M(m, il, PB_R_ROUTER)->data); r.sh_gate_inp = V(m, il, PB_R_SH_GATE_INP); r.n_exp = c.n_exp;
-    r.xq_out = s->xq;
     PbRouteParams q; memset(&q, 0, sizeof q);
     q.t = tt; q.n_exp = c.n_exp; q.top_k = c.top_k; q.e_lo = m->e_lo; q.e_hi = m->e_hi;
     q.sel_e = s->sel_e; q.sel_w = s->sel_w; q.n_used = s->n_used; q.used_e = s->used_e; q.used_off = s->used_off;
     q.ent_tok = s->ent_tok; q.ent_slot = s->ent_slot; q.ent_w = s->ent_w;
+    // two and more tokens of the formats it covers: the expert kernels on the tensor cores, which read the token rows themselves
+    const bool moeh = expert_mma(m, il, tt);
+    if (moeh) { r.scale_out = s->tok_scale; q.virt = s->virt; q.n_virt = s->n_used + 1; } else r.xq_out = s->xq;
     const float* logits; int64_t ldl;
     if (sh) {
         // router logits of the local tokens, written next to a copy of their residual rows; one all-gather
@@ -850,7 +864,9 @@ static int run_moe(pb_state* s, int il, const float* x_in, const float* norm_w, 
     int gu_type = g->type;
     if (g->rdata && up->rdata && shg->rdata && shu->rdata) { e.w_a = g->rdata; e.w_b = up->rdata; e.sh_a = shg->rdata; e.sh_b = shu->rdata; gu_type = PB_T_IQ3S_N4; }   // re-coded copies
     e.rows_e = c.ff_exp; e.rows_sh = c.ff_sh;
-    PB_TRY(pb_launch_expert_gu(ctx, e, gu_type, c.d));
+    if (tt > s->moe_cap) PB_FAIL(ctx, PB_ERR_ARG, "MoE block on %d tokens, buffers hold %d", tt, s->moe_cap);
+    if (moeh) { e.virt = s->virt; e.n_virt = s->n_used + 1; e.x = r.x; e.ldx = r.ldx; e.norm_w = norm_w; e.tok_scale = s->tok_scale; PB_TRY(pb_launch_moeh_gu(ctx, e, gu_type, c.d)); }
+    else PB_TRY(pb_launch_expert_gu(ctx, e, gu_type, c.d));
     pb_qmat* dn = M(m, il, PB_R_EXP_DOWN);
     e.e_base = dn->rows == (int64_t)c.d * c.n_exp ? 0 : m->e_lo;
     pb_qmat* shd = M(m, il, PB_R_SH_DOWN);
@@ -858,7 +874,6 @@ static int run_moe(pb_state* s, int il, const float* x_in, const float* norm_w, 
     int dn_type = dn->type;
     if (dn->rdata && shd->rdata) { e.w_a = dn->rdata; e.sh_a = shd->rdata; dn_type = PB_T_IQ3S_N4; }
     e.rows_e = c.d; e.rows_sh = c.d;
-    if (tt > s->moe_cap) PB_FAIL(ctx, PB_ERR_ARG, "MoE block on %d tokens, buffers hold %d", tt, s->moe_cap);
     e.hq = tt > 1 && c.ff_exp == c.ff_sh ? s->hq : nullptr;   // several tokens: levels of the hidden vectors made once
     PbCombineParams k; memset(&k, 0, sizeof k);
     k.part = s->part; k.part_sh = s->part_sh + (size_t)tok0 * c.d; k.logits = logits + (size_t)tok0 * ldl; k.ldl = ldl; k.t = t; k.d = c.d; k.top_k = c.top_k; k.n_exp = c.n_exp;
@@ -866,8 +881,9 @@ static int run_moe(pb_state* s, int il, const float* x_in, const float* norm_w, 
     if (sh && s->p2p) e.part_tok = s->part_tok;            // finished rows go straight into the memory of the token's owner
     k.y = y; k.ldy = ldy; k.accumulate = accumulate;
     // few tokens on one GPU: the down kernel's last CTA also combines (one launch less per layer)
-    if (m->ep_world == 1 && (int64_t)t * c.d <= 8192) return pb_launch_expert_down(ctx, e, dn_type, c.ff_exp, &k, s->ticket + 1);
-    PB_TRY(pb_launch_expert_down(ctx, e, dn_type, c.ff_exp));
+    if (moeh) PB_TRY(pb_launch_moeh_down(ctx, e, dn_type, c.ff_exp));
+    else if (m->ep_world == 1 && (int64_t)t * c.d <= 8192) return pb_launch_expert_down(ctx, e, dn_type, c.ff_exp, &k, s->ticket + 1);
+    else PB_TRY(pb_launch_expert_down(ctx, e, dn_type, c.ff_exp));
     // expert parallelism: every (token, slot) row was produced on exactly one rank and is zero elsewhere,
     // so the sum is an exact gather and the combine below sees the same bits for every GPU count
     if (sh && s->p2p) { k.exch = s->exch_dev; k.exch_idx = 2 * il + 1; k.part = s->part_rs; }   // the combine kernel announces and waits

@@ -1,406 +1,270 @@
-// Batched dequant-GEMM for 4..16 activation columns on the tensor cores (IQ3_S weights).
+// Batched dequant-GEMM for 2 .. 16 activation columns a launch on the tensor cores, every quantized format (core: pb_hmma.cuh).
 //
-//   y[b][yoff_s + r] (+)= sum_c W_s[r][c] * act(x)[b][c]        b = 0 .. t-1 (t <= 16)
+//   y[b][yoff_s + r] (+)= sum_c W_s[r][c] * act(x)[b][c]        b = 0 .. t-1
 //
-// Used where one weight matrix meets several tokens at once (batched decode, verify windows):
-// the weight bytes are streamed and decoded ONCE for all columns, instead of once per column
-// as in the dp4a GEMV.  Same streaming skeleton (persistent CTAs, producer warp, 1-D bulk
-// copies into a 4-stage ring, bounded mbarrier waits); the arithmetic is
-// mma.sync.m16n8k16 (f16 x f16 -> f32):
-//   - A = 16 rows of decoded weights.  The codebook lives in shared memory as four f16 per
-//     entry; the sub-block multiplier (1 + 2*s <= 31) is folded in exactly (|w| <= 465), the f16
-//     block scale d is applied in f32 once per 256-weight block.
-//   - B = activations split into f16 high and low parts (x = hi + lo, 22 significant bits),
-//     laid out in shared memory in fragment order; an n-tile holds 4 tokens x (hi, lo), so a
-//     thread owns both halves of its tokens and adds them itself.
-//   - the contraction index inside a block is permuted so that thread q of a quad owns the 64
-//     consecutive weights of quarter q (one decode per lane, as in the GEMV); A and B use the
-//     same permutation, so the sum is unchanged.
-// A chunk is 16 rows; the eight consumer warps split its blocks (K) and meet in shared memory.
-// Replaces the reference's batched GEMV / prefill GEMM (k_gemv4*, k_gemm_pf / k_gemm_tc,
-// src/model/qn_cube.rs:71-233, 293-1159) for IQ3_S; other formats keep the dp4a kernel.
-#include "pb_stream.cuh"
+// Used where one weight matrix meets several tokens at once (batched decode, verify windows): the weights are streamed and decoded ONCE for
+// all columns, instead of once per column as in the dp4a GEMV.  Persistent CTAs, one per SM; the 16-row tiles of all segments are dealt to the
+// CTAs in contiguous runs.  A CTA prepares the activations (none / RMSNorm / per-head gated norm, f16 high + low parts) in its shared memory
+// while its warps already load their first weights, then every warp takes whole tiles on its own: no barrier in the loop.  What is left of
+// a run after whole rounds of one tile per warp -- or all of a small matrix -- is cut along the contraction: 2, 4, .. warps share a tile, each
+// takes a run of its blocks, and their sums meet in shared memory.  Without that cut a 12352-row matrix keeps a third of the warps busy, and a
+// 151936-row one (64.2 tiles per CTA) waits a fifth of its time for the last round.
+// Rows of 4096 columns, and small matrices with more than four tokens, are cut along the contraction over a cluster of CTAs as well: each prepares
+// and keeps only its part of the activations (the preparation of 8 tokens x 4096 columns in every CTA took longer than the product: 23 us a
+// launch against 7), and the parts' sums are read from the partners' shared memory, in rank order.
+// Replaces the reference's batched GEMV / prefill GEMM (k_gemv4*, k_gemm_pf / k_gemm_tc, src/model/qn_cube.rs:71-233, 293-1159).
+#include "pb_hmma.cuh"
 #include "pb_internal.h"
 
-#include <cuda_fp16.h>
 #include <stdio.h>
 
-#define GH_CONSUMERS 8
-#define GH_THREADS ((GH_CONSUMERS + 1) * 32)
-#define GH_ROWS 16
+#define GH_WARPS 16
+#define GH_MAXBLK 16         // blocks of 256 columns per row at most
+#define GH_HEAD (16 * GH_MAXBLK * 4)   // bytes in front of the tables: partial sums of squares [16 tokens][blocks]
 
-__device__ __forceinline__ void pb_mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+struct PbGemmHParams {
+    PbGemvQParams q;         // seg[].chunk0 = first 16-row tile of the segment, nchunks = tiles in all
+    PbHGeom g;
+    int stages;              // weight stages of a warp
+    int ks;                  // CTAs of a cluster; each takes bpr / ks blocks of every row
+    uint32_t off_act, off_red, off_stage;
+};
+
+__device__ __forceinline__ void gh_cluster_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ float gh_remote(uint32_t saddr, int rank) {
+    uint32_t a; float v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
 }
 
-// One quarter (64 weights) of an IQ3_S block as 32 half2 words with the sub-block multiplier and
-// the signs applied; returns the block scale d.  tab_h: this lane's copy of the f16 codebook (512 x 4 f16,
-// four interleaved copies: entry i of copy c at (4 i + c) * 8 bytes, so lanes of different copies never share a bank).
-__device__ __forceinline__ float pb_iq3s_quarter_h(uint32_t p, int qt, uint32_t tab_h, uint32_t (&h)[32]) {
-    const float d = pb_h2f((uint16_t)pb_lds16(p));
-    uint32_t qs[4], sg[2];
-    pb_ld_u32x<4>(p + 2 + 16 * qt, qs);
-    pb_ld_u32x<2>(p + 74 + 8 * qt, sg);
-    const uint32_t qh = pb_lds16(p + 66 + 2 * qt);
-    const uint32_t sc = pb_lds8(p + 106 + qt);
-    const __half2 m0 = __half2half2(__int2half_rn(1 + 2 * (int)(sc & 0xF))), m1 = __half2half2(__int2half_rn(1 + 2 * (int)(sc >> 4)));
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-        const uint32_t hb = pb_spread4((qh >> (4 * (u >> 1))) & 0xF);
-        const uint32_t i0 = (u & 1) ? pb_iq3s_index<2>(qs[u >> 1], hb) : pb_iq3s_index<0>(qs[u >> 1], hb);
-        const uint32_t i1 = (u & 1) ? pb_iq3s_index<3>(qs[u >> 1], hb) : pb_iq3s_index<1>(qs[u >> 1], hb);
-        const uint2 g0 = pb_lds64(tab_h + i0 * 32), g1 = pb_lds64(tab_h + i1 * 32);
-        // f16 sign bits by arithmetic: bit k of a nibble -> 0x80 in byte k, then into bytes 1 and 3 of two words
-        const uint32_t sb = sg[u >> 2] >> (8 * (u & 3));
-        const uint32_t ca = ((sb & 0xF) * 0x10204080u) & 0x80808080u, cb = (((sb >> 4) & 0xF) * 0x10204080u) & 0x80808080u;
-        const uint32_t s00 = __byte_perm(ca, 0, 0x1404), s01 = __byte_perm(ca, 0, 0x3424);
-        const uint32_t s10 = __byte_perm(cb, 0, 0x1404), s11 = __byte_perm(cb, 0, 0x3424);
-        const __half2 mm = u < 4 ? m0 : m1;
-        __half2 a;
-        a = __hmul2(*reinterpret_cast<const __half2*>(&g0.x), mm); h[4 * u + 0] = *reinterpret_cast<uint32_t*>(&a) ^ s00;
-        a = __hmul2(*reinterpret_cast<const __half2*>(&g0.y), mm); h[4 * u + 1] = *reinterpret_cast<uint32_t*>(&a) ^ s01;
-        a = __hmul2(*reinterpret_cast<const __half2*>(&g1.x), mm); h[4 * u + 2] = *reinterpret_cast<uint32_t*>(&a) ^ s10;
-        a = __hmul2(*reinterpret_cast<const __half2*>(&g1.y), mm); h[4 * u + 3] = *reinterpret_cast<uint32_t*>(&a) ^ s11;
-    }
-    return d;
-}
-
-// The same 32 half2 words from a block re-coded into 4-bit codes (PB_T_IQ3S_N4, weight = 2 c - 15): a byte
-// permute puts two codes into the mantissas of two f16 with the exponent of 1024 (0x6400 | c = 1024 + c,
-// exact), one subtraction leaves c, one fused multiply-add makes (2 c - 15) * multiplier -- all exact in
-// f16, so the words equal those of pb_iq3s_quarter_h bit for bit.
-__device__ __forceinline__ float pb_n4_quarter_h(uint32_t p, int qt, uint32_t (&h)[32]) {
-    const float d = pb_h2f((uint16_t)(pb_lds32(p) & 0xFFFF));
-    const uint32_t sc = pb_lds8(p + 4 + qt);
-    const float f0 = (float)(1 + 2 * (int)(sc & 0xF)), f1 = (float)(1 + 2 * (int)(sc >> 4));
-    const __half2 a0 = __float2half2_rn(2.0f * f0), b0 = __float2half2_rn(-15.0f * f0);
-    const __half2 a1 = __float2half2_rn(2.0f * f1), b1 = __float2half2_rn(-15.0f * f1);
-    const __half2 k1024 = __float2half2_rn(1024.0f);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const uint2 c = pb_lds64(p + 8 + 32 * qt + 8 * i);
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int u = 2 * i + j;
-            const uint32_t w = j ? c.y : c.x;
-            const uint32_t lo = w & 0x0F0F0F0Fu, hi = (w >> 4) & 0x0F0F0F0Fu;
-            const uint32_t r[4] = {pb_prmt(lo, 0x64006400u, 0x7150u), pb_prmt(lo, 0x64006400u, 0x7352u), pb_prmt(hi, 0x64006400u, 0x7150u), pb_prmt(hi, 0x64006400u, 0x7352u)};
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const __half2 v = __hfma2(__hsub2(*reinterpret_cast<const __half2*>(&r[e]), k1024), u < 4 ? a0 : a1, u < 4 ? b0 : b1);
-                h[4 * u + e] = *reinterpret_cast<const uint32_t*>(&v);
-            }
-        }
-    }
-    return d;
-}
-
-// byte offset of the 8-byte B-fragment slot of (block blk, entry j, n-tile nt, token-in-tile tq, level lv, quarter q).
-// The slots of n-tiles 2p and 2p+1 of one lane are adjacent, so one 128-bit load feeds two mma.
-__device__ __forceinline__ uint32_t pb_xh_off(int blk, int j, int nt, int NT, int tq, int lv, int q) {
-    const int lane = (2 * tq + lv) * 4 + q;
-    if (NT == 1) return (uint32_t)(((blk * 16 + j) * 32 + lane) * 8);
-    return (uint32_t)(((((blk * 16 + j) * (NT / 2) + (nt >> 1)) * 32 + lane) * 2 + (nt & 1)) * 8);
-}
-
-// store 4 consecutive activations (elements c .. c+3, c % 4 == 0) of token b as f16 hi / lo fragments
-__device__ __forceinline__ void pb_xh_store(uint8_t* xh, int NT, int b, int c, float4 v) {
-    const int blk = c >> 8, q = (c >> 6) & 3, j = (c >> 2) & 15, nt = b >> 2, tq = b & 3;
-    const __half2 h01 = __floats2half2_rn(v.x, v.y), h23 = __floats2half2_rn(v.z, v.w);
-    const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
-    const __half2 l01 = __floats2half2_rn(v.x - f01.x, v.y - f01.y), l23 = __floats2half2_rn(v.z - f23.x, v.w - f23.y);
-    *reinterpret_cast<uint2*>(xh + pb_xh_off(blk, j, nt, NT, tq, 0, q)) = make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
-    *reinterpret_cast<uint2*>(xh + pb_xh_off(blk, j, nt, NT, tq, 1, q)) = make_uint2(*reinterpret_cast<const uint32_t*>(&l01), *reinterpret_cast<const uint32_t*>(&l23));
-}
-
-// Activations of all t tokens of a GEMM -> f16 high / low parts in B-fragment order, written once to
-// global memory for all CTAs of all its launches.  The tokens are cut into tiles of `tile` (16 or 8);
-// a tile of tt tokens uses NT = 1 / 2 / 4 n-tiles (4 * NT token slots, the unused ones zero) and lives at
-// xbuf + tile_index * tile_stride: 256 bytes of per-token prescale inverses, then the fragments.
-// grid = number of tiles * tile CTAs (one token slot each), 256 threads.  PLAIN columns get an exact
-// power-of-two prescale into [0.5, 1) (f16 neither overflows nor loses small columns).
-__global__ void __launch_bounds__(256) pb_xh_prep_kernel(const PbGemvQParams p, uint8_t* __restrict__ xbuf, int tile, size_t tile_stride) {
-    constexpr int CT = 256;
-    const int ti = (int)blockIdx.x / tile, b = (int)blockIdx.x - ti * tile;   // tile, slot inside the tile
-    const int tt = min(tile, p.t - ti * tile);                                  // tokens of this tile
-    const int NT = tt <= 4 ? 1 : (tt <= 8 ? 2 : 4);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int cols = p.bpr * 256;
-    __shared__ float red0[8];
-    pb_pdl_wait();
-    pb_pdl_trigger();
-    if (b >= 4 * NT) return;
-    const bool live = b < tt;
-    const float* x = p.x + (size_t)(ti * tile + b) * p.ldx;
-    const float* z = p.z ? p.z + (size_t)(ti * tile + b) * p.ldz : nullptr;
-    uint8_t* xh = xbuf + (size_t)ti * tile_stride + 256;
-    float* xinv = reinterpret_cast<float*>(xbuf + (size_t)ti * tile_stride);
-    if (tid == 0 && blockIdx.y == 0) xinv[b] = 1.0f;
-    if (p.mode == PB_ACT_GNORM) {
-        const int nheads = cols / p.head_dim;   // head_dim == 128 (checked on the host); the heads are spread over grid.y
-        for (int h = warp + 8 * (int)blockIdx.y; h < nheads; h += 8 * (int)gridDim.y) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (live) {
-                v = *reinterpret_cast<const float4*>(x + h * p.head_dim + 4 * lane);
-                const float ss = pb_warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w);
-                const float s = 1.0f / sqrtf(ss / (float)p.head_dim + p.eps);
-                const float4 w = *reinterpret_cast<const float4*>(p.norm_w + 4 * lane);
-                const float4 zz = *reinterpret_cast<const float4*>(z + h * p.head_dim + 4 * lane);
-                v.x = v.x * (s * w.x) * pb_sigm(zz.x); v.y = v.y * (s * w.y) * pb_sigm(zz.y); v.z = v.z * (s * w.z) * pb_sigm(zz.z); v.w = v.w * (s * w.w) * pb_sigm(zz.w);
-            }
-            pb_xh_store(xh, NT, b, h * p.head_dim + 4 * lane, v);
-        }
-        return;
-    }
-    // one CTA-wide reduction: sum of squares (NORM) or largest magnitude (PLAIN)
-    float r = 0.f;
-    if (live) for (int c = tid; c < cols; c += CT) { const float v = x[c]; r = p.mode == PB_ACT_NORM ? r + v * v : fmaxf(r, fabsf(v)); }
-    r = p.mode == PB_ACT_NORM ? pb_warp_sum(r) : pb_warp_max(r);
-    if (lane == 0) red0[warp] = r;
-    __syncthreads();
-    float tot = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; i++) tot = p.mode == PB_ACT_NORM ? tot + red0[i] : fmaxf(tot, red0[i]);
-    float s = 1.0f;
-    if (p.mode == PB_ACT_NORM) s = 1.0f / sqrtf(tot / (float)cols + p.eps);
-    else if (tot > 0.f && tot <= 3.0e38f) {
-        int e; (void)frexpf(tot, &e);
-        s = ldexpf(1.0f, -e);
-        if (tid == 0) xinv[b] = ldexpf(1.0f, e);
-    }
-    for (int c = tid * 4; c < cols; c += CT * 4) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (live) {
-            v = *reinterpret_cast<const float4*>(x + c);
-            if (p.mode == PB_ACT_NORM) { const float4 w = *reinterpret_cast<const float4*>(p.norm_w + c); v.x = v.x * s * w.x; v.y = v.y * s * w.y; v.z = v.z * s * w.z; v.w = v.w * s * w.w; }
-            else { v.x *= s; v.y *= s; v.z *= s; v.w *= s; }
-        }
-        pb_xh_store(xh, NT, b, c, v);
-    }
-}
-
-// NST = stages of the ring (4; 2 for rows wider than 2048 columns, whose fragments leave less room)
-// RC: the weights are the re-coded copy (136-byte blocks, no codebook table)
-template <int NT, int NST, bool RC>
-__global__ void __launch_bounds__(GH_THREADS, 1) pb_gemmh_iq3s_kernel(const PbGemvQParams p) {
-    constexpr int NB = 4 * NT;
+template <int FMT, int NT>
+__global__ void __launch_bounds__(GH_WARPS * 32, 1) pb_gemmh_kernel(const PbGemmHParams h) {
+    const PbGemvQParams& p = h.q;
     extern __shared__ __align__(128) uint8_t smem[];
-    PbRing ring;
-    ring.full = reinterpret_cast<uint64_t*>(smem);
-    ring.empty = ring.full + NST;
-    float* red0 = reinterpret_cast<float*>(smem + 64);            // GH_CONSUMERS floats
-    float* xinv = reinterpret_cast<float*>(smem + 128);           // per token: inverse of the power-of-two prescale
-    uint64_t* xbar = reinterpret_cast<uint64_t*>(smem + 192);     // completion of the fragment copies
-    uint8_t* tab = smem + 256;                                    // f16 codebook, four interleaved copies (16 KB)
-    const int cols = p.bpr * 256;
-    uint8_t* xh = tab + (RC ? 0 : 16384);                         // B fragments: cols * NB * 4 bytes
-    float* red = reinterpret_cast<float*>(xh + (size_t)cols * NB * 4);   // [2][GH_CONSUMERS][16 rows][NB]
-    ring.stages = reinterpret_cast<uint8_t*>(red) + 2 * GH_CONSUMERS * GH_ROWS * NB * 4;
-    ring.stage_bytes = p.stage_bytes;
-
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float* ssq = reinterpret_cast<float*>(smem);
+    uint8_t* tab = smem + GH_HEAD;
+    uint8_t* act = smem + h.off_act;
+    float* red = reinterpret_cast<float*>(smem + h.off_red);          // [GH_WARPS][4 NT tokens][16 rows]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3, nw = (int)blockDim.x >> 5;
+    const int ks = h.ks, rank = ks > 1 ? (int)blockIdx.x % ks : 0, cl = (int)blockIdx.x / ks, ncl = (int)gridDim.x / ks;   // (clusters are consecutive CTAs)
+    const int bpr = p.bpr / ks, kb = rank * bpr;                       // this CTA's blocks of a row: kb .. kb + bpr
+    const uint32_t tokb = (uint32_t)pb_h_tok_bytes<FMT>(256 * bpr);
     pb_pdl_trigger();
-    if (tid == 0) {
-        for (int s = 0; s < NST; s++) { pb_mbar_init(&ring.full[s], 1); pb_mbar_init(&ring.empty[s], GH_CONSUMERS); }
-        pb_mbar_init(xbar, 1);
-        pb_fence_barrier_init();
+    const int tile0 = (int)((int64_t)p.nchunks * cl / ncl), tile1 = (int)((int64_t)p.nchunks * (cl + 1) / ncl);
+    // whole rounds: every warp a tile; then one round of `share` warps per tile
+    const int rounds = (tile1 - tile0) / nw, nfull = rounds * nw, nrest = tile1 - tile0 - nfull;
+    int share = 1;
+    while (nrest > 0 && 2 * share <= bpr && 2 * share * nrest <= nw) share *= 2;
+    const int pieces = rounds + (nrest > 0 ? 1 : 0);
+    // piece i of this warp: its tile (-1: none) and blocks [b0, b1)
+    auto piece = [&](int i, int& b0, int& b1) -> int {
+        if (i < rounds) { b0 = 0; b1 = bpr; return tile0 + i * nw + warp; }
+        const int k = warp / share, part = warp - k * share;
+        b0 = part * (bpr / share); b1 = b0 + bpr / share;
+        return k < nrest ? tile0 + nfull + k : -1;
+    };
+    auto locate = [&](int tile, int& r0) -> int { int s = 0; while (s + 1 < p.nseg && tile >= p.seg[s + 1].chunk0) s++; r0 = (tile - p.seg[s].chunk0) * 16; return s; };
+
+    // ---- weights: the blocks of the warp's pieces go round its ring of stages; the first are requested before anything of the previous
+    //      kernel is awaited
+    const uint32_t ring = pb_smem_u32(smem + h.off_stage) + (uint32_t)(warp * h.stages * h.g.stage_bytes);
+    PbHTile pt; pt.a = pt.b = nullptr; pt.la = pt.lb = 7;
+    int pi = 0, pb0 = 0, pb1 = 0, ptile = -1, pblk = 0, ps = 0;
+    auto tile_of = [&](int tile, PbHTile& t) {
+        int r0;
+        const int s = locate(tile, r0), rows = p.seg[s].rows;
+        const uint8_t* w = p.seg[s].w + (size_t)r0 * p.row_bytes;
+        t.a = w; t.la = min(7, rows - 1 - r0);
+        const bool two = r0 + 8 < rows;                                // (else the second half repeats the first and is not stored)
+        t.b = two ? w + 8 * (size_t)p.row_bytes : w; t.lb = two ? min(7, rows - 9 - r0) : t.la;
+    };
+    auto open = [&]() { ptile = pi < pieces ? piece(pi, pb0, pb1) : -1; if (ptile >= 0) { tile_of(ptile, pt); pblk = pb0; } };
+    auto issue = [&]() {
+        if (ptile >= 0) {
+            pb_h_stage<FMT>(ring + (uint32_t)(ps * h.g.stage_bytes), pt, h.g, kb + pblk, lane);
+            if (++pblk == pb1) { pi++; open(); }
+        } else asm volatile("cp.async.commit_group;" ::: "memory");
+        ps = ps + 1 == h.stages ? 0 : ps + 1;
+    };
+    open();
+    for (int i = 0; i + 1 < h.stages; i++) issue();
+    PbQTabs T = {0u, 0u, 0u};
+    if constexpr (pb_h_mode<FMT>() != PB_H_DIRECT) T = pb_fill_qtabs<FMT>(tab, p.rep, tid, (int)blockDim.x, lane);
+
+    // ---- activations: a block of a token per warp
+    pb_pdl_wait();
+    const int c0 = pb_h_c0<FMT>(lane), c1 = pb_h_c1<FMT>(lane);
+    if (p.mode == PB_ACT_NORM) {
+        for (int i = warp; i < p.t * p.bpr; i += nw) {
+            const int b = i / p.bpr, blk = i - b * p.bpr;
+            const float* x = p.x + (size_t)b * p.ldx + 256 * blk;
+            const float4 u = *reinterpret_cast<const float4*>(x + 4 * lane), v = *reinterpret_cast<const float4*>(x + 128 + 4 * lane);
+            const float ss = pb_warp_sum((u.x * u.x + u.y * u.y + u.z * u.z + u.w * u.w) + (v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w));
+            if (lane == 0) ssq[b * GH_MAXBLK + blk] = ss;
+        }
+        __syncthreads();
+    }
+#pragma unroll 2
+    for (int i = warp; i < p.t * bpr; i += nw) {
+        const int b = i / bpr, blk = i - b * bpr;
+        const int col = 256 * (kb + blk);
+        const float* x = p.x + (size_t)b * p.ldx + col;
+        const float4 u = *reinterpret_cast<const float4*>(x + c0), v = *reinterpret_cast<const float4*>(x + c1);
+        float a[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+        if (p.mode == PB_ACT_NORM) {          // rms(): x * s * w  (qwen4exp_gguf.rs:209)
+            float ss = 0.f;
+            for (int k = 0; k < p.bpr; k++) ss += ssq[b * GH_MAXBLK + k];
+            const float s = 1.0f / sqrtf(ss / (float)(256 * p.bpr) + p.eps);
+            const float4 n0 = *reinterpret_cast<const float4*>(p.norm_w + col + c0), n1 = *reinterpret_cast<const float4*>(p.norm_w + col + c1);
+            const float n[8] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
+#pragma unroll
+            for (int c = 0; c < 8; c++) a[c] = a[c] * s * n[c];
+        } else if (p.mode == PB_ACT_GNORM) {  // per head of 128 (two quarters): rms(x) * w * sigmoid(z)  (linear_core, qwen4exp_gguf.rs:1667)
+            const float* z = p.z + (size_t)b * p.ldz + col;
+            const float4 z0 = *reinterpret_cast<const float4*>(z + c0), z1 = *reinterpret_cast<const float4*>(z + c1);
+            float ss = 0.f;
+#pragma unroll
+            for (int c = 0; c < 8; c++) ss += a[c] * a[c];
+            ss += __shfl_xor_sync(0xffffffffu, ss, 1); ss += __shfl_xor_sync(0xffffffffu, ss, 4); ss += __shfl_xor_sync(0xffffffffu, ss, 8); ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+            const float s = 1.0f / sqrtf(ss / 128.0f + p.eps);
+            const float4 n0 = *reinterpret_cast<const float4*>(p.norm_w + (c0 & 127)), n1 = *reinterpret_cast<const float4*>(p.norm_w + (c1 & 127));
+            const float n[8] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w}, zz[8] = {z0.x, z0.y, z0.z, z0.w, z1.x, z1.y, z1.z, z1.w};
+#pragma unroll
+            for (int c = 0; c < 8; c++) a[c] = a[c] * (s * n[c]) * pb_sigm(zz[c]);
+        }
+        pb_h_put<FMT>(act + (size_t)b * tokb, bpr, blk, lane, a);   // (columns past the tokens read whatever their slots hold and are dropped)
     }
     __syncthreads();
-    const int my_chunks = p.nchunks > (int)blockIdx.x ? (p.nchunks - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
-    if (warp == GH_CONSUMERS) {
-        if (lane == 0) {
-            int k = 0;
-            bool x_issued = false;
-            for (; k < my_chunks; k++) {
-                if (k == NST && !x_issued) {
-                    // the ring is full of weights (which no earlier kernel writes): now wait for the kernel
-                    // that made the fragments and bring them in, in pieces of 16 KB
-                    pb_pdl_wait();
-                    const uint32_t xbytes = (uint32_t)cols * NB * 4;
-                    pb_mbar_expect_tx(xbar, xbytes);
-                    for (uint32_t o = 0; o < xbytes; o += 16384) pb_bulk_g2s(xh + o, p.xh_in + o, min(16384u, xbytes - o), xbar);
-                    x_issued = true;
-                }
-                const int chunk = (int)blockIdx.x + k * (int)gridDim.x;
-                int s = 0;
-                while (s + 1 < p.nseg && chunk >= p.seg[s + 1].chunk0) s++;
-                const int r0 = (chunk - p.seg[s].chunk0) * GH_ROWS;
-                const int nr = min(GH_ROWS, p.seg[s].rows - r0);
-                const uint32_t bytes = ((uint32_t)nr * (uint32_t)p.row_bytes + 15u) & ~15u;
-                const int st = k % NST;
-                if (k >= NST && !pb_mbar_wait_relaxed(&ring.empty[st], ((k / NST) - 1) & 1, p.status, PB_DEV_WAIT_EMPTY_TIMEOUT)) break;
-                pb_mbar_expect_tx(&ring.full[st], bytes);
-                pb_bulk_g2s(ring.stages + (size_t)st * ring.stage_bytes, p.seg[s].w + (size_t)r0 * p.row_bytes, bytes, &ring.full[st]);
+    const PbHLane L = pb_h_lane<FMT>(pb_smem_u32(act), bpr, lane);
+    int cs = 0;
+    for (int i = 0; i < pieces; i++) {
+        int b0, b1, r0 = 0, s = 0;
+        const int tile = piece(i, b0, b1);
+        PbHTile ct; ct.a = ct.b = nullptr; ct.la = ct.lb = 7;
+        if (tile >= 0) { s = locate(tile, r0); if constexpr (pb_h_mode<FMT>() != PB_H_DIRECT) tile_of(tile, ct); }
+        float tot[NT][2];
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++) tot[nt][0] = tot[nt][1] = 0.f;
+        if (tile >= 0)
+            for (int blk = b0; blk < b1; blk++) {
+                if (h.stages == 3) asm volatile("cp.async.wait_group 1;" ::: "memory"); else asm volatile("cp.async.wait_group 0;" ::: "memory");
+                __syncwarp();   // this block has landed for all lanes, and all have left the stage that is refilled now
+                issue();
+                pb_h_block<FMT, NT>(ring + (uint32_t)(cs * h.g.stage_bytes), ct, h.g, T, kb + blk, blk, lane, L, tot);
+                cs = cs + 1 == h.stages ? 0 : cs + 1;
             }
-            if (!x_issued) {
-                pb_pdl_wait();
-                const uint32_t xbytes = (uint32_t)cols * NB * 4;
-                pb_mbar_expect_tx(xbar, xbytes);
-                for (uint32_t o = 0; o < xbytes; o += 16384) pb_bulk_g2s(xh + o, p.xh_in + o, min(16384u, xbytes - o), xbar);
-            }
-            // error path: give the copies in flight a bounded chance to land before the CTA may exit
-            if (k < my_chunks) {
-                for (int j = max(0, k - NST); j < k; j++) pb_mbar_wait(&ring.full[j % NST], (j / NST) & 1, nullptr, 0);
-                pb_mbar_wait(xbar, 0, nullptr, 0);
-            }
-        }
-        return;
-    }
-
-    // ---- consumers: tables ----
-    constexpr int CT = GH_CONSUMERS * 32;
-    if (!RC) {   // the re-coded form needs no codebook (and the fragments start where the table would be)
-        uint2* gh = reinterpret_cast<uint2*>(tab);
-        for (int i = tid; i < 512; i += CT) {
-            const uint32_t g = PB_IQ3S_GRID[i];
-            const __half2 a = __floats2half2_rn((float)(g & 0xFF), (float)((g >> 8) & 0xFF)), b = __floats2half2_rn((float)((g >> 16) & 0xFF), (float)(g >> 24));
-            const uint2 e = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
-            gh[4 * i] = e; gh[4 * i + 1] = e; gh[4 * i + 2] = e; gh[4 * i + 3] = e;
-        }
-    }
-    const uint32_t tab_h = pb_smem_u32(tab) + (lane & 3) * 8;
-    if (tid < NB) xinv[tid] = 1.0f;
-    pb_named_barrier(2, CT);
-    pb_pdl_wait();
-    // ---- f16 hi/lo fragments and prescales made by pb_xh_prep_kernel: wait for the producer's bulk copies ----
-    if (tid < NB) xinv[tid] = p.xinv_in[tid];
-    if (!pb_mbar_wait(xbar, 0, p.status, PB_DEV_WAIT_FULL_TIMEOUT)) return;
-    pb_named_barrier(1, CT);
-
-    const int g = lane >> 2, q = lane & 3;
-    const uint32_t xh_s = pb_smem_u32(xh);
-    for (int k = 0; k < my_chunks; k++) {
-        if (!pb_mbar_wait(&ring.full[k % NST], (k / NST) & 1, p.status, PB_DEV_WAIT_FULL_TIMEOUT)) return;
-        const int chunk = (int)blockIdx.x + k * (int)gridDim.x;
-        int s = 0;
-        while (s + 1 < p.nseg && chunk >= p.seg[s + 1].chunk0) s++;
-        const int r0 = (chunk - p.seg[s].chunk0) * GH_ROWS;
-        const int nr = min(GH_ROWS, p.seg[s].rows - r0);
-        const uint32_t base = pb_smem_u32(ring.stages + (size_t)(k % NST) * ring.stage_bytes);
-        float tot[NT][4];
+        const int shr = i < rounds ? 1 : share;
+        if (shr == 1 && ks == 1) {
+            if (tile >= 0) {
+                const int rows = p.seg[s].rows;
 #pragma unroll
-        for (int nt = 0; nt < NT; nt++) { tot[nt][0] = tot[nt][1] = tot[nt][2] = tot[nt][3] = 0.f; }
-        for (int blk = warp; blk < p.bpr; blk += GH_CONSUMERS) {   // K split: this warp's blocks of the 16 rows
-            uint32_t ha[32], hb[32];
-            // rows g and g + 8 (rows past the end of the matrix decode stale bytes of the stage; never stored)
-            const float da = RC ? pb_n4_quarter_h(base + (uint32_t)g * p.row_bytes + blk * 136, q, ha) : pb_iq3s_quarter_h(base + (uint32_t)g * p.row_bytes + blk * 110, q, tab_h, ha);
-            const float db = RC ? pb_n4_quarter_h(base + (uint32_t)(g + 8) * p.row_bytes + blk * 136, q, hb) : pb_iq3s_quarter_h(base + (uint32_t)(g + 8) * p.row_bytes + blk * 110, q, tab_h, hb);
-            float acc[NT][4];
-#pragma unroll
-            for (int nt = 0; nt < NT; nt++) { acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f; }
-#pragma unroll
-            for (int j = 0; j < 16; j++) {
-                if (NT == 1) {
-                    const uint2 bx = pb_lds64(xh_s + (uint32_t)(((blk * 16 + j) * 32 + lane) * 8));
-                    pb_mma_f16(acc[0], ha[2 * j], hb[2 * j], ha[2 * j + 1], hb[2 * j + 1], bx.x, bx.y);
-                } else {
-#pragma unroll
-                    for (int np = 0; np < NT / 2; np++) {
-                        const uint4 bx = pb_lds128(xh_s + (uint32_t)((((blk * 16 + j) * (NT / 2) + np) * 32 + lane) * 16));
-                        pb_mma_f16(acc[2 * np], ha[2 * j], hb[2 * j], ha[2 * j + 1], hb[2 * j + 1], bx.x, bx.y);
-                        pb_mma_f16(acc[2 * np + 1], ha[2 * j], hb[2 * j], ha[2 * j + 1], hb[2 * j + 1], bx.z, bx.w);
+                for (int nt = 0; nt < NT; nt++) {
+                    const int b = 4 * nt + q;
+                    if (b < p.t) {
+                        float* dst = p.y + (size_t)b * p.ldy + p.seg[s].yoff + r0 + g;
+                        if (r0 + g < rows) dst[0] = p.accumulate ? dst[0] + tot[nt][0] : tot[nt][0];
+                        if (r0 + 8 + g < rows) dst[8] = p.accumulate ? dst[8] + tot[nt][1] : tot[nt][1];
                     }
                 }
             }
+        } else {
+            // the sums of a tile's parts meet in shared memory and are added in block order; a CTA of a cluster adds a share of the round's outputs
+            float* mine = red + (size_t)warp * (4 * NT * 16);
 #pragma unroll
-            for (int nt = 0; nt < NT; nt++) {
-                tot[nt][0] = fmaf(da, acc[nt][0], tot[nt][0]); tot[nt][1] = fmaf(da, acc[nt][1], tot[nt][1]);
-                tot[nt][2] = fmaf(db, acc[nt][2], tot[nt][2]); tot[nt][3] = fmaf(db, acc[nt][3], tot[nt][3]);
-            }
-        }
-        __syncwarp();
-        if (lane == 0) pb_mbar_arrive(&ring.empty[k % NST]);
-        // this warp's partial [16 rows][NB tokens]: thread (g, q) owns rows g, g+8 and token 4*nt + q (hi + lo columns)
-        float* mine = red + (size_t)((k & 1) * GH_CONSUMERS + warp) * GH_ROWS * NB;
-#pragma unroll
-        for (int nt = 0; nt < NT; nt++) {
-            mine[g * NB + 4 * nt + q] = tot[nt][0] + tot[nt][1];
-            mine[(g + 8) * NB + 4 * nt + q] = tot[nt][2] + tot[nt][3];
-        }
-        pb_named_barrier(1, CT);
-        // 256 threads <-> 16 rows x up to 16 tokens
-        for (int o = tid; o < GH_ROWS * NB; o += CT) {
-            const int r = o / NB, b = o - r * NB;
-            if (r < nr && b < p.t) {
-                const float* src = red + (size_t)(k & 1) * GH_CONSUMERS * GH_ROWS * NB + o;
+            for (int nt = 0; nt < NT; nt++) { mine[(4 * nt + q) * 16 + g] = tot[nt][0]; mine[(4 * nt + q) * 16 + g + 8] = tot[nt][1]; }
+            if (ks > 1) gh_cluster_sync(); else __syncthreads();
+            const int first = tile0 + i * nw, nout = (i < rounds ? nw : nrest) * 16 * p.t;
+            for (int o = nout * rank / ks + tid; o < nout * (rank + 1) / ks; o += (int)blockDim.x) {
+                const int k = o / (16 * p.t), e = o - k * 16 * p.t, b = e >> 4, r = e & 15;
+                int rr;
+                const int sg = locate(first + k, rr);
+                if (rr + r >= p.seg[sg].rows) continue;
+                const uint32_t src = pb_smem_u32(red) + (uint32_t)((k * shr * (4 * NT * 16) + b * 16 + r) * 4);
                 float v = 0.f;
-#pragma unroll
-                for (int w = 0; w < GH_CONSUMERS; w++) v += src[(size_t)w * GH_ROWS * NB];
-                v *= xinv[b];
-                float* dst = p.y + b * p.ldy + p.seg[s].yoff + r0 + r;
+                for (int c = 0; c < ks; c++)
+                    for (int w = 0; w < shr; w++) v += ks > 1 ? gh_remote(src + (uint32_t)(w * 4 * NT * 16 * 4), c) : red[(size_t)(k * shr + w) * (4 * NT * 16) + b * 16 + r];
+                float* dst = p.y + (size_t)b * p.ldy + p.seg[sg].yoff + rr + r;
                 *dst = p.accumulate ? *dst + v : v;
             }
+            if (ks > 1) gh_cluster_sync(); else if (i + 1 < pieces) __syncthreads();   // the buffer is rewritten (or, at the end, given up) only when all have read it
         }
-        // the buffer of parity k & 1 is rewritten two chunks later, after the barrier of chunk k + 1
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-template <int NT, int NST, bool RC>
-static int launch_h(pb_ctx* ctx, const PbGemvQArgs& a, const uint8_t* tile_buf) {
-    constexpr int NB = 4 * NT;
-    PbGemvQParams p;
-    memset(&p, 0, sizeof p);
-    p.row_bytes = a.cols / 256 * (RC ? 136 : 110); p.bpr = a.cols / 256; p.nseg = a.nseg;
-    p.x = a.x; p.ldx = a.ldx; p.t = a.t; p.y = a.y; p.ldy = a.ldy; p.status = ctx->dev_status;
-    p.mode = a.mode; p.norm_w = a.norm_w; p.z = a.z; p.ldz = a.ldz; p.head_dim = a.head_dim; p.eps = a.eps; p.accumulate = a.accumulate;
-    p.rows_per_chunk = GH_ROWS;
-    int nchunks = 0;
-    for (int s = 0; s < a.nseg; s++) {
-        p.seg[s].w = RC ? a.seg[s].wr : a.seg[s].w; p.seg[s].rows = (int)a.seg[s].rows; p.seg[s].yoff = (int)a.seg[s].yoff; p.seg[s].chunk0 = nchunks;
-        nchunks += (int)((a.seg[s].rows + GH_ROWS - 1) / GH_ROWS);
-    }
-    p.nchunks = nchunks;
-    p.stage_bytes = (uint32_t)(((size_t)GH_ROWS * p.row_bytes + 16 + 127) & ~(size_t)127);
-    const size_t smem = 256 + (RC ? 0 : 16384) + (size_t)a.cols * NB * 4 + 2 * GH_CONSUMERS * GH_ROWS * NB * 4 + (size_t)NST * p.stage_bytes;
-    if (smem > (size_t)ctx->max_smem_optin) PB_FAIL(ctx, PB_UNSUPPORTED, "gemm: %zu bytes of shared memory needed for cols=%d t=%d", smem, a.cols, a.t);
-    p.xh_in = tile_buf + 256; p.xinv_in = reinterpret_cast<const float*>(tile_buf);
-    auto kern = pb_gemmh_iq3s_kernel<NT, NST, RC>;
-    PB_TRY(pb_ensure_smem(ctx, kern, smem));
-    const int grid = nchunks < ctx->sm_count ? nchunks : ctx->sm_count;
-    pb_launch_k(ctx, kern, dim3(grid), dim3(GH_THREADS), smem, p);
-    ctx->kernels_launched++;
-    PB_CUDA(ctx, cudaGetLastError());
-    return PB_OK;
+// Tokens of one launch and warps per CTA that fit shared memory
+template <int FMT>
+static bool gh_layout(pb_ctx* ctx, int cols, int t, int ks, int& nt, int& nw, PbGemmHParams& h, size_t& smem) {
+    constexpr int rep = pb_tab_rep_max<FMT>();
+    h.g = pb_h_geom<FMT>(cols);
+    for (nt = (t + 3) / 4 > 4 ? 4 : (t + 3) / 4; nt >= 1; nt--)
+        for (nw = GH_WARPS; nw >= 8; nw /= 2)
+            for (h.stages = 3; h.stages >= 2; h.stages--)
+                for (h.q.rep = rep > 8 ? 8 : rep; h.q.rep >= 1; h.q.rep /= 2) {   // copies of the codebook: as many as fit
+                    const uint32_t tabb = pb_h_mode<FMT>() == PB_H_DIRECT ? 0u : pb_tab_bytes<FMT>(h.q.rep);
+                    h.off_act = GH_HEAD + ((tabb + 127) & ~127u);
+                    h.off_red = h.off_act + (uint32_t)(4 * nt) * (uint32_t)pb_h_tok_bytes<FMT>(cols / ks);
+                    h.off_stage = h.off_red + (uint32_t)nw * 4 * nt * 16 * 4;
+                    smem = h.off_stage + (size_t)nw * h.stages * h.g.stage_bytes + 64;   // the decoders read whole words: a few bytes past the last row
+                    if (smem <= (size_t)ctx->max_smem_optin) return true;
+                }
+    return false;
 }
 
-bool pb_gemmh_supported(int type, int cols, int t) { return type == PB_T_IQ3_S && t >= 3 && cols % 256 == 0 && cols >= 256 && cols <= 4096; }
-
-int pb_launch_gemmh(pb_ctx* ctx, const PbGemvQArgs& a) {
-    if (!pb_gemmh_supported(a.type, a.cols, a.t)) PB_FAIL(ctx, PB_UNSUPPORTED, "gemm: type %d cols %d t %d", a.type, a.cols, a.t);
-    if (a.mode == PB_ACT_PREQ) PB_FAIL(ctx, PB_UNSUPPORTED, "gemm: pre-split activations are not accepted");
-    if (a.mode == PB_ACT_GNORM && a.head_dim != 128) PB_FAIL(ctx, PB_UNSUPPORTED, "gemm: gated norm over heads of %d (128 is built)", a.head_dim);
-    if (((uintptr_t)a.x & 15) || (a.ldx & 3)) PB_FAIL(ctx, PB_ERR_ARG, "gemm: activations must be 16-byte aligned");
-    // columns per launch: 16 with a 4-stage ring up to 2048 weight columns, 8 with a 2-stage ring above
-    const bool wide = a.cols > 2048;
-    const int tile = wide ? 8 : 16;
-    const int ntiles = (a.t + tile - 1) / tile;
-    const size_t tile_stride = 256 + (size_t)a.cols * tile * 4;
-    if (ntiles * tile_stride > PB_XH_BYTES) PB_FAIL(ctx, PB_UNSUPPORTED, "gemm: %d tokens of %d columns exceed the %d-byte fragment buffer", a.t, a.cols, (int)PB_XH_BYTES);
-    {   // fragments of all tokens, made once for all launches and CTAs of this GEMM
-        PbGemvQParams p;
-        memset(&p, 0, sizeof p);
-        p.bpr = a.cols / 256; p.x = a.x; p.ldx = a.ldx; p.t = a.t; p.mode = a.mode; p.norm_w = a.norm_w; p.z = a.z; p.ldz = a.ldz; p.head_dim = a.head_dim; p.eps = a.eps;
-        pb_launch_k(ctx, pb_xh_prep_kernel, dim3(ntiles * tile, p.mode == PB_ACT_GNORM ? 4 : 1), dim3(256), (size_t)0, p, ctx->xh_buf, tile, tile_stride);
+template <int FMT>
+static int launch_fmt(pb_ctx* ctx, const PbGemvQArgs& a, bool recoded) {
+    int el, bs;
+    pb_geom(FMT, &el, &bs);
+    int all = 0;
+    for (int s = 0; s < a.nseg; s++) all += (int)((a.seg[s].rows + 15) / 16);
+    // CTAs of a cluster: 1024 columns each above 2048; half a row each where a CTA has at most a round of tiles and the activations of several
+    // tokens would take as long to prepare as the product
+    const int ks = a.cols > 2048 ? a.cols / 1024 : (a.cols == 2048 && all <= 16 * ctx->sm_count && a.t > 4 ? 2 : 1);
+    for (int t0 = 0, n = 0; t0 < a.t; t0 += n) {
+        PbGemmHParams h;
+        memset(&h, 0, sizeof h);
+        h.ks = ks;
+        int nt, nw; size_t smem;
+        if (!gh_layout<FMT>(ctx, a.cols, a.t - t0, ks, nt, nw, h, smem)) PB_FAIL(ctx, PB_UNSUPPORTED, "gemm: %d columns do not fit shared memory", a.cols);
+        n = a.t - t0 < 4 * nt ? a.t - t0 : 4 * nt;
+        PbGemvQParams& p = h.q;
+        p.row_bytes = a.cols / el * bs; p.bpr = a.cols / 256; p.nseg = a.nseg;
+        p.x = a.x + (int64_t)t0 * a.ldx; p.ldx = a.ldx; p.t = n; p.y = a.y + (int64_t)t0 * a.ldy; p.ldy = a.ldy; p.status = ctx->dev_status;
+        p.mode = a.mode; p.norm_w = a.norm_w; p.z = a.z ? a.z + (int64_t)t0 * a.ldz : nullptr; p.ldz = a.ldz; p.head_dim = a.head_dim; p.eps = a.eps; p.accumulate = a.accumulate;
+        int ntiles = 0;
+        for (int s = 0; s < a.nseg; s++) {
+            p.seg[s].w = recoded ? a.seg[s].wr : a.seg[s].w; p.seg[s].rows = (int)a.seg[s].rows; p.seg[s].yoff = (int)a.seg[s].yoff; p.seg[s].chunk0 = ntiles;
+            ntiles += (int)((a.seg[s].rows + 15) / 16);
+        }
+        p.nchunks = ntiles;
+        if (ntiles == 0) return PB_OK;
+#define GO(N) { auto kern = pb_gemmh_kernel<FMT, N>; PB_TRY(pb_ensure_smem(ctx, kern, smem)); const int ncl = pb_max_clusters(ctx, reinterpret_cast<const void*>(kern), nw * 32, smem, ks), grid = (ntiles < ncl ? ntiles : ncl) * ks; pb_launch_kc(ctx, kern, dim3(grid), dim3(nw * 32), smem, ks, h); }
+        if (nt == 1) GO(1) else if (nt == 2) GO(2) else if (nt == 3) GO(3) else GO(4)
+#undef GO
         ctx->kernels_launched++;
         PB_CUDA(ctx, cudaGetLastError());
     }
-    bool recoded = true;   // every segment has a re-coded copy
-    for (int sg = 0; sg < a.nseg && sg < 4; sg++) recoded = recoded && a.seg[sg].wr != nullptr;
-    int rc = PB_OK;
-    for (int ti = 0; ti < ntiles && rc == PB_OK; ti++) {
-        const int t0 = ti * tile;
-        PbGemvQArgs s = a;
-        s.t = a.t - t0 < tile ? a.t - t0 : tile;
-        s.x = a.x + (int64_t)t0 * a.ldx; s.y = a.y + (int64_t)t0 * a.ldy; s.z = a.z ? a.z + (int64_t)t0 * a.ldz : nullptr;
-        const uint8_t* tb = ctx->xh_buf + (size_t)ti * tile_stride;
-        if (recoded) {
-            if (wide) rc = s.t <= 4 ? launch_h<1, 2, true>(ctx, s, tb) : launch_h<2, 2, true>(ctx, s, tb);
-            else rc = s.t <= 4 ? launch_h<1, 4, true>(ctx, s, tb) : (s.t <= 8 ? launch_h<2, 4, true>(ctx, s, tb) : launch_h<4, 4, true>(ctx, s, tb));
-        } else if (wide) rc = s.t <= 4 ? launch_h<1, 2, false>(ctx, s, tb) : launch_h<2, 2, false>(ctx, s, tb);
-        else rc = s.t <= 4 ? launch_h<1, 4, false>(ctx, s, tb) : (s.t <= 8 ? launch_h<2, 4, false>(ctx, s, tb) : launch_h<4, 4, false>(ctx, s, tb));
+    return PB_OK;
+}
+
+bool pb_gemmh_supported(int type, int cols, int t) { return t >= 2 && pb_gemvq_supported(type, cols); }
+
+int pb_launch_gemmh(pb_ctx* ctx, const PbGemvQArgs& a) {
+    if (!pb_gemmh_supported(a.type, a.cols, a.t)) PB_FAIL(ctx, PB_UNSUPPORTED, "gemm: type %d cols %d t %d", a.type, a.cols, a.t);
+    if (a.nseg < 1 || a.nseg > 4) PB_FAIL(ctx, PB_ERR_ARG, "gemm: %d segments", a.nseg);
+    if (a.mode == PB_ACT_PREQ) PB_FAIL(ctx, PB_UNSUPPORTED, "gemm: pre-split activations are not accepted");
+    if (a.mode == PB_ACT_GNORM && a.head_dim != 128) PB_FAIL(ctx, PB_UNSUPPORTED, "gemm: gated norm over heads of %d (128 is built)", a.head_dim);
+    if (((uintptr_t)a.x & 15) || (a.ldx & 3)) PB_FAIL(ctx, PB_ERR_ARG, "gemm: activations must be 16-byte aligned");
+    bool recoded = a.type == PB_T_IQ3_S;   // every segment has a re-coded copy
+    for (int sg = 0; sg < a.nseg; sg++) { recoded = recoded && a.seg[sg].wr != nullptr; if ((uintptr_t)a.seg[sg].w & 15) PB_FAIL(ctx, PB_ERR_ARG, "gemm: weight pointer must be 16-byte aligned"); }
+#define GO(F) case F: return launch_fmt<F>(ctx, a, false)
+    switch (a.type) {
+        case PB_T_IQ3_S: return recoded ? launch_fmt<PB_T_IQ3S_N4>(ctx, a, true) : launch_fmt<PB_T_IQ3_S>(ctx, a, false);
+        GO(PB_T_IQ3S_N4); GO(PB_T_IQ2_XS); GO(PB_T_Q4_K); GO(PB_T_Q8_0); GO(PB_T_IQ3_XXS); GO(PB_T_IQ2_S); GO(PB_T_IQ4_NL); GO(PB_T_IQ4_XS);
+        GO(PB_T_Q2_0); GO(PB_T_IQ2_XXS); GO(PB_T_Q6_K); GO(PB_T_IQ1_M); GO(PB_T_Q4_0); GO(PB_T_Q5_0); GO(PB_T_Q3_K); GO(PB_T_Q5_K);
+        default: PB_FAIL(ctx, PB_UNSUPPORTED, "gemm: type %d", a.type);
     }
-    return rc;
+#undef GO
 }

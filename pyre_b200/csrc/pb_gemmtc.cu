@@ -11,7 +11,7 @@
 //                       bits), prepared once per GEMM by pb_xt_prep_kernel in exactly the operand layout -- with 1-D
 //                       bulk copies.
 //   decoder warps (8)   stream the re-coded IQ3_S rows of the tile (4-bit codes, PB_T_IQ3S_N4: 136 bytes per row and 256
-//                       columns) into a double buffer of raw bytes with 8-byte cp.async (all 256 threads share the
+//                       columns) into a double buffer of raw bytes with 16-byte cp.async (all 256 threads share the
 //                       copies), then one thread = one row x 64 columns per step: f16 weights stored with tcgen05.st
 //                       into the thread's own lane of a weight tile in tensor memory (the A operand is read from
 //                       there, behind the accumulator).  (2c - 15) * (1 + 2s) is
@@ -178,16 +178,16 @@ __global__ void __launch_bounds__(256) pb_xt_prep_kernel(const PbGemvQParams p, 
 
 // raw bytes of one quarter (64 weights) of a re-coded block: {d (f16) | pad, four sub-scale bytes}, 32 bytes of codes
 struct TcRaw { uint2 head; uint2 c[4]; };
-// from the raw ring: `b` = shared-memory address of this row's block (rows 136 bytes apart: 8-byte loads of 16 lanes hit 32 banks)
-__device__ __forceinline__ void tc_load_raw(TcRaw& r, uint32_t b, int qt, bool live) {
+// from the raw ring: `b` = shared-memory address of the block of this row's group of eight (pb_repack.cu), row = row in the group
+__device__ __forceinline__ void tc_load_raw(TcRaw& r, uint32_t b, int row, int qt, bool live) {
     if (!live) { r.head = make_uint2(0u, 0u); r.c[0] = r.c[1] = r.c[2] = r.c[3] = make_uint2(0x77777777u, 0x77777777u); return; }
     // volatile with a memory clobber: these loads must stay behind the wait for the block's copies
-    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.head.x), "=r"(r.head.y) : "r"(b) : "memory");
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.head.x), "=r"(r.head.y) : "r"(b + 1024 + 8 * row) : "memory");
 #pragma unroll
-    for (int i = 0; i < 4; i++) asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.c[i].x), "=r"(r.c[i].y) : "r"(b + 8 + 32 * qt + 8 * i) : "memory");
+    for (int i = 0; i < 2; i++) asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.c[2 * i].x), "=r"(r.c[2 * i].y), "=r"(r.c[2 * i + 1].x), "=r"(r.c[2 * i + 1].y) : "r"(b + 512 * i + (4 * row + qt) * 16) : "memory");
 }
-__device__ __forceinline__ void tc_cp_async8(uint32_t dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+__device__ __forceinline__ void tc_cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 // the mbarrier (initialised with one count per issuing thread) gets this thread's arrival once its copies so far have landed
 __device__ __forceinline__ void tc_cp_async_arrive(uint64_t* bar) {
@@ -328,13 +328,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
         const int row = (warp & 3) * 32 + lane;    // row of the tile
         const bool live = row < nr;
         const uint8_t* wbase = p.seg[s].w + (size_t)r0 * p.row_bytes;
-        // raw bytes: block kb of the tile's rows (136 bytes per row) -> raw[kb % 2]; thread tid copies 8-byte words tid, tid + 256, ..
-        const int nkb = p.cols / 256, nwords = nr * 17;
+        // raw bytes: block kb of the tile's rows (1088 bytes per group of eight rows) -> raw[kb % 2]; thread tid copies 16-byte words tid, tid + 256, ..
+        const int nkb = p.cols / 256, nwords = (nr + 7) / 8 * 68;
         auto issue_raw = [&](int kb) {
             const uint32_t dst = pb_smem_u32(raw + (size_t)(kb % TC_RAW_STAGES) * TC_RAW_BYTES);
             for (int i = tid; i < nwords; i += TC_DECODERS * 32) {
-                const int r = i / 17, w = i - r * 17;
-                tc_cp_async8(dst + (uint32_t)(r * 136 + w * 8), wbase + (size_t)r * p.row_bytes + (size_t)kb * 136 + w * 8);
+                const int gr = i / 68, w = i - gr * 68;
+                tc_cp_async16(dst + (uint32_t)(gr * 1088 + w * 16), wbase + (size_t)gr * 8 * p.row_bytes + (size_t)kb * 1088 + w * 16);
             }
             tc_cp_async_arrive(&raw_full[kb % TC_RAW_STAGES]);
         };
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
         if (nkb > 1) issue_raw(1);
         // per-tile power-of-two shift: the largest |d| of the tile's rows times 465 lands in [2^14, 2^15)
         float dm = 0.f;
-        if (grp == 0 && live) for (int b = 0; b < nkb; b++) dm = fmaxf(dm, fabsf(pb_h2f(__ldg(reinterpret_cast<const uint16_t*>(wbase + (size_t)row * p.row_bytes + (size_t)b * 136)))));
+        if (grp == 0 && live) for (int b = 0; b < nkb; b++) dm = fmaxf(dm, fabsf(pb_h2f(__ldg(reinterpret_cast<const uint16_t*>(wbase + (size_t)(row & ~7) * p.row_bytes + (size_t)b * 1088 + 1024 + 8 * (row & 7))))));
         dm = pb_warp_max(dm);
         if (lane == 0) red[warp] = dm;
         if (tid < TC_NBLK) xinv[tid] = tid < nt ? reinterpret_cast<const float*>(p.xt)[tb * TC_NBLK + tid] : 0.f;
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
             // release the buffer and -- once all 256 threads have released it -- refill it with the block after next
             if ((k & 3) == grp && !pb_mbar_wait(&raw_full[rs], (kb / TC_RAW_STAGES) & 1, p.status, PB_DEV_TC_TIMEOUT)) { ok = false; break; }
             TcRaw cur;
-            tc_load_raw(cur, pb_smem_u32(raw + (size_t)rs * TC_RAW_BYTES) + (uint32_t)row * 136u, k & 3, live);
+            tc_load_raw(cur, pb_smem_u32(raw + (size_t)rs * TC_RAW_BYTES) + (uint32_t)(row >> 3) * 1088u, row & 7, k & 3, live);
             if ((k & 3) == grp + 2) {
                 pb_mbar_arrive(&raw_empty[rs]);
                 if (kb + 2 < nkb) {

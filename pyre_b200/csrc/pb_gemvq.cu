@@ -15,7 +15,7 @@
 //     made shared-memory wavefronts the bound; for large matrices the IQ3_S / IQ2_XS codebook is
 //     replicated once per shared-memory bank so that random lookups never conflict (64 KB of the
 //     227 KB per SM);
-//   - three or more columns of IQ3_S weights go to the tensor-core kernel of pb_gemmh.cu instead.
+//   - two and more columns go to the tensor-core kernels of pb_gemmh.cu instead.
 // Replaces QMat::matmul (src/model/gguf_q.rs:217-242), the k_gemv* / k_gemv_iq4* kernels and
 // the k_rms* prologues (src/model/qn_cube.rs:257-2331) of the reference.
 #include "pb_stream.cuh"
@@ -58,7 +58,8 @@ __global__ void __launch_bounds__(PB_KTHREADS, 1) pb_gemvq_kernel(const PbGemvQP
                 int s = 0;
                 while (s + 1 < p.nseg && chunk >= p.seg[s + 1].chunk0) s++;
                 const int r0 = (chunk - p.seg[s].chunk0) * p.rows_per_chunk;
-                const int nr = min(p.rows_per_chunk, p.seg[s].rows - r0);
+                int nr = min(p.rows_per_chunk, p.seg[s].rows - r0);
+                if (FMT == PB_T_IQ3S_N4) nr = (nr + 7) & ~7;   // whole groups of eight rows
                 const uint32_t bytes = ((uint32_t)nr * (uint32_t)p.row_bytes + 15u) & ~15u;
                 if (!pb_ring_acquire(ring, k, bytes, p.status)) break;
                 pb_ring_copy(ring, k, 0, p.seg[s].w + (size_t)r0 * p.row_bytes, bytes);
@@ -147,11 +148,18 @@ __global__ void __launch_bounds__(PB_KTHREADS, 1) pb_gemvq_kernel(const PbGemvQP
             // chains overlap each other's shared-memory latency (a row past nr decodes stale bytes of the
             // stage and is not stored)
             float* ybase = p.y + p.seg[s].yoff + r0;
+            // re-coded rows come in groups of eight: the warp's rows are all row (warp & 7) of their group
+            const uint32_t oc = pb_n4_code_off(warp & 7, ql), oh = pb_n4_head_off(warp & 7, ql);
             for (int ra = warp; ra < nr; ra += 2 * PB_CONSUMERS) {
                 const int rc = ra + PB_CONSUMERS;
                 const bool two = rc < p.rows_per_chunk;
-                float v0 = pb_decode_dot<FMT>(base + (uint32_t)ra * (uint32_t)p.row_bytes + (ql >> 2) * D::STEP_BYTES, ql & 3, T, xr[0]);
-                float v1 = pb_decode_dot<FMT>(base + (uint32_t)(two ? rc : ra) * (uint32_t)p.row_bytes + (ql >> 2) * D::STEP_BYTES, ql & 3, T, xr[0]);
+                float v0, v1;
+                if constexpr (FMT == PB_T_IQ3S_N4) {
+                    const uint32_t ga = base + (uint32_t)(ra & ~7) * (uint32_t)p.row_bytes, gb = base + (uint32_t)((two ? rc : ra) & ~7) * (uint32_t)p.row_bytes;
+                    PbQuarter wa, wb;
+                    D::quarter(ga + oc, ga + oh, ql & 3, wa); D::quarter(gb + oc, gb + oh, ql & 3, wb);
+                    v0 = pb_quarter_dot<FMT>(wa, xr[0]); v1 = pb_quarter_dot<FMT>(wb, xr[0]);
+                } else { v0 = pb_decode_dot<FMT>(base, ra, p.row_bytes, ql, T, xr[0]); v1 = pb_decode_dot<FMT>(base, two ? rc : ra, p.row_bytes, ql, T, xr[0]); }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) { v0 += __shfl_xor_sync(0xffffffffu, v0, o); v1 += __shfl_xor_sync(0xffffffffu, v1, o); }
                 if (lane == 0) {
@@ -169,17 +177,16 @@ __global__ void __launch_bounds__(PB_KTHREADS, 1) pb_gemvq_kernel(const PbGemvQP
 #pragma unroll
             for (int b = 0; b < NB; b++) acc[b] = 0.f;
             if (valid) {
-                const uint32_t rowp = base + (uint32_t)r * (uint32_t)p.row_bytes;
 #pragma unroll
                 for (int ps = 0; ps < PASSES; ps++) {
                     const int qi = ps * 32 + ql;
                     if (qi < nquarters) {
                         if (FMT == PB_T_IQ3_S && NB == 1) {
-                            acc[0] += pb_iq3s_quarter_dot(rowp + (qi >> 2) * D::STEP_BYTES, qi & 3, T, xr[ps]);
+                            acc[0] += pb_iq3s_quarter_dot(base + (uint32_t)r * (uint32_t)p.row_bytes + (qi >> 2) * D::STEP_BYTES, qi & 3, T, xr[ps]);
                             continue;
                         }
                         PbQuarter wq;
-                        D::quarter(rowp + (qi >> 2) * D::STEP_BYTES, qi & 3, T, wq);
+                        pb_quarter_at<FMT>(base, r, p.row_bytes, qi, T, wq);
                         if (NB == 1) {
                             acc[0] += pb_quarter_dot<FMT>(wq, xr[ps]);
                         } else {
@@ -228,7 +235,7 @@ static int launch_q(pb_ctx* ctx, const PbGemvQArgs& a, int row_bytes) {
     const size_t xbytes = ((size_t)NB * pb_xq_words(a.cols) * 4 + 127) & ~(size_t)127;
     const size_t fixed = 256 + p.tab_bytes + xbytes;
     int align_rows = 1;
-    while ((align_rows * row_bytes) % 16) align_rows *= 2;
+    while ((align_rows * row_bytes) % 16 || (FMT == PB_T_IQ3S_N4 && align_rows < 8)) align_rows *= 2;
     if (fixed + (size_t)PB_STAGES * (align_rows * row_bytes + 144) > (size_t)ctx->max_smem_optin)
         PB_FAIL(ctx, PB_UNSUPPORTED, "gemv: cols=%d with %d columns does not fit shared memory", a.cols, a.t);
     size_t stage_cap = ((size_t)ctx->max_smem_optin - fixed) / PB_STAGES;
@@ -294,14 +301,6 @@ int pb_launch_gemvq(pb_ctx* ctx, const PbGemvQArgs& a) {
         bool all = true;
         for (int s = 0; s < a.nseg && s < 4; s++) all = all && a.seg[s].wr != nullptr;
         if (use_tc && all && a.t >= pb_gemmtc_min_tokens()) return pb_launch_gemmtc(ctx, a);
-    }
-    if (a.mode != PB_ACT_PREQ && pb_gemvi_supported(a.type, a.cols, a.t)) {
-        bool all = true;
-        int64_t rows = 0;
-        for (int s = 0; s < a.nseg && s < 4; s++) { all = all && (a.type == PB_T_IQ3S_N4 ? a.seg[s].w : a.seg[s].wr) != nullptr; rows += a.seg[s].rows; }
-        // measured: from about ten million weights on it beats the dp4a kernel with two tokens, below that they tie
-        static const int64_t min_weights = getenv("PYRE_B200_IMMA_MIN_WEIGHTS") ? atoll(getenv("PYRE_B200_IMMA_MIN_WEIGHTS")) : ((int64_t)10 << 20);
-        if (all && rows * a.cols >= min_weights) return pb_launch_gemvi(ctx, a);
     }
     if (a.mode != PB_ACT_PREQ && pb_gemmh_supported(a.type, a.cols, a.t)) {
         static const bool use_mma = !(getenv("PYRE_B200_MMA") && atoi(getenv("PYRE_B200_MMA")) == 0);

@@ -1,0 +1,376 @@
+// Tensor-core core for quantized weights that meet a few tokens: warp-level mma.sync m16n8k16, f16 x f16 -> f32.
+//
+// A warp owns a tile of 16 weight rows over a run of 256-column blocks.  No warp waits for another: the weights of a block come into the
+// warp's own ring of shared-memory stages by asynchronous copies issued two blocks ahead, are decoded straight into the A operand, and meet
+// the tokens' activations, which the CTA prepared once in shared memory as B operands.
+//
+//   - Lane (g, q) = (lane >> 2, lane & 3) holds the 64 weights of quarter q of row g of the tile's two halves of eight rows.  The
+//     contraction index is permuted so that the four k of an mma that a lane holds are weights of its own quarter; A and B use the same
+//     permutation.
+//   - Weights enter as f16 integers (code times integer sub-block multiplier, at most 2048: exact), the f16 block scale d is applied in f32 to
+//     the sum over the block (PB_H_DIRECT, PB_H_FOLD); formats whose scales do not fold (Q8_0, Q6_K, ..) enter as the f16 high and low
+//     parts of the scaled weight, 22 significant bits (PB_H_SPLIT).
+//   - Activations are scaled by a power of two per token and block so that the largest lies in [2^9, 2^11), and split into f16 high and low parts
+//     (22 significant bits); column 2 j of an n-tile is the high part of token j, column 2 j + 1 its low part.
+//   - A token's columns do not depend on the other tokens: the result of a token is the same however tokens are grouped.
+#pragma once
+#include "pb_stream.cuh"
+#include <cuda_fp16.h>
+
+__device__ __forceinline__ void pb_hmma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ __half2 pb_as_h2(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
+__device__ __forceinline__ uint32_t pb_as_u32(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
+// (w & mask) | bits in one logic operation
+__device__ __forceinline__ uint32_t pb_and_or(uint32_t w, uint32_t mask, uint32_t bits) {
+    uint32_t d; asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(w), "r"(mask), "r"(bits)); return d;
+}
+// small non-negative integer (< 1024) in both halves of an f16 pair: the exponent of 1024 makes the mantissa the integer itself
+__device__ __forceinline__ __half2 pb_h2_int(uint32_t n) { return __hsub2(pb_as_h2((n * 0x00010001u) | 0x64006400u), pb_as_h2(0x64006400u)); }
+// activations in shared memory are rewritten between phases of a kernel: these loads stay where they are written
+__device__ __forceinline__ uint4 pb_ldsa128(uint32_t a) { uint4 v; asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a)); return v; }
+__device__ __forceinline__ uint32_t pb_ldsa32(uint32_t a) { uint32_t v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
+__device__ __forceinline__ uint2 pb_ldsa64(uint32_t a) { uint2 v; asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a)); return v; }
+
+enum { PB_H_DIRECT = 0,   // 4-bit codes decoded by the nibble
+       PB_H_FOLD = 1,     // int8 values, integer multipliers folded into the weights
+       PB_H_SPLIT = 2 };  // int8 values, scaled weights as high + low parts
+template <int FMT> __host__ __device__ constexpr int pb_h_mode() {
+    return FMT == PB_T_IQ3S_N4 || FMT == PB_T_Q4_K ? PB_H_DIRECT : (FMT == PB_T_IQ3_S || FMT == PB_T_IQ2_XS ? PB_H_FOLD : PB_H_SPLIT);
+}
+// a minimum per 32 weights, which meets the group sums of the activations in one more mma
+template <int FMT> __host__ __device__ constexpr bool pb_h_offs() { return FMT == PB_T_Q4_K || FMT == PB_T_Q5_K; }
+// order of the k index: words of eight consecutive weights as (0 2)(4 6)(1 3)(5 7), or (Q4_K) of four weights of each of the quarter's two groups
+template <int FMT> __host__ __device__ constexpr bool pb_h_twin() { return FMT == PB_T_Q4_K; }
+
+// ---------------------------------------------------------------- weights of one block of a tile -> a stage
+// A tile is two halves of eight rows (they may belong to different matrices).
+struct PbHTile { const uint8_t *a, *b; int la, lb; };   // first row of each half, last valid row of each (0 .. 7)
+struct PbHGeom { int row_bytes, step_bytes, npiece, pitch, stage_bytes; };   // bytes of a row, of a block of 256 columns; 16-byte pieces per row of a stage, its row pitch, its size
+template <int FMT> __host__ __device__ constexpr bool pb_h_grouped() { return FMT == PB_T_IQ3S_N4; }   // rows in groups of eight (pb_repack.cu)
+template <int FMT>
+static inline PbHGeom pb_h_geom(int cols) {
+    int el, bs;
+    pb_geom(FMT, &el, &bs);
+    PbHGeom h;
+    h.row_bytes = cols / el * bs; h.step_bytes = 256 / el * bs;
+    if (pb_h_grouped<FMT>()) { h.npiece = 68; h.pitch = 136; h.stage_bytes = 2 * 1088; }
+    else if (h.step_bytes % 16 == 0 && h.row_bytes % 16 == 0) { h.npiece = h.step_bytes / 16; h.pitch = (h.npiece | 1) * 16; h.stage_bytes = 16 * h.pitch; }
+    else { h.npiece = (h.step_bytes + 14 + 15) / 16; h.pitch = (h.npiece | 1) * 16; h.stage_bytes = 16 * h.pitch; }   // an odd number of 16-byte words: the rows start on different banks
+    return h;
+}
+__device__ __forceinline__ void pb_h_cp16(uint32_t dst, const uint8_t* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+// rows start at any even byte: the copy covers the 16-byte pieces around them and keeps their alignment
+template <int FMT>
+__device__ __forceinline__ void pb_h_stage(uint32_t stage, const PbHTile& t, const PbHGeom& h, int blk, int lane) {
+    if constexpr (pb_h_grouped<FMT>()) {
+        const uint8_t *a = t.a + blk * 1088 + 16 * lane, *b = t.b + blk * 1088 + 16 * lane;
+        stage += 16 * lane;
+        pb_h_cp16(stage, a); pb_h_cp16(stage + 512, a + 512); pb_h_cp16(stage + 1088, b); pb_h_cp16(stage + 1600, b + 512);
+        if (lane < 8) pb_h_cp16(stage + (lane < 4 ? 1024 : 2112 - 64), lane < 4 ? a + 1024 : b + 960);   // the rows' heads: 64 bytes of each half
+    } else {
+        for (int i = lane; i < 16 * h.npiece; i += 32) {
+            const int r = i / h.npiece, c = i - r * h.npiece;
+            const uint8_t* p = (r < 8 ? t.a + (size_t)min(r, t.la) * h.row_bytes : t.b + (size_t)min(r - 8, t.lb) * h.row_bytes) + (size_t)blk * h.step_bytes;
+            pb_h_cp16(stage + (uint32_t)(r * h.pitch + 16 * c), p - (reinterpret_cast<uintptr_t>(p) & 15) + 16 * c);
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// ---------------------------------------------------------------- nibble formats: the lane's bytes of a block
+template <int FMT> struct PbHRaw;
+template <> struct PbHRaw<PB_T_IQ3S_N4> {
+    uint4 c0, c1; uint2 h;
+    __device__ __forceinline__ void load(uint32_t p, int g, int q) {   // p = the half's block
+        const uint32_t a = p + (uint32_t)((4 * g + q) * 16);
+        c0 = pb_ldsa128(a); c1 = pb_ldsa128(a + 512); h = pb_ldsa64(p + 1024 + 8 * g);
+    }
+};
+template <> struct PbHRaw<PB_T_Q4_K> {
+    uint4 c0, c1, h;
+    __device__ __forceinline__ void load(uint32_t p, int, int q) {         // p = the row's block
+        h = pb_ldsa128(p); c0 = pb_ldsa128(p + 16 + 32 * q); c1 = pb_ldsa128(p + 32 + 32 * q);
+    }
+};
+// decoder over the raw registers: word u -> four f16 pairs
+template <int FMT> struct PbHDec;
+template <> struct PbHDec<PB_T_IQ3S_N4> {
+    __half2 m2[2], m15[2];   // 2 m and -15 m of the quarter's two groups
+    __device__ __forceinline__ void head(const PbHRaw<PB_T_IQ3S_N4>& r, int q) {
+        const uint32_t sc = r.h.y >> (8 * q);
+        const __half2 s0 = pb_h2_int(sc & 0xF), s1 = pb_h2_int((sc >> 4) & 0xF);      // multiplier m = 1 + 2 s <= 31
+        const __half2 k4 = pb_as_h2(0x44004400u), k2 = pb_as_h2(0x40004000u), km30 = pb_as_h2(0xCF80CF80u), km15 = pb_as_h2(0xCB80CB80u);   // 4, 2, -30, -15
+        m2[0] = __hfma2(s0, k4, k2); m15[0] = __hfma2(s0, km30, km15);
+        m2[1] = __hfma2(s1, k4, k2); m15[1] = __hfma2(s1, km30, km15);
+    }
+    __device__ static __forceinline__ float d(const PbHRaw<PB_T_IQ3S_N4>& r) { return pb_h2f((uint16_t)(r.h.x & 0xFFFF)); }
+    __device__ static __forceinline__ float dmin(const PbHRaw<PB_T_IQ3S_N4>&) { return 0.f; }
+    __device__ static __forceinline__ uint32_t offs(const PbHRaw<PB_T_IQ3S_N4>&, int) { return 0u; }
+    // (2 c - 15) m: the code sits in the mantissa of an f16 with exponent 1024 (low nibbles) or 64 (high nibbles); both steps are exact
+    __device__ __forceinline__ void word(const PbHRaw<PB_T_IQ3S_N4>& r, int u, uint32_t (&o)[4]) const {
+        const uint4& c = u < 4 ? r.c0 : r.c1;
+        const uint32_t w = (u & 3) == 0 ? c.x : ((u & 3) == 1 ? c.y : ((u & 3) == 2 ? c.z : c.w)), w8 = w >> 8;
+        const __half2 k1024 = pb_as_h2(0x64006400u), k64 = pb_as_h2(0x54005400u), a = m2[u >> 2], b = m15[u >> 2];
+        o[0] = pb_as_u32(__hfma2(__hsub2(pb_as_h2(pb_and_or(w, 0x000F000Fu, 0x64006400u)), k1024), a, b));
+        o[1] = pb_as_u32(__hfma2(__hsub2(pb_as_h2(pb_and_or(w, 0x00F000F0u, 0x54005400u)), k64), a, b));
+        o[2] = pb_as_u32(__hfma2(__hsub2(pb_as_h2(pb_and_or(w8, 0x000F000Fu, 0x64006400u)), k1024), a, b));
+        o[3] = pb_as_u32(__hfma2(__hsub2(pb_as_h2(pb_and_or(w8, 0x00F000F0u, 0x54005400u)), k64), a, b));
+    }
+};
+template <> struct PbHDec<PB_T_Q4_K> {
+    __half2 s[2], sk[2];     // scale of the two groups; -1024 scale (low nibbles), -64 scale (high nibbles)
+    // scale_min_k4 (gguf_q.rs:62-64) of groups 2 q and 2 q + 1: both groups' values in bytes 0 and 1
+    __device__ static __forceinline__ uint32_t scales(const uint4& h, int q) {
+        return q < 2 ? (h.y >> (16 * q)) & 0x3F3Fu : ((h.w >> (16 * (q - 2))) & 0x0F0Fu) | (((h.y >> (16 * (q - 2))) & 0xC0C0u) >> 2);
+    }
+    __device__ __forceinline__ void head(const PbHRaw<PB_T_Q4_K>& r, int q) {
+        const uint32_t s2 = scales(r.h, q);
+        s[0] = pb_h2_int(s2 & 0xFF); s[1] = pb_h2_int((s2 >> 8) & 0xFF);
+        sk[0] = __hmul2(s[0], pb_as_h2(0xE400E400u)); sk[1] = __hmul2(s[1], pb_as_h2(0xD400D400u));   // exact
+    }
+    __device__ static __forceinline__ float d(const PbHRaw<PB_T_Q4_K>& r) { return pb_h2f((uint16_t)(r.h.x & 0xFFFF)); }
+    __device__ static __forceinline__ float dmin(const PbHRaw<PB_T_Q4_K>& r) { return pb_h2f((uint16_t)(r.h.x >> 16)); }
+    // f16 pair of the two groups' integer minima
+    __device__ static __forceinline__ uint32_t offs(const PbHRaw<PB_T_Q4_K>& r, int q) {
+        const uint32_t m2 = q < 2 ? (r.h.z >> (16 * q)) & 0x3F3Fu : ((r.h.w >> (16 * (q - 2) + 4)) & 0x0F0Fu) | (((r.h.z >> (16 * (q - 2))) & 0xC0C0u) >> 2);
+        return pb_as_u32(__hsub2(pb_as_h2((m2 & 0xFF) | ((m2 & 0xFF00) << 8) | 0x64006400u), pb_as_h2(0x64006400u)));
+    }
+    // q * scale <= 945: (1024 + q) s - 1024 s and (64 + q) s - 64 s, exact
+    __device__ __forceinline__ void word(const PbHRaw<PB_T_Q4_K>& r, int u, uint32_t (&o)[4]) const {
+        const uint4& c = u < 4 ? r.c0 : r.c1;
+        const uint32_t w = (u & 3) == 0 ? c.x : ((u & 3) == 1 ? c.y : ((u & 3) == 2 ? c.z : c.w)), w8 = w >> 8;
+        o[0] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w, 0x000F000Fu, 0x64006400u)), s[0], sk[0]));
+        o[1] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w8, 0x000F000Fu, 0x64006400u)), s[0], sk[0]));
+        o[2] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w, 0x00F000F0u, 0x54005400u)), s[1], sk[1]));
+        o[3] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w8, 0x00F000F0u, 0x54005400u)), s[1], sk[1]));
+    }
+};
+
+// ---------------------------------------------------------------- activations in shared memory
+// Token slot: per block and word u of 8 weights one 128-byte row [high | low][quarter][8 halves]; then per block the inverse prescale (f32); then,
+// for formats with minima, per block and quarter the f16 pair of the two groups' sums and what that rounding lost (8 bytes).
+template <int FMT> __host__ __device__ constexpr int pb_h_tok_bytes(int cols) { return cols * 4 + ((cols / 256 * 4 + 15) & ~15) + (pb_h_offs<FMT>() ? cols / 256 * 32 : 0); }
+__device__ __forceinline__ uint32_t pb_h_scale_off(int bpr) { return (uint32_t)bpr * 1024u; }
+__device__ __forceinline__ uint32_t pb_h_sums_off(int bpr) { return (uint32_t)bpr * 1024u + (uint32_t)((bpr * 4 + 15) & ~15); }
+
+// columns of a block that lane (q = lane & 3, u = lane >> 2) prepares: [c0, c0 + 4) and [c1, c1 + 4)
+template <int FMT> __device__ __forceinline__ int pb_h_c0(int lane) { return 64 * (lane & 3) + (pb_h_twin<FMT>() ? 4 : 8) * (lane >> 2); }
+template <int FMT> __device__ __forceinline__ int pb_h_c1(int lane) { return pb_h_c0<FMT>(lane) + (pb_h_twin<FMT>() ? 32 : 4); }
+
+// One warp stores block blk of a token: v = the lane's eight activations (columns c0 .., c1 ..).
+template <int FMT>
+__device__ __forceinline__ void pb_h_put(uint8_t* slot, int bpr, int blk, int lane, const float (&x)[8]) {
+    const int q = lane & 3, u = lane >> 2;
+    constexpr bool twin = pb_h_twin<FMT>();
+    float m = fmaxf(fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3]))), fmaxf(fmaxf(fabsf(x[4]), fabsf(x[5])), fmaxf(fabsf(x[6]), fabsf(x[7]))));
+    m = pb_warp_max(m);
+    float p = 1.0f, ip = 1.0f;
+    if (m > 1e-30f && m < 1e30f) {   // 2^(9 - exponent) and its inverse, built from the exponent bits
+        const int e = (int)((__float_as_uint(m) >> 23) & 0xFF) - 127;
+        p = __uint_as_float((uint32_t)(9 - e + 127) << 23); ip = __uint_as_float((uint32_t)(e - 9 + 127) << 23);
+    }
+    if (lane == 0) *reinterpret_cast<float*>(slot + pb_h_scale_off(bpr) + 4 * blk) = ip;
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = x[i] * p;
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {   // pairs (0 2)(4 6)(1 3)(5 7), or (0 2)(1 3) of each group
+        const int e0 = twin ? (k < 2 ? k : k + 2) : (k < 2 ? 4 * k : 4 * (k - 2) + 1);
+        const __half2 h = __floats2half2_rn(v[e0], v[e0 + 2]);
+        const float2 r = __half22float2(h);
+        hi[k] = pb_as_u32(h); lo[k] = pb_as_u32(__floats2half2_rn(v[e0] - r.x, v[e0 + 2] - r.y));
+    }
+    uint8_t* row = slot + (size_t)blk * 1024 + u * 128 + q * 16;
+    *reinterpret_cast<uint4*>(row) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4*>(row + 64) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    if (pb_h_offs<FMT>()) {
+        // sums of the quarter's two groups of 32: over the eight lanes u of the quarter (one group each half of the words unless twin)
+        float s0 = (v[0] + v[1]) + (v[2] + v[3]), s1 = (v[4] + v[5]) + (v[6] + v[7]);
+        if (!twin) { s0 += s1; s1 = u >= 4 ? s0 : 0.f; s0 = u >= 4 ? 0.f : s0; }
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) { s0 += __shfl_xor_sync(0xffffffffu, s0, o); s1 += __shfl_xor_sync(0xffffffffu, s1, o); }
+        if (u == 0) {
+            const __half2 h = __floats2half2_rn(s0, s1);
+            const float2 r = __half22float2(h);
+            *reinterpret_cast<uint2*>(slot + pb_h_sums_off(bpr) + blk * 32 + q * 8) = make_uint2(pb_as_u32(h), pb_as_u32(__floats2half2_rn(s0 - r.x, s1 - r.y)));
+        }
+    }
+}
+// The lane's addresses of the activations of tokens 4 nt + ..: b = B rows of token (g >> 1), sums = its group sums, scale = prescales of token q
+struct PbHLane { uint32_t b, sums, scale, tok4; };
+template <int FMT>
+__device__ __forceinline__ PbHLane pb_h_lane(uint32_t slot0, int bpr, int lane) {
+    const int g = lane >> 2, q = lane & 3;
+    const uint32_t tokb = (uint32_t)pb_h_tok_bytes<FMT>(256 * bpr), s = slot0 + (uint32_t)(g >> 1) * tokb;
+    PbHLane l;
+    l.b = s + (uint32_t)((g & 1) * 64 + q * 16); l.sums = s + pb_h_sums_off(bpr) + 8u * q; l.scale = slot0 + (uint32_t)q * tokb + pb_h_scale_off(bpr); l.tok4 = 4 * tokb;
+    return l;
+}
+
+// ---------------------------------------------------------------- one block of one tile
+// tot[nt][0] = row g of the first half, tot[nt][1] = row g of the second half, token 4 nt + q.
+template <int FMT, int NT>
+__device__ __forceinline__ void pb_h_add(const float (&acc)[NT][4], int nt, int blk, float fa, float fb, float oa, float ob, const PbHLane& L, float (&tot)[NT][2]) {
+    float va = __fadd_rn(__fmul_rn(fa, acc[nt][0]), __fmul_rn(fa, acc[nt][1])), vb = __fadd_rn(__fmul_rn(fb, acc[nt][2]), __fmul_rn(fb, acc[nt][3]));
+    if (pb_h_offs<FMT>()) { va += oa; vb += ob; }
+    const float s = __uint_as_float(pb_ldsa32(L.scale + (uint32_t)nt * L.tok4 + 4u * blk));
+    tot[nt][0] = __fadd_rn(tot[nt][0], __fmul_rn(va, s)); tot[nt][1] = __fadd_rn(tot[nt][1], __fmul_rn(vb, s));
+}
+template <int FMT, int NT>
+__device__ __forceinline__ void pb_h_block_nib(uint32_t stage, const PbHGeom& h, int blk, int lane, const PbHLane& L, float (&tot)[NT][2]) {
+    const int g = lane >> 2, q = lane & 3;
+    PbHRaw<FMT> ra, rb;
+    if constexpr (pb_h_grouped<FMT>()) { ra.load(stage, g, q); rb.load(stage + 1088, g, q); }
+    else { ra.load(stage + (uint32_t)(g * h.pitch), g, q); rb.load(stage + (uint32_t)((g + 8) * h.pitch), g, q); }
+    PbHDec<FMT> wa, wb;
+    wa.head(ra, q); wb.head(rb, q);
+    float acc[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; nt++) { acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f; }
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        uint32_t a[4], b[4];
+        wa.word(ra, u, a); wb.word(rb, u, b);
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++) {
+            const uint4 x = pb_ldsa128(L.b + (uint32_t)nt * L.tok4 + (uint32_t)(blk * 1024 + u * 128));
+            pb_hmma(acc[nt], a[0], b[0], a[1], b[1], x.x, x.y);
+            pb_hmma(acc[nt], a[2], b[2], a[3], b[3], x.z, x.w);
+        }
+    }
+    const float da = PbHDec<FMT>::d(ra), db = PbHDec<FMT>::d(rb);
+#pragma unroll
+    for (int nt = 0; nt < NT; nt++) {
+        float oa = 0.f, ob = 0.f;
+        if (pb_h_offs<FMT>()) {
+            uint2 s = pb_ldsa64(L.sums + (uint32_t)nt * L.tok4 + (uint32_t)(blk * 32));
+            if (g & 1) s = make_uint2(0u, 0u);         // low columns: the high columns carry both parts of the sums
+            const uint32_t ma = PbHDec<FMT>::offs(ra, q), mb = PbHDec<FMT>::offs(rb, q);
+            float mc[4] = {0.f, 0.f, 0.f, 0.f};
+            pb_hmma(mc, ma, mb, ma, mb, s.x, s.y);
+            oa = -PbHDec<FMT>::dmin(ra) * mc[0]; ob = -PbHDec<FMT>::dmin(rb) * mc[2];
+        }
+        pb_h_add<FMT, NT>(acc, nt, blk, da, db, oa, ob, L, tot);
+    }
+}
+
+// ---------------------------------------------------------------- int8 formats (the decoders of the dp4a kernels)
+// Integer multipliers of a quarter (per 16 weights) and the f32 factor of the whole block
+template <int FMT> __device__ __forceinline__ void pb_h_mults(uint32_t p, int qt, float& d, uint32_t (&m)[4]);
+template <> __device__ __forceinline__ void pb_h_mults<PB_T_IQ3_S>(uint32_t p, int qt, float& d, uint32_t (&m)[4]) {
+    d = pb_h2f((uint16_t)pb_lds16(p));
+    const uint32_t sc = pb_lds8(p + 106 + qt);
+    m[0] = m[1] = 1 + 2 * (sc & 0xF); m[2] = m[3] = 1 + 2 * (sc >> 4);
+}
+template <> __device__ __forceinline__ void pb_h_mults<PB_T_IQ2_XS>(uint32_t p, int qt, float& d, uint32_t (&m)[4]) {
+    d = pb_h2f((uint16_t)pb_lds16(p)) * 0.125f;              // d (0.5 + s) / 4 = d / 8 (1 + 2 s)
+    const uint32_t sc = pb_lds16(p + 66 + 2 * qt);
+#pragma unroll
+    for (int h = 0; h < 4; h++) m[h] = 1 + 2 * ((sc >> (4 * h)) & 0xF);
+}
+// bytes (0, 2) or (1, 3) of a word of four signed bytes, already flipped to unsigned, as the mantissas of 1024 + 128 + v
+__device__ __forceinline__ uint32_t pb_h_bytes(uint32_t w, bool odd) { return pb_prmt(w, 0x64646464u, odd ? 0x4341u : 0x4240u); }
+
+template <int FMT, int NT>
+__device__ __forceinline__ void pb_h_block_int(uint32_t pa, uint32_t pb, const PbQTabs& T, int blk, int lane, const PbHLane& L, float (&tot)[NT][2]) {
+    using D = PbQDec<FMT>;
+    const int q = lane & 3;
+    float acc[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; nt++) { acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f; }
+    PbQuarter wa, wb;
+    D::quarter(pa, q, T, wa); D::quarter(pb, q, T, wb);
+    float fa, fb;                                              // f32 factor of the block's sum
+    if constexpr (pb_h_mode<FMT>() == PB_H_FOLD) {
+        uint32_t ma[4], mb[4];
+        pb_h_mults<FMT>(pa, q, fa, ma); pb_h_mults<FMT>(pb, q, fb, mb);
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const __half2 sa = pb_h2_int(ma[u >> 1]), sb = pb_h2_int(mb[u >> 1]), k = pb_as_h2(0xE480E480u);   // -1152
+            const __half2 ka = __hmul2(sa, k), kb = __hmul2(sb, k);                                             // exact: at most 9 significant bits
+            uint32_t a[4], b[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                a[e] = pb_as_u32(__hfma2(pb_as_h2(pb_h_bytes((uint32_t)wa.w[2 * u + (e & 1)] ^ 0x80808080u, e >= 2)), sa, ka));
+                b[e] = pb_as_u32(__hfma2(pb_as_h2(pb_h_bytes((uint32_t)wb.w[2 * u + (e & 1)] ^ 0x80808080u, e >= 2)), sb, kb));
+            }
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++) {
+                const uint4 x = pb_ldsa128(L.b + (uint32_t)nt * L.tok4 + (uint32_t)(blk * 1024 + u * 128));
+                pb_hmma(acc[nt], a[0], b[0], a[1], b[1], x.x, x.y);
+                pb_hmma(acc[nt], a[2], b[2], a[3], b[3], x.z, x.w);
+            }
+        }
+    } else {
+        // power of two that puts the largest scale of the row's block into [1, 2); scales as f16 high + low parts
+        auto norm = [&](PbQuarter& w, float& f) {
+            float m = fmaxf(fmaxf(fabsf(w.sc[0]), fabsf(w.sc[1])), fmaxf(fabsf(w.sc[2]), fabsf(w.sc[3])));
+            if (D::HAS_MIN) m = fmaxf(m, fmaxf(fabsf(w.mn[0]), fabsf(w.mn[1])) * (1.0f / 64.f));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1)); m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+            float p = 1.0f; f = 1.0f;
+            if (m > 1e-30f && m < 1e30f) { const uint32_t e = (__float_as_uint(m) >> 23) & 0xFF; p = __uint_as_float((254u - e) << 23); f = __uint_as_float(e << 23); }
+#pragma unroll
+            for (int h = 0; h < 4; h++) w.sc[h] *= p;
+            if (D::HAS_MIN) { w.mn[0] *= p; w.mn[1] *= p; }
+        };
+        norm(wa, fa); norm(wb, fb);
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const float sfa = wa.sc[u >> 1], sfb = wb.sc[u >> 1];
+            const __half ha = __float2half_rn(sfa), hb = __float2half_rn(sfb);
+            const __half2 sah = __half2half2(ha), sbh = __half2half2(hb), sal = __half2half2(__float2half_rn(sfa - __half2float(ha))), sbl = __half2half2(__float2half_rn(sfb - __half2float(hb)));
+            const __half2 k = pb_as_h2(0x64806480u);            // 1152
+            uint32_t a[4], b[4], al[4], bl[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                // scaled weight = high + low: the remainder of the high product is exact in one fused multiply-add
+                const __half2 va = __hsub2(pb_as_h2(pb_h_bytes((uint32_t)wa.w[2 * u + (e & 1)] ^ 0x80808080u, e >= 2)), k);
+                const __half2 vb = __hsub2(pb_as_h2(pb_h_bytes((uint32_t)wb.w[2 * u + (e & 1)] ^ 0x80808080u, e >= 2)), k);
+                const __half2 pa2 = __hmul2(va, sah), pb2 = __hmul2(vb, sbh);
+                a[e] = pb_as_u32(pa2); b[e] = pb_as_u32(pb2);
+                al[e] = pb_as_u32(__hfma2(va, sal, __hfma2(va, sah, __hneg2(pa2)))); bl[e] = pb_as_u32(__hfma2(vb, sbl, __hfma2(vb, sbh, __hneg2(pb2))));
+            }
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++) {
+                const uint4 x = pb_ldsa128(L.b + (uint32_t)nt * L.tok4 + (uint32_t)(blk * 1024 + u * 128));
+                pb_hmma(acc[nt], a[0], b[0], a[1], b[1], x.x, x.y);
+                pb_hmma(acc[nt], a[2], b[2], a[3], b[3], x.z, x.w);
+                pb_hmma(acc[nt], al[0], bl[0], al[1], bl[1], x.x, x.y);
+                pb_hmma(acc[nt], al[2], bl[2], al[3], bl[3], x.z, x.w);
+            }
+        }
+    }
+#pragma unroll
+    for (int nt = 0; nt < NT; nt++) {
+        float oa = 0.f, ob = 0.f;
+        if (D::HAS_MIN && pb_h_offs<FMT>()) {
+            uint2 s = pb_ldsa64(L.sums + (uint32_t)nt * L.tok4 + (uint32_t)(blk * 32));
+            if ((lane >> 2) & 1) s = make_uint2(0u, 0u);
+            const __half2 ma = __floats2half2_rn(wa.mn[0], wa.mn[1]), mb = __floats2half2_rn(wb.mn[0], wb.mn[1]);
+            const float2 ra = __half22float2(ma), rb = __half22float2(mb);
+            const uint32_t la = pb_as_u32(__floats2half2_rn(wa.mn[0] - ra.x, wa.mn[1] - ra.y)), lb = pb_as_u32(__floats2half2_rn(wb.mn[0] - rb.x, wb.mn[1] - rb.y));
+            float mc[4] = {0.f, 0.f, 0.f, 0.f};
+            pb_hmma(mc, pb_as_u32(ma), pb_as_u32(mb), pb_as_u32(ma), pb_as_u32(mb), s.x, s.y);
+            pb_hmma(mc, la, lb, la, lb, s.x, s.y);
+            oa = -fa * mc[0]; ob = -fb * mc[2];
+        }
+        pb_h_add<FMT, NT>(acc, nt, blk, fa, fb, oa, ob, L, tot);
+    }
+}
+
+// the block in stage `stage` of tile t, whichever the format: block wblk of the weight rows, block blk of the prepared activations
+template <int FMT, int NT>
+__device__ __forceinline__ void pb_h_block(uint32_t stage, const PbHTile& t, const PbHGeom& h, const PbQTabs& T, int wblk, int blk, int lane, const PbHLane& L, float (&tot)[NT][2]) {
+    if constexpr (pb_h_mode<FMT>() == PB_H_DIRECT) pb_h_block_nib<FMT, NT>(stage, h, blk, lane, L, tot);
+    else {
+        const int g = lane >> 2;
+        const uint32_t oa = (uint32_t)(reinterpret_cast<uintptr_t>(t.a) + (uint32_t)min(g, t.la) * (uint32_t)h.row_bytes + (uint32_t)wblk * (uint32_t)h.step_bytes) & 15u;
+        const uint32_t ob = (uint32_t)(reinterpret_cast<uintptr_t>(t.b) + (uint32_t)min(g, t.lb) * (uint32_t)h.row_bytes + (uint32_t)wblk * (uint32_t)h.step_bytes) & 15u;
+        pb_h_block_int<FMT, NT>(stage + (uint32_t)(g * h.pitch) + oa, stage + (uint32_t)((g + 8) * h.pitch) + ob, T, blk, lane, L, tot);
+    }
+}

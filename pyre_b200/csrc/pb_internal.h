@@ -4,7 +4,6 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <string.h>
-#include <map>
 #include <string>
 #include <vector>
 
@@ -15,7 +14,7 @@ struct pb_ctx {
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;   // the stream every kernel of this context is launched on
     int* dev_status = nullptr;       // device status word (see PB_DEV_* in pb_common.cuh)
-    uint8_t* xh_buf = nullptr;       // PB_XH_BYTES: activation fragments of the tensor-core GEMM (pb_gemmh.cu)
+    uint8_t* xh_buf = nullptr;       // PB_XH_BYTES: activation tiles of the tcgen05 GEMM (pb_gemmtc.cu)
     int* host_status = nullptr;      // pinned host mirror, filled by an async copy before each sync
     int sm_count = 148;
     int max_smem_optin = 0;
@@ -32,9 +31,6 @@ struct pb_ctx {
     bool pdl_chain = false;  // the previous op on the stream was one of our kernels
     void* ep_comm = nullptr;
     int ep_rank = 0, ep_world = 1;
-    // largest dynamic shared-memory size set so far per kernel function: the attribute belongs to the device's
-    // copy of the function, so the cache lives in the context, not in the process
-    std::map<const void*, size_t> smem_cfg;
     // tracing: stamp slots handed to the launches of the streaming kernels while enabled (pb_ctx_stamps_enable)
     unsigned long long* stamps = nullptr; int stamp_slots = 0, stamp_next = 0;
     std::vector<int> stamp_ids;   // kernel id (PB_K_*) per handed-out slot
@@ -111,30 +107,31 @@ struct pb_qmat {
 // Kernel launch on the context's stream; inside the token step consecutive kernels are chained with
 // programmatic stream serialization (every such kernel calls pb_pdl_wait before touching dependent data).
 template <typename K, typename... A>
-static inline void pb_launch_k(pb_ctx* ctx, K kern, dim3 grid, dim3 block, size_t smem, A... args) {
+// pb_launch_kc: in clusters of `cluster` CTAs.
+static inline void pb_launch_kc(pb_ctx* ctx, K kern, dim3 grid, dim3 block, size_t smem, int cluster, A... args) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof cfg);
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = ctx->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (ctx->use_pdl && ctx->pdl_scope > 0 && ctx->pdl_chain) { at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[n].val.programmaticStreamSerializationAllowed = 1; n++; }
+    if (cluster > 1) { at[n].id = cudaLaunchAttributeClusterDimension; at[n].val.clusterDim.x = (unsigned)cluster; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1; n++; }
     cfg.attrs = at;
-    cfg.numAttrs = (ctx->use_pdl && ctx->pdl_scope > 0 && ctx->pdl_chain) ? 1 : 0;
+    cfg.numAttrs = (unsigned)n;
     ctx->pdl_chain = ctx->pdl_scope > 0;
     cudaLaunchKernelEx(&cfg, kern, args...);   // errors are picked up by cudaGetLastError at the call site
 }
 
-// Raise the kernel's dynamic shared-memory limit on this context's device when `smem` exceeds what was set before.
+template <typename K, typename... A>
+static inline void pb_launch_k(pb_ctx* ctx, K kern, dim3 grid, dim3 block, size_t smem, A... args) { pb_launch_kc(ctx, kern, grid, block, smem, 1, args...); }
+// Raise the kernel's dynamic shared-memory limit on this context's device when `smem` exceeds what was set before.  The limit belongs to
+// the device's copy of the function, which all contexts on that device share: it only ever grows (pb_api.cu).
+int pb_ensure_smem_fn(pb_ctx* ctx, const void* kern, size_t smem);
 template <typename K>
-static inline int pb_ensure_smem(pb_ctx* ctx, K kern, size_t smem) {
-    const void* key = reinterpret_cast<const void*>(kern);
-    auto it = ctx->smem_cfg.find(key);
-    if (it != ctx->smem_cfg.end() && it->second >= smem) return PB_OK;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) { char b[256]; snprintf(b, sizeof b, "cudaFuncSetAttribute(%zu bytes of shared memory): %s", smem, cudaGetErrorString(e)); ctx->err = b; return PB_ERR_CUDA; }
-    ctx->smem_cfg[key] = smem;
-    return PB_OK;
-}
+static inline int pb_ensure_smem(pb_ctx* ctx, K kern, size_t smem) { return pb_ensure_smem_fn(ctx, reinterpret_cast<const void*>(kern), smem); }
+
+// clusters of `cluster` CTAs of this kernel that fit the device at once (asked once per configuration)
+int pb_max_clusters(pb_ctx* ctx, const void* kern, int threads, size_t smem, int cluster);
 
 // next stamp slot (PB_STAMP_WORDS words), or null when tracing is off or the slots are used up; kernel_id is recorded on the host
 unsigned long long* pb_stamp_slot(pb_ctx* ctx, int kernel_id);
@@ -171,7 +168,7 @@ struct PbGemvArgs {
     int64_t ldy;
 };
 int pb_launch_gemv(pb_ctx* ctx, const PbGemvArgs& a);
-int pb_launch_repack_iq3s(pb_ctx* ctx, const uint8_t* src, uint8_t* dst, int64_t nblocks);
+int pb_launch_repack_iq3s(pb_ctx* ctx, const uint8_t* src, uint8_t* dst, int64_t rows, int bpr);   // dst: ceil(rows / 8) groups of bpr * 1088 bytes
 
 // pb_gemvq.cu: integer-core GEMV over up to four same-shaped-row matrices with a fused
 // activation prologue and an optional accumulate (residual) epilogue.
@@ -180,7 +177,7 @@ enum { PB_ACT_PLAIN = 0,   // x as given
        PB_ACT_GNORM = 2,   // per head of head_dim: rms(x) * norm_w[head_dim], times sigmoid(z)
        PB_ACT_PREQ = 3 };  // activations already split into int8 levels (xq_in)
 struct PbGemvSegArg { const uint8_t* w; int64_t rows; int64_t yoff; const uint8_t* wr; };   // wr: re-coded rows (pb_qmat::rdata) or null
-#define PB_XH_BYTES (((size_t)16 << 20) + 8192)   // operand buffer of the tensor-core GEMMs: t * cols * 4 bytes + a header (e.g. 1024 tokens of 4096 columns)
+#define PB_XH_BYTES (((size_t)16 << 20) + 8192)   // operand buffer of the tcgen05 GEMM: t * cols * 4 bytes + a header (e.g. 1024 tokens of 4096 columns)
 struct PbGemvQArgs {
     int type, cols, nseg;
     PbGemvSegArg seg[4];
@@ -202,19 +199,15 @@ struct PbGemvQParams {
     float* y; int64_t ldy;
     int mode; const float* norm_w; const float* z; int64_t ldz; int head_dim; float eps;
     const uint32_t* xq_in;
-    const uint8_t* xh_in; const float* xinv_in;   // pb_gemmh.cu: f16 fragments and prescale inverses made by its prep kernel
     int accumulate;
     int* status;
     unsigned long long* stamps;
 };
 bool pb_gemvq_supported(int type, int cols);
 int pb_launch_gemvq(pb_ctx* ctx, const PbGemvQArgs& a);
-// pb_gemmh.cu: tensor-core path for 3..16 columns of IQ3_S weights
+// pb_gemmh.cu: warp-level tensor-core path from two columns on, every quantized format
 bool pb_gemmh_supported(int type, int cols, int t);
 int pb_launch_gemmh(pb_ctx* ctx, const PbGemvQArgs& a);
-// pb_gemvi.cu: int8 tensor-core path for one and two columns of IQ3_S weights that have a re-coded copy
-bool pb_gemvi_supported(int type, int cols, int t);
-int pb_launch_gemvi(pb_ctx* ctx, const PbGemvQArgs& a);
 // pb_gemmtc.cu: tcgen05 path for 16 and more columns of IQ3_S weights that have a re-coded copy
 bool pb_gemmtc_supported(int type, int cols, int t);
 int pb_launch_gemmtc(pb_ctx* ctx, const PbGemvQArgs& a);
@@ -230,7 +223,8 @@ struct PbRouterParams {
     const float* sh_gate_inp;                 // f32 [cols] or null
     int n_exp;
     float* logits; int64_t ldl;               // [t][ldl >= n_exp + 1], entry n_exp = shared-gate logit
-    uint32_t* xq_out;                         // [t][pb_xq_words(cols)] int8-split activations
+    uint32_t* xq_out;                         // [t][pb_xq_words(cols)] int8-split activations, or null
+    float* scale_out;                         // [t] RMS scales for the tensor-core expert kernels, or null
     // phase 0: everything.  Sharded tokens split it around the all-gather: phase 1 = logits of the local
     // tokens plus a raw copy of their rows into xcopy (row stride ldl); phase 2 = split + routing of all
     // gathered tokens (no GEMV)
@@ -254,7 +248,9 @@ struct PbExpertParams {
     const uint32_t* xq;                       // gate/up: int8-split activations per token
     const uint8_t* w_a; const uint8_t* w_b;   // gate/up: gate_exps, up_exps; down: down_exps, unused
     const uint8_t* sh_a; const uint8_t* sh_b; // shared expert counterparts
+    int4* virt; int* n_virt;                  // several tokens: distinct local experts in groups of up to PB_VGROUP entries {expert, first entry, entries, 0}, and their number
     float* h; float* h_sh;                    // hidden [entry][ff], [t][ff_sh]
+#define PB_VGROUP 8
     uint32_t* hq;                             // down, several tokens: int8-split hidden vectors [t * top_k + t][pb_xq_words(ff)], else null
     float* part; float* part_sh;              // down: [t][top_k][d], [t][d]
     float* const* part_tok;                   // down, peer exchange: part_tok[token] = [top_k][d] block in the memory of the token's owner (else null)
@@ -268,6 +264,10 @@ struct PbExpertParams {
 struct PbCombineParams {
     const float* part; const float* part_sh; const float* logits; int64_t ldl;
     int t, d, top_k, n_exp;
+    // tensor-core kernels (pb_moeh.cu): groups of entries, raw token rows with their RMS scales and the norm weight (null: x is normalized)
+    const int4* virt; const int* n_virt;
+    const float* x; int64_t ldx; const float* norm_w; const float* tok_scale;
+    int nslots;                               // token slots of a CTA
     float* y; int64_t ldy; int accumulate;
     // peer exchange (device copy of the descriptor): before reading `part`, announce exchange exch_idx (kind 1: this
     // rank's expert rows are stored in their owners' memory) and wait for every rank's announcement
@@ -284,6 +284,10 @@ struct PbDeltaParams {
     const float* conv_w; const float* a; const float* dt;
     float* conv;                              // [batch][conv_k slots][ch] ring
     float* ssm;                               // [batch][nv][dk][dv]
+// pb_moeh.cu: the expert kernels of two and more tokens on the tensor cores
+bool pb_moeh_supported(int type, int d, int ff, int t);
+int pb_launch_moeh_gu(pb_ctx* ctx, const PbExpertParams& p, int type, int cols);
+int pb_launch_moeh_down(pb_ctx* ctx, const PbExpertParams& p, int type, int cols);
     const int64_t* pos;                       // [batch]
     float* out; int64_t ldo;                  // [batch][nv*dv] readout before the gated norm
     int nk, nv, dk, dv, conv_k, batch;

@@ -100,7 +100,7 @@ __device__ __forceinline__ void pb_route_token_cta(const PbRouteParams& p, int b
 __device__ __forceinline__ void pb_route_lists(const PbRouteParams& p, int* rsm) {
     int* cnt = rsm;                 // [1024] entries per expert (local experts only)
     int* cursor = rsm + 1024;       // [1024] start offset of the expert's entries, then a fill cursor
-    __shared__ int wsum[2][8];
+    __shared__ int wsum[3][8];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int e = tid; e < 1024; e += 256) { cnt[e] = 0; cursor[e] = 0; }
     __syncthreads();
@@ -111,20 +111,29 @@ __device__ __forceinline__ void pb_route_lists(const PbRouteParams& p, int* rsm)
     __syncthreads();
     // distinct local experts in ascending id with entry offsets: block-wide exclusive scans of
     // (used flag, entry count) over expert ids; thread t owns experts 4t .. 4t+3
-    int c4[4], f = 0, c = 0;
+    int c4[4], f = 0, c = 0, v = 0;   // distinct experts, entries, groups of PB_VGROUP entries
 #pragma unroll
-    for (int q = 0; q < 4; q++) { const int e = 4 * tid + q; c4[q] = e < p.n_exp ? cnt[e] : 0; f += c4[q] > 0; c += c4[q]; }
-    int fi = f, ci = c;
+    for (int q = 0; q < 4; q++) { const int e = 4 * tid + q; c4[q] = e < p.n_exp ? cnt[e] : 0; f += c4[q] > 0; c += c4[q]; v += (c4[q] + PB_VGROUP - 1) / PB_VGROUP; }
+    int fi = f, ci = c, vi = v;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) { const int a = __shfl_up_sync(0xffffffffu, fi, o), d = __shfl_up_sync(0xffffffffu, ci, o); if (lane >= o) { fi += a; ci += d; } }
-    if (lane == 31) { wsum[0][warp] = fi; wsum[1][warp] = ci; }
+    for (int o = 1; o < 32; o <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, fi, o), d = __shfl_up_sync(0xffffffffu, ci, o), b = __shfl_up_sync(0xffffffffu, vi, o);
+        if (lane >= o) { fi += a; ci += d; vi += b; }
+    }
+    if (lane == 31) { wsum[0][warp] = fi; wsum[1][warp] = ci; wsum[2][warp] = vi; }
     __syncthreads();
-    int fb = 0, cb = 0;
-    for (int w2 = 0; w2 < warp; w2++) { fb += wsum[0][w2]; cb += wsum[1][w2]; }
-    int n = fb + fi - f, off = cb + ci - c;   // exclusive prefixes for expert 4 * tid
+    int fb = 0, cb = 0, vb = 0;
+    for (int w2 = 0; w2 < warp; w2++) { fb += wsum[0][w2]; cb += wsum[1][w2]; vb += wsum[2][w2]; }
+    int n = fb + fi - f, off = cb + ci - c, vn = vb + vi - v;   // exclusive prefixes for expert 4 * tid
 #pragma unroll
-    for (int q = 0; q < 4; q++) if (c4[q] > 0) { const int e = 4 * tid + q; p.used_e[n] = e; p.used_off[n] = off; cursor[e] = off; n++; off += c4[q]; }
-    if (tid == 255) { p.used_off[n] = off; *p.n_used = n; }
+    for (int q = 0; q < 4; q++)
+        if (c4[q] > 0) {
+            const int e = 4 * tid + q;
+            p.used_e[n] = e; p.used_off[n] = off; cursor[e] = off;
+            if (p.virt) for (int k = 0; k < c4[q]; k += PB_VGROUP) p.virt[vn++] = make_int4(e, off + k, min(PB_VGROUP, c4[q] - k), 0);
+            n++; off += c4[q];
+        }
+    if (tid == 255) { p.used_off[n] = off; *p.n_used = n; if (p.virt) *p.n_virt = vn; }
     __syncthreads();
     for (int i = tid; i < p.t * p.top_k; i += 256) {
         const int e = __ldcg(p.sel_e + i);
@@ -196,10 +205,10 @@ __global__ void __launch_bounds__(256) pb_router_kernel(const PbRouterParams p, 
     // per-token RMS scale (rms(): 1 / sqrt(mean(x^2) + eps), qwen4exp_gguf.rs:209); one warp per token
     for (int b = b_lo + warp; b < b_hi; b += 8) {
         const float s = p.norm_w ? pb_row_rms_scale(p.x + b * p.ldx, p.cols, p.eps, lane) : 1.0f;
-        if (lane == 0) scale[b] = s;
+        if (lane == 0) { scale[b] = s; if (p.scale_out && blockIdx.x == 0) p.scale_out[b] = s; }
     }
     __syncthreads();
-    const int ng = p.cols / 32;
+    const int ng = p.phase == 1 || p.xq_out ? p.cols / 32 : 0;
     for (int g0 = blockIdx.x * 4; g0 < ng; g0 += gridDim.x * 4) {
         for (int b = b_lo + warp; b < b_hi; b += 8) {
             float4 v = *reinterpret_cast<const float4*>(p.x + b * p.ldx + 32 * g0 + 4 * lane);
@@ -294,7 +303,6 @@ __global__ void __launch_bounds__(256) pb_router_kernel(const PbRouterParams p, 
 
 template <int FMT, int PASSES>
 __global__ void __launch_bounds__(PB_KTHREADS, 1) pb_expert_gu_kernel(const PbExpertParams p) {
-    using D = PbQDec<FMT>;
     extern __shared__ __align__(128) uint8_t smem[];
     PbRing ring;
     ring.full = reinterpret_cast<uint64_t*>(smem);
@@ -416,8 +424,8 @@ __global__ void __launch_bounds__(PB_KTHREADS, 1) pb_expert_gu_kernel(const PbEx
             for (int ps = 0; ps < PASSES; ps++) {
                 const int qi = ps * 32 + ql;
                 if (qi < nquarters) {
-                    D::quarter(base + (uint32_t)r * p.row_bytes + (qi >> 2) * D::STEP_BYTES, qi & 3, T, wg[ps]);
-                    D::quarter(base + half + (uint32_t)r * p.row_bytes + (qi >> 2) * D::STEP_BYTES, qi & 3, T, wu[ps]);
+                    pb_quarter_at<FMT>(base, r, p.row_bytes, qi, T, wg[ps]);
+                    pb_quarter_at<FMT>(base + half, r, p.row_bytes, qi, T, wu[ps]);
                 }
             }
             for (int en = e0; en < e1; en++) {
@@ -481,7 +489,6 @@ __global__ void __launch_bounds__(128) pb_split_h_kernel(const PbExpertParams p)
 
 template <int FMT, int PASSES>
 __global__ void __launch_bounds__(PB_KTHREADS, 1) pb_expert_down_kernel(const PbExpertParams p, const PbCombineParams cp, unsigned int* ticket) {
-    using D = PbQDec<FMT>;
     extern __shared__ __align__(128) uint8_t smem[];
     PbRing ring;
     ring.full = reinterpret_cast<uint64_t*>(smem);
@@ -586,7 +593,7 @@ __global__ void __launch_bounds__(PB_KTHREADS, 1) pb_expert_down_kernel(const Pb
 #pragma unroll
                 for (int ps = 0; ps < PASSES; ps++) {
                     const int qi = ps * 32 + ql;
-                    if (qi < nquarters) D::quarter(base + (uint32_t)r * p.row_bytes + (qi >> 2) * D::STEP_BYTES, qi & 3, T, wq[ps]);
+                    if (qi < nquarters) pb_quarter_at<FMT>(base, r, p.row_bytes, qi, T, wq[ps]);
                 }
                 for (int en = e0; en < e1; en++) {
                     int tok, slot = 0; float wgt = 1.0f;
@@ -627,7 +634,7 @@ __global__ void __launch_bounds__(PB_KTHREADS, 1) pb_expert_down_kernel(const Pb
                     const int qi = ps * 32 + ql;
                     if (qi < nquarters) {
                         PbQuarter wq; PbXQuarter xv;
-                        D::quarter(base + (uint32_t)r * p.row_bytes + (qi >> 2) * D::STEP_BYTES, qi & 3, T, wq);
+                        pb_quarter_at<FMT>(base, r, p.row_bytes, qi, T, wq);
                         pb_load_xquarter<PbQDec<FMT>::AFFINE>(xq, cols, qi, xv);
                         acc += pb_quarter_dot<FMT>(wq, xv);
                     }
@@ -664,7 +671,6 @@ __global__ void __launch_bounds__(PB_KTHREADS, 1) pb_expert_down_kernel(const Pb
 #define PB_DR_MAXE 16
 template <int FMT>
 __global__ void __launch_bounds__(PB_KTHREADS, 1) pb_expert_down_rows_kernel(const PbExpertParams p, const PbCombineParams cp) {
-    using D = PbQDec<FMT>;
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);                       // [PB_DR_MAXE]
     float* res = reinterpret_cast<float*>(smem + 128);                        // [PB_DR_MAXE][16 rows]
@@ -729,7 +735,7 @@ __global__ void __launch_bounds__(PB_KTHREADS, 1) pb_expert_down_rows_kernel(con
         if (!pb_mbar_wait(&full[k], 0, p.status, PB_DEV_WAIT_FULL_TIMEOUT)) break;
         if (i == 0) pb_stamp(p.stamps, 4, st_first);
         PbQuarter wq; PbXQuarter xv;
-        D::quarter(pb_smem_u32(stages + (size_t)k * slice) + (uint32_t)r * p.row_bytes + (ql >> 2) * D::STEP_BYTES, ql & 3, T, wq);
+        pb_quarter_at<FMT>(pb_smem_u32(stages + (size_t)k * slice), r, p.row_bytes, ql, T, wq);
         pb_load_xquarter<PbQDec<FMT>::AFFINE>(xq + (size_t)k * xw, cols, ql, xv);
         float acc = pb_quarter_dot<FMT>(wq, xv);
         for (int o = nquarters >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);

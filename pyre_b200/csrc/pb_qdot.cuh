@@ -178,21 +178,23 @@ template <> struct PbQDec<PB_T_Q4_K> {
 template <> struct PbQDec<PB_T_IQ3S_N4> {
     static constexpr int STEP_BYTES = 136;
     static constexpr bool HAS_MIN = false, SCALE16 = false, AFFINE = true;
-    __device__ static __forceinline__ void quarter(uint32_t p, int qt, const PbQTabs&, PbQuarter& o) {
-        const uint32_t hdr = pb_lds32(p);
-        const float d = pb_h2f((uint16_t)(hdr & 0xFFFF));
-        const uint32_t sc = pb_lds8(p + 4 + qt);
+    // a = shared address of the quarter's first 16 bytes, hp = of the row's head (pb_repack.cu)
+    __device__ static __forceinline__ void quarter(uint32_t a, uint32_t hp, int qt, PbQuarter& o) {
+        const uint2 hdr = pb_lds64(hp);
+        const float d = pb_h2f((uint16_t)(hdr.x & 0xFFFF));
+        const uint32_t sc = (hdr.y >> (8 * qt)) & 0xFF;
         const float d0 = d * (float)(1 + 2 * (int)(sc & 0xF)), d1 = d * (float)(1 + 2 * (int)(sc >> 4));
         o.sc[0] = o.sc[1] = d0; o.sc[2] = o.sc[3] = d1;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint2 c = pb_lds64(p + 8 + 32 * qt + 8 * i);
-            o.w[4 * i + 0] = (int)(c.x & 0x0F0F0F0Fu); o.w[4 * i + 1] = (int)((c.x >> 4) & 0x0F0F0F0Fu);
-            o.w[4 * i + 2] = (int)(c.y & 0x0F0F0F0Fu); o.w[4 * i + 3] = (int)((c.y >> 4) & 0x0F0F0F0Fu);
+        for (int i = 0; i < 2; i++) {
+            const uint4 c = pb_lds128(a + 512 * i);
+            o.w[8 * i + 0] = (int)(c.x & 0x0F0F0F0Fu); o.w[8 * i + 1] = (int)((c.x >> 4) & 0x0F0F0F0Fu);
+            o.w[8 * i + 2] = (int)(c.y & 0x0F0F0F0Fu); o.w[8 * i + 3] = (int)((c.y >> 4) & 0x0F0F0F0Fu);
+            o.w[8 * i + 4] = (int)(c.z & 0x0F0F0F0Fu); o.w[8 * i + 5] = (int)((c.z >> 4) & 0x0F0F0F0Fu);
+            o.w[8 * i + 6] = (int)(c.w & 0x0F0F0F0Fu); o.w[8 * i + 7] = (int)((c.w >> 4) & 0x0F0F0F0Fu);
         }
     }
 };
-
 // ---- IQ3_XXS: per 32 weights eight 8-bit grid indices (entries of four magnitudes) and one u32 with four 7-bit sign
 // patterns and a 4-bit scale (gguf_q.rs:136-140).  Grid entries from shared memory (256 x 4 bytes), signs through the
 // 256-entry mask table after the parity bit is restored, as IQ2_XS.
@@ -505,6 +507,16 @@ template <> struct PbQDec<PB_T_Q6_K> {
     }
 };
 
+// offset of quarter qi of row r7 (0 .. 7) inside a group of eight re-coded rows, and of its head
+__device__ __forceinline__ uint32_t pb_n4_code_off(int r7, int qi) { return (uint32_t)(qi >> 2) * 1088u + (uint32_t)((4 * r7 + (qi & 3)) * 16); }
+__device__ __forceinline__ uint32_t pb_n4_head_off(int r7, int qi) { return (uint32_t)(qi >> 2) * 1088u + 1024u + 8u * (uint32_t)r7; }
+// Quarter qi of row r of a run of rows that starts at shared address `base` (for the re-coded form: at a group of eight rows)
+template <int FMT>
+__device__ __forceinline__ void pb_quarter_at(uint32_t base, int r, int row_bytes, int qi, const PbQTabs& T, PbQuarter& o) {
+    if constexpr (FMT == PB_T_IQ3S_N4) { const uint32_t gp = base + (uint32_t)(r & ~7) * (uint32_t)row_bytes; PbQDec<FMT>::quarter(gp + pb_n4_code_off(r & 7, qi), gp + pb_n4_head_off(r & 7, qi), qi & 3, o); }
+    else PbQDec<FMT>::quarter(base + (uint32_t)r * (uint32_t)row_bytes + (uint32_t)(qi >> 2) * PbQDec<FMT>::STEP_BYTES, qi & 3, T, o);
+}
+
 // unsigned bytes of a times signed bytes of b
 __device__ __forceinline__ int pb_dp4a_us(int a, int b, int c) {
     int d; asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d;
@@ -600,11 +612,11 @@ __device__ __forceinline__ float pb_iq3s_quarter_dot(uint32_t p, int qt, const P
     return acc;
 }
 
-// decode one quarter and dot it with one column's activations
+// decode quarter qi of row r of the run at `base` and dot it with one column's activations
 template <int FMT>
-__device__ __forceinline__ float pb_decode_dot(uint32_t p, int qt, const PbQTabs& T, const PbXQuarter& x) {
-    if (FMT == PB_T_IQ3_S) return pb_iq3s_quarter_dot(p, qt, T, x);
+__device__ __forceinline__ float pb_decode_dot(uint32_t base, int r, int row_bytes, int qi, const PbQTabs& T, const PbXQuarter& x) {
+    if constexpr (FMT == PB_T_IQ3_S) return pb_iq3s_quarter_dot(base + (uint32_t)r * (uint32_t)row_bytes + (uint32_t)(qi >> 2) * PbQDec<FMT>::STEP_BYTES, qi & 3, T, x);
     PbQuarter w;
-    PbQDec<FMT>::quarter(p, qt, T, w);
+    pb_quarter_at<FMT>(base, r, row_bytes, qi, T, w);
     return pb_quarter_dot<FMT>(w, x);
 }

@@ -130,7 +130,6 @@ struct PsOpFetch {
 
 template <int PASSES>
 __device__ __forceinline__ bool ps_gemv(PsCtx& c, const PbStepOp& op) {
-    using D = PbQDec<PS_FMT>;
     const PsGemvOp& g = op.g;
     const int cols = g.cols, mode = g.mode;
     const int tid = c.tid, warp = c.warp, lane = c.lane;
@@ -217,8 +216,8 @@ __device__ __forceinline__ bool ps_gemv(PsCtx& c, const PbStepOp& op) {
             for (int ra = warp; ra < nr; ra += 2 * PB_CONSUMERS) {
                 const int rc = ra + PB_CONSUMERS;
                 const bool two = rc < rpc;
-                float v0 = pb_decode_dot<PS_FMT>(base + (uint32_t)ra * (uint32_t)row_bytes + (ql >> 2) * D::STEP_BYTES, ql & 3, T, xr);
-                float v1 = pb_decode_dot<PS_FMT>(base + (uint32_t)(two ? rc : ra) * (uint32_t)row_bytes + (ql >> 2) * D::STEP_BYTES, ql & 3, T, xr);
+                float v0 = pb_decode_dot<PS_FMT>(base, ra, row_bytes, ql, T, xr);
+                float v1 = pb_decode_dot<PS_FMT>(base, two ? rc : ra, row_bytes, ql, T, xr);
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) { v0 += __shfl_xor_sync(0xffffffffu, v0, o); v1 += __shfl_xor_sync(0xffffffffu, v1, o); }
                 if (lane == 0) {
@@ -232,13 +231,12 @@ __device__ __forceinline__ bool ps_gemv(PsCtx& c, const PbStepOp& op) {
                 const bool valid = r < nr;
                 float acc = 0.f;
                 if (valid) {
-                    const uint32_t rowp = base + (uint32_t)r * (uint32_t)row_bytes;
 #pragma unroll
                     for (int ps = 0; ps < PASSES; ps++) {
                         const int qi = ps * 32 + ql;
                         if (qi < nquarters) {
                             PbQuarter wq;
-                            D::quarter(rowp + (qi >> 2) * D::STEP_BYTES, qi & 3, T, wq);
+                            pb_quarter_at<PS_FMT>(base, r, row_bytes, qi, T, wq);
                             if (PASSES == 1) acc += pb_quarter_dot<PS_FMT>(wq, xr);
                             else { PbXQuarter xq2; pb_load_xquarter<true>(c.xq, cols, qi, xq2); acc += pb_quarter_dot<PS_FMT>(wq, xq2); }
                         }
@@ -262,7 +260,7 @@ __device__ __forceinline__ bool ps_gemv_produce(PsCtx& c, const PbStepOp& op) {
         while (sgi + 1 < g.nseg && chunk >= g.seg[sgi + 1].chunk0) sgi++;
         const int r0 = (chunk - g.seg[sgi].chunk0) * g.rows_per_chunk;
         const int nr = min(g.rows_per_chunk, g.seg[sgi].rows - r0);
-        const uint32_t bytes = ((uint32_t)nr * (uint32_t)g.row_bytes + 15u) & ~15u;
+        const uint32_t bytes = (uint32_t)((nr + 7) & ~7) * (uint32_t)g.row_bytes;   // whole groups of eight rows
         if (!ps_acquire(c, c.k, bytes)) return false;
         ps_copy(c, c.k, 0, g.seg[sgi].w + (size_t)r0 * g.row_bytes, bytes);
     }
@@ -419,14 +417,13 @@ __device__ __forceinline__ void ps_route(PsCtx& c, const PsMoeOp& m) {
 }
 
 __device__ __forceinline__ bool ps_gu_chunk(PsCtx& c, const PsMoeOp& m, int ci, const PbXQuarter& xr, int lpr, int ql, int half, int r) {
-    using D = PbQDec<PS_FMT>;
     const PbQTabs T = {0u, 0u, 0u};
     const int rg = m.rg, cpe = m.ff / rg;
     if (!ps_wait_full(c, c.k)) return false;
     // the shared expert's chunks come first (their rows never wait for the routing)
     const int slot = ci < cpe ? m.top_k : ci / cpe - 1, r0 = (ci % cpe) * rg;
-    const uint32_t base = pb_smem_u32(ps_stage(c, c.k)) + (uint32_t)half * (uint32_t)rg * (uint32_t)m.row_bytes_gu + (uint32_t)r * (uint32_t)m.row_bytes_gu;
-    float v = pb_decode_dot<PS_FMT>(base + (ql >> 2) * D::STEP_BYTES, ql & 3, T, xr);
+    const uint32_t base = pb_smem_u32(ps_stage(c, c.k)) + (uint32_t)half * (uint32_t)rg * (uint32_t)m.row_bytes_gu;
+    float v = pb_decode_dot<PS_FMT>(base, r, m.row_bytes_gu, ql, T, xr);
     for (int o = lpr >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     const int par = c.k & 1;
     if (ql == 0) c.m->gu[par][half][r] = v;
@@ -516,7 +513,6 @@ __device__ __forceinline__ bool ps_gu_produce(PsCtx& c, const PbStepOp& op) {
 // so the weighted sum over the experts (ascending expert id, then the shared expert as in pb_combine_one) is formed
 // inside the CTA and added to the residual directly (the arithmetic of pb_expert_down_rows_kernel).
 __device__ __forceinline__ bool ps_down(PsCtx& c, const PbStepOp& op) {
-    using D = PbQDec<PS_FMT>;
     const PsMoeOp& m = op.m;
     const int cols = m.ff, xw = pb_xq_words(cols), tid = c.tid, warp = c.warp, lane = c.lane;
     const int top_k = m.top_k, nsl = top_k + 1, spc = m.spc, row_bytes = m.row_bytes_dn;
@@ -563,7 +559,7 @@ __device__ __forceinline__ bool ps_down(PsCtx& c, const PbStepOp& op) {
             ps_fine(c, 4 + cur);
         }
         PbQuarter wq; PbXQuarter xv;
-        D::quarter(pb_smem_u32(ps_stage(c, kbase + cur)) + (uint32_t)(k % spc) * slice + (uint32_t)r * (uint32_t)row_bytes + (ql >> 2) * D::STEP_BYTES, ql & 3, T, wq);
+        pb_quarter_at<PS_FMT>(pb_smem_u32(ps_stage(c, kbase + cur)) + (uint32_t)(k % spc) * slice, r, row_bytes, ql, T, wq);
         pb_load_xquarter<true>(c.xq + (size_t)k * xw, cols, ql, xv);
         float acc = pb_quarter_dot<PS_FMT>(wq, xv);
         for (int o = nquarters >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
