@@ -148,8 +148,9 @@ __device__ __forceinline__ void pb_route_lists(const PbRouteParams& p, int* rsm)
 // levels for the expert kernels, so that work is spread over the grid.
 #define PB_ROUTER_TPG 8   // tokens per router CTA (one warp each for the RMS scales)
 #define PB_ROUTER_TICKETS 8   // ticket[0 .. 8): whole-launch counters (router, expert kernels); ticket[8 + g]: token group g of the router
+template <bool QUADS>
 __global__ void __launch_bounds__(256) pb_router_kernel(const PbRouterParams p, const PbRouteParams rp, unsigned int* ticket) {
-    extern __shared__ float rs[];   // 2048 ints for the routing pass, then scale[t]
+    extern __shared__ float rs[];   // 2048 ints for the routing pass, then scale[t], then the partial sums of several tokens
     float* scale = rs + 2048;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const bool st_first = tid == 0 && blockIdx.x == 0 && blockIdx.y == 0;
@@ -158,8 +159,15 @@ __global__ void __launch_bounds__(256) pb_router_kernel(const PbRouterParams p, 
     // trip to DRAM overlaps that kernel's tail
     const int row = blockIdx.x * 8 + warp;
     const float* wrow = p.phase != 2 && row <= p.n_exp ? (row < p.n_exp ? p.router + (size_t)row * p.cols : p.sh_gate_inp) : nullptr;
+    // one token: a warp holds a row; several tokens: four rows x a quarter of the columns (rows 4 (warp & 1) .. of the CTA's eight)
     PbRouterRow2048 rr;
-    if (p.cols == 2048 && wrow) rr.load(wrow, p.norm_w, lane);
+    PbRouterQuad rq;
+    if constexpr (QUADS) {
+        const float* rows[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) { const int rw = blockIdx.x * 8 + 4 * (warp & 1) + r; rows[r] = rw < p.n_exp ? p.router + (size_t)rw * p.cols : (rw == p.n_exp ? p.sh_gate_inp : nullptr); }
+        rq.load(rows, p.norm_w, warp >> 1, lane);
+    } else if (p.cols == 2048 && wrow) rr.load(wrow, p.norm_w, lane);
     pb_pdl_wait();
     pb_pdl_trigger();
     pb_stamp(p.stamps, 2, st_first);
@@ -172,7 +180,7 @@ __global__ void __launch_bounds__(256) pb_router_kernel(const PbRouterParams p, 
     }
     // grid.y cuts the tokens into groups of PB_ROUTER_TPG: this CTA handles tokens [b_lo, b_hi)
     const int b_lo = (int)blockIdx.y * PB_ROUTER_TPG, b_hi = min(p.t, b_lo + PB_ROUTER_TPG);
-    if (p.t == 1 && p.cols == 2048 && p.phase == 0 && p.norm_w && !p.exch) {
+    if (!QUADS && p.t == 1 && p.cols == 2048 && p.phase == 0 && p.norm_w && !p.exch && p.xq_out) {
         // One token on one GPU: every warp fetches the activation row once, in the layout that the RMS scale, the row product and
         // (for the CTAs that split a piece of it) the split all use, instead of one trip to L2 for each of the three.  Same arithmetic
         // as pb_row_rms_scale, PbRouterRow2048::dot and the general loops below.
@@ -226,7 +234,24 @@ __global__ void __launch_bounds__(256) pb_router_kernel(const PbRouterParams p, 
         }
     }
     pb_stamp(p.stamps, 3, st_first);   // activations split
-    if (p.phase != 2 && row <= p.n_exp) {
+    if constexpr (QUADS) {
+        float* qs = scale + ((p.t + 31) & ~31);   // [8 tokens][4 quarters][8 rows]
+#pragma unroll 2
+        for (int b = b_lo; b < b_hi; b++) {
+            const float acc = rq.dot(p.x + b * p.ldx, warp >> 1, lane);
+            if ((lane & 7) == 0) qs[(b - b_lo) * 32 + (warp >> 1) * 8 + 4 * (warp & 1) + (lane >> 3)] = acc;
+        }
+        __syncthreads();
+        for (int i = tid; i < 8 * (b_hi - b_lo); i += 256) {
+            const int b = b_lo + (i >> 3), rw = blockIdx.x * 8 + (i & 7);
+            const float* v = qs + (i >> 3) * 32 + (i & 7);
+            const float acc = ((v[0] + v[8]) + (v[16] + v[24])) * scale[b];
+            if (rw <= p.n_exp) {
+                p.logits[b * p.ldl + rw] = acc;
+                if (p.exch) for (int q = 0; q < p.exch->world; q++) p.exch->peer_xg[q][p.peer_off + b * p.ldl + p.cols + rw] = acc;
+            }
+        }
+    } else if (p.phase != 2 && row <= p.n_exp) {
         if (p.cols == 2048 && wrow) {
             // the row, times the norm weight, stays in registers for all tokens
 #pragma unroll 2
@@ -782,10 +807,13 @@ int pb_launch_router(pb_ctx* ctx, const PbRouterParams& p, const PbRouteParams& 
     if (p.cols % 128) PB_FAIL(ctx, PB_UNSUPPORTED, "router: width %d is not a multiple of 128", p.cols);
     if (rp.top_k > PB_MAX_TOPK || rp.n_exp > 1024) PB_FAIL(ctx, PB_UNSUPPORTED, "route: top_k %d / n_exp %d beyond %d / 1024", rp.top_k, rp.n_exp, PB_MAX_TOPK);
     const int grid = p.phase == 2 ? (p.cols / 128 > 0 ? p.cols / 128 : 1) : (p.n_exp + 1 + 7) / 8;   // phase 2 only splits (4 groups of 32 per CTA) and routes
-    const size_t smem = (size_t)(2048 + ((p.t + 31) & ~31)) * 4;
+    const size_t smem = (size_t)(2048 + ((p.t + 31) & ~31) + 32 * PB_ROUTER_TPG) * 4;
     PbRouterParams ps = p;
     ps.stamps = pb_stamp_slot(ctx, PB_K_ROUTER);
-    pb_launch_k(ctx, pb_router_kernel, dim3(grid, (p.t + PB_ROUTER_TPG - 1) / PB_ROUTER_TPG), dim3(256), smem, ps, rp, ticket);
+    const dim3 gd(grid, (p.t + PB_ROUTER_TPG - 1) / PB_ROUTER_TPG);
+    // several tokens of the model's width: four rows x a quarter of the columns per warp
+    if (p.cols == 2048 && p.phase != 2 && p.t > 1) pb_launch_k(ctx, pb_router_kernel<true>, gd, dim3(256), smem, ps, rp, ticket);
+    else pb_launch_k(ctx, pb_router_kernel<false>, gd, dim3(256), smem, ps, rp, ticket);
     ctx->kernels_launched++;
     PB_CUDA(ctx, cudaGetLastError());
     return PB_OK;

@@ -37,6 +37,47 @@ struct PbRouterRow2048 {
     }
 };
 
+// Four router rows x a quarter of their 2048 columns, held by one warp for several tokens: one fetch of the token's 512 values serves four
+// rows (a row per warp is bound by those fetches: 120 us for 256 tokens x 513 rows, this form 73 us).  The quarters of a row meet in shared memory.
+struct PbRouterQuad {
+    float4 w[4][4];
+    __device__ __forceinline__ void load(const float* const (&rows)[4], const float* norm_w, int kq, int lane) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int c = 512 * kq + lane * 4 + 128 * k;
+            float4 n = make_float4(1.f, 1.f, 1.f, 1.f);
+            if (norm_w) n = *reinterpret_cast<const float4*>(norm_w + c);
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (rows[r]) v = *reinterpret_cast<const float4*>(rows[r] + c);
+                v.x *= n.x; v.y *= n.y; v.z *= n.z; v.w *= n.w;
+                w[r][k] = v;
+            }
+        }
+    }
+    // lane l ends up with the sum of row (l >> 3) & 3 over the warp's columns
+    __device__ __forceinline__ float dot(const float* x, int kq, int lane) const {
+        float4 v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = *reinterpret_cast<const float4*>(x + 512 * kq + lane * 4 + 128 * k);
+        float a[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; k++) { s0 = fmaf(w[r][k].x, v[k].x, s0); s1 = fmaf(w[r][k].y, v[k].y, s1); s0 = fmaf(w[r][k].z, v[k].z, s0); s1 = fmaf(w[r][k].w, v[k].w, s1); }
+            a[r] = s0 + s1;
+        }
+        // rows (0 1 | 2 3) by lane bit 4, then (0 | 1), (2 | 3) by bit 3
+        const bool h = lane & 16, l = lane & 8;
+        float b0 = (h ? a[2] : a[0]) + __shfl_xor_sync(0xffffffffu, h ? a[0] : a[2], 16), b1 = (h ? a[3] : a[1]) + __shfl_xor_sync(0xffffffffu, h ? a[1] : a[3], 16);
+        float c = (l ? b1 : b0) + __shfl_xor_sync(0xffffffffu, l ? b0 : b1, 8);
+        c += __shfl_xor_sync(0xffffffffu, c, 4); c += __shfl_xor_sync(0xffffffffu, c, 2); c += __shfl_xor_sync(0xffffffffu, c, 1);
+        return c;
+    }
+};
+
 // The same product for one token without keeping the row: (w n) is formed per element on the way (same roundings).
 __device__ __forceinline__ float pb_router_row2048_dot1(const float* wrow, const float* norm_w, const float* x, float scale, int lane) {
     float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
