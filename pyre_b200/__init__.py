@@ -9,7 +9,9 @@ anywhere, but creating a :class:`Ctx` without the library or without a GPU raise
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
+import weakref
 from pathlib import Path
 
 import numpy as np
@@ -105,6 +107,48 @@ def _f32(a):
     return np.ascontiguousarray(a, dtype=np.float32)
 
 
+class _PinnedPool:
+    """Page-locked result buffers of a context, handed out again once the arrays over them are gone.  A result in a fresh pageable array costs
+    a staging copy, a host copy and the page faults of the array (a third of a verify window's 6 x 151936 logits); one in a buffer of this pool
+    is a single DMA.  At most CAP idle bytes are kept.  Deques make take and give safe against finalizers of any thread without a lock."""
+
+    CAP = 64 << 20
+    MIN = 16 << 10          # below this a plain array is as fast
+
+    def __init__(self, ctx):
+        self.ctx, self.idle, self.idle_bytes = ctx, {}, 0
+
+    def empty(self, shape, dtype) -> np.ndarray:
+        n = int(np.prod(shape, dtype=np.int64)) * np.dtype(dtype).itemsize
+        if n < self.MIN:
+            return np.empty(shape, dtype)
+        size = -(-n // 4096) * 4096
+        try:
+            ptr = self.idle[size].pop()
+            self.idle_bytes -= size
+        except (KeyError, IndexError):
+            p = C.c_void_p()
+            if lib().pb_host_alloc(self.ctx.h, C.c_size_t(size), C.byref(p)):
+                return np.empty(shape, dtype)
+            ptr = p.value
+        buf = (C.c_uint8 * size).from_address(ptr)
+        weakref.finalize(buf, self._give, ptr, size).atexit = False
+        return np.frombuffer(buf, dtype=np.uint8, count=n).view(dtype).reshape(shape)
+
+    def _give(self, ptr, size):
+        if self.ctx is None or self.idle_bytes + size > self.CAP:
+            lib().pb_host_free(None, C.c_void_p(ptr))
+        else:
+            self.idle_bytes += size
+            self.idle.setdefault(size, collections.deque()).append(ptr)
+
+    def close(self):
+        self.ctx = None
+        for q in list(self.idle.values()):
+            while q:
+                lib().pb_host_free(None, C.c_void_p(q.pop()))
+
+
 class Ctx:
     """One GPU, one worker thread (the reference's Cube, src/model/qn_cube.rs:6237-6250)."""
 
@@ -114,6 +158,11 @@ class Ctx:
         if rc:
             raise PyreError(rc, "pb_ctx_create failed (is a CUDA device visible?)")
         self.device = device
+        self._pool = _PinnedPool(self)
+
+    def _result(self, shape, dtype=np.float32) -> np.ndarray:
+        """An array for a call's result, page-locked where that pays; like np.empty otherwise."""
+        return self._pool.empty(shape, dtype)
 
     def check(self, rc: int):
         if rc:
@@ -136,7 +185,6 @@ class Ctx:
         buf = (C.c_uint8 * max(n, 1)).from_address(ptr.value)
         arr = np.frombuffer(buf, dtype=np.uint8, count=n).view(dtype).reshape(shape)
         free = lib().pb_host_free
-        import weakref
         weakref.finalize(buf, lambda a=ptr.value: free(None, C.c_void_p(a)))     # without the context: the array may outlive it
         return arr
 
@@ -183,6 +231,7 @@ class Ctx:
 
     def close(self):
         if self.h:
+            self._pool.close()
             lib().pb_ctx_destroy(self.h)
             self.h = C.c_void_p()
 
@@ -261,7 +310,7 @@ class QMat:
         """y[t][rows] = x[t][cols] . W^T through the host-buffer entry point (QMat::matmul)."""
         x = _f32(x).reshape(-1, self.cols)
         t = x.shape[0] if t is None else t
-        y = np.empty((t, self.rows), dtype=np.float32)
+        y = self.ctx._result((t, self.rows))
         self.ctx.check(lib().pb_gemv(self.ctx.h, self.h, _p(x), C.c_int(t), _p(y)))
         return y
 

@@ -73,6 +73,37 @@ int pb_scratch(pb_ctx* ctx, size_t bytes, void** out) {
     return PB_OK;
 }
 
+bool pb_host_pinned(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
+    return a.type == cudaMemoryTypeHost;
+}
+static int pin_room(pb_ctx* ctx, size_t bytes) {
+    if (bytes <= ctx->pin_bytes) return PB_OK;
+    PB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    const size_t want = (bytes + ((size_t)1 << 20)) & ~(((size_t)1 << 20) - 1);
+    uint8_t* p = nullptr;
+    if (cudaMallocHost(&p, want) != cudaSuccess) { cudaGetLastError(); PB_FAIL(ctx, PB_ERR_OOM, "page-locked staging of %zu bytes failed", want); }
+    if (ctx->pin) { memcpy(p, ctx->pin, ctx->pin_bytes); cudaFreeHost(ctx->pin); }
+    ctx->pin = p; ctx->pin_bytes = want;
+    return PB_OK;
+}
+int pb_h2d(pb_ctx* ctx, void* dst, const void* src, size_t bytes, size_t off) {
+    if (off + bytes > PB_PIN_MAX || pb_host_pinned(src)) { PB_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream)); return PB_OK; }
+    PB_TRY(pin_room(ctx, off + bytes));
+    memcpy(ctx->pin + off, src, bytes);
+    PB_CUDA(ctx, cudaMemcpyAsync(dst, ctx->pin + off, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    return PB_OK;
+}
+int pb_d2h(pb_ctx* ctx, void* dst, const void* src, size_t bytes, size_t off, const void** staged) {
+    *staged = nullptr;
+    if (off + bytes > PB_PIN_MAX || pb_host_pinned(dst)) { PB_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream)); return PB_OK; }
+    PB_TRY(pin_room(ctx, off + bytes));
+    PB_CUDA(ctx, cudaMemcpyAsync(ctx->pin + off, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    *staged = ctx->pin + off;
+    return PB_OK;
+}
+
 // Synchronise the stream and turn a non-zero device status word into PB_ERR_DEVICE.
 int pb_sync_check(pb_ctx* ctx, const char* who) {
     PB_CUDA(ctx, cudaMemcpyAsync(ctx->host_status, ctx->dev_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -125,6 +156,7 @@ int pb_ctx_destroy(pb_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     pb_ep_destroy(ctx);
     if (ctx->scratch) cudaFree(ctx->scratch);
+    if (ctx->pin) cudaFreeHost(ctx->pin);
     if (ctx->stamps) cudaFree(ctx->stamps);
     if (ctx->dev_status) cudaFree(ctx->dev_status);
     if (ctx->xh_buf) cudaFree(ctx->xh_buf);
@@ -364,10 +396,12 @@ int pb_gemv(pb_ctx* ctx, const pb_qmat* m, const float* x_host, int t, float* y_
     PB_TRY(pb_scratch(ctx, xb + yb, &tmp));
     float* xd = (float*)tmp;
     float* yd = (float*)((uint8_t*)tmp + xb);
-    PB_CUDA(ctx, cudaMemcpyAsync(xd, x_host, (size_t)t * m->cols * 4, cudaMemcpyHostToDevice, ctx->stream));
+    const void* staged;
+    PB_TRY(pb_h2d(ctx, xd, x_host, (size_t)t * m->cols * 4, 0));
     PB_TRY(pb_gemv_dev(ctx, m, xd, t, yd));
-    PB_CUDA(ctx, cudaMemcpyAsync(y_host, yd, yb, cudaMemcpyDeviceToHost, ctx->stream));
+    PB_TRY(pb_d2h(ctx, y_host, yd, yb, xb, &staged));
     PB_TRY(pb_sync_check(ctx, "pb_gemv"));
+    if (staged) memcpy(y_host, staged, yb);
     return PB_OK;
 }
 

@@ -1259,15 +1259,10 @@ static int step_once(pb_state* s) {
 // Logits leave through a pinned buffer of the state: a device -> pageable-host copy is staged by the driver in small pieces
 // (about 0.1 ms for one 608 KB row), a copy into pinned memory runs at link speed and the host copies it on.
 // A destination in page-locked host memory (pb_host_alloc, or the caller's own registered buffer) takes the copy directly.
-static bool host_pinned(const void* p) {
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
-    return a.type == cudaMemoryTypeHost;
-}
 static int logits_stage(pb_state* s, size_t n, float* dst = nullptr, bool* direct = nullptr) {
     pb_ctx* ctx = s->m->ctx;
     if (direct) *direct = false;
-    if (dst && direct && host_pinned(dst)) {
+    if (dst && direct && pb_host_pinned(dst)) {
         PB_CUDA(ctx, cudaMemcpyAsync(dst, s->logits, n * 4, cudaMemcpyDeviceToHost, ctx->stream));
         *direct = true;
         return PB_OK;
@@ -1802,11 +1797,16 @@ int pb_moe_forward(pb_state* s, int layer, const float* x_host, int t, float* y_
     PB_TRY(layer_ok(s, layer, -1, "pb_moe_forward"));
     if (!x_host || !y_host || t < 0 || t > s->batch) PB_FAIL(ctx, PB_ERR_ARG, "pb_moe_forward: t=%d (state batch %d)", t, s->batch);
     if (t == 0) return PB_OK;
-    PB_CUDA(ctx, cudaMemcpyAsync(s->xin, x_host, (size_t)t * c.d * 4, cudaMemcpyHostToDevice, ctx->stream));
+    const size_t xb = (size_t)t * c.d * 4, sb = (size_t)t * c.top_k * 4;
+    const void *ys = nullptr, *ss = nullptr;
+    PB_TRY(pb_h2d(ctx, s->xin, x_host, xb, 0));
     PB_TRY(run_moe(s, layer, s->xin, nullptr, t, s->yout, c.d, 0));
-    PB_CUDA(ctx, cudaMemcpyAsync(y_host, s->yout, (size_t)t * c.d * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    if (sel_host) PB_CUDA(ctx, cudaMemcpyAsync(sel_host, s->sel_e, (size_t)t * c.top_k * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    return pb_sync_check(ctx, "pb_moe_forward");
+    if (sel_host) PB_TRY(pb_d2h(ctx, sel_host, s->sel_e, sb, xb, &ss));
+    PB_TRY(pb_d2h(ctx, y_host, s->yout, xb, xb + ((sb + 255) & ~(size_t)255), &ys));
+    PB_TRY(pb_sync_check(ctx, "pb_moe_forward"));
+    if (ss) memcpy(sel_host, ss, sb);
+    if (ys) memcpy(y_host, ys, xb);
+    return PB_OK;
 }
 
 int pb_deltanet_step(pb_state* s, int layer, const float* x_host, float* y_host) {

@@ -20,6 +20,7 @@ struct pb_ctx {
     int max_smem_optin = 0;
     std::string err;
     // grow-only device scratch for host-buffer entry points
+    uint8_t* pin = nullptr; size_t pin_bytes = 0;   // page-locked staging of the host-buffer entry points, grow-only
     void* scratch = nullptr;
     size_t scratch_bytes = 0;
     uint64_t kernels_launched = 0;
@@ -106,8 +107,8 @@ struct pb_qmat {
 
 // Kernel launch on the context's stream; inside the token step consecutive kernels are chained with
 // programmatic stream serialization (every such kernel calls pb_pdl_wait before touching dependent data).
-template <typename K, typename... A>
 // pb_launch_kc: in clusters of `cluster` CTAs.
+template <typename K, typename... A>
 static inline void pb_launch_kc(pb_ctx* ctx, K kern, dim3 grid, dim3 block, size_t smem, int cluster, A... args) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof cfg);
@@ -121,9 +122,9 @@ static inline void pb_launch_kc(pb_ctx* ctx, K kern, dim3 grid, dim3 block, size
     ctx->pdl_chain = ctx->pdl_scope > 0;
     cudaLaunchKernelEx(&cfg, kern, args...);   // errors are picked up by cudaGetLastError at the call site
 }
-
 template <typename K, typename... A>
 static inline void pb_launch_k(pb_ctx* ctx, K kern, dim3 grid, dim3 block, size_t smem, A... args) { pb_launch_kc(ctx, kern, grid, block, smem, 1, args...); }
+
 // Raise the kernel's dynamic shared-memory limit on this context's device when `smem` exceeds what was set before.  The limit belongs to
 // the device's copy of the function, which all contexts on that device share: it only ever grows (pb_api.cu).
 int pb_ensure_smem_fn(pb_ctx* ctx, const void* kern, size_t smem);
@@ -138,6 +139,12 @@ unsigned long long* pb_stamp_slot(pb_ctx* ctx, int kernel_id);
 enum { PB_K_GEMVQ = 1, PB_K_ROUTER = 2, PB_K_EXPERT_GU = 3, PB_K_EXPERT_DOWN = 4, PB_K_DELTANET = 5, PB_K_ATTN = 6, PB_K_STEP = 7 };
 
 int pb_scratch(pb_ctx* ctx, size_t bytes, void** out);
+// Host buffers of the entry points: a copy from or into pageable memory blocks the host while the driver stages it piece by piece, so the library
+// stages it itself in page-locked memory of the context (up to PB_PIN_MAX bytes; larger ones and page-locked buffers are copied directly).
+#define PB_PIN_MAX ((size_t)8 << 20)
+bool pb_host_pinned(const void* p);
+int pb_h2d(pb_ctx* ctx, void* dst, const void* src, size_t bytes, size_t pin_off);   // pin_off: this copy's place in the staging buffer
+int pb_d2h(pb_ctx* ctx, void* dst, const void* src, size_t bytes, size_t pin_off, const void** staged);   // *staged: where the bytes are after the synchronisation, null when they are in dst
 int pb_sync_check(pb_ctx* ctx, const char* who);
 
 // pb_dequant.cu
@@ -241,22 +248,26 @@ struct PbRouteParams {
     int* sel_e; float* sel_w;                 // [t][top_k], ascending expert id
     int* n_used; int* used_e; int* used_off;  // distinct local experts, entry offsets [n_used + 1]
     int* ent_tok; int* ent_slot; float* ent_w;
+    int4* virt; int* n_virt;                  // several tokens: distinct local experts in groups of up to PB_VGROUP entries {expert, first entry, entries, 0}, and their number
 };
+#define PB_VGROUP 8
 struct PbExpertParams {
     const int* n_used; const int* used_e; const int* used_off;
     const int* ent_tok; const int* ent_slot; const float* ent_w;
     const uint32_t* xq;                       // gate/up: int8-split activations per token
     const uint8_t* w_a; const uint8_t* w_b;   // gate/up: gate_exps, up_exps; down: down_exps, unused
     const uint8_t* sh_a; const uint8_t* sh_b; // shared expert counterparts
-    int4* virt; int* n_virt;                  // several tokens: distinct local experts in groups of up to PB_VGROUP entries {expert, first entry, entries, 0}, and their number
     float* h; float* h_sh;                    // hidden [entry][ff], [t][ff_sh]
-#define PB_VGROUP 8
     uint32_t* hq;                             // down, several tokens: int8-split hidden vectors [t * top_k + t][pb_xq_words(ff)], else null
     float* part; float* part_sh;              // down: [t][top_k][d], [t][d]
     float* const* part_tok;                   // down, peer exchange: part_tok[token] = [top_k][d] block in the memory of the token's owner (else null)
     int rows_e, rows_sh, has_shared, t, top_k, n_exp, e_base;
     int sh_tok0, sh_ntok;                     // tokens [sh_tok0, sh_tok0 + sh_ntok) get the shared expert here
     int bpr, row_bytes, rows_per_chunk; uint32_t stage_bytes, tab_bytes; int rep;
+    // tensor-core kernels (pb_moeh.cu): groups of entries, raw token rows with their RMS scales and the norm weight (null: x is normalized)
+    const int4* virt; const int* n_virt;
+    const float* x; int64_t ldx; const float* norm_w; const float* tok_scale;
+    int nslots;                               // token slots of a CTA
     int nx;                                   // activation-level vectors of a chunk's first nx entries ride along with its weights
     int* status;
     unsigned long long* stamps;
@@ -264,10 +275,6 @@ struct PbExpertParams {
 struct PbCombineParams {
     const float* part; const float* part_sh; const float* logits; int64_t ldl;
     int t, d, top_k, n_exp;
-    // tensor-core kernels (pb_moeh.cu): groups of entries, raw token rows with their RMS scales and the norm weight (null: x is normalized)
-    const int4* virt; const int* n_virt;
-    const float* x; int64_t ldx; const float* norm_w; const float* tok_scale;
-    int nslots;                               // token slots of a CTA
     float* y; int64_t ldy; int accumulate;
     // peer exchange (device copy of the descriptor): before reading `part`, announce exchange exch_idx (kind 1: this
     // rank's expert rows are stored in their owners' memory) and wait for every rank's announcement
@@ -277,6 +284,10 @@ int pb_launch_router(pb_ctx* ctx, const PbRouterParams& p, const PbRouteParams& 
 int pb_launch_expert_gu(pb_ctx* ctx, const PbExpertParams& p, int type, int cols);
 int pb_launch_expert_down(pb_ctx* ctx, const PbExpertParams& p, int type, int cols, const PbCombineParams* cp = nullptr, unsigned int* ticket = nullptr);
 int pb_launch_moe_combine(pb_ctx* ctx, const PbCombineParams& p);
+// pb_moeh.cu: the expert kernels of two and more tokens on the tensor cores
+bool pb_moeh_supported(int type, int d, int ff, int t);
+int pb_launch_moeh_gu(pb_ctx* ctx, const PbExpertParams& p, int type, int cols);
+int pb_launch_moeh_down(pb_ctx* ctx, const PbExpertParams& p, int type, int cols);
 
 // ---------------------------------------------------------------- pb_deltanet.cu
 struct PbDeltaParams {
@@ -284,10 +295,6 @@ struct PbDeltaParams {
     const float* conv_w; const float* a; const float* dt;
     float* conv;                              // [batch][conv_k slots][ch] ring
     float* ssm;                               // [batch][nv][dk][dv]
-// pb_moeh.cu: the expert kernels of two and more tokens on the tensor cores
-bool pb_moeh_supported(int type, int d, int ff, int t);
-int pb_launch_moeh_gu(pb_ctx* ctx, const PbExpertParams& p, int type, int cols);
-int pb_launch_moeh_down(pb_ctx* ctx, const PbExpertParams& p, int type, int cols);
     const int64_t* pos;                       // [batch]
     float* out; int64_t ldo;                  // [batch][nv*dv] readout before the gated norm
     int nk, nv, dk, dv, conv_k, batch;

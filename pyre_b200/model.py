@@ -93,7 +93,7 @@ class State:
                 raise ValueError("forward: out must be a C-contiguous float32 array [batch][vocab]")
             logits = out
         else:
-            logits = np.empty((self.batch, self.model.cfg.vocab), dtype=np.float32)
+            logits = self.ctx._result((self.batch, self.model.cfg.vocab))
         self.ctx.check(lib().pb_forward(self.h, _p(ids), C.c_int(ids.shape[1]), _p(logits)))
         return logits
 
@@ -112,7 +112,7 @@ class State:
 
     def forward_multi(self, ids) -> np.ndarray:
         ids = np.ascontiguousarray(ids, dtype=np.uint32).reshape(-1)
-        logits = np.empty((ids.size, self.model.cfg.vocab), dtype=np.float32)
+        logits = self.ctx._result((ids.size, self.model.cfg.vocab))
         self.ctx.check(lib().pb_verify(self.h, _p(ids), C.c_int(ids.size), _p(logits)))
         return logits
 
@@ -210,20 +210,20 @@ class State:
     def moe_forward(self, layer: int, x: np.ndarray):
         x = _f32(x).reshape(-1, self.model.cfg.d)
         t = x.shape[0]
-        y = np.empty_like(x)
+        y = self.ctx._result(x.shape)
         sel = np.empty((t, self.model.cfg.top_k), dtype=np.int32)
         self.ctx.check(lib().pb_moe_forward(self.h, C.c_int(layer), _p(x), C.c_int(t), _p(y), _p(sel)))
         return y, sel
 
     def deltanet_step(self, layer: int, x: np.ndarray) -> np.ndarray:
         x = _f32(x).reshape(self.batch, self.model.cfg.d)
-        y = np.empty_like(x)
+        y = self.ctx._result(x.shape)
         self.ctx.check(lib().pb_deltanet_step(self.h, C.c_int(layer), _p(x), _p(y)))
         return y
 
     def attn_step(self, layer: int, x: np.ndarray) -> np.ndarray:
         x = _f32(x).reshape(self.batch, self.model.cfg.d)
-        y = np.empty_like(x)
+        y = self.ctx._result(x.shape)
         self.ctx.check(lib().pb_attn_step(self.h, C.c_int(layer), _p(x), _p(y)))
         return y
 
