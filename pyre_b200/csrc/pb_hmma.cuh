@@ -22,6 +22,11 @@ __device__ __forceinline__ void pb_hmma(float (&c)[4], uint32_t a0, uint32_t a1,
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// the same with a zero accumulator in
+__device__ __forceinline__ void pb_hmma0(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
 __device__ __forceinline__ __half2 pb_as_h2(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
 __device__ __forceinline__ uint32_t pb_as_u32(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
 // (w & mask) | bits in one logic operation
@@ -110,6 +115,7 @@ template <> struct PbHDec<PB_T_IQ3S_N4> {
     __device__ static __forceinline__ float d(const PbHRaw<PB_T_IQ3S_N4>& r) { return pb_h2f((uint16_t)(r.h.x & 0xFFFF)); }
     __device__ static __forceinline__ float dmin(const PbHRaw<PB_T_IQ3S_N4>&) { return 0.f; }
     __device__ static __forceinline__ uint32_t offs(const PbHRaw<PB_T_IQ3S_N4>&, int) { return 0u; }
+    __device__ __forceinline__ uint32_t centre() const { return 0u; }
     // (2 c - 15) m: the code sits in the mantissa of an f16 with exponent 1024 (low nibbles) or 64 (high nibbles); both steps are exact
     __device__ __forceinline__ void word(const PbHRaw<PB_T_IQ3S_N4>& r, int u, uint32_t (&o)[4]) const {
         const uint4& c = u < 4 ? r.c0 : r.c1;
@@ -122,7 +128,7 @@ template <> struct PbHDec<PB_T_IQ3S_N4> {
     }
 };
 template <> struct PbHDec<PB_T_Q4_K> {
-    __half2 s[2], sk[2];     // scale of the two groups; -1024 scale (low nibbles), -64 scale (high nibbles)
+    __half2 s[2], sk[2];     // scale of the two groups, -72 scale
     // scale_min_k4 (gguf_q.rs:62-64) of groups 2 q and 2 q + 1: both groups' values in bytes 0 and 1
     __device__ static __forceinline__ uint32_t scales(const uint4& h, int q) {
         return q < 2 ? (h.y >> (16 * q)) & 0x3F3Fu : ((h.w >> (16 * (q - 2))) & 0x0F0Fu) | (((h.y >> (16 * (q - 2))) & 0xC0C0u) >> 2);
@@ -130,7 +136,7 @@ template <> struct PbHDec<PB_T_Q4_K> {
     __device__ __forceinline__ void head(const PbHRaw<PB_T_Q4_K>& r, int q) {
         const uint32_t s2 = scales(r.h, q);
         s[0] = pb_h2_int(s2 & 0xFF); s[1] = pb_h2_int((s2 >> 8) & 0xFF);
-        sk[0] = __hmul2(s[0], pb_as_h2(0xE400E400u)); sk[1] = __hmul2(s[1], pb_as_h2(0xD400D400u));   // exact
+        sk[0] = __hmul2(s[0], pb_as_h2(0xD480D480u)); sk[1] = __hmul2(s[1], pb_as_h2(0xD480D480u));   // exact: 9 x 6 bits
     }
     __device__ static __forceinline__ float d(const PbHRaw<PB_T_Q4_K>& r) { return pb_h2f((uint16_t)(r.h.x & 0xFFFF)); }
     __device__ static __forceinline__ float dmin(const PbHRaw<PB_T_Q4_K>& r) { return pb_h2f((uint16_t)(r.h.x >> 16)); }
@@ -139,14 +145,17 @@ template <> struct PbHDec<PB_T_Q4_K> {
         const uint32_t m2 = q < 2 ? (r.h.z >> (16 * q)) & 0x3F3Fu : ((r.h.w >> (16 * (q - 2) + 4)) & 0x0F0Fu) | (((r.h.z >> (16 * (q - 2))) & 0xC0C0u) >> 2);
         return pb_as_u32(__hsub2(pb_as_h2((m2 & 0xFF) | ((m2 & 0xFF00) << 8) | 0x64006400u), pb_as_h2(0x64006400u)));
     }
-    // q * scale <= 945: (1024 + q) s - 1024 s and (64 + q) s - 64 s, exact
+    // f16 pair of 8 x scale of the two groups
+    __device__ __forceinline__ uint32_t centre() const { return pb_as_u32(__hmul2(__halves2half2(__low2half(s[0]), __low2half(s[1])), pb_as_h2(0x48004800u))); }
+    // (q - 8) scale = (64 + q) s - 72 s, exact: codes around zero, so that activations with a mean do not make large sums that the minima then cancel;
+    // the 8 scale comes back with the minima
     __device__ __forceinline__ void word(const PbHRaw<PB_T_Q4_K>& r, int u, uint32_t (&o)[4]) const {
         const uint4& c = u < 4 ? r.c0 : r.c1;
-        const uint32_t w = (u & 3) == 0 ? c.x : ((u & 3) == 1 ? c.y : ((u & 3) == 2 ? c.z : c.w)), w8 = w >> 8;
-        o[0] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w, 0x000F000Fu, 0x64006400u)), s[0], sk[0]));
-        o[1] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w8, 0x000F000Fu, 0x64006400u)), s[0], sk[0]));
+        const uint32_t w = (u & 3) == 0 ? c.x : ((u & 3) == 1 ? c.y : ((u & 3) == 2 ? c.z : c.w));
+        o[0] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w << 4, 0x00F000F0u, 0x54005400u)), s[0], sk[0]));
+        o[1] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w >> 4, 0x00F000F0u, 0x54005400u)), s[0], sk[0]));
         o[2] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w, 0x00F000F0u, 0x54005400u)), s[1], sk[1]));
-        o[3] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w8, 0x00F000F0u, 0x54005400u)), s[1], sk[1]));
+        o[3] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w >> 8, 0x00F000F0u, 0x54005400u)), s[1], sk[1]));
     }
 };
 
@@ -221,6 +230,12 @@ __device__ __forceinline__ void pb_h_add(const float (&acc)[NT][4], int nt, int 
     const float s = __uint_as_float(pb_ldsa32(L.scale + (uint32_t)nt * L.tok4 + 4u * blk));
     tot[nt][0] = __fadd_rn(tot[nt][0], __fmul_rn(va, s)); tot[nt][1] = __fadd_rn(tot[nt][1], __fmul_rn(vb, s));
 }
+// The tensor core adds into its f32 accumulator by truncation, an error that grows with the chain: chains of four mma, added up in rounded f32, keep
+// a sum as precise as the integer dot products of the dp4a kernels (2048 columns, relative to |x| |w|: 2e-9; one chain per block: 7e-9).
+__device__ __forceinline__ void pb_h_flush(float (&acc)[4], const float (&c)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) acc[i] += c[i];
+}
 template <int FMT, int NT>
 __device__ __forceinline__ void pb_h_block_nib(uint32_t stage, const PbHGeom& h, int blk, int lane, const PbHLane& L, float (&tot)[NT][2]) {
     const int g = lane >> 2, q = lane & 3;
@@ -229,6 +244,7 @@ __device__ __forceinline__ void pb_h_block_nib(uint32_t stage, const PbHGeom& h,
     else { ra.load(stage + (uint32_t)(g * h.pitch), g, q); rb.load(stage + (uint32_t)((g + 8) * h.pitch), g, q); }
     PbHDec<FMT> wa, wb;
     wa.head(ra, q); wb.head(rb, q);
+    float c[NT][4];
     float acc[NT][4];
 #pragma unroll
     for (int nt = 0; nt < NT; nt++) { acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f; }
@@ -239,8 +255,9 @@ __device__ __forceinline__ void pb_h_block_nib(uint32_t stage, const PbHGeom& h,
 #pragma unroll
         for (int nt = 0; nt < NT; nt++) {
             const uint4 x = pb_ldsa128(L.b + (uint32_t)nt * L.tok4 + (uint32_t)(blk * 1024 + u * 128));
-            pb_hmma(acc[nt], a[0], b[0], a[1], b[1], x.x, x.y);
-            pb_hmma(acc[nt], a[2], b[2], a[3], b[3], x.z, x.w);
+            if (u & 1) pb_hmma(c[nt], a[0], b[0], a[1], b[1], x.x, x.y); else pb_hmma0(c[nt], a[0], b[0], a[1], b[1], x.x, x.y);
+            pb_hmma(c[nt], a[2], b[2], a[3], b[3], x.z, x.w);
+            if (u & 1) pb_h_flush(acc[nt], c[nt]);
         }
     }
     const float da = PbHDec<FMT>::d(ra), db = PbHDec<FMT>::d(rb);
@@ -253,7 +270,10 @@ __device__ __forceinline__ void pb_h_block_nib(uint32_t stage, const PbHGeom& h,
             const uint32_t ma = PbHDec<FMT>::offs(ra, q), mb = PbHDec<FMT>::offs(rb, q);
             float mc[4] = {0.f, 0.f, 0.f, 0.f};
             pb_hmma(mc, ma, mb, ma, mb, s.x, s.y);
-            oa = -PbHDec<FMT>::dmin(ra) * mc[0]; ob = -PbHDec<FMT>::dmin(rb) * mc[2];
+            float cc[4];
+            const uint32_t ca = wa.centre(), cb = wb.centre();
+            pb_hmma0(cc, ca, cb, ca, cb, s.x, s.y);
+            oa = da * cc[0] - PbHDec<FMT>::dmin(ra) * mc[0]; ob = db * cc[2] - PbHDec<FMT>::dmin(rb) * mc[2];
         }
         pb_h_add<FMT, NT>(acc, nt, blk, da, db, oa, ob, L, tot);
     }
@@ -289,6 +309,7 @@ __device__ __forceinline__ void pb_h_block_int(uint32_t pa, uint32_t pb, const P
     if constexpr (pb_h_mode<FMT>() == PB_H_FOLD) {
         uint32_t ma[4], mb[4];
         pb_h_mults<FMT>(pa, q, fa, ma); pb_h_mults<FMT>(pb, q, fb, mb);
+        float c[NT][4];
 #pragma unroll
         for (int u = 0; u < 8; u++) {
             const __half2 sa = pb_h2_int(ma[u >> 1]), sb = pb_h2_int(mb[u >> 1]), k = pb_as_h2(0xE480E480u);   // -1152
@@ -302,8 +323,9 @@ __device__ __forceinline__ void pb_h_block_int(uint32_t pa, uint32_t pb, const P
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
                 const uint4 x = pb_ldsa128(L.b + (uint32_t)nt * L.tok4 + (uint32_t)(blk * 1024 + u * 128));
-                pb_hmma(acc[nt], a[0], b[0], a[1], b[1], x.x, x.y);
-                pb_hmma(acc[nt], a[2], b[2], a[3], b[3], x.z, x.w);
+                if (u & 1) pb_hmma(c[nt], a[0], b[0], a[1], b[1], x.x, x.y); else pb_hmma0(c[nt], a[0], b[0], a[1], b[1], x.x, x.y);
+                pb_hmma(c[nt], a[2], b[2], a[3], b[3], x.z, x.w);
+                if (u & 1) pb_h_flush(acc[nt], c[nt]);
             }
         }
     } else {
@@ -338,10 +360,12 @@ __device__ __forceinline__ void pb_h_block_int(uint32_t pa, uint32_t pb, const P
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
                 const uint4 x = pb_ldsa128(L.b + (uint32_t)nt * L.tok4 + (uint32_t)(blk * 1024 + u * 128));
-                pb_hmma(acc[nt], a[0], b[0], a[1], b[1], x.x, x.y);
-                pb_hmma(acc[nt], a[2], b[2], a[3], b[3], x.z, x.w);
-                pb_hmma(acc[nt], al[0], bl[0], al[1], bl[1], x.x, x.y);
-                pb_hmma(acc[nt], al[2], bl[2], al[3], bl[3], x.z, x.w);
+                float c[4];                                      // the low parts first: their sums are small, and so is what truncation takes from them
+                pb_hmma0(c, al[0], bl[0], al[1], bl[1], x.x, x.y);
+                pb_hmma(c, al[2], bl[2], al[3], bl[3], x.z, x.w);
+                pb_hmma(c, a[0], b[0], a[1], b[1], x.x, x.y);
+                pb_hmma(c, a[2], b[2], a[3], b[3], x.z, x.w);
+                pb_h_flush(acc[nt], c);
             }
         }
     }
