@@ -1,0 +1,405 @@
+// Attention of a window: consecutive tokens of one sequence (a prompt chunk, a verify window) over the sequence's cache, on the tensor cores.
+//
+// The tokens of a window read the same keys and values, so a CTA takes a tile of 64 query rows (64 / G tokens x the G heads of a KV head) and
+// walks positions in tiles of 64 (flash attention): every byte of the cache is fetched and decoded once per 64 rows instead of once per token,
+// and the f32 rows of the recent window go through the tensor cores too.  Splits along the positions fill the GPU;
+// pb_attnw_combine_kernel merges them, normalizes and applies the sigmoid output gate.  Restates attn_core (dense branch) and the layout
+// rule of kv_push of the reference (src/model/qwen4exp_gguf.rs:1558-1615, 1517-1534); the token-per-CTA kernels of pb_attn.cu stay for
+// decode steps, masks and other head shapes.
+//
+//   Precision: queries, keys, probabilities and values enter as f16 high + low parts (22 significant bits); a product is the three mma
+//   high x high, low x high, high x low.  Keys and values are scaled per tile by a power of two, queries per row.
+//   Packed or f32: token j treats as packed the positions below q4_j, what a token-by-token run would have packed by then.  The boundaries
+//   of a tile's tokens differ by steps of 64, so the positions are walked as two runs -- packed [0, max q4), f32 [min q4, last position] --
+//   and the mask drops what is not a row's.
+//   Warps: 8; warp = (16 rows m, half h).  Scores: half of the tile's positions; output: half of the 256 dims.  Q stays in registers.
+//   Memory: one f16 tile (high, low) serves K and then V; the raw bytes of the next operand arrive by asynchronous copies in a staging
+//   buffer meanwhile: V during the score products, the next K during the output products.
+#include "pb_common.cuh"
+#include "pb_internal.h"
+
+#include <cuda_fp16.h>
+#include <stdio.h>
+
+#define AW_THREADS 256
+#define AW_M 64                       // query rows of a CTA
+#define AW_N 64                       // positions of a tile
+#define AW_HD 256
+#define AW_ROW 528                    // bytes between rows of an f16 tile: 512 + 16, so that the 8 rows of an ldmatrix fall on different banks
+#define AW_PROW 144                   // the same for the probabilities (64 halves)
+#define AW_TILE (AW_N * AW_ROW)
+#define AW_OFF_P (2 * AW_TILE)        // K or V high, low; then P high, P low
+#define AW_OFF_RAW (AW_OFF_P + 2 * AW_M * AW_PROW)
+#define AW_OFF_MISC (AW_OFF_RAW + AW_N * AW_HD * 4)
+#define AW_SMEM (AW_OFF_MISC + 2048)
+
+__device__ __forceinline__ void aw_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void aw_ldm4(uint32_t (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void aw_ldm4t(uint32_t (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void aw_split(float a, float b, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 r = __half22float2(h);
+    const __half2 l = __floats2half2_rn(a - r.x, b - r.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h); lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+__device__ __forceinline__ void aw_cp16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ float aw_exp2i(int k) { k = k < -126 ? -126 : (k > 127 ? 127 : k); return __int_as_float((k + 127) << 23); }
+// exponent e with max < 2^e, or 0 for an empty tile
+__device__ __forceinline__ int aw_expo(float m) { return m > 1e-30f && m < 1e30f ? (int)((__float_as_uint(m) >> 23) & 0xFF) - 126 : 0; }
+
+__device__ __forceinline__ int64_t aw_q4(const PbAttnParams& p, int64_t n, int64_t prev) {
+    if (p.kv_bits != 4) return 0;
+    const int64_t rule = n > p.kv_recent ? ((n - p.kv_recent) / 64) * 64 : 0;
+    const int64_t q = rule > prev ? rule : prev;
+    return q < n ? q : n;
+}
+
+// raw bytes of 64 positions from pb on -> staging.  Packed: [64][32] words K (or [8][256] position-transposed words V), then [64][8] scales
+__device__ __forceinline__ void aw_fetch(const PbAttnParams& p, uint32_t raw, size_t hrow, bool v, bool packed, int64_t p0, int64_t plast, int tid) {
+    if (packed) {
+        const uint8_t* w = reinterpret_cast<const uint8_t*>((v ? p.vw : p.kw) + hrow * p.max_ctx * (AW_HD / 8)) + p0 * 128;
+        const uint8_t* s = reinterpret_cast<const uint8_t*>((v ? p.vs : p.ks) + hrow * p.max_ctx * (AW_HD / 32)) + p0 * 32;
+        for (int i = tid; i < 640; i += AW_THREADS) aw_cp16(raw + 16 * i, i < 512 ? w + 16 * i : s + 16 * (i - 512));
+    } else {
+        const float* r = (v ? p.vr : p.kr) + hrow * p.ring_cap * AW_HD;
+        const int rw = tid >> 6, c = tid & 63;          // 64 threads bring one row
+        int64_t slot = (p0 + rw) % p.ring_cap;
+        for (int i = rw; i < AW_N; i += 4) {
+            const bool in = p0 + i <= plast;              // rows past the last position are never read: the converter takes them as zeros
+            if (in) aw_cp16(raw + (uint32_t)(i * 1024 + c * 16), r + slot * AW_HD + 4 * c);
+            slot += 4; if (slot >= p.ring_cap) slot -= p.ring_cap;
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+
+// nibbles at bit sh and sh + 16 of offset-binary words -> their signed values
+__device__ __forceinline__ float2 aw_nib2(uint32_t x, int sh) {
+    const uint32_t t = ((x >> sh) & 0x000F000Fu) | 0x64006400u;           // 1024 + n
+    return __half22float2(__hsub2(*reinterpret_cast<const __half2*>(&t), __float2half2_rn(1032.0f)));
+}
+
+// staged tile -> f16 high and low tiles, scaled by 2^-e with e from the tile's largest magnitude; returns e.  All threads; the caller has
+// synchronized on the staged bytes.  mx: this conversion's slot (zero), nx: the next one's.
+__device__ __forceinline__ int aw_convert(uint8_t* smem, const uint8_t* raw, bool v, bool packed, int nrow, unsigned* mx, unsigned* nx, int tid) {
+    const int warp = tid >> 5, lane = tid & 31;
+    const float* scales = reinterpret_cast<const float*>(raw + 8192);
+    float m = 0.f;
+    if (packed) m = fmaxf(scales[tid], scales[tid + 256]) * 8.0f;
+    else for (int i = warp; i < nrow; i += 8) {
+        const float4 x = *reinterpret_cast<const float4*>(raw + i * 1024 + lane * 16), y = *reinterpret_cast<const float4*>(raw + i * 1024 + 512 + lane * 16);
+        m = fmaxf(m, fmaxf(fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))), fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w)))));
+    }
+    m = pb_warp_max(m);
+    if (lane == 0) atomicMax(mx, __float_as_uint(m));   // non-negative floats order like their bits
+    __syncthreads();
+    const int e = aw_expo(__uint_as_float(*mx));
+    if (tid == 0) *nx = 0u;
+    const float sc = aw_exp2i(-e);
+    if (!packed) {
+#pragma unroll 4
+        for (int i = warp; i < AW_N; i += 8) {
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (i < nrow) x = *reinterpret_cast<const float4*>(raw + i * 1024 + k * 512 + lane * 16);
+                uint2 hi, lo;
+                aw_split(x.x * sc, x.y * sc, hi.x, lo.x); aw_split(x.z * sc, x.w * sc, hi.y, lo.y);
+                *reinterpret_cast<uint2*>(smem + i * AW_ROW + k * 256 + lane * 8) = hi;
+                *reinterpret_cast<uint2*>(smem + AW_TILE + i * AW_ROW + k * 256 + lane * 8) = lo;
+            }
+        }
+    } else if (!v) {   // a word = 8 dims of one position; lane = word
+#pragma unroll 4
+        for (int i = warp; i < AW_N; i += 8) {
+            const uint32_t w = *reinterpret_cast<const uint32_t*>(raw + i * 128 + lane * 4);
+            const float s = scales[i * 8 + (lane >> 2)] * sc;
+            const float2 a = aw_nib2(w, 0), b = aw_nib2(w, 4), c = aw_nib2(w, 8), d = aw_nib2(w, 12);   // dims (0 4) (1 5) (2 6) (3 7)
+            uint4 hi, lo;
+            aw_split(a.x * s, b.x * s, hi.x, lo.x); aw_split(c.x * s, d.x * s, hi.y, lo.y);
+            aw_split(a.y * s, b.y * s, hi.z, lo.z); aw_split(c.y * s, d.y * s, hi.w, lo.w);
+            *reinterpret_cast<uint4*>(smem + i * AW_ROW + lane * 16) = hi;
+            *reinterpret_cast<uint4*>(smem + AW_TILE + i * AW_ROW + lane * 16) = lo;
+        }
+    } else {           // a word = 8 positions of one dim; a thread takes two dims of a group of 8 positions
+#pragma unroll 2
+        for (int k = 0; k < 4; k++) {
+            const int it = tid + 256 * k, pg = it >> 7, d2 = it & 127;
+            const uint2 w = *reinterpret_cast<const uint2*>(raw + pg * 1024 + d2 * 8);
+            const uint32_t wl = __byte_perm(w.x, w.y, 0x5410), wh = __byte_perm(w.x, w.y, 0x7632);
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float s = scales[(pg * 8 + j) * 8 + (d2 >> 4)] * sc;
+                const float2 a = aw_nib2(j < 4 ? wl : wh, 4 * (j & 3));
+                uint32_t hi, lo;
+                aw_split(a.x * s, a.y * s, hi, lo);
+                *reinterpret_cast<uint32_t*>(smem + (pg * 8 + j) * AW_ROW + d2 * 4) = hi;
+                *reinterpret_cast<uint32_t*>(smem + AW_TILE + (pg * 8 + j) * AW_ROW + d2 * 4) = lo;
+            }
+        }
+    }
+    __syncthreads();
+    return e;
+}
+
+// grid (splits, row tiles, KV heads)
+template <int G>
+__global__ void __launch_bounds__(AW_THREADS, 1) pb_attnw_kernel(const PbAttnParams p) {
+    extern __shared__ __align__(128) uint8_t aw_smem[];
+    constexpr int TPT = AW_M / G;   // tokens of a tile
+    const int sp = blockIdx.x, kvh = blockIdx.z, tok0 = blockIdx.y * TPT;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3, wm = warp >> 1, wh = warp & 1;
+    uint8_t* raw = aw_smem + AW_OFF_RAW;
+    int* qe = reinterpret_cast<int*>(aw_smem + AW_OFF_MISC);                  // [64] exponent of a query row
+    float* rmax = reinterpret_cast<float*>(aw_smem + AW_OFF_MISC + 256);      // [2][64] maxima, later sums, of the position halves
+    unsigned* mx = reinterpret_cast<unsigned*>(aw_smem + AW_OFF_MISC + 768);  // [2] largest magnitude of the tile being converted
+    const uint32_t sm = pb_smem_u32(aw_smem), sraw = pb_smem_u32(raw);
+    pb_pdl_wait();
+    pb_pdl_trigger();
+    if (tid < 2) mx[tid] = 0u;
+    const int ntok = min(TPT, p.batch - tok0);
+    const int64_t pos0 = p.pos[tok0], plast = p.pos[tok0 + ntok - 1], prev = p.kv_bits == 4 ? p.q4n[1] : 0;
+    const int64_t q4lo = aw_q4(p, pos0 + 1, prev), q4hi = aw_q4(p, plast + 1, prev);
+    const int npk = (int)((q4hi + AW_N - 1) / AW_N), ntl = npk + (int)((plast - q4lo) / AW_N + 1);   // packed tiles, all tiles
+    const int tb = (int)((int64_t)ntl * sp / gridDim.x), te = (int)((int64_t)ntl * (sp + 1) / gridDim.x);
+    if (tb >= te) {
+        if (tid < ntok * G) {
+            const int tok = tok0 + tid / G;
+            float* ml = p.part_ml + ((((size_t)tok * p.n_kv + kvh) * p.nsplit + sp) * G + tid % G) * 2;
+            ml[0] = -INFINITY; ml[1] = 0.f;
+        }
+        return;
+    }
+    auto tile_p0 = [&](int t) -> int64_t { return t < npk ? (int64_t)t * AW_N : q4lo + (int64_t)(t - npk) * AW_N; };
+    aw_fetch(p, sraw, (size_t)kvh, false, tb < npk, tile_p0(tb), plast, tid);
+
+    // queries of the tile: rms_inplace(q, qn), rope, times 1/sqrt(hd)  (:1603-1606); a lane owns dims lane + 32 k of a row (n_rot = 64)
+    for (int r = warp; r < AW_M; r += 8) {
+        const int tok = tok0 + r / G;
+        float qv[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) qv[k] = 0.f;
+        if (r / G < ntok) {
+            const float* qraw = p.proj + (size_t)tok * p.ldp + (size_t)(kvh * G + r % G) * 2 * AW_HD;
+            float ss = 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; k++) { qv[k] = qraw[lane + 32 * k]; ss += qv[k] * qv[k]; }
+            ss = pb_warp_sum(ss);
+            const float s = 1.0f / sqrtf(ss / (float)AW_HD + p.eps), scale = 1.0f / sqrtf((float)AW_HD);
+            float sn, co;
+            sincosf((float)p.pos[tok] * p.rope_inv[lane], &sn, &co);
+            const float ms = p.rope_inv[32];
+            if (ms != 1.0f) { co *= ms; sn *= ms; }
+#pragma unroll
+            for (int k = 0; k < 8; k++) qv[k] *= s * p.qn[lane + 32 * k];
+            const float x0 = qv[0], x1 = qv[1];
+            qv[0] = x0 * co - x1 * sn; qv[1] = x1 * co + x0 * sn;
+#pragma unroll
+            for (int k = 0; k < 8; k++) qv[k] *= scale;
+        }
+        float m = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; k++) m = fmaxf(m, fabsf(qv[k]));
+        const int e = aw_expo(pb_warp_max(m));
+        if (lane == 0) qe[r] = e;
+        const float sc = aw_exp2i(-e);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const float x = qv[k] * sc;
+            const __half hi = __float2half_rn(x);
+            *reinterpret_cast<__half*>(aw_smem + r * AW_ROW + (lane + 32 * k) * 2) = hi;
+            *reinterpret_cast<__half*>(aw_smem + AW_TILE + r * AW_ROW + (lane + 32 * k) * 2) = __float2half_rn(x - __half2float(hi));
+        }
+    }
+    __syncthreads();
+    uint32_t qh[16][4], ql[16][4];
+    const uint32_t afrag = sm + (uint32_t)((16 * wm + (lane & 15)) * AW_ROW + (lane >> 4) * 16);
+#pragma unroll
+    for (int k = 0; k < 16; k++) { aw_ldm4(qh[k], afrag + k * 32); aw_ldm4(ql[k], afrag + AW_TILE + k * 32); }
+    const int row0 = 16 * wm + g;
+    int64_t rpos[2], rq4[2]; int re[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int r = row0 + 8 * i, tk = r / G;
+        rpos[i] = tk < ntok ? p.pos[tok0 + tk] : -1;
+        rq4[i] = tk < ntok ? aw_q4(p, rpos[i] + 1, prev) : 0;
+        re[i] = qe[r];
+    }
+    float mrun[2] = {-INFINITY, -INFINITY}, lrun[2] = {0.f, 0.f};
+    float o[16][4];
+#pragma unroll
+    for (int i = 0; i < 16; i++) { o[i][0] = 0.f; o[i][1] = 0.f; o[i][2] = 0.f; o[i][3] = 0.f; }
+    int ev = 0, nconv = 0;
+    const uint32_t kfrag = sm + (uint32_t)((32 * wh + (lane >> 4) * 8 + (lane & 7)) * AW_ROW + ((lane >> 3) & 1) * 16);
+    const uint32_t vfrag = sm + (uint32_t)((((lane >> 3) & 1) * 8 + (lane & 7)) * AW_ROW + wh * 256 + (lane >> 4) * 16);
+    const uint32_t pfrag = sm + AW_OFF_P + (uint32_t)((16 * wm + (lane & 15)) * AW_PROW + (lane >> 4) * 16);
+
+    for (int t = tb; t < te; t++) {
+        const bool packed = t < npk;
+        const int64_t p0 = tile_p0(t);
+        const int nrow = packed ? AW_N : (int)min((int64_t)AW_N, plast - p0 + 1);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        const int ek = aw_convert(aw_smem, raw, false, packed, nrow, mx + (nconv & 1), mx + ((nconv + 1) & 1), tid); nconv++;
+        aw_fetch(p, sraw, (size_t)kvh, true, packed, p0, plast, tid);
+        float s[4][4];
+#pragma unroll
+        for (int n = 0; n < 4; n++) { s[n][0] = 0.f; s[n][1] = 0.f; s[n][2] = 0.f; s[n][3] = 0.f; }
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            uint32_t b0[4], b1[4];
+            aw_ldm4(b0, kfrag + k * 32); aw_ldm4(b1, kfrag + 16 * AW_ROW + k * 32);
+            aw_mma(s[0], qh[k], b0[0], b0[1]); aw_mma(s[1], qh[k], b0[2], b0[3]); aw_mma(s[2], qh[k], b1[0], b1[1]); aw_mma(s[3], qh[k], b1[2], b1[3]);
+            aw_mma(s[0], ql[k], b0[0], b0[1]); aw_mma(s[1], ql[k], b0[2], b0[3]); aw_mma(s[2], ql[k], b1[0], b1[1]); aw_mma(s[3], ql[k], b1[2], b1[3]);
+            aw_ldm4(b0, kfrag + AW_TILE + k * 32); aw_ldm4(b1, kfrag + AW_TILE + 16 * AW_ROW + k * 32);
+            aw_mma(s[0], qh[k], b0[0], b0[1]); aw_mma(s[1], qh[k], b0[2], b0[3]); aw_mma(s[2], qh[k], b1[0], b1[1]); aw_mma(s[3], qh[k], b1[2], b1[3]);
+        }
+        float alpha[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const float f = aw_exp2i(re[i] + ek);
+            // offsets of the first and past the last position this row sees in the tile
+            const int lo = packed ? 0 : (int)max((int64_t)0, min(rq4[i] - p0, (int64_t)AW_N)), hi = (int)max((int64_t)0, min((packed ? rq4[i] : rpos[i] + 1) - p0, (int64_t)AW_N));
+            float m = -INFINITY;
+#pragma unroll
+            for (int n = 0; n < 4; n++)
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    const int c = 32 * wh + 8 * n + 2 * q + j;
+                    const float x = c >= lo && c < hi ? s[n][2 * i + j] * f : -INFINITY;
+                    s[n][2 * i + j] = x;
+                    m = fmaxf(m, x);
+                }
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1)); m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+            if (q == 0) rmax[wh * 64 + row0 + 8 * i] = m;
+        }
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + wm) : "memory");   // the two warps of these rows
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int r = row0 + 8 * i;
+            const float mn = fmaxf(mrun[i], fmaxf(rmax[r], rmax[64 + r]));
+            alpha[i] = mn == -INFINITY ? 1.0f : expf(mrun[i] - mn);
+            float l = 0.f;
+#pragma unroll
+            for (int n = 0; n < 4; n++) {
+                const float a = mn == -INFINITY ? 0.f : expf(s[n][2 * i] - mn), b = mn == -INFINITY ? 0.f : expf(s[n][2 * i + 1] - mn);
+                l += a + b;
+                uint32_t hi, lo;
+                aw_split(a * 1024.0f, b * 1024.0f, hi, lo);   // 2^10: small probabilities keep their bits in f16
+                uint8_t* d = aw_smem + AW_OFF_P + r * AW_PROW + (32 * wh + 8 * n + 2 * q) * 2;
+                *reinterpret_cast<uint32_t*>(d) = hi; *reinterpret_cast<uint32_t*>(d + AW_M * AW_PROW) = lo;
+            }
+            lrun[i] = lrun[i] * alpha[i] + l;
+            mrun[i] = mn;
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        const int e = aw_convert(aw_smem, raw, true, packed, nrow, mx + (nconv & 1), mx + ((nconv + 1) & 1), tid); nconv++;
+        if (t + 1 < te) aw_fetch(p, sraw, (size_t)kvh, false, t + 1 < npk, tile_p0(t + 1), plast, tid);
+        const float sh = t == tb ? 1.0f : aw_exp2i(ev - e);
+        ev = e;
+        alpha[0] *= sh; alpha[1] *= sh;
+#pragma unroll
+        for (int n = 0; n < 16; n++) { o[n][0] *= alpha[0]; o[n][1] *= alpha[0]; o[n][2] *= alpha[1]; o[n][3] *= alpha[1]; }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            uint32_t ph[4], pl[4];
+            aw_ldm4(ph, pfrag + k * 32); aw_ldm4(pl, pfrag + AW_M * AW_PROW + k * 32);
+#pragma unroll
+            for (int n = 0; n < 8; n += 2) {
+                uint32_t b0[4], b1[4];
+                aw_ldm4t(b0, vfrag + k * 16 * AW_ROW + n * 32); aw_ldm4t(b1, vfrag + k * 16 * AW_ROW + n * 32 + 32);
+                float (&o0)[4] = o[2 * n], (&o1)[4] = o[2 * n + 1], (&o2)[4] = o[2 * n + 2], (&o3)[4] = o[2 * n + 3];
+                aw_mma(o0, ph, b0[0], b0[1]); aw_mma(o1, ph, b0[2], b0[3]); aw_mma(o2, ph, b1[0], b1[1]); aw_mma(o3, ph, b1[2], b1[3]);
+                aw_mma(o0, pl, b0[0], b0[1]); aw_mma(o1, pl, b0[2], b0[3]); aw_mma(o2, pl, b1[0], b1[1]); aw_mma(o3, pl, b1[2], b1[3]);
+                aw_ldm4t(b0, vfrag + AW_TILE + k * 16 * AW_ROW + n * 32); aw_ldm4t(b1, vfrag + AW_TILE + k * 16 * AW_ROW + n * 32 + 32);
+                aw_mma(o0, ph, b0[0], b0[1]); aw_mma(o1, ph, b0[2], b0[3]); aw_mma(o2, ph, b1[0], b1[1]); aw_mma(o3, ph, b1[2], b1[3]);
+            }
+        }
+    }
+
+    const float f = aw_exp2i(ev - 10);
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        float l = lrun[i];
+        l += __shfl_xor_sync(0xffffffffu, l, 1); l += __shfl_xor_sync(0xffffffffu, l, 2);
+        const int r = row0 + 8 * i;
+        if (q == 0 && wh == 1) rmax[r] = l;
+        lrun[i] = l;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int r = row0 + 8 * i;
+        if (r / G >= ntok) continue;
+        const size_t row = (((size_t)(tok0 + r / G) * p.n_kv + kvh) * p.nsplit + sp) * G + r % G;
+        if (q == 0 && wh == 0) { p.part_ml[row * 2] = mrun[i]; p.part_ml[row * 2 + 1] = lrun[i] + rmax[r]; }
+        float* d = p.part_acc + row * AW_HD + wh * 128 + 2 * q;
+#pragma unroll
+        for (int n = 0; n < 16; n++) *reinterpret_cast<float2*>(d + 8 * n) = make_float2(o[n][2 * i] * f, o[n][2 * i + 1] * f);
+    }
+}
+
+// grid (tokens, heads / 4), 256 threads: merge the splits, normalize, gate with sigmoid(gate)  (:1607-1610); 64 threads own a head
+__global__ void __launch_bounds__(256) pb_attnw_combine_kernel(const PbAttnParams p) {
+    const int tok = blockIdx.x, h = blockIdx.y * 4 + (threadIdx.x >> 6), c = threadIdx.x & 63, G = p.n_head / p.n_kv;
+    pb_pdl_wait();
+    pb_pdl_trigger();
+    if (h >= p.n_head) return;
+    const size_t base = (((size_t)tok * p.n_kv + h / G) * p.nsplit) * G + h % G;
+    const float4 gate = *reinterpret_cast<const float4*>(p.proj + (size_t)tok * p.ldp + (size_t)h * 2 * AW_HD + AW_HD + 4 * c);
+    float M = -INFINITY, L = 0.f;
+    for (int s = 0; s < p.nsplit; s++) M = fmaxf(M, p.part_ml[(base + (size_t)s * G) * 2]);
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int s = 0; s < p.nsplit; s++) {
+        const float2 ml = *reinterpret_cast<const float2*>(p.part_ml + (base + (size_t)s * G) * 2);
+        if (ml.x == -INFINITY) continue;      // this split saw none of the row's positions: its sums were not written
+        const float f = expf(ml.x - M);
+        const float4 a = *reinterpret_cast<const float4*>(p.part_acc + (base + (size_t)s * G) * AW_HD + 4 * c);
+        L += ml.y * f;
+        o.x = fmaf(a.x, f, o.x); o.y = fmaf(a.y, f, o.y); o.z = fmaf(a.z, f, o.z); o.w = fmaf(a.w, f, o.w);
+    }
+    const float r = 1.0f / L;
+    *reinterpret_cast<float4*>(p.att + (size_t)tok * p.lda + (size_t)h * AW_HD + 4 * c) =
+        make_float4(o.x * r * pb_sigm(gate.x), o.y * r * pb_sigm(gate.y), o.z * r * pb_sigm(gate.z), o.w * r * pb_sigm(gate.w));
+}
+
+bool pb_attnw_supported(const PbAttnParams& p) {
+    const int G = p.n_kv > 0 ? p.n_head / p.n_kv : 0;
+    return p.window && !p.qsa_on && p.hd == AW_HD && p.n_rot == 64 && p.n_head % p.n_kv == 0 && (G == 8 || G == 4 || G == 2 || G == 1) && (p.ldp & 3) == 0 && (p.lda & 3) == 0;
+}
+
+// Splits of the positions: as many as keep the row tiles x KV heads x splits on the SMs at once, within `room` partial rows per KV head
+int pb_attnw_splits(pb_ctx* ctx, const PbAttnParams& p, int64_t room) {
+    const int G = p.n_head / p.n_kv, tiles = (p.batch * G + AW_M - 1) / AW_M * p.n_kv;
+    int64_t ns = ctx->sm_count / tiles;
+    if (ns > room / p.batch) ns = room / p.batch;
+    return ns < 1 ? 1 : (ns > 64 ? 64 : (int)ns);
+}
+
+int pb_launch_attn_window(pb_ctx* ctx, const PbAttnParams& p) {
+    const int G = p.n_head / p.n_kv;
+    const dim3 grid(p.nsplit, (p.batch * G + AW_M - 1) / AW_M, p.n_kv);
+#define GO(GG)                                                                             \
+    {                                                                                      \
+        PB_TRY(pb_ensure_smem(ctx, pb_attnw_kernel<GG>, (size_t)AW_SMEM));                 \
+        pb_launch_k(ctx, pb_attnw_kernel<GG>, grid, dim3(AW_THREADS), (size_t)AW_SMEM, p); \
+    }
+    if (G == 8) GO(8) else if (G == 4) GO(4) else if (G == 2) GO(2) else GO(1)
+#undef GO
+    ctx->kernels_launched++;
+    PB_CUDA(ctx, cudaGetLastError());
+    pb_launch_k(ctx, pb_attnw_combine_kernel, dim3(p.batch, (p.n_head + 3) / 4), dim3(256), (size_t)0, p);
+    ctx->kernels_launched++;
+    PB_CUDA(ctx, cudaGetLastError());
+    return PB_OK;
+}

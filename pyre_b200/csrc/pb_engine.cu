@@ -778,15 +778,16 @@ static int run_attn(pb_state* s, int il, const float* x_in, const float* norm_w,
         // to the positions <= its own in one launch (token j treats as packed what it would have found packed token by
         // token).  A verify window that is cut short afterwards gets its boundary back in pb_keep.
         p.window = 1; p.pos = s->wpos; p.batch = s->win_t;
+        const bool tiles = pb_attnw_supported(p);   // the model's head shape without a mask: 64 query rows share each cache tile
         const bool mma = s->nsplit_packed > 0;
         // splits per token: four for a chunk of hundreds of tokens, more for a window of a few, so that the grid fills the GPU
         int ws = ctx->sm_count / (c.n_kv * s->win_t);
         ws = ws < PB_WIN_SPLITS ? PB_WIN_SPLITS : (ws > 64 ? 64 : ws);
         if ((size_t)ws * s->win_t > (size_t)PB_PREFILL_CHUNK * PB_WIN_SPLITS) ws = PB_WIN_SPLITS;
-        p.nsplit = mma ? ws : 1; p.nsplit_packed = mma ? ws - 1 : 0;
+        p.nsplit = tiles ? pb_attnw_splits(ctx, p, (int64_t)PB_PREFILL_CHUNK * PB_WIN_SPLITS) : mma ? ws : 1; p.nsplit_packed = mma ? ws - 1 : 0;
         PB_TRY(pb_launch_kv_append(ctx, p));
         PB_TRY(pb_launch_kv_pack(ctx, p));
-        PB_TRY(pb_launch_attn(ctx, p));
+        PB_TRY(tiles ? pb_launch_attn_window(ctx, p) : pb_launch_attn(ctx, p));
     } else if (s->win_t > 0) {
         // causal inside the window: token j is appended, then attends to positions <= its own
         // (models with an indexer take this form for prefill chunks too: every token makes its own selection)

@@ -354,6 +354,9 @@ int pb_launch_mtp_mask(pb_ctx* ctx, uint32_t* mask, int* on, int64_t lo, int64_t
 int pb_launch_mtp_best(pb_ctx* ctx, const float* lg, int n, uint32_t* out);
 int pb_launch_kv_append(pb_ctx* ctx, const PbAttnParams& p);
 int pb_launch_attn(pb_ctx* ctx, const PbAttnParams& p);
+bool pb_attnw_supported(const PbAttnParams& p);   // windows on the tensor cores (pb_attnw.cu)
+int pb_attnw_splits(pb_ctx* ctx, const PbAttnParams& p, int64_t room);
+int pb_launch_attn_window(pb_ctx* ctx, const PbAttnParams& p);
 int pb_launch_kv_pack(pb_ctx* ctx, const PbAttnParams& p);   // window mode, after pb_launch_kv_append
 int pb_launch_kv4_pack(pb_ctx* ctx, const float* x, int64_t n, uint32_t* w, float* sc, int bias);   // bias 0: kv4.rs nibbles; 8: cache form
 int pb_launch_kv4_pack_vt(pb_ctx* ctx, const float* x, int64_t npos, int hd, uint32_t* w, float* sc, int bias);   // position-transposed V words
