@@ -117,34 +117,38 @@ __global__ void __launch_bounds__(256) pb_kv4_unpack_kernel(const uint32_t* __re
     if (i < n) x[i] = pb_kv4_dequant(w[i / 8], (int)(i % 8), sc[i / 32]);
 }
 
-// Moves the packed boundary of sequence b to where `len` rows put it (kv_push :1520: whole multiples of 64 positions):
-// the rows in between are read from the f32 ring and stored in 4-bit form.  All AT_THREADS threads of one CTA.
-__device__ __forceinline__ void pb_kv_pack_upto(const PbAttnParams& p, int b, int64_t len, int tid, int warp, int lane) {
-    const int hd = p.hd, nkv = p.n_kv;
-    const int64_t have = p.q4n[b];
-    const int64_t want = len > p.kv_recent ? ((len - p.kv_recent) / 64) * 64 : 0;
-    if (want <= have) return;
-    const int bpp = hd / 32;                                  // blocks per position per head
-    const int64_t nblk = (want - have) * nkv * bpp;
-    for (int64_t i = warp; i < nblk; i += AT_WARPS) {
-        const int blk = (int)(i % bpp); const int h = (int)((i / bpp) % nkv); const int64_t pp = have + i / ((int64_t)bpp * nkv);
-        const size_t src = (((size_t)b * nkv + h) * p.ring_cap + (pp % p.ring_cap)) * hd + blk * 32 + lane;
-        const size_t row = ((size_t)b * nkv + h) * p.max_ctx + pp;
-        pb_kv4_pack_block(p.kr[src], lane, p.kw + row * (hd / 8) + blk * 4, p.ks + row * bpp + blk, 8);
+// Packs the rows [have, want) of sequence b (multiples of 64 positions) from the f32 ring; this CTA's share is part `part` of `nparts`.
+// A warp brings a whole row of K, or eight positions of 32 dims of V, with eight loads in flight and eight reductions side by side: with one
+// block of 32 per turn every block waited for its own trip to L2 (64 positions x 2 heads on one CTA: 200 us).
+__device__ __forceinline__ void pb_kv_pack_rows(const PbAttnParams& p, int b, int64_t have, int64_t want, int part, int nparts, int warp, int lane) {
+    const int hd = p.hd, nkv = p.n_kv, bpp = hd / 32;         // blocks per position per head
+    const int first = part * AT_WARPS + warp, step = nparts * AT_WARPS;
+    const int nk = (int)(want - have) * nkv;
+    for (int i = first; i < nk; i += step) {
+        const int h = i % nkv; const int64_t pp = have + i / nkv;
+        const size_t head = (size_t)b * nkv + h, row = head * p.max_ctx + pp;
+        const float* src = p.kr + (head * p.ring_cap + (pp % p.ring_cap)) * hd + lane;
+        for (int k0 = 0; k0 < bpp; k0 += 8) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = k0 + k < bpp ? src[(k0 + k) * 32] : 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; k++) if (k0 + k < bpp) pb_kv4_pack_block(v[k], lane, p.kw + row * (hd / 8) + (k0 + k) * 4, p.ks + row * bpp + k0 + k, 8);
+        }
     }
     // V: groups of 8 positions (have and want are multiples of 64)
-    const int64_t nvt = (want - have) / 8 * nkv * bpp;
-    for (int64_t i = warp; i < nvt; i += AT_WARPS) {
-        const int blk = (int)(i % bpp); const int h = (int)((i / bpp) % nkv); const int64_t pg = have / 8 + i / ((int64_t)bpp * nkv);
+    const int nv = (int)((want - have) / 8) * nkv * bpp;
+    for (int i = first; i < nv; i += step) {
+        const int blk = i % bpp, h = (i / bpp) % nkv; const int64_t pg = have / 8 + i / (bpp * nkv);
         const size_t head = (size_t)b * nkv + h;
         float v[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) v[j] = p.vr[(head * p.ring_cap + ((pg * 8 + j) % p.ring_cap)) * hd + blk * 32 + lane];
         p.vw[head * p.max_ctx * (hd / 8) + (size_t)pg * hd + blk * 32 + lane] = pb_kv4_pack_vt8(v, lane, p.vs + (head * p.max_ctx + pg * 8) * bpp + blk, bpp, 8);
     }
-    __syncthreads();
-    if (tid == 0) p.q4n[b] = want;
 }
+// where `len` rows put the packed boundary (kv_push :1520: whole multiples of 64 positions)
+__device__ __forceinline__ int64_t pb_kv_boundary(const PbAttnParams& p, int64_t len) { return len > p.kv_recent ? ((len - p.kv_recent) / 64) * 64 : 0; }
 
 // ------------------------------------------------------------------------------------ append
 
@@ -214,21 +218,26 @@ __global__ void __launch_bounds__(AT_THREADS) pb_kv_append_kernel(const PbAttnPa
             vd[i] = vraw[h * hd + i];
         }
     }
+    if (p.window && b == 0 && tid == 0) *p.q4prev = p.q4n[0];
     if (p.kv_bits != 4 || p.window) return;
+    const int64_t have = p.q4n[b], want = pb_kv_boundary(p, pos + 1);
+    if (want <= have) return;
     __syncthreads();
-    pb_kv_pack_upto(p, b, pos + 1, tid, warp, lane);
+    pb_kv_pack_rows(p, b, have, want, 0, 1, warp, lane);
+    __syncthreads();
+    if (tid == 0) p.q4n[b] = want;
 }
 
-// window mode: one CTA moves the packed boundary of sequence 0 to where the window's last token puts it, and keeps the
-// boundary from before the window in q4n[1]
+// window mode: moves the packed boundary of sequence 0 to where the window's last token puts it; the append kernel has kept the boundary
+// from before the window in q4prev
 __global__ void __launch_bounds__(AT_THREADS) pb_kv_pack_kernel(const PbAttnParams p) {
     const int tid = threadIdx.x;
     pb_pdl_wait();
     pb_pdl_trigger();
-    const int64_t have = p.q4n[0];
-    __syncthreads();
-    if (tid == 0) p.q4n[1] = have;
-    pb_kv_pack_upto(p, 0, p.pos[p.batch - 1] + 1, tid, tid >> 5, tid & 31);
+    const int64_t have = *p.q4prev, want = pb_kv_boundary(p, p.pos[p.batch - 1] + 1);
+    if (want <= have) return;
+    pb_kv_pack_rows(p, 0, have, want, (int)blockIdx.x, (int)gridDim.x, tid >> 5, tid & 31);
+    if (tid == 0 && blockIdx.x == 0) p.q4n[0] = want;
 }
 
 // ------------------------------------------------------------------------------------ partial
@@ -440,7 +449,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) pb_attn_partial_kernel(const Pb
     // window mode: this token sees as packed what a token-by-token run would have packed when it was appended
     int64_t q4n = 0;
     if (p.kv_bits == 4) {
-        if (p.window) { const int64_t rule = n > p.kv_recent ? ((n - p.kv_recent) / 64) * 64 : 0, prev = p.q4n[1]; q4n = rule > prev ? rule : prev; }
+        if (p.window) { const int64_t rule = n > p.kv_recent ? ((n - p.kv_recent) / 64) * 64 : 0, prev = *p.q4prev; q4n = rule > prev ? rule : prev; }
         else q4n = p.q4n[b];
     }
     const float* proj = p.proj + (size_t)b * p.ldp;
@@ -764,7 +773,7 @@ int pb_launch_kv_append(pb_ctx* ctx, const PbAttnParams& p) {
 
 int pb_launch_kv_pack(pb_ctx* ctx, const PbAttnParams& p) {
     if (!p.window || p.kv_bits != 4) return PB_OK;
-    pb_launch_k(ctx, pb_kv_pack_kernel, dim3(1), dim3(AT_THREADS), (size_t)(0), p);
+    pb_launch_k(ctx, pb_kv_pack_kernel, dim3(64), dim3(AT_THREADS), (size_t)(0), p);
     ctx->kernels_launched++;
     PB_CUDA(ctx, cudaGetLastError());
     return PB_OK;

@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(AW_THREADS, 1) pb_attnw_kernel(const PbAttnPar
     pb_pdl_trigger();
     if (tid < 2) mx[tid] = 0u;
     const int ntok = min(TPT, p.batch - tok0);
-    const int64_t pos0 = p.pos[tok0], plast = p.pos[tok0 + ntok - 1], prev = p.kv_bits == 4 ? p.q4n[1] : 0;
+    const int64_t pos0 = p.pos[tok0], plast = p.pos[tok0 + ntok - 1], prev = p.kv_bits == 4 ? *p.q4prev : 0;
     const int64_t q4lo = aw_q4(p, pos0 + 1, prev), q4hi = aw_q4(p, plast + 1, prev);
     const int npk = (int)((q4hi + AW_N - 1) / AW_N), ntl = npk + (int)((plast - q4lo) / AW_N + 1);   // packed tiles, all tiles
     const int tb = (int)((int64_t)ntl * sp / gridDim.x), te = (int)((int64_t)ntl * (sp + 1) / gridDim.x);

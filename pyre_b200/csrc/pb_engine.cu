@@ -107,6 +107,7 @@ struct pb_state {
     // speculative verify: DeltaNet (conv ring, ssm) after each of the first t-1 tokens of the last window
     std::vector<float*> ck_conv, ck_ssm;   // [n_lin * PB_MAX_WINDOW]
     float** ck_tab = nullptr; float** ck_live = nullptr;   // the same pointers and the live buffers as device tables (pb_launch_ck_restore)
+    int64_t* q4prev = nullptr;    // packed boundary from before the window that runs
     int64_t* q4n_all = nullptr;   // packed boundaries of all attention layers [n_attn][batch]; PbKv::q4n points into it
     int verify_t = 0; int64_t verify_pos0 = 0;
     uint64_t steps = 0, kernels_per_step = 0;
@@ -572,6 +573,7 @@ static int state_create(pb_model* m, int batch, bool sharded, pb_state** out) {
     // 4-bit cache: the f32 ring holds the recent positions, the 64 that wait for the next packing step, and (batch-1 states)
     // a whole prefill chunk appended before its packing step
     s->ring_cap = c.kv_bits == 4 ? (int64_t)c.kv_recent + 64 + (solo ? PB_PREFILL_CHUNK : 0) : (int64_t)c.max_ctx;
+    if (rc == PB_OK) rc = dalloc(s, &s->q4prev, (size_t)1);
     if (rc == PB_OK) rc = dalloc(s, &s->q4n_all, (size_t)(m->n_attn > 0 ? m->n_attn : 1) * B);
     for (int i = 0; i < m->n_attn && rc == PB_OK; i++) {
         PbKv& k = s->kv[i];
@@ -734,7 +736,7 @@ static void attn_params(pb_state* s, int il, PbAttnParams& p) {
     p.n_rot = c.n_rot; p.eps = c.eps; p.n_head = c.n_head; p.n_kv = c.n_kv; p.hd = c.hd;
     p.kw = k.kw; p.ks = k.ks; p.vw = k.vw; p.vs = k.vs; p.kr = k.kr; p.vr = k.vr;
     p.max_ctx = c.kv_bits == 4 ? c.max_ctx : 1; p.ring_cap = s->ring_cap; p.kv_bits = c.kv_bits; p.kv_recent = c.kv_recent;
-    p.pos = s->pos; p.q4n = k.q4n; p.part_ml = s->part_ml; p.part_acc = s->part_acc; p.nsplit = s->nsplit; p.nsplit_packed = s->nsplit_packed;
+    p.pos = s->pos; p.q4n = k.q4n; p.q4prev = s->q4prev; p.part_ml = s->part_ml; p.part_acc = s->part_acc; p.nsplit = s->nsplit; p.nsplit_packed = s->nsplit_packed;
     { static const float rw = getenv("PYRE_B200_ATTN_RINGW") ? (float)atof(getenv("PYRE_B200_ATTN_RINGW")) : 2.5f; p.ring_weight = rw > 0.f ? rw : 2.5f; }   // measured: 2.5 .. 3.5 give the shortest batch-1 step, 2 .. 2.5 the shortest batch-32 step
     p.att = s->att; p.lda = (int64_t)c.n_head * c.hd; p.batch = s->batch;
 }

@@ -317,6 +317,7 @@ struct PbAttnParams {
     float* kr; float* vr;                                // f32 ring [batch][n_kv][ring_cap][hd]
     int64_t max_ctx; int64_t ring_cap; int kv_bits; int kv_recent;
     const int64_t* pos; int64_t* q4n;                    // [batch]
+    int64_t* q4prev;                                     // window: the boundary from before it
     float* part_ml; float* part_acc; int nsplit;
     int nsplit_packed;                                   // splits [0, nsplit_packed) walk the packed positions on the tensor cores
     float ring_weight;                                   // cost of a scalar tile of 8 f32 positions in packed tiles of 32 (split shares)
@@ -324,7 +325,7 @@ struct PbAttnParams {
     int batch;
     // window: the `batch` entries are consecutive tokens of sequence 0 (a prefill chunk): they share its cache; the append
     // kernel only writes the f32 ring, pb_launch_kv_pack then moves the packed boundary once for the whole window and
-    // keeps the previous boundary in q4n[1]; token j treats as packed what a token-by-token run would have packed by then
+    // the previous boundary stays in q4prev; token j treats as packed what a token-by-token run would have packed by then
     int window;
     // QSA block-sparse attention (pb_qsa.cu): when qsa_on[b] is set, sequence b attends only to the positions whose bit is
     // set in qsa_mask[b * qsa_ld + position / 32]; null = dense

@@ -67,3 +67,27 @@ def test_deltanet_run_lengths(ctx, n):
     for (ca, sa), (cb, sb) in zip((a.get_lin(0), a.get_lin(1)), (b.get_lin(0), b.get_lin(1))):
         assert rel_err(ca, cb) < tol and rel_err(sa, sb) < tol
     a.destroy(); b.destroy(); m.destroy()
+
+
+@pytest.mark.parametrize("n_head,n_kv", [(4, 2), (8, 1), (2, 2)])
+@pytest.mark.parametrize("prefix,t", [(0, 3), (60, 9), (127, 15), (250, 7), (383, 12)])
+def test_window_attention_matches_single_steps(ctx, n_head, n_kv, prefix, t):
+    """Windows whose tokens straddle the 64-position tiles and the boundary of the packed cache, one to three of which fill a row tile
+    (t < 16: the projections keep exact weights), then single steps over what the window left in the cache."""
+    cfg = small_cfg(pb, n_layers=2, full_every=1, n_head=n_head, n_kv=n_kv, kv_bits=4, kv_recent=64)
+    m = synth.build_model(ctx, cfg, synth.model_spec(cfg, 11), 11)
+    a, b = m.new_state(1), m.new_state(1)
+    ids = np.random.default_rng(prefix + t).integers(0, cfg.vocab, t).astype(np.uint32)
+    for s in (a, b):
+        if prefix:
+            for ai in range(2):
+                s.fill_kv_synth(ai, prefix, 3)
+            s.set_pos(prefix)
+    la = a.forward(ids)
+    for i in ids:
+        lb = b.forward(np.array([i], np.uint32))
+    assert rel_err(la, lb) < 1e-4
+    for _ in range(3):
+        assert rel_err(a.forward(ids[:1]), b.forward(ids[:1])) < 1e-3    # a rounding of a value may fall the other way in the packed cache
+    assert ctx.device_status() == 0
+    a.destroy(); b.destroy(); m.destroy()
