@@ -248,9 +248,12 @@ struct PbRouteParams {
     int* sel_e; float* sel_w;                 // [t][top_k], ascending expert id
     int* n_used; int* used_e; int* used_off;  // distinct local experts, entry offsets [n_used + 1]
     int* ent_tok; int* ent_slot; float* ent_w;
-    int4* virt; int* n_virt;                  // several tokens: distinct local experts in groups of up to PB_VGROUP entries {expert, first entry, entries, 0}, and their number
+    int4* virt; int* n_virt;                  // several tokens: distinct local experts in groups of up to PB_VGROUP entries {expert, first entry, entries, cost of the groups before}, and their number
 };
 #define PB_VGROUP 8
+// Cost of a group of n entries in the expert kernels, in thirds of a group of up to four: five to eight entries take a second n-tile of mma and, as
+// fewer such groups share a phase, more preparation (measured: 1.3 of a small group)
+__host__ __device__ static inline int pb_vgroup_cost(int n) { return n <= 0 ? 0 : (n <= 4 ? 3 : 4); }
 struct PbExpertParams {
     const int* n_used; const int* used_e; const int* used_off;
     const int* ent_tok; const int* ent_slot; const float* ent_w;

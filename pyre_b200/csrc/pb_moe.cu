@@ -100,7 +100,7 @@ __device__ __forceinline__ void pb_route_token_cta(const PbRouteParams& p, int b
 __device__ __forceinline__ void pb_route_lists(const PbRouteParams& p, int* rsm) {
     int* cnt = rsm;                 // [1024] entries per expert (local experts only)
     int* cursor = rsm + 1024;       // [1024] start offset of the expert's entries, then a fill cursor
-    __shared__ int wsum[3][8];
+    __shared__ int wsum[4][8];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int e = tid; e < 1024; e += 256) { cnt[e] = 0; cursor[e] = 0; }
     __syncthreads();
@@ -111,26 +111,26 @@ __device__ __forceinline__ void pb_route_lists(const PbRouteParams& p, int* rsm)
     __syncthreads();
     // distinct local experts in ascending id with entry offsets: block-wide exclusive scans of
     // (used flag, entry count) over expert ids; thread t owns experts 4t .. 4t+3
-    int c4[4], f = 0, c = 0, v = 0;   // distinct experts, entries, groups of PB_VGROUP entries
+    int c4[4], f = 0, c = 0, v = 0, w = 0;   // distinct experts, entries, groups of PB_VGROUP entries, cost of the groups
 #pragma unroll
-    for (int q = 0; q < 4; q++) { const int e = 4 * tid + q; c4[q] = e < p.n_exp ? cnt[e] : 0; f += c4[q] > 0; c += c4[q]; v += (c4[q] + PB_VGROUP - 1) / PB_VGROUP; }
-    int fi = f, ci = c, vi = v;
+    for (int q = 0; q < 4; q++) { const int e = 4 * tid + q; c4[q] = e < p.n_exp ? cnt[e] : 0; f += c4[q] > 0; c += c4[q]; v += (c4[q] + PB_VGROUP - 1) / PB_VGROUP; w += c4[q] / PB_VGROUP * pb_vgroup_cost(PB_VGROUP) + pb_vgroup_cost(c4[q] % PB_VGROUP); }
+    int fi = f, ci = c, vi = v, wi = w;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const int a = __shfl_up_sync(0xffffffffu, fi, o), d = __shfl_up_sync(0xffffffffu, ci, o), b = __shfl_up_sync(0xffffffffu, vi, o);
-        if (lane >= o) { fi += a; ci += d; vi += b; }
+        const int a = __shfl_up_sync(0xffffffffu, fi, o), d = __shfl_up_sync(0xffffffffu, ci, o), b = __shfl_up_sync(0xffffffffu, vi, o), h = __shfl_up_sync(0xffffffffu, wi, o);
+        if (lane >= o) { fi += a; ci += d; vi += b; wi += h; }
     }
-    if (lane == 31) { wsum[0][warp] = fi; wsum[1][warp] = ci; wsum[2][warp] = vi; }
+    if (lane == 31) { wsum[0][warp] = fi; wsum[1][warp] = ci; wsum[2][warp] = vi; wsum[3][warp] = wi; }
     __syncthreads();
-    int fb = 0, cb = 0, vb = 0;
-    for (int w2 = 0; w2 < warp; w2++) { fb += wsum[0][w2]; cb += wsum[1][w2]; vb += wsum[2][w2]; }
-    int n = fb + fi - f, off = cb + ci - c, vn = vb + vi - v;   // exclusive prefixes for expert 4 * tid
+    int fb = 0, cb = 0, vb = 0, wb = 0;
+    for (int w2 = 0; w2 < warp; w2++) { fb += wsum[0][w2]; cb += wsum[1][w2]; vb += wsum[2][w2]; wb += wsum[3][w2]; }
+    int n = fb + fi - f, off = cb + ci - c, vn = vb + vi - v, wn = wb + wi - w;   // exclusive prefixes for expert 4 * tid
 #pragma unroll
     for (int q = 0; q < 4; q++)
         if (c4[q] > 0) {
             const int e = 4 * tid + q;
             p.used_e[n] = e; p.used_off[n] = off; cursor[e] = off;
-            if (p.virt) for (int k = 0; k < c4[q]; k += PB_VGROUP) p.virt[vn++] = make_int4(e, off + k, min(PB_VGROUP, c4[q] - k), 0);
+            if (p.virt) for (int k = 0; k < c4[q]; k += PB_VGROUP) { const int z = min(PB_VGROUP, c4[q] - k); p.virt[vn++] = make_int4(e, off + k, z, wn); wn += pb_vgroup_cost(z); }
             n++; off += c4[q];
         }
     if (tid == 255) { p.used_off[n] = off; *p.n_used = n; if (p.virt) *p.n_virt = vn; }

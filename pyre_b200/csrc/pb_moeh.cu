@@ -3,7 +3,8 @@
 // The router lists the distinct selected experts in groups of up to eight of their (token, slot) entries (pb_route_lists); the shared expert adds
 // groups of eight tokens.  Unit of work: eight rows of gate and the same eight rows of up of one group (GU: the two halves of one mma
 // tile, so a lane ends up with both products and forms the hidden value itself), or sixteen output rows (DOWN).  The units, ordered by group, are
-// cut into equal runs, one per CTA (one CTA of sixteen warps per SM); inside a CTA the warps take the units of a run in turn.  The CTA first
+// cut into runs of equal cost, one per CTA (one CTA of sixteen warps per SM; with runs of as many units the CTAs that got the shared expert's full
+// groups ended 20 to 30 % after the mean); inside a CTA the warps take the units of a run in turn.  The CTA first
 // prepares the activations of as many groups as its shared memory holds (one token per warp), then runs their units without any
 // further barrier; a run that spans more groups repeats this.  A group of more than eight entries streams its weights again, from L2.
 //
@@ -27,7 +28,7 @@ __global__ void __launch_bounds__(MH_THREADS, 1) pb_moeh_kernel(const PbExpertPa
     extern __shared__ __align__(128) uint8_t smem[];
     int4* vtab = reinterpret_cast<int4*>(smem);                        // [MH_MAXV] {expert or -1 (shared), first entry / token, entries, first slot}
     int* stok = reinterpret_cast<int*>(smem + MH_MAXV * 16);           // [slots] group of the slot
-    __shared__ int nphase, nslots_used;
+    __shared__ int nphase, nslots_used, bound[2];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
     const uint32_t ring = pb_smem_u32(smem + MH_HEAD) + (uint32_t)(warp * MH_STAGES * h.stage_bytes);
     uint8_t* act = smem + MH_HEAD + (size_t)MH_WARPS * MH_STAGES * h.stage_bytes;
@@ -38,9 +39,23 @@ __global__ void __launch_bounds__(MH_THREADS, 1) pb_moeh_kernel(const PbExpertPa
     pb_pdl_wait();          // lists, activations / hidden vectors come from earlier kernels
     const int nv = *p.n_virt, nsh = p.has_shared ? (p.sh_ntok + PB_VGROUP - 1) / PB_VGROUP : 0;
     const int upg = p.rows_e / (DOWN ? 16 : 8);                          // units per group
-    const int64_t total = (int64_t)(nv + nsh) * upg;
-    const int u1 = (int)(total * (blockIdx.x + 1) / gridDim.x);
-    int u0 = (int)(total * blockIdx.x / gridDim.x);
+    // the CTA's run: the cost in front of a group stands in its list entry; the thread whose group holds a boundary finds its unit
+    if (tid < 2) bound[tid] = (nv + nsh) * upg;
+    const int4 lv = nv > 0 ? p.virt[nv - 1] : make_int4(0, 0, 0, 0);
+    const int croute = lv.w + pb_vgroup_cost(lv.z), zlast = p.sh_ntok - (nsh - 1) * PB_VGROUP;
+    const int64_t total = ((int64_t)croute + (nsh > 0 ? (nsh - 1) * pb_vgroup_cost(PB_VGROUP) + pb_vgroup_cost(zlast) : 0)) * upg;
+    const int64_t at0 = total * blockIdx.x / gridDim.x, at1 = total * (blockIdx.x + 1) / gridDim.x;
+    __syncthreads();
+    for (int v = tid; v < nv + nsh; v += MH_THREADS) {
+        const int4 e = v < nv ? p.virt[v] : make_int4(0, 0, v == nv + nsh - 1 ? zlast : PB_VGROUP, croute + (v - nv) * pb_vgroup_cost(PB_VGROUP));
+        const int c = pb_vgroup_cost(e.z);
+        const int64_t lo = (int64_t)e.w * upg, hi = lo + (int64_t)c * upg;
+        if (at0 >= lo && at0 < hi) bound[0] = v * upg + (int)(at0 - lo) / c;
+        if (at1 >= lo && at1 < hi) bound[1] = v * upg + (int)(at1 - lo) / c;
+    }
+    __syncthreads();
+    const int u1 = bound[1];
+    int u0 = bound[0];
     while (u0 < u1) {
         // ---- groups of this phase: as many as the slots hold
         const int v0 = u0 / upg;
