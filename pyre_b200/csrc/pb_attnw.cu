@@ -182,41 +182,50 @@ __global__ void __launch_bounds__(AW_THREADS, 1) pb_attnw_kernel(const PbAttnPar
     aw_fetch(p, sraw, (size_t)kvh, false, tb < npk, tile_p0(tb), plast, tid);
 
     // queries of the tile: rms_inplace(q, qn), rope, times 1/sqrt(hd)  (:1603-1606); a lane owns dims lane + 32 k of a row (n_rot = 64)
-    for (int r = warp; r < AW_M; r += 8) {
-        const int tok = tok0 + r / G;
-        float qv[8];
+    // (four rows at a time: their loads share one trip to L2)
+    float wn[8];
 #pragma unroll
-        for (int k = 0; k < 8; k++) qv[k] = 0.f;
-        if (r / G < ntok) {
+    for (int k = 0; k < 8; k++) wn[k] = p.qn[lane + 32 * k];
+    const float rinv = p.rope_inv[lane], ms = p.rope_inv[32];
+    for (int rb = warp; rb < AW_M; rb += 32) {
+        float qa[4][8], pf[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = rb + 8 * i, tok = tok0 + r / G;
             const float* qraw = p.proj + (size_t)tok * p.ldp + (size_t)(kvh * G + r % G) * 2 * AW_HD;
+            pf[i] = r / G < ntok ? (float)p.pos[tok] : 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; k++) qa[i][k] = r / G < ntok ? qraw[lane + 32 * k] : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = rb + 8 * i;
+            float (&qv)[8] = qa[i];
             float ss = 0.f;
 #pragma unroll
-            for (int k = 0; k < 8; k++) { qv[k] = qraw[lane + 32 * k]; ss += qv[k] * qv[k]; }
+            for (int k = 0; k < 8; k++) ss += qv[k] * qv[k];
             ss = pb_warp_sum(ss);
             const float s = 1.0f / sqrtf(ss / (float)AW_HD + p.eps), scale = 1.0f / sqrtf((float)AW_HD);
             float sn, co;
-            sincosf((float)p.pos[tok] * p.rope_inv[lane], &sn, &co);
-            const float ms = p.rope_inv[32];
+            sincosf(pf[i] * rinv, &sn, &co);
             if (ms != 1.0f) { co *= ms; sn *= ms; }
 #pragma unroll
-            for (int k = 0; k < 8; k++) qv[k] *= s * p.qn[lane + 32 * k];
+            for (int k = 0; k < 8; k++) qv[k] *= s * wn[k];
             const float x0 = qv[0], x1 = qv[1];
             qv[0] = x0 * co - x1 * sn; qv[1] = x1 * co + x0 * sn;
+            float m = 0.f;
 #pragma unroll
-            for (int k = 0; k < 8; k++) qv[k] *= scale;
-        }
-        float m = 0.f;
+            for (int k = 0; k < 8; k++) { qv[k] *= scale; m = fmaxf(m, fabsf(qv[k])); }
+            const int e = aw_expo(pb_warp_max(m));
+            if (lane == 0) qe[r] = e;
+            const float sc = aw_exp2i(-e);
 #pragma unroll
-        for (int k = 0; k < 8; k++) m = fmaxf(m, fabsf(qv[k]));
-        const int e = aw_expo(pb_warp_max(m));
-        if (lane == 0) qe[r] = e;
-        const float sc = aw_exp2i(-e);
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const float x = qv[k] * sc;
-            const __half hi = __float2half_rn(x);
-            *reinterpret_cast<__half*>(aw_smem + r * AW_ROW + (lane + 32 * k) * 2) = hi;
-            *reinterpret_cast<__half*>(aw_smem + AW_TILE + r * AW_ROW + (lane + 32 * k) * 2) = __float2half_rn(x - __half2float(hi));
+            for (int k = 0; k < 8; k++) {
+                const float x = qv[k] * sc;
+                const __half hi = __float2half_rn(x);
+                *reinterpret_cast<__half*>(aw_smem + r * AW_ROW + (lane + 32 * k) * 2) = hi;
+                *reinterpret_cast<__half*>(aw_smem + AW_TILE + r * AW_ROW + (lane + 32 * k) * 2) = __float2half_rn(x - __half2float(hi));
+            }
         }
     }
     __syncthreads();
@@ -353,23 +362,37 @@ __global__ void __launch_bounds__(256) pb_attnw_combine_kernel(const PbAttnParam
     const int tok = blockIdx.x, h = blockIdx.y * 4 + (threadIdx.x >> 6), c = threadIdx.x & 63, G = p.n_head / p.n_kv;
     pb_pdl_wait();
     pb_pdl_trigger();
-    if (h >= p.n_head) return;
-    const size_t base = (((size_t)tok * p.n_kv + h / G) * p.nsplit) * G + h % G;
-    const float4 gate = *reinterpret_cast<const float4*>(p.proj + (size_t)tok * p.ldp + (size_t)h * 2 * AW_HD + AW_HD + 4 * c);
-    float M = -INFINITY, L = 0.f;
-    for (int s = 0; s < p.nsplit; s++) M = fmaxf(M, p.part_ml[(base + (size_t)s * G) * 2]);
+    const int hr = h < p.n_head ? h : p.n_head - 1;     // (a CTA's last heads may be past the end: they repeat one and store nothing)
+    const size_t base = (((size_t)tok * p.n_kv + hr / G) * p.nsplit) * G + hr % G;
+    const float4 gate = *reinterpret_cast<const float4*>(p.proj + (size_t)tok * p.ldp + (size_t)hr * 2 * AW_HD + AW_HD + 4 * c);
+    // (at most 64 splits: thread c has split c's maximum and sum)
+    __shared__ float fs[4][64], wm[4][2], wl[4][2];
+    const int hq = threadIdx.x >> 6, wq = (threadIdx.x >> 5) & 1;
+    const float2 ml = c < p.nsplit ? *reinterpret_cast<const float2*>(p.part_ml + (base + (size_t)c * G) * 2) : make_float2(-INFINITY, 0.f);
+    const float wmx = pb_warp_max(ml.x);
+    if ((threadIdx.x & 31) == 0) wm[hq][wq] = wmx;
+    __syncthreads();
+    const float M = fmaxf(wm[hq][0], wm[hq][1]), fc = ml.x == -INFINITY ? 0.f : expf(ml.x - M);
+    fs[hq][c] = fc;
+    const float ls = pb_warp_sum(ml.y * fc);
+    if ((threadIdx.x & 31) == 0) wl[hq][wq] = ls;
+    __syncthreads();
+    const float L = wl[hq][0] + wl[hq][1];
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-    for (int s = 0; s < p.nsplit; s++) {
-        const float2 ml = *reinterpret_cast<const float2*>(p.part_ml + (base + (size_t)s * G) * 2);
-        if (ml.x == -INFINITY) continue;      // this split saw none of the row's positions: its sums were not written
-        const float f = expf(ml.x - M);
-        const float4 a = *reinterpret_cast<const float4*>(p.part_acc + (base + (size_t)s * G) * AW_HD + 4 * c);
-        L += ml.y * f;
-        o.x = fmaf(a.x, f, o.x); o.y = fmaf(a.y, f, o.y); o.z = fmaf(a.z, f, o.z); o.w = fmaf(a.w, f, o.w);
+    for (int s0 = 0; s0 < p.nsplit; s0 += 8) {
+        float4 a[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {          // (a split that saw none of the row's positions did not write its sums)
+            a[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (s0 + k < p.nsplit && fs[hq][s0 + k] != 0.f) a[k] = *reinterpret_cast<const float4*>(p.part_acc + (base + (size_t)(s0 + k) * G) * AW_HD + 4 * c);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            if (s0 + k < p.nsplit) { const float f = fs[hq][s0 + k]; o.x = fmaf(a[k].x, f, o.x); o.y = fmaf(a[k].y, f, o.y); o.z = fmaf(a[k].z, f, o.z); o.w = fmaf(a[k].w, f, o.w); }
+        }
     }
     const float r = 1.0f / L;
-    *reinterpret_cast<float4*>(p.att + (size_t)tok * p.lda + (size_t)h * AW_HD + 4 * c) =
+    if (h < p.n_head) *reinterpret_cast<float4*>(p.att + (size_t)tok * p.lda + (size_t)h * AW_HD + 4 * c) =
         make_float4(o.x * r * pb_sigm(gate.x), o.y * r * pb_sigm(gate.y), o.z * r * pb_sigm(gate.z), o.w * r * pb_sigm(gate.w));
 }
 
