@@ -4,8 +4,8 @@
 //
 // This is the path of prefill chunks, wide verify windows and batched decode: the reference switches to its tensor-core
 // GEMM at 16 tokens as well (gmm, src/model/qwen4exp_gguf.rs:3264-3266; k_gemm_tc, src/model/qn_cube.rs:153, host side
-// gemm_pfx :6559-6587).  One CTA owns a tile of 128 weight rows x up to 128 tokens and walks the contraction in steps of
-// 64 columns through a ring of 6 stages (a weight tile in tensor memory + the activation tiles in shared memory):
+// gemm_pfx :6559-6587).  One CTA owns a tile of 128 weight rows x up to 256 tokens and walks the contraction in steps of
+// 64 columns through a ring of 3 or 6 stages (a weight tile in tensor memory + the activation tiles in shared memory):
 //
 //   producer warp       brings the activations of each step -- f16 high and low parts (x = hi + lo, 22 significant
 //                       bits), prepared once per GEMM by pb_xt_prep_kernel in exactly the operand layout -- with 1-D
@@ -31,18 +31,19 @@
 #include <stdio.h>
 
 #define TC_ROWS 128                 // weight rows per tile = MMA M
-#define TC_NBLK 128                 // tokens per CTA; the MMA's N is twice the (padded) token count: high and low parts side by side
+#define TC_NARROW 128               // tokens per CTA, narrow form: the MMA's N is twice the (padded) token count, high and low parts side by side
+#define TC_WIDE 256                 // wide form: the two parts are two MMAs into the same columns, and one decode of a weight tile serves twice the tokens
 #define TC_KSTEP 64                 // contraction columns per step
 #define TC_STAGES 6                 // ring depth: a stage = a decoded weight tile in tensor memory (32 columns behind the accumulator's
-                                    // 256) + the activation tiles of the same step in shared memory (32 KB at 128 tokens)
-#define TC_ACC_COLS (2 * TC_NBLK)   // accumulator columns: high and low parts of up to 128 tokens
+                                    // 256) + the activation tiles of the same step in shared memory (wide: 3 stages)
+#define TC_ACC_COLS 256             // accumulator columns
 #define TC_A_COLS (TC_KSTEP / 2)    // a weight tile is 128 lanes x 32 columns: two f16 per 32-bit cell
 #define TC_TMEM_COLS 512            // 256 + 6 x 32 = 448, rounded to the power of two: the whole tensor memory of the SM (one CTA per SM)
-#define TC_RAW_STAGES 2             // raw double buffer: one block (256 columns = 4 steps) each
+#define TC_RAW_STAGES 2             // raw double buffer: one block (256 columns = 4 steps) each (deeper rings measured the same)
 #define TC_RAW_BYTES (TC_ROWS * 136)
 #define TC_DECODERS 8
 #define TC_THREADS ((TC_DECODERS + 2) * 32)
-#define TC_B_BYTES (2 * TC_NBLK * TC_KSTEP * 2)                   // high and low activation tiles: 32 KB
+#define TC_B_BYTES (2 * TC_NARROW * TC_KSTEP * 2)                 // high and low activation tiles of a stage: 32 KB, in the wide form twice that
 #define TC_XT_HEAD 4096             // bytes of per-token prescale inverses in front of the activation tiles
 
 enum : int { PB_DEV_TC_TIMEOUT = 6 };
@@ -107,29 +108,29 @@ __device__ __forceinline__ void pb_xt_store(uint8_t* blk, int np, int n, int c, 
     *reinterpret_cast<uint2*>(blk + pb_xt_off(np, n, c, 0)) = make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
     *reinterpret_cast<uint2*>(blk + pb_xt_off(np, n, c, 1)) = make_uint2(*reinterpret_cast<const uint32_t*>(&l01), *reinterpret_cast<const uint32_t*>(&l23));
 }
-__host__ __device__ __forceinline__ int pb_xt_np(int t, int tb) { const int n = t - tb * TC_NBLK < TC_NBLK ? t - tb * TC_NBLK : TC_NBLK; return (n + 15) & ~15; }
+__host__ __device__ __forceinline__ int pb_xt_np(int t, int tb, int nb) { const int n = t - tb * nb < nb ? t - tb * nb : nb; return (n + 15) & ~15; }   // nb: tokens of a block
 
 // One CTA per token slot (the slots past t of the last block are written as zeros).  The activation function is the
 // one of the other GEMV kernels: PLAIN (with an exact power-of-two prescale into [0.5, 1) so that f16 neither overflows
 // nor loses small columns), NORM (RMS norm times weight), GNORM (per-head RMS norm times weight times sigmoid(z)).
-// xbuf: TC_XT_HEAD bytes of prescale inverses [t], then per block of TC_NBLK tokens, per step of 64 columns, the high
+// xbuf: TC_XT_HEAD bytes of prescale inverses [t], then per block of nb tokens, per step of 64 columns, the high
 // tile and the low tile, each np x 64 f16 as swizzled 128-byte rows.
-__global__ void __launch_bounds__(256) pb_xt_prep_kernel(const PbGemvQParams p, uint8_t* __restrict__ xbuf) {
+__global__ void __launch_bounds__(256) pb_xt_prep_kernel(const PbGemvQParams p, int nb, uint8_t* __restrict__ xbuf) {
     constexpr int CT = 256;
     const int slot = (int)blockIdx.x;
-    const int tb = slot / TC_NBLK, n = slot - tb * TC_NBLK;
-    const int np = pb_xt_np(p.t, tb);
+    const int tb = slot / nb, n = slot - tb * nb;
+    const int np = pb_xt_np(p.t, tb, nb);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int cols = p.bpr * 256;
     __shared__ float red0[8];
     pb_pdl_wait();
     pb_pdl_trigger();
     if (n >= np) return;
-    const int tok = tb * TC_NBLK + n;
+    const int tok = tb * nb + n;
     const bool live = tok < p.t;
     const float* x = p.x + (size_t)tok * p.ldx;
     const float* z = p.z ? p.z + (size_t)tok * p.ldz : nullptr;
-    uint8_t* blk = xbuf + TC_XT_HEAD + (size_t)tb * ((size_t)cols / 64) * (2 * (size_t)TC_NBLK * 128);
+    uint8_t* blk = xbuf + TC_XT_HEAD + (size_t)tb * ((size_t)cols / 64) * (2 * (size_t)nb * 128);
     float* xinv = reinterpret_cast<float*>(xbuf);
     if (tid == 0 && live) xinv[tok] = 1.0f;
     if (p.mode == PB_ACT_GNORM) {
@@ -242,10 +243,14 @@ struct TcParams {
     const uint8_t* xt;      // prepared activations (pb_xt_prep_kernel)
     float* y; int64_t ldy;
     int accumulate;
+    int ks;                 // CTAs of a cluster: each takes cols / ks columns of its tile, their sums meet through distributed shared memory
     int* status;
 };
 
+template <bool WIDE>
 __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcParams p) {
+    constexpr int NB = WIDE ? TC_WIDE : TC_NARROW, NST = WIDE ? TC_STAGES / 2 : TC_STAGES;   // tokens of a CTA, stages of the ring
+    constexpr size_t STB = WIDE ? 2 * TC_B_BYTES : TC_B_BYTES;                               // and their bytes
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);             // [TC_STAGES] 128 decoder arrivals + the producer's, and the bulk-copy bytes
     uint64_t* empty = full + TC_STAGES;                             // [TC_STAGES] tcgen05.commit: the MMAs that read the stage are done
@@ -254,20 +259,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
     uint64_t* acc_full = raw_empty + TC_RAW_STAGES;                 // accumulator complete
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 384);
     float* red = reinterpret_cast<float*>(smem + 416);              // [8] per-warp maxima of d
-    float* xinv = reinterpret_cast<float*>(smem + 512);             // [TC_NBLK]
     uint8_t* b_ring = smem + 1024;                                  // [TC_STAGES][high tile | low tile], swizzled 128-byte rows
     uint8_t* raw = b_ring + TC_STAGES * TC_B_BYTES;               // [TC_RAW_STAGES][128 rows][136 bytes]
+    float* part = reinterpret_cast<float*>(b_ring);                 // [tokens][TC_ROWS] sums of this CTA's share of the contraction, once the MMAs are done
     static_assert((TC_STAGES * 2 + TC_RAW_STAGES * 2 + 1) * 8 <= 384 && TC_ACC_COLS + TC_STAGES * TC_A_COLS <= TC_TMEM_COLS, "barriers fit in front of the TMEM slot");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    const int tile = (int)blockIdx.x, tb = (int)blockIdx.y;
+    const int ks = p.ks, rank = (int)blockIdx.x % ks, tile = (int)blockIdx.x / ks, tb = (int)blockIdx.y;   // (clusters are consecutive CTAs)
     int s = 0;
     while (s + 1 < p.nseg && tile >= p.seg[s + 1].chunk0) s++;
     const int r0 = (tile - p.seg[s].chunk0) * TC_ROWS;
     const int nr = min(TC_ROWS, p.seg[s].rows - r0);
-    const int np = pb_xt_np(p.t, tb);                 // padded tokens of this block = MMA N
-    const int nt = min(TC_NBLK, p.t - tb * TC_NBLK);  // live tokens
-    const int nk = p.cols / TC_KSTEP;
+    const int np = pb_xt_np(p.t, tb, NB);             // padded tokens of this block = MMA N
+    const int nt = min(NB, p.t - tb * NB);  // live tokens
+    const int nkt = p.cols / TC_KSTEP, nk = nkt / ks, kb0 = rank * (nk / 4);   // steps of a row, of this CTA, and its first block
     const uint32_t bbytes = 2u * (uint32_t)np * 128u;
 
     if (tid == 0) {
@@ -282,40 +287,45 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    pb_pdl_wait();    // the activation tiles, and y when accumulating, come from earlier launches
+    // (pb_pdl_wait below, per role: the activation tiles, and y when accumulating, come from earlier launches; the weights do not)
 
     if (warp == TC_DECODERS) {
-        // ------------------------------------------------------------ producer: activation tiles, TC_STAGES steps ahead
+        // ------------------------------------------------------------ producer: activation tiles, a ring ahead
+        pb_pdl_wait();
         if (lane == 0) {
-            const uint8_t* src = p.xt + TC_XT_HEAD + (size_t)tb * (size_t)nk * (2 * (size_t)TC_NBLK * 128);
+            const uint8_t* src = p.xt + TC_XT_HEAD + (size_t)tb * (size_t)nkt * (2 * (size_t)NB * 128) + (size_t)rank * nk * bbytes;
             int k = 0;
             for (; k < nk; k++) {
-                const int st = k % TC_STAGES;
-                if (k >= TC_STAGES && !pb_mbar_wait(&empty[st], ((k / TC_STAGES) - 1) & 1, p.status, PB_DEV_TC_TIMEOUT)) break;
+                const int st = k % NST;
+                if (k >= NST && !pb_mbar_wait(&empty[st], ((k / NST) - 1) & 1, p.status, PB_DEV_TC_TIMEOUT)) break;
                 pb_mbar_expect_tx(&full[st], bbytes);
-                pb_bulk_g2s(b_ring + (size_t)st * TC_B_BYTES, src + (size_t)k * bbytes, bbytes, &full[st]);
+                pb_bulk_g2s(b_ring + (size_t)st * STB, src + (size_t)k * bbytes, bbytes, &full[st]);
             }
             // error path: the copies in flight get a bounded chance to land before the CTA may exit
             // (a stage's barrier also counts the decoders' arrivals: on the error path it may never complete; the wait is bounded)
-            if (k < nk) for (int j = max(0, k - TC_STAGES); j < k; j++) pb_mbar_wait(&full[j % TC_STAGES], (j / TC_STAGES) & 1, nullptr, 0);
+            if (k < nk) for (int j = max(0, k - NST); j < k; j++) pb_mbar_wait(&full[j % NST], (j / NST) & 1, nullptr, 0);
         }
     } else if (warp == TC_DECODERS + 1) {
         // ------------------------------------------------------------ MMA issue
-        // the high and the low tile are stacked along N: one instruction of N = 2 np columns per 16 columns of K reads the
-        // weight tile once; the epilogue adds the two halves of the accumulator
-        const uint32_t idesc = tc_idesc(TC_ROWS, 2 * np);
+        // narrow form: the high and the low tile are stacked along N: one instruction of N = 2 np columns per 16 columns of K
+        // reads the weight tile once, and the epilogue adds the two halves of the accumulator
+        pb_pdl_wait();
+        const uint32_t idesc = tc_idesc(TC_ROWS, WIDE ? np : 2 * np);
         bool ok = true;
         for (int k = 0; k < nk && ok; k++) {
-            const int st = k % TC_STAGES;
-            ok = pb_mbar_wait(&full[st], (k / TC_STAGES) & 1, p.status, PB_DEV_TC_TIMEOUT);
+            const int st = k % NST;
+            ok = pb_mbar_wait(&full[st], (k / NST) & 1, p.status, PB_DEV_TC_TIMEOUT);
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
             tc_fence_after();
             if (lane == 0) {
                 const uint32_t a_t = tmem + TC_ACC_COLS + (uint32_t)st * TC_A_COLS;
-                const uint32_t b_s = pb_smem_u32(b_ring + (size_t)st * TC_B_BYTES);
+                const uint32_t b_s = pb_smem_u32(b_ring + (size_t)st * STB);
 #pragma unroll
-                for (int kk = 0; kk < TC_KSTEP / 16; kk++) tc_mma_f16_ts(tmem, a_t + kk * 8, tc_desc(b_s + kk * 32), idesc, (k | kk) ? 1u : 0u);
+                for (int kk = 0; kk < TC_KSTEP / 16; kk++) {
+                    tc_mma_f16_ts(tmem, a_t + kk * 8, tc_desc(b_s + kk * 32), idesc, (k | kk) ? 1u : 0u);
+                    if (WIDE) tc_mma_f16_ts(tmem, a_t + kk * 8, tc_desc(b_s + (uint32_t)np * 128u + kk * 32), idesc, 1u);
+                }
                 tc_commit(&empty[st]);
             }
             __syncwarp();
@@ -327,9 +337,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
         const int grp = warp >> 2;                 // two groups of four warps take alternate steps
         const int row = (warp & 3) * 32 + lane;    // row of the tile
         const bool live = row < nr;
-        const uint8_t* wbase = p.seg[s].w + (size_t)r0 * p.row_bytes;
-        // raw bytes: block kb of the tile's rows (1088 bytes per group of eight rows) -> raw[kb % 2]; thread tid copies 16-byte words tid, tid + 256, ..
-        const int nkb = p.cols / 256, nwords = (nr + 7) / 8 * 68;
+        const uint8_t* wbase = p.seg[s].w + (size_t)r0 * p.row_bytes + (size_t)kb0 * 1088;   // (within a group of eight rows a block is 1088 bytes)
+        // raw bytes: block kb of the tile's rows -> raw[kb % TC_RAW_STAGES]; thread tid copies 16-byte words tid, tid + 256, ..
+        const int nkb = nk / 4, nwords = (nr + 7) / 8 * 68;
         auto issue_raw = [&](int kb) {
             const uint32_t dst = pb_smem_u32(raw + (size_t)(kb % TC_RAW_STAGES) * TC_RAW_BYTES);
             for (int i = tid; i < nwords; i += TC_DECODERS * 32) {
@@ -338,61 +348,103 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
             }
             tc_cp_async_arrive(&raw_full[kb % TC_RAW_STAGES]);
         };
-        issue_raw(0);
-        if (nkb > 1) issue_raw(1);
+        for (int i = 0; i < TC_RAW_STAGES && i < nkb; i++) issue_raw(i);
         // per-tile power-of-two shift: the largest |d| of the tile's rows times 465 lands in [2^14, 2^15)
         float dm = 0.f;
-        if (grp == 0 && live) for (int b = 0; b < nkb; b++) dm = fmaxf(dm, fabsf(pb_h2f(__ldg(reinterpret_cast<const uint16_t*>(wbase + (size_t)(row & ~7) * p.row_bytes + (size_t)b * 1088 + 1024 + 8 * (row & 7))))));
+        // (the two groups take alternate blocks; eight loads at a time: one after the other they were a trip to HBM each)
+        if (live) for (int b0 = grp; b0 < nkb; b0 += 16) {
+            float dv[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) dv[i] = b0 + 2 * i < nkb ? fabsf(pb_h2f(__ldg(reinterpret_cast<const uint16_t*>(wbase + (size_t)(row & ~7) * p.row_bytes + (size_t)(b0 + 2 * i) * 1088 + 1024 + 8 * (row & 7))))) : 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; i++) dm = fmaxf(dm, dv[i]);
+        }
         dm = pb_warp_max(dm);
         if (lane == 0) red[warp] = dm;
-        if (tid < TC_NBLK) xinv[tid] = tid < nt ? reinterpret_cast<const float*>(p.xt)[tb * TC_NBLK + tid] : 0.f;
+        pb_pdl_wait();
         pb_named_barrier(1, TC_DECODERS * 32);
-        dm = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+        dm = fmaxf(fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3])), fmaxf(fmaxf(red[4], red[5]), fmaxf(red[6], red[7])));
         int sh = 0;
         if (dm > 0.f && dm < 3.0e38f) { int e; (void)frexpf(dm * 465.0f, &e); sh = 15 - e; }   // dm * 465 * 2^sh in [2^14, 2^15)
         const float shift = ldexpf(1.0f, sh), unshift = ldexpf(1.0f, -sh);
 
         bool ok = true;
         for (int k = grp; k < nk; k += 2) {
-            const int st = k % TC_STAGES, kb = k >> 2, rs = kb % TC_RAW_STAGES;
+            const int st = k % NST, kb = k >> 2, rs = kb % TC_RAW_STAGES;
             // this group's steps of a block are quarters grp and grp + 2: wait for the bytes at the first; after the second,
-            // release the buffer and -- once all 256 threads have released it -- refill it with the block after next
+            // release the buffer and -- once all 256 threads have released it -- refill it
             if ((k & 3) == grp && !pb_mbar_wait(&raw_full[rs], (kb / TC_RAW_STAGES) & 1, p.status, PB_DEV_TC_TIMEOUT)) { ok = false; break; }
             TcRaw cur;
             tc_load_raw(cur, pb_smem_u32(raw + (size_t)rs * TC_RAW_BYTES) + (uint32_t)(row >> 3) * 1088u, row & 7, k & 3, live);
             if ((k & 3) == grp + 2) {
                 pb_mbar_arrive(&raw_empty[rs]);
-                if (kb + 2 < nkb) {
+                if (kb + TC_RAW_STAGES < nkb) {
                     if (!pb_mbar_wait(&raw_empty[rs], (kb / TC_RAW_STAGES) & 1, p.status, PB_DEV_TC_TIMEOUT)) { ok = false; break; }
-                    issue_raw(kb + 2);
+                    issue_raw(kb + TC_RAW_STAGES);
                 }
             }
-            if (k >= TC_STAGES && !pb_mbar_wait(&empty[st], ((k / TC_STAGES) - 1) & 1, p.status, PB_DEV_TC_TIMEOUT)) { ok = false; break; }
+            if (k >= NST && !pb_mbar_wait(&empty[st], ((k / NST) - 1) & 1, p.status, PB_DEV_TC_TIMEOUT)) { ok = false; break; }
             tc_decode_store(cur, k, tmem + ((uint32_t)((warp & 3) * 32) << 16) + TC_ACC_COLS + (uint32_t)st * TC_A_COLS, shift);
             tc_fence_before();                    // the stores are complete (wait::st); order them before the MMA warp's instructions
             pb_mbar_arrive(&full[st]);
         }
-        // ---- epilogue: warp w reads lanes 32 (w % 4) .. + 31 (its rows); warps 0-3 take tokens below 64, 4-7 the rest; columns
-        //      [0, np) hold the high parts' sums, [np, 2 np) the low parts'
+        // ---- epilogue: warp w reads lanes 32 (w % 4) .. + 31 (its rows); warps 0-3 take the first half of the tokens, 4-7 the rest; columns
+        //      [0, np) hold the sums, or (narrow) the high parts' with the low parts' in [np, 2 np)
         if (ok && pb_mbar_wait(acc_full, 0, p.status, PB_DEV_TC_TIMEOUT)) {
             tc_fence_after();
-            for (int c0 = grp * (TC_NBLK / 2); c0 < (grp + 1) * (TC_NBLK / 2) && c0 < np; c0 += 32) {
+            const int half = ((np + 1) / 2 + 31) / 32 * 32;
+            for (int c0 = grp * half; c0 < (grp + 1) * half && c0 < np; c0 += 32) {
+                // the prescales and (accumulating) the old values of the 32 tokens share one trip to L2
+                float* dst = p.y + (size_t)(tb * NB + c0) * p.ldy + p.seg[s].yoff + r0 + row;
+                const float xi = c0 + lane < nt ? reinterpret_cast<const float*>(p.xt)[tb * NB + c0 + lane] : 0.f;
+                float old[32];
+#pragma unroll
+                for (int j = 0; j < 32; j++) old[j] = p.accumulate && ks == 1 && live && c0 + j < nt ? dst[(size_t)j * p.ldy] : 0.f;
                 uint32_t v[32], vl[32];
                 tc_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
-                tc_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(np + c0), vl);
-                if (live) {
+                if (!WIDE) tc_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(np + c0), vl);
 #pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        const int b = c0 + j;
-                        if (b < nt) {
-                            float* dst = p.y + (size_t)(tb * TC_NBLK + b) * p.ldy + p.seg[s].yoff + r0 + row;
-                            const float o = (__uint_as_float(v[j]) + __uint_as_float(vl[j])) * (unshift * xinv[b]);
-                            *dst = p.accumulate ? *dst + o : o;
-                        }
-                    }
+                for (int j = 0; j < 32; j++) {
+                    const float sum = WIDE ? __uint_as_float(v[j]) : __uint_as_float(v[j]) + __uint_as_float(vl[j]);
+                    const float o = sum * (unshift * __shfl_sync(0xffffffffu, xi, j));
+                    if (!live || c0 + j >= nt) continue;
+                    if (ks > 1) part[(c0 + j) * TC_ROWS + row] = o;
+                    else dst[(size_t)j * p.ldy] = old[j] + o;
                 }
             }
         }
+    }
+    __syncwarp();
+    if (ks > 1) {
+        // the CTAs of the cluster add their sums in the order of the contraction, each a share of the tokens
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const uint32_t src = pb_smem_u32(part);
+        const int i1 = nt * (rank + 1) / ks * TC_ROWS;
+        for (int ib = nt * rank / ks * TC_ROWS + tid; ib < i1; ib += 4 * TC_THREADS) {   // four outputs at a time
+            float v[4][8], old[4];
+            float* dst[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int i = ib + u * TC_THREADS, b = i / TC_ROWS, row = i - b * TC_ROWS;
+                dst[u] = i < i1 && row < nr ? p.y + (size_t)(tb * NB + b) * p.ldy + p.seg[s].yoff + r0 + row : nullptr;
+                old[u] = dst[u] && p.accumulate ? *dst[u] : 0.f;
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    v[u][c] = 0.f;
+                    if (c < ks && dst[u]) {
+                        uint32_t a;
+                        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(src + 4u * (uint32_t)i), "r"(c));
+                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[u][c]) : "r"(a) : "memory");
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (dst[u]) { float o = v[u][0]; 
+#pragma unroll
+                    for (int c = 1; c < 8; c++) o += v[u][c]; *dst[u] = old[u] + o; }
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // no CTA leaves while its sums are read
     }
     asm volatile("cp.async.wait_all;" ::: "memory");   // (error paths) no copy of this thread is still in flight when the CTA exits
     tc_fence_before();
@@ -413,7 +465,7 @@ int pb_gemmtc_min_tokens() {
 }
 
 int pb_gemmtc_max_tokens(int cols) {
-    const size_t n = (PB_XH_BYTES - TC_XT_HEAD) / ((size_t)cols * 4) / TC_NBLK * TC_NBLK;
+    const size_t n = (PB_XH_BYTES - TC_XT_HEAD) / ((size_t)cols * 4) / TC_WIDE * TC_WIDE;
     return (int)(n < TC_XT_HEAD / 4 ? n : TC_XT_HEAD / 4);
 }
 
@@ -424,31 +476,43 @@ int pb_launch_gemmtc(pb_ctx* ctx, const PbGemvQArgs& a) {
     if (((uintptr_t)a.x & 15) || (a.ldx & 3)) PB_FAIL(ctx, PB_ERR_ARG, "tensor-core gemm: activations must be 16-byte aligned");
     if (a.nseg < 1 || a.nseg > 4) PB_FAIL(ctx, PB_ERR_ARG, "tensor-core gemm: %d segments", a.nseg);
     for (int sg = 0; sg < a.nseg; sg++) if (!a.seg[sg].wr) PB_FAIL(ctx, PB_UNSUPPORTED, "tensor-core gemm: segment %d has no re-coded copy", sg);
-    const int nblk = (a.t + TC_NBLK - 1) / TC_NBLK;
-    const size_t need = TC_XT_HEAD + (size_t)nblk * TC_NBLK * a.cols * 4;
+    int ntiles = 0;
+    for (int sg = 0; sg < a.nseg; sg++) ntiles += (int)((a.seg[sg].rows + TC_ROWS - 1) / TC_ROWS);
+    if (ntiles == 0) return PB_OK;
+    const size_t smem = 1024 + (size_t)TC_STAGES * TC_B_BYTES + (size_t)TC_RAW_STAGES * TC_RAW_BYTES;
+    // Tokens per CTA and CTAs per tile, by the rounds the SMs need: a CTA walks its columns serially, a wide one takes half as long again per block
+    // and twice as long around it (256 tokens of 12352 x 2048: two rounds of narrow ones 47 us, one of wide ones 39); a matrix with
+    // fewer tiles than SMs is cut along its columns, and the parts' sums meet at the end (256 tokens of 2048 x 4096: 64 us uncut, 26 in four).
+    int nb = TC_NARROW, cut = 1, best = 0;
+    for (int w = TC_NARROW; w <= (a.t > TC_NARROW ? TC_WIDE : TC_NARROW); w *= 2)
+        for (int ks = 1; ks <= 8 && a.cols / 256 % ks == 0 && (ks == 1 || a.cols / 256 / ks >= 2); ks *= 2) {
+            const void* k = w == TC_WIDE ? reinterpret_cast<const void*>(pb_gemmtc_iq3s_kernel<true>) : reinterpret_cast<const void*>(pb_gemmtc_iq3s_kernel<false>);
+            PB_TRY(pb_ensure_smem_fn(ctx, k, smem));
+            const int room = pb_max_clusters(ctx, k, TC_THREADS, smem, ks), rounds = (ntiles * ((a.t + w - 1) / w) + room - 1) / room;
+            const int cost = rounds * ((w == TC_WIDE ? 12 : 6) + (ks > 1 ? 4 : 0) + a.cols / 256 / ks * (w == TC_WIDE ? 3 : 2));
+            if (best == 0 || cost < best) { best = cost; nb = w; cut = ks; }
+        }
+    const int nblk = (a.t + nb - 1) / nb;
+    const size_t need = TC_XT_HEAD + (size_t)nblk * nb * a.cols * 4;
     if ((size_t)a.t * 4 > TC_XT_HEAD || need > PB_XH_BYTES) PB_FAIL(ctx, PB_UNSUPPORTED, "tensor-core gemm: %d tokens of %d columns exceed the %zu-byte operand buffer", a.t, a.cols, (size_t)PB_XH_BYTES);
     {
         PbGemvQParams q;
         memset(&q, 0, sizeof q);
         q.bpr = a.cols / 256; q.x = a.x; q.ldx = a.ldx; q.t = a.t; q.mode = a.mode; q.norm_w = a.norm_w; q.z = a.z; q.ldz = a.ldz; q.head_dim = a.head_dim; q.eps = a.eps;
-        pb_launch_k(ctx, pb_xt_prep_kernel, dim3((nblk - 1) * TC_NBLK + pb_xt_np(a.t, nblk - 1)), dim3(256), (size_t)0, q, ctx->xh_buf);
+        pb_launch_k(ctx, pb_xt_prep_kernel, dim3((nblk - 1) * nb + pb_xt_np(a.t, nblk - 1, nb)), dim3(256), (size_t)0, q, nb, ctx->xh_buf);
         ctx->kernels_launched++;
         PB_CUDA(ctx, cudaGetLastError());
     }
     TcParams p;
     memset(&p, 0, sizeof p);
     p.nseg = a.nseg; p.row_bytes = a.cols / 256 * 136; p.cols = a.cols; p.t = a.t; p.xt = ctx->xh_buf; p.y = a.y; p.ldy = a.ldy; p.accumulate = a.accumulate; p.status = ctx->dev_status;
-    int ntiles = 0;
-    for (int sg = 0; sg < a.nseg; sg++) {
-        p.seg[sg].w = a.seg[sg].wr; p.seg[sg].rows = (int)a.seg[sg].rows; p.seg[sg].yoff = (int)a.seg[sg].yoff; p.seg[sg].chunk0 = ntiles;
-        ntiles += (int)((a.seg[sg].rows + TC_ROWS - 1) / TC_ROWS);
+    for (int sg = 0, n = 0; sg < a.nseg; sg++) {
+        p.seg[sg].w = a.seg[sg].wr; p.seg[sg].rows = (int)a.seg[sg].rows; p.seg[sg].yoff = (int)a.seg[sg].yoff; p.seg[sg].chunk0 = n;
+        n += (int)((a.seg[sg].rows + TC_ROWS - 1) / TC_ROWS);
     }
-    p.ntiles = ntiles;
-    if (ntiles == 0) return PB_OK;
-    const size_t smem = 1024 + (size_t)TC_STAGES * TC_B_BYTES + (size_t)TC_RAW_STAGES * TC_RAW_BYTES;
-    auto kern = pb_gemmtc_iq3s_kernel;
-    PB_TRY(pb_ensure_smem(ctx, kern, smem));
-    pb_launch_k(ctx, kern, dim3(ntiles, nblk), dim3(TC_THREADS), smem, p);
+    p.ntiles = ntiles; p.ks = cut;
+    if (nb == TC_WIDE) pb_launch_kc(ctx, pb_gemmtc_iq3s_kernel<true>, dim3(ntiles * cut, nblk), dim3(TC_THREADS), smem, cut, p);
+    else pb_launch_kc(ctx, pb_gemmtc_iq3s_kernel<false>, dim3(ntiles * cut, nblk), dim3(TC_THREADS), smem, cut, p);
     ctx->kernels_launched++;
     PB_CUDA(ctx, cudaGetLastError());
     return PB_OK;
