@@ -125,14 +125,10 @@ __global__ void __launch_bounds__(PB_KTHREADS, 1) pb_gemvq_kernel(const PbGemvQP
     const int rpw = 32 / lpr;                           // rows one warp handles side by side
     const int sub = lane / lpr, ql = lane - sub * lpr;
 
-    PbXQuarter xr[NB == 1 ? PASSES : 1];
-    if (NB == 1) {
-#pragma unroll
-        for (int ps = 0; ps < PASSES; ps++) {
-            const int qi = ps * 32 + ql;
-            if (qi < nquarters) pb_load_xquarter<PbQDec<FMT>::AFFINE>(xq, cols, qi, xr[ps]);
-        }
-    }
+    // one column: the lane's activations stay in registers; of wider rows (two passes) a warp has few, and both passes' would not fit: they are
+    // loaded as they are used
+    PbXQuarter xr[1];
+    if (NB == 1 && PASSES == 1 && ql < nquarters) pb_load_xquarter<PbQDec<FMT>::AFFINE>(xq, cols, ql, xr[0]);
 
     for (int k = 0; k < my_chunks; k++) {
         if (!pb_ring_wait(ring, k, p.status)) return;
@@ -145,26 +141,30 @@ __global__ void __launch_bounds__(PB_KTHREADS, 1) pb_gemvq_kernel(const PbGemvQP
         const uint32_t base = pb_smem_u32(pb_ring_stage(ring, k));
         if ((FMT == PB_T_IQ3_S || FMT == PB_T_IQ3S_N4) && NB == 1 && PASSES == 1 && lpr == 32) {
             // one column, full-width rows: two rows per iteration, so that the two independent decode
-            // chains overlap each other's shared-memory latency (a row past nr decodes stale bytes of the
-            // stage and is not stored)
+            // chains overlap each other's shared-memory latency
             float* ybase = p.y + p.seg[s].yoff + r0;
-            // re-coded rows come in groups of eight: the warp's rows are all row (warp & 7) of their group
-            const uint32_t oc = pb_n4_code_off(warp & 7, ql), oh = pb_n4_head_off(warp & 7, ql);
-            for (int ra = warp; ra < nr; ra += 2 * PB_CONSUMERS) {
+            // re-coded rows come in groups of eight: the warp's rows are all row (warp & 7) of their group, at a fixed distance
+            const uint32_t rb16 = 16u * (uint32_t)p.row_bytes, hd = pb_n4_head_off(warp & 7, ql) - pb_n4_code_off(warp & 7, ql);
+            uint32_t ga = base + (uint32_t)(warp & ~7) * (uint32_t)p.row_bytes + pb_n4_code_off(warp & 7, ql);
+            for (int ra = warp; ra < nr; ra += 2 * PB_CONSUMERS, ga += 2 * rb16) {
                 const int rc = ra + PB_CONSUMERS;
-                const bool two = rc < p.rows_per_chunk;
-                float v0, v1;
+                const bool two = rc < nr;
+                float v0, v1 = 0.f;
                 if constexpr (FMT == PB_T_IQ3S_N4) {
-                    const uint32_t ga = base + (uint32_t)(ra & ~7) * (uint32_t)p.row_bytes, gb = base + (uint32_t)((two ? rc : ra) & ~7) * (uint32_t)p.row_bytes;
                     PbQuarter wa, wb;
-                    D::quarter(ga + oc, ga + oh, ql & 3, wa); D::quarter(gb + oc, gb + oh, ql & 3, wb);
-                    v0 = pb_quarter_dot<FMT>(wa, xr[0]); v1 = pb_quarter_dot<FMT>(wb, xr[0]);
-                } else { v0 = pb_decode_dot<FMT>(base, ra, p.row_bytes, ql, T, xr[0]); v1 = pb_decode_dot<FMT>(base, two ? rc : ra, p.row_bytes, ql, T, xr[0]); }
+                    if (two) {
+                        D::quarter(ga, ga + hd, ql & 3, wa); D::quarter(ga + rb16, ga + rb16 + hd, ql & 3, wb);
+                        v0 = pb_quarter_dot<FMT>(wa, xr[0]); v1 = pb_quarter_dot<FMT>(wb, xr[0]);
+                    } else { D::quarter(ga, ga + hd, ql & 3, wa); v0 = pb_quarter_dot<FMT>(wa, xr[0]); }
+                } else { v0 = pb_decode_dot<FMT>(base, ra, p.row_bytes, ql, T, xr[0]); if (two) v1 = pb_decode_dot<FMT>(base, rc, p.row_bytes, ql, T, xr[0]); }
+                // the two rows share the reduction: the lower half of the warp goes on with row ra, the upper with rc (the same sums in the same order)
+                const bool up = lane & 16;
+                float v = (up ? v1 : v0) + __shfl_xor_sync(0xffffffffu, up ? v0 : v1, 16);
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) { v0 += __shfl_xor_sync(0xffffffffu, v0, o); v1 += __shfl_xor_sync(0xffffffffu, v1, o); }
-                if (lane == 0) {
-                    ybase[ra] = p.accumulate ? ybase[ra] + v0 : v0;
-                    if (two && rc < nr) ybase[rc] = p.accumulate ? ybase[rc] + v1 : v1;
+                for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if ((lane & 15) == 0 && (!up || two)) {
+                    float* dst = ybase + (up ? rc : ra);
+                    *dst = p.accumulate ? *dst + v : v;
                 }
             }
             pb_ring_release(ring, k, lane);
@@ -181,14 +181,15 @@ __global__ void __launch_bounds__(PB_KTHREADS, 1) pb_gemvq_kernel(const PbGemvQP
                 for (int ps = 0; ps < PASSES; ps++) {
                     const int qi = ps * 32 + ql;
                     if (qi < nquarters) {
+                        if (NB == 1 && PASSES > 1) pb_load_xquarter<PbQDec<FMT>::AFFINE>(xq, cols, qi, xr[0]);
                         if (FMT == PB_T_IQ3_S && NB == 1) {
-                            acc[0] += pb_iq3s_quarter_dot(base + (uint32_t)r * (uint32_t)p.row_bytes + (qi >> 2) * D::STEP_BYTES, qi & 3, T, xr[ps]);
+                            acc[0] += pb_iq3s_quarter_dot(base + (uint32_t)r * (uint32_t)p.row_bytes + (qi >> 2) * D::STEP_BYTES, qi & 3, T, xr[0]);
                             continue;
                         }
                         PbQuarter wq;
                         pb_quarter_at<FMT>(base, r, p.row_bytes, qi, T, wq);
                         if (NB == 1) {
-                            acc[0] += pb_quarter_dot<FMT>(wq, xr[ps]);
+                            acc[0] += pb_quarter_dot<FMT>(wq, xr[0]);
                         } else {
 #pragma unroll 1
                             for (int b = 0; b < NB; b++) {

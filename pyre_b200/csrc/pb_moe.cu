@@ -117,8 +117,15 @@ __device__ __forceinline__ void pb_route_lists(const PbRouteParams& p, int* rsm)
     int fi = f, ci = c, vi = v, wi = w;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const int a = __shfl_up_sync(0xffffffffu, fi, o), d = __shfl_up_sync(0xffffffffu, ci, o), b = __shfl_up_sync(0xffffffffu, vi, o), h = __shfl_up_sync(0xffffffffu, wi, o);
-        if (lane >= o) { fi += a; ci += d; vi += b; wi += h; }
+        const int a = __shfl_up_sync(0xffffffffu, fi, o), d = __shfl_up_sync(0xffffffffu, ci, o);
+        if (lane >= o) { fi += a; ci += d; }
+    }
+    if (p.virt) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int b = __shfl_up_sync(0xffffffffu, vi, o), h = __shfl_up_sync(0xffffffffu, wi, o);
+            if (lane >= o) { vi += b; wi += h; }
+        }
     }
     if (lane == 31) { wsum[0][warp] = fi; wsum[1][warp] = ci; wsum[2][warp] = vi; wsum[3][warp] = wi; }
     __syncthreads();

@@ -163,18 +163,20 @@ template <> struct PbQDec<PB_T_Q4_K> {
             if (j < 4) { s[e] = sb(j) & 63; m[e] = sb(j + 4) & 63; }
             else { s[e] = (sb(j + 4) & 0xF) | ((sb(j - 4) >> 6) << 4); m[e] = (sb(j + 4) >> 4) | ((sb(j) >> 6) << 4); }
         }
-        o.sc[0] = o.sc[1] = d * (float)s[0]; o.sc[2] = o.sc[3] = d * (float)s[1];
+        o.sc[0] = o.sc[1] = d * (float)s[0]; o.sc[2] = o.sc[3] = 0.0625f * (d * (float)s[1]);   // (the second group's codes stay in the high nibbles)
         o.mn[0] = mn * (float)m[0]; o.mn[1] = mn * (float)m[1];
         const uint4 a = pb_lds128(p + 16 + 32 * qt), b = pb_lds128(p + 32 + 32 * qt);
         const uint32_t q[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-        for (int k = 0; k < 8; k++) { o.w[k] = (int)(q[k] & 0x0F0F0F0Fu); o.w[8 + k] = (int)((q[k] >> 4) & 0x0F0F0F0Fu); }
+        for (int k = 0; k < 8; k++) { o.w[k] = (int)(q[k] & 0x0F0F0F0Fu); o.w[8 + k] = (int)(q[k] & 0xF0F0F0F0u); }
     }
 };
 
 // IQ3_S re-coded into 4-bit codes c (weight = 2 c - 15): the quarter holds the codes, unsigned, and
 // pb_quarter_dot removes the offset with the integer sums of the activation levels:
-// sum (2 c - 15) q = 2 sum c q - 15 sum q, exact in integers.
+// sum (2 c - 15) q = 2 sum c q - 15 sum q, exact in integers.  The codes in the high nibbles stay there (16 c): eight times the sum is
+// 16 sum_low + sum_high - 120 sum q, one multiply-add with the last two, and the weight scale carries the 1/8.  One token against a large matrix is
+// bound by instructions, and the shifts were 8 of 190 per row and lane.
 template <> struct PbQDec<PB_T_IQ3S_N4> {
     static constexpr int STEP_BYTES = 136;
     static constexpr bool HAS_MIN = false, SCALE16 = false, AFFINE = true;
@@ -183,15 +185,15 @@ template <> struct PbQDec<PB_T_IQ3S_N4> {
         const uint2 hdr = pb_lds64(hp);
         const float d = pb_h2f((uint16_t)(hdr.x & 0xFFFF));
         const uint32_t sc = (hdr.y >> (8 * qt)) & 0xFF;
-        const float d0 = d * (float)(1 + 2 * (int)(sc & 0xF)), d1 = d * (float)(1 + 2 * (int)(sc >> 4));
+        const float d8 = 0.125f * d, d0 = d8 * (float)(1 + 2 * (int)(sc & 0xF)), d1 = d8 * (float)(1 + 2 * (int)(sc >> 4));
         o.sc[0] = o.sc[1] = d0; o.sc[2] = o.sc[3] = d1;
 #pragma unroll
         for (int i = 0; i < 2; i++) {
             const uint4 c = pb_lds128(a + 512 * i);
-            o.w[8 * i + 0] = (int)(c.x & 0x0F0F0F0Fu); o.w[8 * i + 1] = (int)((c.x >> 4) & 0x0F0F0F0Fu);
-            o.w[8 * i + 2] = (int)(c.y & 0x0F0F0F0Fu); o.w[8 * i + 3] = (int)((c.y >> 4) & 0x0F0F0F0Fu);
-            o.w[8 * i + 4] = (int)(c.z & 0x0F0F0F0Fu); o.w[8 * i + 5] = (int)((c.z >> 4) & 0x0F0F0F0Fu);
-            o.w[8 * i + 6] = (int)(c.w & 0x0F0F0F0Fu); o.w[8 * i + 7] = (int)((c.w >> 4) & 0x0F0F0F0Fu);
+            o.w[8 * i + 0] = (int)(c.x & 0x0F0F0F0Fu); o.w[8 * i + 1] = (int)(c.x & 0xF0F0F0F0u);
+            o.w[8 * i + 2] = (int)(c.y & 0x0F0F0F0Fu); o.w[8 * i + 3] = (int)(c.y & 0xF0F0F0F0u);
+            o.w[8 * i + 4] = (int)(c.z & 0x0F0F0F0Fu); o.w[8 * i + 5] = (int)(c.z & 0xF0F0F0F0u);
+            o.w[8 * i + 6] = (int)(c.w & 0x0F0F0F0Fu); o.w[8 * i + 7] = (int)(c.w & 0xF0F0F0F0u);
         }
     }
 };
@@ -533,9 +535,11 @@ __device__ __forceinline__ int pb_dp4a_us(int a, int b, int c) {
 struct PbXQuarter {
     int q[PB_XLEVELS][16];
     float s[PB_XLEVELS][2], sum[2];
-    int is[PB_XLEVELS][2];   // -15 * integer sum of each level over a 32-group (loaded only for offset-coded formats)
+    int is[PB_XLEVELS][2];   // -120 * integer sum of each level over a 32-group (loaded only for offset-coded formats)
 };
 
+// formats whose decoded bytes are unsigned codes up to 240
+template <int FMT> __host__ __device__ constexpr bool pb_q_unsigned() { return FMT == PB_T_IQ3S_N4 || FMT == PB_T_Q4_K; }
 template <int FMT>
 __device__ __forceinline__ float pb_quarter_dot(const PbQuarter& w, const PbXQuarter& x) {
     using D = PbQDec<FMT>;
@@ -544,17 +548,20 @@ __device__ __forceinline__ float pb_quarter_dot(const PbQuarter& w, const PbXQua
     constexpr int WPH = 16 / NH;
 #pragma unroll
     for (int h = 0; h < NH; h++) {
-        int isum[PB_XLEVELS];
+        const int g = h * WPH / 8;
+        int isum[PB_XLEVELS], high[PB_XLEVELS];
 #pragma unroll
-        for (int l = 0; l < PB_XLEVELS; l++) isum[l] = 0;
+        for (int l = 0; l < PB_XLEVELS; l++) { isum[l] = 0; high[l] = D::AFFINE ? x.is[l][g] : 0; }   // x.is = -120 * (sum of the level over the group)
 #pragma unroll
         for (int k = 0; k < WPH; k++)
 #pragma unroll
-            for (int l = 0; l < PB_XLEVELS; l++) isum[l] = D::AFFINE ? pb_dp4a_us(w.w[h * WPH + k], x.q[l][h * WPH + k], isum[l]) : __dp4a(w.w[h * WPH + k], x.q[l][h * WPH + k], isum[l]);
-        const int g = h * WPH / 8;
+            for (int l = 0; l < PB_XLEVELS; l++) {
+                int& a = D::AFFINE && (k & 1) ? high[l] : isum[l];
+                a = pb_q_unsigned<FMT>() ? pb_dp4a_us(w.w[h * WPH + k], x.q[l][h * WPH + k], a) : __dp4a(w.w[h * WPH + k], x.q[l][h * WPH + k], a);
+            }
         if (D::AFFINE) {
 #pragma unroll
-            for (int l = 0; l < PB_XLEVELS; l++) isum[l] = 2 * isum[l] + x.is[l][g];   // x.is = -15 * (sum of the level over the group)
+            for (int l = 0; l < PB_XLEVELS; l++) isum[l] = 16 * isum[l] + high[l];
         }
         float t = x.s[PB_XLEVELS - 1][g] * (float)isum[PB_XLEVELS - 1];   // smallest level first
 #pragma unroll

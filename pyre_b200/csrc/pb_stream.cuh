@@ -60,7 +60,7 @@ __device__ __forceinline__ void pb_ring_release(const PbRing& r, int k, int lane
 __device__ __forceinline__ int pb_xq_off(int qi, int i, int nq) { return (i * nq + qi) * 4; }
 
 // Quantized activations of one column: PB_XLEVELS arrays of cols/4 words, then PB_XLEVELS scale
-// arrays and the group sums, cols/32 floats each, then PB_XLEVELS arrays of cols/32 integers: -15 times the
+// arrays and the group sums, cols/32 floats each, then PB_XLEVELS arrays of cols/32 integers: -120 times the
 // sum of each level's int8 values over a group (the offset term of weight formats coded as 2 c - 15)
 __host__ __device__ static inline int pb_xq_words(int cols) { return PB_XLEVELS * (cols / 4) + (2 * PB_XLEVELS + 1) * (cols / 32); }
 
@@ -117,7 +117,7 @@ __device__ __forceinline__ void pb_split_groups4(float4 v, int lane, int g0, int
     if (k == 0) {
         const int tot[3] = {(p01 & 0xFFFF) - 4096, (p01 >> 16) - 4096, p2};
 #pragma unroll
-        for (int l = 0; l < PB_XLEVELS; l++) { sc[l * ng + g] = sl[l]; reinterpret_cast<int*>(sc)[(PB_XLEVELS + 1 + l) * ng + g] = -15 * tot[l]; }   // stored ready for 2 A - 15 S
+        for (int l = 0; l < PB_XLEVELS; l++) { sc[l * ng + g] = sl[l]; reinterpret_cast<int*>(sc)[(PB_XLEVELS + 1 + l) * ng + g] = -120 * tot[l]; }   // stored ready for 8 (2 A - 15 S)
         if (WITH_SUM) sc[PB_XLEVELS * ng + g] = sum;
     }
 }
