@@ -326,7 +326,7 @@ def run_ours(args):
         step_bytes = stats.weight_bytes_per_step + stats.kv_bytes_per_step + stats.state_bytes_per_step
         peak, which = measured_peaks()
         line = {"metric": "decode_tok_per_s", "value": round(value, 2), "unit": "tok/s", "n_gpus": world, "steps": args.steps, "warmup": max(args.warmup, 3),
-                "ms_per_step": round(ms / args.steps, 4), "higher_is_better": True, "scaling": "weak" if (args.replicas or sharded or world == 1) else "strong", "vs_baseline": None, "dtype": "int8 (dp4a: decoded weights x int8-split activations) at batch 1, f16 tensor cores (mma.sync with f16 hi/lo activations for 3-15 tokens and attention, tcgen05 for prefill chunks); f32 accumulate",
+                "ms_per_step": round(ms / args.steps, 4), "higher_is_better": True, "scaling": "weak" if (args.replicas or sharded or world == 1) else "strong", "vs_baseline": None, "dtype": "int8 (dp4a: decoded weights x int8-split activations) at batch 1, f16 tensor cores (mma.sync with f16 hi/lo activations from 2 tokens on and for attention, tcgen05 for prefill chunks); f32 accumulate",
                 "data": "synthetic", "config": workload_config(B, world, args.replicas, args.replicated_ep),
                 "e2e": {"value": round(e2e_v, 2), "unit": "tok/s", "h2d_bytes_per_step": 4 * B * mult, "d2h_bytes_per_step": 4 * B * cfg.vocab * mult, "ms_per_step": round(ms_e2e / args.steps, 4)},
                 "gpu_launches": int(stats.kernels_launched) * args.steps,
@@ -468,7 +468,7 @@ def run_ours(args):
         full.destroy()
         # greedy ids of sharded decoding against one GPU holding all experts (8 layers of the same shapes, 32 tokens).  The
         # single-GPU run steps every sequence in a state of the same batch size as a rank's share (here 1): the dense
-        # kernels are chosen by batch size (dp4a for 1-2 tokens, tensor cores above; attention splits by sequences per GPU),
+        # kernels are chosen by batch size (dp4a for one token, tensor cores above; attention splits by sequences per GPU),
         # and results are bit-identical only between runs that use the same ones.  What the flag checks is the exchange.
         cfg_s = full_cfg(pb, batch_room=64, n_layers=8)
         spec_s = synth.model_spec(cfg_s, SEED + 2)
