@@ -20,7 +20,7 @@
 #define PB_MAX_WINDOW 8   // draft windows of the reference are at most 8 tokens (src/spec.rs:185)
 #define PB_PREFILL_CHUNK 256   // prompt tokens per batched pass; prompts are cut on the absolute grid of this size (src/engine_qn.rs:34-38, 92-139)
 #define PB_WIN_SPLITS 4        // attention splits per (token, KV head) of a prefill chunk: three walk the packed positions, one the f32 ring
-#define PB_WIN_KEYS (4 * (PB_MAX_WINDOW + 1) + 1)   // graphs per (t <= 8, ckpt, all_logits), plus one for a full prefill chunk
+#define PB_WIN_KEYS (4 * (PB_MAX_WINDOW + 1) + 2)   // graphs per (t <= 8, ckpt, all_logits), plus two for a full prefill chunk: without and with logits
 static size_t conv_elems(const pb_cfg& c, int B) { return (size_t)B * c.conv_k * (2 * c.lin_nk * c.lin_dk + c.lin_nv * c.lin_dv); }
 static size_t ssm_elems(const pb_cfg& c, int B) { return (size_t)B * c.lin_nv * c.lin_dk * c.lin_dv; }
 
@@ -1170,7 +1170,7 @@ static int run_step(pb_state* s) {
 // recurrences (DeltaNet state, KV append + attention) run token by token.  Logits of all positions go to
 // s->logits [t][vocab] when all_logits, else only the last position's to row 0.  Model::forward_multi,
 // src/model/qwen4exp_gguf.rs:2365-2480.
-static int run_window(pb_state* s, int t, bool ckpt, bool all_logits) {
+static int run_window(pb_state* s, int t, bool ckpt, bool all_logits, bool logits) {
     pb_model* m = s->m; pb_ctx* ctx = m->ctx; const pb_cfg& c = m->cfg;
     struct Scope { pb_ctx* c; pb_state* s; Scope(pb_ctx* x, pb_state* y, int t, bool k) : c(x), s(y) { c->pdl_scope++; c->pdl_chain = false; s->win_t = t; s->win_ckpt = k; }
                    ~Scope() { c->pdl_scope--; c->pdl_chain = false; s->win_t = 0; s->win_ckpt = false; } } scope(ctx, s, t, ckpt);
@@ -1187,6 +1187,7 @@ static int run_window(pb_state* s, int t, bool ckpt, bool all_logits) {
             PB_TRY(run_moe(s, il, s->x, V(m, il, PB_R_FFN_NORM), t, s->x, c.d, 1));
         }
     }
+    if (!logits) return pb_launch_window_pos(ctx, s->pos, s->wpos, t, 1);   // a chunk that another one follows: nobody reads its logits
     pb_qmat* out = M(m, -1, PB_R_OUTPUT) ? M(m, -1, PB_R_OUTPUT) : embd;
     PbGemvQArgs a; memset(&a, 0, sizeof a);
     a.type = out->type; a.cols = c.d; a.nseg = 1; seg(a, 0, out, 0);
@@ -1198,23 +1199,23 @@ static int run_window(pb_state* s, int t, bool ckpt, bool all_logits) {
 
 // run_window as a CUDA graph per (t, ckpt, all_logits): eager the first time (kernel attributes), captured the
 // second, replayed afterwards -- a window is ~1500 launches, whose host cost would otherwise dominate.
-static int window_once(pb_state* s, int t, bool ckpt, bool all_logits) {
+static int window_once(pb_state* s, int t, bool ckpt, bool all_logits, bool logits = true) {
     pb_ctx* ctx = s->m->ctx;
     // graphs: windows of up to 8 tokens per (t, ckpt, all_logits), and the full prefill chunk; other lengths (the ragged
     // ends of a prompt) run eagerly
-    const int key = t <= PB_MAX_WINDOW ? t * 4 + (ckpt ? 2 : 0) + (all_logits ? 1 : 0) : (t == PB_PREFILL_CHUNK && !ckpt && !all_logits ? PB_WIN_KEYS - 1 : -1);
+    const int key = t <= PB_MAX_WINDOW ? t * 4 + (ckpt ? 2 : 0) + (all_logits ? 1 : 0) : (t == PB_PREFILL_CHUNK && !ckpt && !all_logits ? PB_WIN_KEYS - (logits ? 1 : 2) : -1);
     if (key < 0) {
-        PB_TRY(run_window(s, t, ckpt, all_logits));
+        PB_TRY(run_window(s, t, ckpt, all_logits, logits));
     } else if (s->win_graph[key]) {
         PB_CUDA(ctx, cudaGraphLaunch(s->win_graph[key], ctx->stream));
     } else if (s->win_runs[key] == 0) {
-        PB_TRY(run_window(s, t, ckpt, all_logits));
+        PB_TRY(run_window(s, t, ckpt, all_logits, logits));
         s->win_runs[key] = 1;
     } else {
         cudaGraph_t g = nullptr;
         PB_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         const uint64_t k0 = ctx->kernels_launched;
-        const int rc = run_window(s, t, ckpt, all_logits);
+        const int rc = run_window(s, t, ckpt, all_logits, logits);
         ctx->kernels_launched = k0;
         cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
         if (rc != PB_OK) { if (g) cudaGraphDestroy(g); return rc; }
@@ -1319,7 +1320,7 @@ int pb_forward(pb_state* s, const uint32_t* ids_host, int t, float* logits_host)
             n = t - j0 < to_grid ? t - j0 : (int)to_grid;
             for (int j = 0; j < n; j++) s->pin_u32[j] = ids_host[j0 + j];
             PB_CUDA(ctx, cudaMemcpyAsync(s->ids, s->pin_u32, (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
-            PB_TRY(window_once(s, n, false, false));
+            PB_TRY(window_once(s, n, false, false, j0 + n >= t));
             if (j0 + n < t) PB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));   // the pinned id buffer is reused
         }
         s->verify_t = 0;
