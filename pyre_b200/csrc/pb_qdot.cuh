@@ -182,9 +182,8 @@ template <> struct PbQDec<PB_T_IQ3S_N4> {
     static constexpr bool HAS_MIN = false, SCALE16 = false, AFFINE = true;
     // a = shared address of the quarter's first 16 bytes, hp = of the row's head (pb_repack.cu)
     __device__ static __forceinline__ void quarter(uint32_t a, uint32_t hp, int qt, PbQuarter& o) {
-        const uint2 hdr = pb_lds64(hp);
-        const float d = pb_h2f((uint16_t)(hdr.x & 0xFFFF));
-        const uint32_t sc = (hdr.y >> (8 * qt)) & 0xFF;
+        const float d = pb_h2f((uint16_t)pb_lds16(hp));
+        const uint32_t sc = pb_lds8(hp + 4 + qt);
         const float d8 = 0.125f * d, d0 = d8 * (float)(1 + 2 * (int)(sc & 0xF)), d1 = d8 * (float)(1 + 2 * (int)(sc >> 4));
         o.sc[0] = o.sc[1] = d0; o.sc[2] = o.sc[3] = d1;
 #pragma unroll
