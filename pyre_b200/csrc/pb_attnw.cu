@@ -15,6 +15,8 @@
 //   Warps: 8; warp = (16 rows m, half h).  Scores: half of the tile's positions; output: half of the 256 dims.  Q stays in registers.
 //   Memory: one f16 tile (high, low) serves K and then V; the raw bytes of the next operand arrive by asynchronous copies in a staging
 //   buffer meanwhile: V during the score products, the next K during the output products.
+//   What bounds it: the conversion of a tile to f16 parts and the mma, one after the other between barriers (8 us per tile of 64 x 64 rows; the mma
+//   alone would take 3).  256 tokens at position 3840: 313 us and 11 us for the merge; a CTA per token took 167 us for the merge alone.
 #include "pb_common.cuh"
 #include "pb_internal.h"
 

@@ -11,6 +11,7 @@
 // What bounds it: for a few entries per expert the weight stream, beyond that the decode (about two instructions per weight).  An earlier
 // form split the contraction over the warps and added the partial sums in shared memory behind a barrier per 32 rows: the barrier kept the issue slots
 // 44 % busy (143 / 77 us for gate-up / down at 32 tokens of the 2048 x 512 x 512-expert block, the dp4a kernels 132 / 105).
+// Now 512 experts of 2048 x 512: 67 / 38 us at 32 tokens, 134 / 76 at 128, 216 / 120 at 256 (the mean CTA; dp4a 132 / 105 at 32).
 // Replaces the reference's k_xgu* / k_xdown* (src/model/qn_cube.rs:3482-5419) for several tokens.
 #include "pb_hmma.cuh"
 #include "pb_internal.h"
