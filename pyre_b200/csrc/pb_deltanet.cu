@@ -54,8 +54,9 @@ __global__ void __launch_bounds__(DN_THREADS) pb_deltanet_kernel(const PbDeltaPa
 // The reference loops the tokens inside k_delta_m (src/model/qn_cube.rs:2839-2913).
 #define PB_DR_TB 8       // tokens per block of inputs
 
-// scratch rows of the run: normalized q | k per K head, conv'd v, {decay, beta} per V head, k.q per K head
-struct PbDeltaRun { float* qk; float* v; float2* gb; float* kq; };
+// scratch rows of the run: normalized q | k per K head, conv'd v, {decay, beta} per V head, k.q per K head; for runs in blocks of eight
+// tokens per block and K head the products k_t.k_s and q_t.k_s (s <= t, the rest zero)
+struct PbDeltaRun { float* qk; float* v; float2* gb; float* kq; float* gram; };
 
 // TB tokens per CTA: 8 for a chunk (the taps of neighbouring tokens are loaded once), 1 for a window, whose few tokens then spread over the GPU.
 // grid (token blocks, nk + nv), dk (q / k heads) or dv (v heads) threads at most 256 -- one channel (or one of q and one of k) per thread
@@ -68,6 +69,8 @@ __global__ void __launch_bounds__(256) pb_deltanet_inputs_kernel(const PbDeltaPa
     const bool isv = (int)blockIdx.y >= nk;
     const int head = isv ? (int)blockIdx.y - nk : (int)blockIdx.y;
     __shared__ float red[2][3][8];
+    constexpr int LD = 132;                                 // rows of a block's k and q, 4 banks apart
+    __shared__ __align__(16) float kqs[TB == 8 ? 2 : 1][TB == 8 ? 8 * LD : 1];
     const int n = isv ? dv : dk;
     const bool live = tid < n;
     const int c0 = isv ? 2 * nk * dk + head * dv + tid : head * dk + tid, c1 = nk * dk + head * dk + tid;   // q and k channel, or the v channel
@@ -126,8 +129,23 @@ __global__ void __launch_bounds__(256) pb_deltanet_inputs_kernel(const PbDeltaPa
             const float fq = 1.0f / sqrtf(tq + 1e-6f) * (1.0f / sqrtf((float)dk)), fk = 1.0f / sqrtf(tk + 1e-6f);
             float* dst = r.qk + ((size_t)j * nk + head) * 2 * dk;
             if (live) { dst[tid] = a * fq; dst[dk + tid] = b * fk; }
+            if (TB == 8 && r.gram) { kqs[0][i * LD + tid] = b * fk; kqs[1][i * LD + tid] = a * fq; }   // (dk = 128: every thread has a channel)
             if (tid == 0) r.kq[(size_t)j * nk + head] = td * fq * fk;
         }
+    }
+    if (TB == 8 && r.gram && !isv) {
+        __syncthreads();
+        const int which = tid >> 6, t = (tid >> 3) & 7, s = tid & 7;   // 128 threads: k_t.k_s and q_t.k_s
+        float d = 0.f;
+        if (s <= t && t0 + t < t1) {
+            float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int c = 0; c < 128; c += 4) {
+                const float4 x = *reinterpret_cast<const float4*>(&kqs[which][t * LD + c]), y = *reinterpret_cast<const float4*>(&kqs[0][s * LD + c]);
+                u.x = fmaf(x.x, y.x, u.x); u.y = fmaf(x.y, y.y, u.y); u.z = fmaf(x.z, y.z, u.z); u.w = fmaf(x.w, y.w, u.w);
+            }
+            d = (u.x + u.y) + (u.z + u.w);
+        }
+        r.gram[((size_t)blockIdx.x * nk + head) * 128 + tid] = d;
     }
 }
 
@@ -238,21 +256,186 @@ __global__ void __launch_bounds__(128) pb_deltanet_run_kernel(const PbDeltaParam
     }
 }
 
+// The same walk in blocks of eight tokens.  Inside a block only the eight corrections of a column depend on each other:
+//   g_t S_{t-1}^T k_t = G_t (S_0^T k_t) + sum_{s<t} (G_t / G_s) (k_s.k_t) delta_s,     G_t = g_0 .. g_t
+// so the sixteen products S_0^T k_t and S_0^T q_t of a block are formed from the state as the block found it, without waiting for one another,
+// then a triangular system of eight unknowns per column is solved by substitution, and the state takes its eight rank-one updates at once.  A
+// warp holds four columns, its lanes eight groups of sixteen rows x four columns; eight warps an SM.  What bounds it: issue slots (the token-by-token
+// walk is bound by the latency of one token).  1024 tokens of 32 heads of 128 x 128: 344 us token by token, 238 in blocks (four warps of eight
+// columns each: 245).  A token's values never enter an earlier token's: the sums run over s < t only.
+#define DB_C 8               // tokens of a block
+__global__ void __launch_bounds__(256) pb_deltanet_block_kernel(const PbDeltaParams p, int T, const PbDeltaRun r) {
+    constexpr int DK = 128, C = DB_C, NT = 256;
+    const int nk = p.nk, nv = p.nv, dv = p.dv;
+    const int splits = dv / DN_COLS, h = blockIdx.x / splits, j0 = (blockIdx.x % splits) * DN_COLS, kh = h % nk;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = lane >> 2, col = lane & 3;
+    struct __align__(16) In { float qk[C][2 * DK]; float v[C][DN_COLS]; float gram[2 * C * C]; float2 gb[C]; };
+    __shared__ In in[2];
+    __shared__ __align__(16) float mat[2][C][C], dec[2][C];            // decayed products (k.k, q.k); G_t and G_7 / G_s
+    __shared__ __align__(16) float ab[8][2][4][C], del[8][C][4];       // per warp: S^T k and S^T q of its columns, corrections
+    pb_pdl_wait();
+    pb_pdl_trigger();
+    auto fetch = [&](int t0, int buf) {
+        const int n = min(C, T - t0);
+        constexpr int PQ = 2 * DK / 4, PV = DN_COLS / 4;
+        In& d = in[buf];
+        for (int i = tid; i < C * (PQ + PV); i += NT) {
+            const int t = i / (PQ + PV), c = i - t * (PQ + PV);
+            float* dst = c < PQ ? &d.qk[t][4 * c] : &d.v[t][4 * (c - PQ)];
+            if (t < n) {
+                const float* src = c < PQ ? r.qk + ((size_t)(t0 + t) * nk + kh) * 2 * DK + 4 * c : r.v + (size_t)(t0 + t) * nv * dv + h * dv + j0 + 4 * (c - PQ);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(pb_smem_u32(dst)), "l"(src) : "memory");
+            } else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (tid >= NT - 2 * C * C / 4) { const int i = tid - (NT - 2 * C * C / 4); asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(pb_smem_u32(&d.gram[4 * i])), "l"(r.gram + ((size_t)(t0 / C) * nk + kh) * (2 * C * C) + 4 * i) : "memory"); }
+        else if (tid >= NT - 2 * C * C / 4 - C) {
+            const int t = tid - (NT - 2 * C * C / 4 - C);
+            if (t < n) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(pb_smem_u32(&d.gb[t])), "l"(r.gb + (size_t)(t0 + t) * nv + h) : "memory");
+            else d.gb[t] = make_float2(1.f, 0.f);       // past the run: no decay, no correction
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0, 0);
+    // the lane's rows 32 j + 4 rg + {0..3}, j = 0..3, of its column, as pairs of rows
+    float* S = p.ssm + ((size_t)h * DK) * dv + j0 + 4 * warp + col;
+    unsigned long long s[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int row = 32 * (i >> 1) + 4 * rg + 2 * (i & 1);
+        s[i] = pb_f2(S[(size_t)row * dv], S[(size_t)(row + 1) * dv]);
+    }
+    int buf = 0;
+    for (int t0 = 0; t0 < T; t0 += C, buf ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                    // this block's inputs have landed; the other buffer and the tables are free
+        if (t0 + C < T) fetch(t0 + C, buf ^ 1);
+        const In& d = in[buf];
+        const int n = min(C, T - t0);
+        if (tid < 2 * C * C) {   // thread (t, which, s): the product decayed from s to t; then G_t and G_7 / G_s
+            const int t = tid >> 4, which = (tid >> 3) & 1, q = tid & 7;
+            float f = 1.f;
+#pragma unroll
+            for (int i = 1; i < C; i++) if (i > q && i <= t) f *= d.gb[i].x;
+            mat[which][t][q] = f * d.gram[which * C * C + t * C + q];   // (the entries that are read: s < t, or s <= t for q.k)
+        } else if (tid < 2 * C * C + 2 * C) {
+            const int which = (tid >> 3) & 1, q = tid & 7;
+            float e = 1.f;
+#pragma unroll
+            for (int i = 0; i < C; i++) if (which == 0 ? i <= q : i > q) e *= d.gb[i].x;
+            dec[which][q] = e;
+        }
+        // S_0^T k_t and S_0^T q_t of the lane's rows, all of the block before anything is summed over the lanes
+        float v[2][C];
+#pragma unroll
+        for (int t = 0; t < C; t++) {
+            unsigned long long a[2] = {0ull, 0ull}, b[2] = {0ull, 0ull};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(&d.qk[t][32 * j + 4 * rg]), k = *reinterpret_cast<const ulonglong2*>(&d.qk[t][DK + 32 * j + 4 * rg]);
+                a[0] = j ? pb_fma2(s[2 * j], k.x, a[0]) : pb_mul2(s[0], k.x); a[1] = j ? pb_fma2(s[2 * j + 1], k.y, a[1]) : pb_mul2(s[1], k.y);
+                b[0] = j ? pb_fma2(s[2 * j], q.x, b[0]) : pb_mul2(s[0], q.x); b[1] = j ? pb_fma2(s[2 * j + 1], q.y, b[1]) : pb_mul2(s[1], q.y);
+            }
+            const float2 x = pb_f2_get(pb_add2(a[0], a[1])), y = pb_f2_get(pb_add2(b[0], b[1]));
+            v[0][t] = x.x + x.y; v[1][t] = y.x + y.y;
+        }
+        {   // sums over the eight row groups (lane bits 2 .. 4): bit 4 keeps k or q, bit 3 half of the tokens, bit 2 a quarter
+            const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+            float w[C], u[C / 2], z[C / 4];
+#pragma unroll
+            for (int t = 0; t < C; t++) w[t] = (b4 ? v[1][t] : v[0][t]) + __shfl_xor_sync(0xffffffffu, b4 ? v[0][t] : v[1][t], 16);
+#pragma unroll
+            for (int t = 0; t < C / 2; t++) u[t] = (b3 ? w[t + 4] : w[t]) + __shfl_xor_sync(0xffffffffu, b3 ? w[t] : w[t + 4], 8);
+#pragma unroll
+            for (int t = 0; t < C / 4; t++) z[t] = (b2 ? u[t + 2] : u[t]) + __shfl_xor_sync(0xffffffffu, b2 ? u[t] : u[t + 2], 4);
+            *reinterpret_cast<float2*>(&ab[warp][lane >> 4][col][(b3 ? 4 : 0) + (b2 ? 2 : 0)]) = make_float2(z[0], z[1]);
+        }
+        __syncthreads();                                    // the tables are complete (and the warp's sums)
+        // corrections of the lane's column, all of them by each of the column's eight lanes: delta_t = (v_t - g_t mem_t) beta_t (:1663); a correction
+        // is taken out of the later tokens as soon as it is known
+        float de[C], m[C][C];
+        {
+            const float4 x = *reinterpret_cast<const float4*>(&ab[warp][0][col][0]), y = *reinterpret_cast<const float4*>(&ab[warp][0][col][4]);
+            const float4 g = *reinterpret_cast<const float4*>(&dec[0][0]), e = *reinterpret_cast<const float4*>(&dec[0][4]);
+            const float av[C] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w}, gv[C] = {g.x, g.y, g.z, g.w, e.x, e.y, e.z, e.w};
+#pragma unroll
+            for (int t = 0; t < C; t++) {
+                if (t > 0) { const float4 o = *reinterpret_cast<const float4*>(&mat[0][t][0]); m[t][0] = o.x; m[t][1] = o.y; m[t][2] = o.z; m[t][3] = o.w; }
+                if (t > 4) { const float4 o = *reinterpret_cast<const float4*>(&mat[0][t][4]); m[t][4] = o.x; m[t][5] = o.y; m[t][6] = o.z; m[t][7] = o.w; }
+                de[t] = fmaf(-gv[t], av[t], d.v[t][4 * warp + col]);
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < C; t++) {
+            de[t] = t < n ? de[t] * d.gb[t].y : 0.f;
+#pragma unroll
+            for (int q = t + 1; q < C; q++) de[q] = fmaf(-m[q][t], de[t], de[q]);
+        }
+        {   // each of the column's lanes forms one of the outputs: token rg
+            const float4 x = *reinterpret_cast<const float4*>(&mat[1][rg][0]), y = *reinterpret_cast<const float4*>(&mat[1][rg][4]);
+            const float w[C] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+            float o = dec[0][rg] * ab[warp][1][col][rg], own = de[0];
+#pragma unroll
+            for (int q = 0; q < C; q++) { if (q <= rg) o = fmaf(w[q], de[q], o); if (q == rg) own = de[q]; }
+            if (rg < n) p.out[(size_t)(t0 + rg) * p.ldo + h * dv + j0 + 4 * warp + col] = o;   // readout before the gated norm
+            del[warp][rg][col] = own * dec[1][rg];
+        }
+        __syncwarp();
+        const float g = dec[0][C - 1];
+        const unsigned long long g2 = pb_f2(g, g);
+#pragma unroll
+        for (int i = 0; i < 8; i++) s[i] = pb_mul2(s[i], g2);
+#pragma unroll
+        for (int t = 0; t < C; t++) {
+            const float e = del[warp][t][col];
+            const unsigned long long e2 = pb_f2(e, e);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(&d.qk[t][DK + 32 * j + 4 * rg]);
+                s[2 * j] = pb_fma2(k.x, e2, s[2 * j]); s[2 * j + 1] = pb_fma2(k.y, e2, s[2 * j + 1]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int row = 32 * (i >> 1) + 4 * rg + 2 * (i & 1);
+        const float2 a = pb_f2_get(s[i]);
+        S[(size_t)row * dv] = a.x; S[(size_t)(row + 1) * dv] = a.y;
+    }
+    // the conv ring keeps the last K inputs.  Channels: this slice's v columns; q and k of a K head by the first slice of the first V head that reads it
+    constexpr int K = 4;
+    const int ch = 2 * nk * DK + nv * dv;
+    const int64_t pos0 = p.pos[0];
+    const int nel = DN_COLS + (h == kh && j0 == 0 ? 2 * DK : 0);
+    for (int i = tid; i < nel; i += NT) {
+        const int c = i < DN_COLS ? 2 * nk * DK + h * dv + j0 + i : (i - DN_COLS < DK ? kh * DK + i - DN_COLS : nk * DK + kh * DK + i - DN_COLS - DK);
+        for (int j = max(0, T - K); j < T; j++) p.conv[(size_t)((pos0 + j) % K) * ch + c] = p.proj[(size_t)j * p.ldp + c];
+    }
+}
+
 // T consecutive tokens of sequence 0; false when the shape is outside what the kernels are built for
 bool pb_deltanet_seq_supported(const PbDeltaParams& p) { return p.conv_k == 4 && p.dv % DN_COLS == 0 && p.dv <= 256 && (p.dk == 128 || p.dk == 64 || p.dk == 32); }
-size_t pb_deltanet_seq_scratch(const PbDeltaParams& p, int T) { return (size_t)T * (2 * p.nk * p.dk + p.nv * p.dv + 2 * p.nv + p.nk) + 16; }   // floats
+size_t pb_deltanet_seq_scratch(const PbDeltaParams& p, int T) { return (size_t)T * (2 * p.nk * p.dk + p.nv * p.dv + 2 * p.nv + p.nk) + (size_t)((T + 7) / 8) * p.nk * 128 + 16; }   // floats
 int pb_launch_deltanet_seq(pb_ctx* ctx, const PbDeltaParams& p, int T, float* scratch, const PbDeltaCk* ckp) {
     if (!pb_deltanet_seq_supported(p)) PB_FAIL(ctx, PB_UNSUPPORTED, "deltanet run: dk=%d dv=%d conv_k=%d not supported", p.dk, p.dv, p.conv_k);
     PbDeltaCk ck; memset(&ck, 0, sizeof ck);
     if (ckp) ck = *ckp;
     PbDeltaRun r;
     r.qk = scratch; r.v = r.qk + (size_t)T * 2 * p.nk * p.dk; r.gb = reinterpret_cast<float2*>(r.v + (size_t)T * p.nv * p.dv); r.kq = reinterpret_cast<float*>(r.gb + (size_t)T * p.nv);
+    // blocks of eight tokens from two full blocks on, for the one head size they are built for; verify windows need the state after every token
+    const bool blocks = !ckp && T >= 16 && p.dk == 128 && p.dv <= 128;
+    r.gram = blocks ? reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(r.kq + (size_t)T * p.nk) + 15) & ~(uintptr_t)15) : nullptr;
     const int wide = p.dk > p.dv ? p.dk : p.dv;
-    if (T >= 32) pb_launch_k(ctx, pb_deltanet_inputs_kernel<8>, dim3((T + 7) / 8, p.nk + p.nv), dim3((wide + 31) & ~31), (size_t)0, p, T, r);
+    if (T >= 32 || blocks) pb_launch_k(ctx, pb_deltanet_inputs_kernel<8>, dim3((T + 7) / 8, p.nk + p.nv), dim3((wide + 31) & ~31), (size_t)0, p, T, r);
     else pb_launch_k(ctx, pb_deltanet_inputs_kernel<1>, dim3(T, p.nk + p.nv), dim3((wide + 31) & ~31), (size_t)0, p, T, r);
     ctx->kernels_launched++;
     PB_CUDA(ctx, cudaGetLastError());
     const dim3 grid(p.nv * (p.dv / DN_COLS));
+    if (blocks) {
+        pb_launch_k(ctx, pb_deltanet_block_kernel, grid, dim3(256), (size_t)0, p, T, r);
+        ctx->kernels_launched++;
+        PB_CUDA(ctx, cudaGetLastError());
+        return PB_OK;
+    }
 #define GO(DK) { if (ckp) pb_launch_k(ctx, pb_deltanet_run_kernel<DK, true>, grid, dim3(128), (size_t)0, p, T, r, ck); else pb_launch_k(ctx, pb_deltanet_run_kernel<DK, false>, grid, dim3(128), (size_t)0, p, T, r, ck); }
     if (p.dk == 128) GO(128) else if (p.dk == 64) GO(64) else GO(32)
 #undef GO

@@ -1,0 +1,29 @@
+"""Prompt passes and the kernels that only they and large batches reach: runs of the DeltaNet recurrence in blocks of eight tokens, the router as a GEMM,
+several prompt chunks in one pass, expert groups of up to 24 entries."""
+import numpy as np
+import pytest
+
+import pyre_b200 as pb
+from pyre_b200 import synth
+from conftest import rel_err
+from helpers import oracle_cfg, oracle_model, small_cfg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [16, 23, 24])
+def test_deltanet_blocks_of_tokens(ctx, n):
+    """Two full blocks, and a last block of seven tokens: the state that n single steps leave (below 32 tokens the projections' weights are exact;
+    two layers and the gates amplify the last bits of f32 sums)."""
+    cfg = small_cfg(pb, n_layers=2, full_every=0)
+    m = synth.build_model(ctx, cfg, synth.model_spec(cfg, 9), 9)
+    a, b = m.new_state(1), m.new_state(1)
+    ids = np.random.default_rng(n).integers(0, cfg.vocab, n).astype(np.uint32)
+    la = a.forward(ids)
+    for t in ids:
+        lb = b.forward(np.array([t], np.uint32))
+    assert rel_err(la, lb) < 1e-4
+    for (ca, sa), (cb, sb) in zip((a.get_lin(0), a.get_lin(1)), (b.get_lin(0), b.get_lin(1))):
+        assert rel_err(ca, cb) < 1e-4 and rel_err(sa, sb) < 1e-4
+    assert ctx.device_status() == 0
+    a.destroy(); b.destroy(); m.destroy()
