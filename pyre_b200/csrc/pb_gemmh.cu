@@ -1,4 +1,4 @@
-// Batched dequant-GEMM for 2 .. 16 activation columns a launch on the tensor cores, every quantized format (core: pb_hmma.cuh).  (Two columns of a
+// Batched dequant-GEMM for 2 .. 16 (small matrices 32) activation columns a launch on the tensor cores, every quantized format (core: pb_hmma.cuh).  (Two columns of a
 // small matrix in a format with a long decode stay on the dp4a kernel: pb_gemvq.cu.)
 //
 //   y[b][yoff_s + r] (+)= sum_c W_s[r][c] * act(x)[b][c]        b = 0 .. t-1
@@ -19,10 +19,12 @@
 #include "pb_internal.h"
 
 #include <stdio.h>
+#include <stdlib.h>
 
 #define GH_WARPS 16
 #define GH_MAXBLK 16         // blocks of 256 columns per row at most
-#define GH_HEAD (16 * GH_MAXBLK * 4)   // bytes in front of the tables: partial sums of squares [16 tokens][blocks]
+#define GH_MAXNT 8           // n-tiles of four tokens at most
+#define GH_HEAD (4 * GH_MAXNT * GH_MAXBLK * 4)   // bytes in front of the tables: partial sums of squares [tokens][blocks]
 
 struct PbGemmHParams {
     PbGemvQParams q;         // seg[].chunk0 = first 16-row tile of the segment, nchunks = tiles in all
@@ -92,7 +94,7 @@ __global__ void __launch_bounds__(GH_WARPS * 32, 1) pb_gemmh_kernel(const PbGemm
     open();
     for (int i = 0; i + 1 < h.stages; i++) issue();
     PbQTabs T = {0u, 0u, 0u};
-    if constexpr (pb_h_mode<FMT>() != PB_H_DIRECT) T = pb_fill_qtabs<FMT>(tab, p.rep, tid, (int)blockDim.x, lane);
+    if constexpr (pb_h_mode<FMT>() != PB_H_DIRECT) T = pb_h_fill_tabs<FMT>(tab, p.rep, tid, (int)blockDim.x, lane);
 
     // ---- activations: a block of a token per warp
     pb_pdl_wait();
@@ -201,11 +203,11 @@ template <int FMT>
 static bool gh_layout(pb_ctx* ctx, int cols, int t, int ks, int& nt, int& nw, PbGemmHParams& h, size_t& smem) {
     constexpr int rep = pb_tab_rep_max<FMT>();
     h.g = pb_h_geom<FMT>(cols);
-    for (nt = (t + 3) / 4 > 4 ? 4 : (t + 3) / 4; nt >= 1; nt--)
+    for (nt = t > 4 * GH_MAXNT ? GH_MAXNT : ((t + 3) / 4 > 4 ? ((t + 3) / 4 + 1) & ~1 : (t + 3) / 4); nt >= 1; nt -= nt > 4 ? 2 : 1)   // (forms are built for 1, 2, 3, 4, 6 and 8)
         for (nw = GH_WARPS; nw >= 8; nw /= 2)
             for (h.stages = 3; h.stages >= 2; h.stages--)
                 for (h.q.rep = rep > 8 ? 8 : rep; h.q.rep >= 1; h.q.rep /= 2) {   // copies of the codebook: as many as fit
-                    const uint32_t tabb = pb_h_mode<FMT>() == PB_H_DIRECT ? 0u : pb_tab_bytes<FMT>(h.q.rep);
+                    const uint32_t tabb = pb_h_tab_bytes<FMT>(h.q.rep);
                     h.off_act = GH_HEAD + ((tabb + 127) & ~127u);
                     h.off_red = h.off_act + (uint32_t)(4 * nt) * (uint32_t)pb_h_tok_bytes<FMT>(cols / ks);
                     h.off_stage = h.off_red + (uint32_t)nw * 4 * nt * 16 * 4;
@@ -223,14 +225,20 @@ static int launch_fmt(pb_ctx* ctx, const PbGemvQArgs& a, bool recoded) {
     for (int s = 0; s < a.nseg; s++) all += (int)((a.seg[s].rows + 15) / 16);
     // CTAs of a cluster: 1024 columns each above 2048; half a row each where a CTA has at most a round of tiles and the activations of several
     // tokens would take as long to prepare as the product
-    const int ks = a.cols > 2048 ? a.cols / 1024 : (a.cols == 2048 && all <= 16 * ctx->sm_count && a.t > 4 ? 2 : 1);
+    const int ks16 = a.cols > 2048 ? a.cols / 1024 : (a.cols == 2048 && all <= 16 * ctx->sm_count && a.t > 4 ? 2 : 1);
+    // More than 16 tokens in one launch: 512 columns per CTA (32 tokens' activations fit beside the weights), worth it where every CTA of a cluster has at
+    // most one round of tiles; with more, the exchange of the parts' sums in every round costs more than the second launch (us for 24 tokens of IQ3_S, two
+    // launches / one: 2048 x 512 15.5 / 10.4, 4096 x 2048 22.7 / 16.5, 2048 x 4096 23.5 / 16.5, 12351 x 2048 31 / 28, 151936 x 2048 138 / 221).
+    const int ks32 = a.cols > 512 ? a.cols / 512 : 1;
+    const int most = all <= 16 * (ctx->sm_count / ks32) ? 4 * GH_MAXNT : 16;
     for (int t0 = 0, n = 0; t0 < a.t; t0 += n) {
         PbGemmHParams h;
         memset(&h, 0, sizeof h);
-        h.ks = ks;
         int nt, nw; size_t smem;
-        if (!gh_layout<FMT>(ctx, a.cols, a.t - t0, ks, nt, nw, h, smem)) PB_FAIL(ctx, PB_UNSUPPORTED, "gemm: %d columns do not fit shared memory", a.cols);
-        n = a.t - t0 < 4 * nt ? a.t - t0 : 4 * nt;
+        const int r = a.t - t0 < most ? a.t - t0 : most, ks = r > 16 ? ks32 : ks16;
+        h.ks = ks;
+        if (!gh_layout<FMT>(ctx, a.cols, r, ks, nt, nw, h, smem)) PB_FAIL(ctx, PB_UNSUPPORTED, "gemm: %d columns do not fit shared memory", a.cols);
+        n = r < 4 * nt ? r : 4 * nt;
         PbGemvQParams& p = h.q;
         p.row_bytes = a.cols / el * bs; p.bpr = a.cols / 256; p.nseg = a.nseg;
         p.x = a.x + (int64_t)t0 * a.ldx; p.ldx = a.ldx; p.t = n; p.y = a.y + (int64_t)t0 * a.ldy; p.ldy = a.ldy; p.status = ctx->dev_status;
@@ -243,7 +251,7 @@ static int launch_fmt(pb_ctx* ctx, const PbGemvQArgs& a, bool recoded) {
         p.nchunks = ntiles;
         if (ntiles == 0) return PB_OK;
 #define GO(N) { auto kern = pb_gemmh_kernel<FMT, N>; PB_TRY(pb_ensure_smem(ctx, kern, smem)); const int ncl = pb_max_clusters(ctx, reinterpret_cast<const void*>(kern), nw * 32, smem, ks), grid = (ntiles < ncl ? ntiles : ncl) * ks; pb_launch_kc(ctx, kern, dim3(grid), dim3(nw * 32), smem, ks, h); }
-        if (nt == 1) GO(1) else if (nt == 2) GO(2) else if (nt == 3) GO(3) else GO(4)
+        if (nt == 1) GO(1) else if (nt == 2) GO(2) else if (nt == 3) GO(3) else if (nt == 4) GO(4) else if (nt == 6) GO(6) else GO(8)
 #undef GO
         ctx->kernels_launched++;
         PB_CUDA(ctx, cudaGetLastError());
@@ -251,6 +259,10 @@ static int launch_fmt(pb_ctx* ctx, const PbGemvQArgs& a, bool recoded) {
     return PB_OK;
 }
 
+int pb_gemmh_piece(int type, int cols) {
+    static const bool use_mma = !(getenv("PYRE_B200_MMA") && atoi(getenv("PYRE_B200_MMA")) == 0);
+    return use_mma && pb_gemvq_supported(type, cols) ? 32 : 16;
+}
 bool pb_gemmh_supported(int type, int cols, int t) { return t >= 2 && pb_gemvq_supported(type, cols); }
 
 int pb_launch_gemmh(pb_ctx* ctx, const PbGemvQArgs& a) {

@@ -101,42 +101,50 @@ template <> struct PbHRaw<PB_T_Q4_K> {
         h = pb_ldsa128(p); c0 = pb_ldsa128(p + 16 + 32 * q); c1 = pb_ldsa128(p + 32 + 32 * q);
     }
 };
-// decoder over the raw registers: word u -> four f16 pairs
+// decoder over the raw registers: word u -> four f16 pairs.  A nibble left where it lies in its 16-bit half is a subnormal f16, c 2^-24 or
+// c 2^-20: one mask and one fused multiply-add give 2^-14 times the integer weight, exactly (every product and sum is a multiple of 2^-14 below
+// 2^-4, and every weight that is not zero a normal number); the block's factor takes the 2^14 back.  Nine instructions for eight weights; with the
+// nibble in the mantissa of 1024 or 64 and the offset subtracted first it was thirteen (2 tokens x 151936 rows of IQ3_S 47 us, 41 so;
+// Q4_K 70 and 66).
+#define PB_H_UNIT 16384.0f
 template <int FMT> struct PbHDec;
 template <> struct PbHDec<PB_T_IQ3S_N4> {
-    __half2 m2[2], m15[2];   // 2 m and -15 m of the quarter's two groups
+    __half2 lo[2], hi[2], off[2];   // m 2^11, m 2^7 and -15 m 2^-14 of the quarter's two groups, m = 1 + 2 s <= 31
     __device__ __forceinline__ void head(const PbHRaw<PB_T_IQ3S_N4>& r, int q) {
         const uint32_t sc = r.h.y >> (8 * q);
-        const __half2 s0 = pb_h2_int(sc & 0xF), s1 = pb_h2_int((sc >> 4) & 0xF);      // multiplier m = 1 + 2 s <= 31
-        const __half2 k4 = pb_as_h2(0x44004400u), k2 = pb_as_h2(0x40004000u), km30 = pb_as_h2(0xCF80CF80u), km15 = pb_as_h2(0xCB80CB80u);   // 4, 2, -30, -15
-        m2[0] = __hfma2(s0, k4, k2); m15[0] = __hfma2(s0, km30, km15);
-        m2[1] = __hfma2(s1, k4, k2); m15[1] = __hfma2(s1, km30, km15);
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const __half2 s = pb_h2_int((sc >> (4 * i)) & 0xF);
+            lo[i] = __hfma2(s, pb_as_h2(0x6C006C00u), pb_as_h2(0x68006800u));     // 4096 s + 2048
+            hi[i] = __hfma2(s, pb_as_h2(0x5C005C00u), pb_as_h2(0x58005800u));     // 256 s + 128
+            off[i] = __hfma2(s, pb_as_h2(0x97809780u), pb_as_h2(0x93809380u));    // -30 2^-14 s - 15 2^-14
+        }
     }
     __device__ static __forceinline__ float d(const PbHRaw<PB_T_IQ3S_N4>& r) { return pb_h2f((uint16_t)(r.h.x & 0xFFFF)); }
     __device__ static __forceinline__ float dmin(const PbHRaw<PB_T_IQ3S_N4>&) { return 0.f; }
     __device__ static __forceinline__ uint32_t offs(const PbHRaw<PB_T_IQ3S_N4>&, int) { return 0u; }
     __device__ __forceinline__ uint32_t centre() const { return 0u; }
-    // (2 c - 15) m: the code sits in the mantissa of an f16 with exponent 1024 (low nibbles) or 64 (high nibbles); both steps are exact
+    // (2 c - 15) m
     __device__ __forceinline__ void word(const PbHRaw<PB_T_IQ3S_N4>& r, int u, uint32_t (&o)[4]) const {
         const uint4& c = u < 4 ? r.c0 : r.c1;
         const uint32_t w = (u & 3) == 0 ? c.x : ((u & 3) == 1 ? c.y : ((u & 3) == 2 ? c.z : c.w)), w8 = w >> 8;
-        const __half2 k1024 = pb_as_h2(0x64006400u), k64 = pb_as_h2(0x54005400u), a = m2[u >> 2], b = m15[u >> 2];
-        o[0] = pb_as_u32(__hfma2(__hsub2(pb_as_h2(pb_and_or(w, 0x000F000Fu, 0x64006400u)), k1024), a, b));
-        o[1] = pb_as_u32(__hfma2(__hsub2(pb_as_h2(pb_and_or(w, 0x00F000F0u, 0x54005400u)), k64), a, b));
-        o[2] = pb_as_u32(__hfma2(__hsub2(pb_as_h2(pb_and_or(w8, 0x000F000Fu, 0x64006400u)), k1024), a, b));
-        o[3] = pb_as_u32(__hfma2(__hsub2(pb_as_h2(pb_and_or(w8, 0x00F000F0u, 0x54005400u)), k64), a, b));
+        o[0] = pb_as_u32(__hfma2(pb_as_h2(w & 0x000F000Fu), lo[u >> 2], off[u >> 2]));
+        o[1] = pb_as_u32(__hfma2(pb_as_h2(w & 0x00F000F0u), hi[u >> 2], off[u >> 2]));
+        o[2] = pb_as_u32(__hfma2(pb_as_h2(w8 & 0x000F000Fu), lo[u >> 2], off[u >> 2]));
+        o[3] = pb_as_u32(__hfma2(pb_as_h2(w8 & 0x00F000F0u), hi[u >> 2], off[u >> 2]));
     }
 };
 template <> struct PbHDec<PB_T_Q4_K> {
-    __half2 s[2], sk[2];     // scale of the two groups, -72 scale
+    __half2 lo, hi, off[2];  // 2^10 scale of the first group (low nibbles), 2^6 scale of the second (high nibbles), -8 2^-14 scale of each
     // scale_min_k4 (gguf_q.rs:62-64) of groups 2 q and 2 q + 1: both groups' values in bytes 0 and 1
     __device__ static __forceinline__ uint32_t scales(const uint4& h, int q) {
         return q < 2 ? (h.y >> (16 * q)) & 0x3F3Fu : ((h.w >> (16 * (q - 2))) & 0x0F0Fu) | (((h.y >> (16 * (q - 2))) & 0xC0C0u) >> 2);
     }
     __device__ __forceinline__ void head(const PbHRaw<PB_T_Q4_K>& r, int q) {
         const uint32_t s2 = scales(r.h, q);
-        s[0] = pb_h2_int(s2 & 0xFF); s[1] = pb_h2_int((s2 >> 8) & 0xFF);
-        sk[0] = __hmul2(s[0], pb_as_h2(0xD480D480u)); sk[1] = __hmul2(s[1], pb_as_h2(0xD480D480u));   // exact: 9 x 6 bits
+        const __half2 s0 = pb_h2_int(s2 & 0xFF), s1 = pb_h2_int((s2 >> 8) & 0xFF), k8 = pb_as_h2(0x90009000u);   // k8 = -8 2^-14
+        lo = __hmul2(s0, pb_as_h2(0x64006400u)); hi = __hmul2(s1, pb_as_h2(0x54005400u));
+        off[0] = __hmul2(s0, k8); off[1] = __hmul2(s1, k8);
     }
     __device__ static __forceinline__ float d(const PbHRaw<PB_T_Q4_K>& r) { return pb_h2f((uint16_t)(r.h.x & 0xFFFF)); }
     __device__ static __forceinline__ float dmin(const PbHRaw<PB_T_Q4_K>& r) { return pb_h2f((uint16_t)(r.h.x >> 16)); }
@@ -146,16 +154,16 @@ template <> struct PbHDec<PB_T_Q4_K> {
         return pb_as_u32(__hsub2(pb_as_h2((m2 & 0xFF) | ((m2 & 0xFF00) << 8) | 0x64006400u), pb_as_h2(0x64006400u)));
     }
     // f16 pair of 8 x scale of the two groups
-    __device__ __forceinline__ uint32_t centre() const { return pb_as_u32(__hmul2(__halves2half2(__low2half(s[0]), __low2half(s[1])), pb_as_h2(0x48004800u))); }
-    // (q - 8) scale = (64 + q) s - 72 s, exact: codes around zero, so that activations with a mean do not make large sums that the minima then cancel;
-    // the 8 scale comes back with the minima
+    __device__ __forceinline__ uint32_t centre() const { return pb_as_u32(__hmul2(__halves2half2(__low2half(off[0]), __low2half(off[1])), pb_as_h2(0xF400F400u))); }   // off times -2^14
+    // (q - 8) scale: codes around zero, so that activations with a mean do not make large sums that the minima then cancel; the 8 scale comes back
+    // with the minima
     __device__ __forceinline__ void word(const PbHRaw<PB_T_Q4_K>& r, int u, uint32_t (&o)[4]) const {
         const uint4& c = u < 4 ? r.c0 : r.c1;
-        const uint32_t w = (u & 3) == 0 ? c.x : ((u & 3) == 1 ? c.y : ((u & 3) == 2 ? c.z : c.w));
-        o[0] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w << 4, 0x00F000F0u, 0x54005400u)), s[0], sk[0]));
-        o[1] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w >> 4, 0x00F000F0u, 0x54005400u)), s[0], sk[0]));
-        o[2] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w, 0x00F000F0u, 0x54005400u)), s[1], sk[1]));
-        o[3] = pb_as_u32(__hfma2(pb_as_h2(pb_and_or(w >> 8, 0x00F000F0u, 0x54005400u)), s[1], sk[1]));
+        const uint32_t w = (u & 3) == 0 ? c.x : ((u & 3) == 1 ? c.y : ((u & 3) == 2 ? c.z : c.w)), w8 = w >> 8;
+        o[0] = pb_as_u32(__hfma2(pb_as_h2(w & 0x000F000Fu), lo, off[0]));
+        o[1] = pb_as_u32(__hfma2(pb_as_h2(w8 & 0x000F000Fu), lo, off[0]));
+        o[2] = pb_as_u32(__hfma2(pb_as_h2(w & 0x00F000F0u), hi, off[1]));
+        o[3] = pb_as_u32(__hfma2(pb_as_h2(w8 & 0x00F000F0u), hi, off[1]));
     }
 };
 
@@ -170,11 +178,10 @@ __device__ __forceinline__ uint32_t pb_h_sums_off(int bpr) { return (uint32_t)bp
 template <int FMT> __device__ __forceinline__ int pb_h_c0(int lane) { return 64 * (lane & 3) + (pb_h_twin<FMT>() ? 4 : 8) * (lane >> 2); }
 template <int FMT> __device__ __forceinline__ int pb_h_c1(int lane) { return pb_h_c0<FMT>(lane) + (pb_h_twin<FMT>() ? 32 : 4); }
 
-// One warp stores block blk of a token: v = the lane's eight activations (columns c0 .., c1 ..).
+// A warp's block of a token, eight activations a lane (columns c0 .., c1 ..), times the power of two that puts the block's largest into [2^9, 2^10): f16
+// high and low parts as pairs (0 2)(4 6)(1 3)(5 7), or (0 2)(1 3) of each group.  x is scaled in place; the result is the inverse of the power.
 template <int FMT>
-__device__ __forceinline__ void pb_h_put(uint8_t* slot, int bpr, int blk, int lane, const float (&x)[8]) {
-    const int q = lane & 3, u = lane >> 2;
-    constexpr bool twin = pb_h_twin<FMT>();
+__device__ __forceinline__ float pb_h_split(float (&x)[8], uint32_t (&hi)[4], uint32_t (&lo)[4]) {
     float m = fmaxf(fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3]))), fmaxf(fmaxf(fabsf(x[4]), fabsf(x[5])), fmaxf(fabsf(x[6]), fabsf(x[7]))));
     m = pb_warp_max(m);
     float p = 1.0f, ip = 1.0f;
@@ -182,18 +189,28 @@ __device__ __forceinline__ void pb_h_put(uint8_t* slot, int bpr, int blk, int la
         const int e = (int)((__float_as_uint(m) >> 23) & 0xFF) - 127;
         p = __uint_as_float((uint32_t)(9 - e + 127) << 23); ip = __uint_as_float((uint32_t)(e - 9 + 127) << 23);
     }
-    if (lane == 0) *reinterpret_cast<float*>(slot + pb_h_scale_off(bpr) + 4 * blk) = ip;
+#pragma unroll
+    for (int i = 0; i < 8; i++) x[i] *= p;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int e0 = pb_h_twin<FMT>() ? (k < 2 ? k : k + 2) : (k < 2 ? 4 * k : 4 * (k - 2) + 1);
+        const __half2 h = __floats2half2_rn(x[e0], x[e0 + 2]);
+        const float2 r = __half22float2(h);
+        hi[k] = pb_as_u32(h); lo[k] = pb_as_u32(__floats2half2_rn(x[e0] - r.x, x[e0 + 2] - r.y));
+    }
+    return ip;
+}
+// One warp stores block blk of a token: x = the lane's eight activations.
+template <int FMT>
+__device__ __forceinline__ void pb_h_put(uint8_t* slot, int bpr, int blk, int lane, const float (&x)[8]) {
+    const int q = lane & 3, u = lane >> 2;
+    constexpr bool twin = pb_h_twin<FMT>();
     float v[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) v[i] = x[i] * p;
+    for (int i = 0; i < 8; i++) v[i] = x[i];
     uint32_t hi[4], lo[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {   // pairs (0 2)(4 6)(1 3)(5 7), or (0 2)(1 3) of each group
-        const int e0 = twin ? (k < 2 ? k : k + 2) : (k < 2 ? 4 * k : 4 * (k - 2) + 1);
-        const __half2 h = __floats2half2_rn(v[e0], v[e0 + 2]);
-        const float2 r = __half22float2(h);
-        hi[k] = pb_as_u32(h); lo[k] = pb_as_u32(__floats2half2_rn(v[e0] - r.x, v[e0 + 2] - r.y));
-    }
+    const float ip = pb_h_split<FMT>(v, hi, lo);
+    if (lane == 0) *reinterpret_cast<float*>(slot + pb_h_scale_off(bpr) + 4 * blk) = ip;
     uint8_t* row = slot + (size_t)blk * 1024 + u * 128 + q * 16;
     *reinterpret_cast<uint4*>(row) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     *reinterpret_cast<uint4*>(row + 64) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
@@ -244,20 +261,40 @@ __device__ __forceinline__ void pb_h_block_nib(uint32_t stage, const PbHGeom& h,
     else { ra.load(stage + (uint32_t)(g * h.pitch), g, q); rb.load(stage + (uint32_t)((g + 8) * h.pitch), g, q); }
     PbHDec<FMT> wa, wb;
     wa.head(ra, q); wb.head(rb, q);
-    float c[NT][4];
     float acc[NT][4];
 #pragma unroll
     for (int nt = 0; nt < NT; nt++) { acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f; }
+    if constexpr (NT <= 2) {
+        float c[NT][4];
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-        uint32_t a[4], b[4];
-        wa.word(ra, u, a); wb.word(rb, u, b);
+        for (int u = 0; u < 8; u++) {
+            uint32_t a[4], b[4];
+            wa.word(ra, u, a); wb.word(rb, u, b);
 #pragma unroll
-        for (int nt = 0; nt < NT; nt++) {
-            const uint4 x = pb_ldsa128(L.b + (uint32_t)nt * L.tok4 + (uint32_t)(blk * 1024 + u * 128));
-            if (u & 1) pb_hmma(c[nt], a[0], b[0], a[1], b[1], x.x, x.y); else pb_hmma0(c[nt], a[0], b[0], a[1], b[1], x.x, x.y);
-            pb_hmma(c[nt], a[2], b[2], a[3], b[3], x.z, x.w);
-            if (u & 1) pb_h_flush(acc[nt], c[nt]);
+            for (int nt = 0; nt < NT; nt++) {
+                const uint4 x = pb_ldsa128(L.b + (uint32_t)nt * L.tok4 + (uint32_t)(blk * 1024 + u * 128));
+                if (u & 1) pb_hmma(c[nt], a[0], b[0], a[1], b[1], x.x, x.y); else pb_hmma0(c[nt], a[0], b[0], a[1], b[1], x.x, x.y);
+                pb_hmma(c[nt], a[2], b[2], a[3], b[3], x.z, x.w);
+                if (u & 1) pb_h_flush(acc[nt], c[nt]);
+            }
+        }
+    } else {
+        // more n-tiles: both words of a chain are decoded first, so that one chain's accumulator is alive at a time
+#pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+            uint32_t a[2][4], b[2][4];
+            wa.word(ra, u, a[0]); wb.word(rb, u, b[0]); wa.word(ra, u + 1, a[1]); wb.word(rb, u + 1, b[1]);
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++) {
+                const uint32_t xa = L.b + (uint32_t)nt * L.tok4 + (uint32_t)(blk * 1024 + u * 128);
+                const uint4 x = pb_ldsa128(xa), y = pb_ldsa128(xa + 128);
+                float c[4];
+                pb_hmma0(c, a[0][0], b[0][0], a[0][1], b[0][1], x.x, x.y);
+                pb_hmma(c, a[0][2], b[0][2], a[0][3], b[0][3], x.z, x.w);
+                pb_hmma(c, a[1][0], b[1][0], a[1][1], b[1][1], y.x, y.y);
+                pb_hmma(c, a[1][2], b[1][2], a[1][3], b[1][3], y.z, y.w);
+                pb_h_flush(acc[nt], c);
+            }
         }
     }
     const float da = PbHDec<FMT>::d(ra), db = PbHDec<FMT>::d(rb);
@@ -275,7 +312,7 @@ __device__ __forceinline__ void pb_h_block_nib(uint32_t stage, const PbHGeom& h,
             pb_hmma0(cc, ca, cb, ca, cb, s.x, s.y);
             oa = da * cc[0] - PbHDec<FMT>::dmin(ra) * mc[0]; ob = db * cc[2] - PbHDec<FMT>::dmin(rb) * mc[2];
         }
-        pb_h_add<FMT, NT>(acc, nt, blk, da, db, oa, ob, L, tot);
+        pb_h_add<FMT, NT>(acc, nt, blk, da * PB_H_UNIT, db * PB_H_UNIT, oa, ob, L, tot);
     }
 }
 
@@ -293,6 +330,35 @@ template <> __device__ __forceinline__ void pb_h_mults<PB_T_IQ2_XS>(uint32_t p, 
 #pragma unroll
     for (int h = 0; h < 4; h++) m[h] = 1 + 2 * ((sc >> (4 * h)) & 0xF);
 }
+// Codebook of this core: as the dp4a kernels have it (pb_fill_qtabs), but for IQ2_XS, whose three magnitudes 8, 25, 43 fit a nibble each: one word of
+// eight byte selectors per entry, and the signs come from the index bits by arithmetic (pb_h_word_iq2xs).  With eight bytes per entry and the 16-byte rows of a
+// sign table the look-ups took two thirds of the shared-memory wavefronts (16 tokens x 151936 rows: 147 us, 129 so).
+template <int FMT> __host__ __device__ constexpr uint32_t pb_h_tab_bytes(int rep) { return pb_h_mode<FMT>() == PB_H_DIRECT ? 0u : (FMT == PB_T_IQ2_XS ? 512u * 4u * (uint32_t)rep : pb_tab_bytes<FMT>(rep)); }
+template <int FMT>
+__device__ __forceinline__ PbQTabs pb_h_fill_tabs(uint8_t* tab, int rep, int tid, int nthreads, int lane) {
+    if constexpr (FMT == PB_T_IQ2_XS) {
+        uint32_t* g = reinterpret_cast<uint32_t*>(tab);
+        for (int i = tid; i < 512 * rep; i += nthreads) {
+            const uint64_t e = PB_IQ2XS_GRID[i / rep];
+            uint32_t v = 0;
+            for (int j = 0; j < 8; j++) { const uint32_t b = (uint32_t)(e >> (8 * j)) & 0xFFu; v |= (b == 8u ? 0u : (b == 25u ? 1u : 2u)) << (4 * j); }
+            g[i] = v;
+        }
+        PbQTabs T = {0u, 0u, 0u};
+        T.stride = 4u * (uint32_t)rep; T.grid = pb_smem_u32(tab) + (uint32_t)(lane & (rep - 1)) * 4u;
+        return T;
+    } else return pb_fill_qtabs<FMT>(tab, rep, tid, nthreads, lane);
+}
+// Eight weights of an IQ2_XS index (9 bits of grid, 7 of signs, the eighth their parity) as f16 pairs (0 2)(4 6)(1 3)(5 7), times s; k = -1024 s
+__device__ __forceinline__ void pb_h_word_iq2xs(const PbQTabs& T, uint32_t q, __half2 s, __half2 k, uint32_t (&o)[4]) {
+    const uint32_t sel = pb_lds32(T.grid + (q & 511u) * T.stride);
+    const uint32_t s7 = q >> 9, s8 = s7 | ((uint32_t)(__popc(s7) & 1) << 7), z = s8 | (s8 << 14);   // sign bits i and i + 2 sixteen places apart (14 + 2)
+    const uint32_t g0 = pb_prmt(0x002B1908u, 0u, sel), g1 = pb_prmt(0x002B1908u, 0u, sel >> 16);      // magnitudes as bytes
+    o[0] = pb_as_u32(__hfma2(pb_as_h2(pb_prmt(g0, 0x64646464u, 0x4240u)), s, k)) ^ ((z << 15) & 0x80008000u);
+    o[1] = pb_as_u32(__hfma2(pb_as_h2(pb_prmt(g1, 0x64646464u, 0x4240u)), s, k)) ^ ((z << 11) & 0x80008000u);
+    o[2] = pb_as_u32(__hfma2(pb_as_h2(pb_prmt(g0, 0x64646464u, 0x4341u)), s, k)) ^ ((z << 14) & 0x80008000u);
+    o[3] = pb_as_u32(__hfma2(pb_as_h2(pb_prmt(g1, 0x64646464u, 0x4341u)), s, k)) ^ ((z << 10) & 0x80008000u);
+}
 // bytes (0, 2) or (1, 3) of a word of four signed bytes, already flipped to unsigned, as the mantissas of 1024 + 128 + v
 __device__ __forceinline__ uint32_t pb_h_bytes(uint32_t w, bool odd) { return pb_prmt(w, 0x64646464u, odd ? 0x4341u : 0x4240u); }
 
@@ -304,9 +370,34 @@ __device__ __forceinline__ void pb_h_block_int(uint32_t pa, uint32_t pb, const P
 #pragma unroll
     for (int nt = 0; nt < NT; nt++) { acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f; }
     PbQuarter wa, wb;
-    D::quarter(pa, q, T, wa); D::quarter(pb, q, T, wb);
+    if constexpr (FMT != PB_T_IQ2_XS) { D::quarter(pa, q, T, wa); D::quarter(pb, q, T, wb); }
     float fa, fb;                                              // f32 factor of the block's sum
-    if constexpr (pb_h_mode<FMT>() == PB_H_FOLD) {
+    if constexpr (FMT == PB_T_IQ2_XS) {
+        uint32_t ma[4], mb[4], qa[4], qb[4];                   // integer multipliers and index words
+        pb_h_mults<FMT>(pa, q, fa, ma); pb_h_mults<FMT>(pb, q, fb, mb);
+        pb_ld_u32x<4>(pa + 2 + 16 * q, qa); pb_ld_u32x<4>(pb + 2 + 16 * q, qb);
+#pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+            const __half2 sa = pb_h2_int(ma[u >> 1]), sb = pb_h2_int(mb[u >> 1]), k = pb_as_h2(0xE400E400u), ka = __hmul2(sa, k), kb = __hmul2(sb, k);   // -1024
+            uint32_t a[2][4], b[2][4];
+#pragma unroll
+            for (int v = 0; v < 2; v++) {
+                pb_h_word_iq2xs(T, (qa[u >> 1] >> (16 * v)) & 0xFFFFu, sa, ka, a[v]);
+                pb_h_word_iq2xs(T, (qb[u >> 1] >> (16 * v)) & 0xFFFFu, sb, kb, b[v]);
+            }
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++) {
+                const uint32_t xa = L.b + (uint32_t)nt * L.tok4 + (uint32_t)(blk * 1024 + u * 128);
+                const uint4 x = pb_ldsa128(xa), y = pb_ldsa128(xa + 128);
+                float c[4];
+                pb_hmma0(c, a[0][0], b[0][0], a[0][1], b[0][1], x.x, x.y);
+                pb_hmma(c, a[0][2], b[0][2], a[0][3], b[0][3], x.z, x.w);
+                pb_hmma(c, a[1][0], b[1][0], a[1][1], b[1][1], y.x, y.y);
+                pb_hmma(c, a[1][2], b[1][2], a[1][3], b[1][3], y.z, y.w);
+                pb_h_flush(acc[nt], c);
+            }
+        }
+    } else if constexpr (pb_h_mode<FMT>() == PB_H_FOLD) {
         uint32_t ma[4], mb[4];
         pb_h_mults<FMT>(pa, q, fa, ma); pb_h_mults<FMT>(pb, q, fb, mb);
         float c[NT][4];
