@@ -251,10 +251,10 @@ struct PbRouteParams {
     int* ent_tok; int* ent_slot; float* ent_w;
     int4* virt; int* n_virt;                  // several tokens: distinct local experts in groups of up to PB_VGROUP entries {expert, first entry, entries, cost of the groups before}, and their number
 };
-#define PB_VGROUP 8
-// Cost of a group of n entries in the expert kernels, in thirds of a group of up to four: five to eight entries take a second n-tile of mma and, as
-// fewer such groups share a phase, more preparation (measured: 1.3 of a small group)
-__host__ __device__ static inline int pb_vgroup_cost(int n) { return n <= 0 ? 0 : (n <= 4 ? 3 : 4); }
+#define PB_VGROUP 12
+// Cost of a group of n entries in the expert kernels, in sixths of a group of up to four: five to eight entries take a second n-tile of mma and, as
+// fewer such groups share a phase, more preparation (measured: 1.3 of a small group), nine to twelve a third
+__host__ __device__ static inline int pb_vgroup_cost(int n) { return n <= 0 ? 0 : (n <= 4 ? 6 : (n <= 8 ? 8 : 11)); }
 struct PbExpertParams {
     const int* n_used; const int* used_e; const int* used_off;
     const int* ent_tok; const int* ent_slot; const float* ent_w;

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(MH_THREADS, 1) pb_moeh_kernel(const PbExpertPa
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) { const int a = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += a; }
             e.w = incl - s;
-            const bool in = v <= (u1 - 1) / upg && incl - s + PB_VGROUP <= p.nslots;   // the columns past a group's entries read the slots behind it (and are dropped)
+            const bool in = v <= (u1 - 1) / upg && incl - s + ((s + 3) & ~3) <= p.nslots;   // the columns past a group's entries read the slots behind it (and are dropped)
             const unsigned m = __ballot_sync(0xffffffffu, in);
             const int n = m == 0xffffffffu ? 32 : __ffs(~m) - 1;         // leading groups that fit (at least one: nslots >= PB_VGROUP)
             vtab[lane] = e;
@@ -133,18 +133,19 @@ __global__ void __launch_bounds__(MH_THREADS, 1) pb_moeh_kernel(const PbExpertPa
             const int vi = u / upg - v0, j = u - (v0 + vi) * upg;
             const int4 e = vtab[vi];
             const PbHLane L = pb_h_lane<FMT>(pb_smem_u32(act) + (uint32_t)e.w * tokb, bpr, lane);
-            float tot[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+            float tot[3][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
             for (int blk = 0; blk < bpr; blk++) {
                 asm volatile("cp.async.wait_group %0;" ::"n"(MH_STAGES - 2) : "memory");
                 __syncwarp();   // this block has landed for all lanes, and all have left the stage that is refilled now
                 issue();
                 const uint32_t st = ring + (uint32_t)(cs * h.stage_bytes);
                 if (e.z <= 4) pb_h_block<FMT, 1>(st, pt, h, T, blk, blk, lane, L, reinterpret_cast<float (&)[1][2]>(tot));
-                else pb_h_block<FMT, 2>(st, pt, h, T, blk, blk, lane, L, tot);
+                else if (e.z <= 8) pb_h_block<FMT, 2>(st, pt, h, T, blk, blk, lane, L, reinterpret_cast<float (&)[2][2]>(tot));
+                else pb_h_block<FMT, 3>(st, pt, h, T, blk, blk, lane, L, tot);
                 cs = cs + 1 == MH_STAGES ? 0 : cs + 1;
             }
 #pragma unroll
-            for (int nt = 0; nt < 2; nt++) {
+            for (int nt = 0; nt < 3; nt++) {
                 const int k = 4 * nt + q;
                 if (k < e.z) {
                     const float a = tot[nt][0], b = tot[nt][1];
