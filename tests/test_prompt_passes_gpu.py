@@ -27,3 +27,21 @@ def test_deltanet_blocks_of_tokens(ctx, n):
         assert rel_err(ca, cb) < 1e-4 and rel_err(sa, sb) < 1e-4
     assert ctx.device_status() == 0
     a.destroy(); b.destroy(); m.destroy()
+
+
+@pytest.mark.parametrize("t", [128, 131, 261])
+def test_router_as_a_gemm(ctx, t):
+    """70 experts (a ragged second tile of router rows), one, two and three token tiles, the last with a few tokens: selection and block against the oracle."""
+    import oracle
+    cfg = small_cfg(pb, n_layers=1, full_every=0, d=2048, n_exp=70)
+    spec = synth.model_spec(cfg, 6)
+    m = synth.build_model(ctx, cfg, spec, 6)
+    _, mats = oracle_model(cfg, spec, 6)
+    st = m.new_state(t)
+    x = np.random.default_rng(t).standard_normal((t, cfg.d)).astype(np.float32)
+    y, sel = st.moe_forward(0, x)
+    yo, selo, _ = oracle.moe(oracle_cfg(cfg), *(mats[(0, r)] for r in ("ROUTER", "EXP_GATE", "EXP_UP", "EXP_DOWN", "SH_GATE", "SH_UP", "SH_DOWN", "SH_GATE_INP")), x)
+    assert np.array_equal(np.sort(sel, axis=1), np.sort(selo, axis=1))
+    assert rel_err(y, yo) < 1e-5
+    assert ctx.device_status() == 0
+    st.destroy(); m.destroy()
