@@ -15,10 +15,13 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <new>
+#include <utility>
 #include <vector>
 
 #define PB_MAX_WINDOW 8   // draft windows of the reference are at most 8 tokens (src/spec.rs:185)
 #define PB_PREFILL_CHUNK 256   // prompt tokens per batched pass; prompts are cut on the absolute grid of this size (src/engine_qn.rs:34-38, 92-139)
+#define PB_PROMPT_ROWS 1024    // prompt tokens of one pass over the layers where the model's prompt workspace is used: whole chunks, and the rest of the prompt behind them
+#define PB_PROMPT_TAIL 16      // a rest shorter than this runs as a pass of its own: its products are made by the kernels of few tokens
 #define PB_WIN_SPLITS 4        // attention splits per (token, KV head) of a prefill chunk: three walk the packed positions, one the f32 ring
 #define PB_WIN_KEYS (8 * (PB_MAX_WINDOW + 1) + 2)   // graphs per (t <= 8, ckpt, all_logits, logits), plus two for a full prefill chunk: without and with logits
 static size_t conv_elems(const pb_cfg& c, int B) { return (size_t)B * c.conv_k * (2 * c.lin_nk * c.lin_dk + c.lin_nv * c.lin_dv); }
@@ -26,8 +29,23 @@ static size_t ssm_elems(const pb_cfg& c, int B) { return (size_t)B * c.lin_nv * 
 
 struct PbSlot { pb_qmat* mat = nullptr; float* vec = nullptr; int64_t nvec = 0; };
 
+struct pb_state;
+// Row buffers of a pass over more than one prompt chunk: one set per model, made by the first prompt that is long enough.  The states of a model
+// share their context's stream and its thread, so one pass at a time uses it; a pass exchanges the pointers with the state's own.
+struct PbPromptWs {
+    bool tried = false;
+    void* mem = nullptr;
+    uint32_t* ids = nullptr; int64_t* wpos = nullptr; unsigned int* ticket = nullptr;
+    float *x = nullptr, *proj = nullptr, *olin = nullptr, *att = nullptr, *rlogits = nullptr, *dn_run = nullptr;
+    int *sel_e = nullptr, *ent_tok = nullptr, *ent_slot = nullptr; float *sel_w = nullptr, *ent_w = nullptr, *tok_scale = nullptr; int4* virt = nullptr;
+    float *h = nullptr, *h_sh = nullptr, *part = nullptr, *part_sh = nullptr;
+    int moe_cap = PB_PROMPT_ROWS;
+    void exchange(pb_state* s);
+};
+
 struct pb_model {
     pb_ctx* ctx = nullptr;
+    PbPromptWs ws;
     pb_cfg cfg{};
     std::vector<PbSlot> slots;      // [(n_layers + 1)][PB_R_COUNT], index 0 = global
     std::vector<int> kind, idx;     // per layer: 1 = full attention, 0 = DeltaNet; index among its kind
@@ -121,6 +139,13 @@ struct pb_state {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;   // GPU time of the token-loop calls (pb_stats.device_ns)
     bool ev_open = false; uint64_t device_ns = 0;
 };
+void PbPromptWs::exchange(pb_state* s) {
+    std::swap(ids, s->ids); std::swap(wpos, s->wpos); std::swap(ticket, s->ticket);
+    std::swap(x, s->x); std::swap(proj, s->proj); std::swap(olin, s->olin); std::swap(att, s->att); std::swap(rlogits, s->rlogits); std::swap(dn_run, s->dn_run);
+    std::swap(sel_e, s->sel_e); std::swap(ent_tok, s->ent_tok); std::swap(ent_slot, s->ent_slot); std::swap(sel_w, s->sel_w); std::swap(ent_w, s->ent_w);
+    std::swap(tok_scale, s->tok_scale); std::swap(virt, s->virt); std::swap(h, s->h); std::swap(h_sh, s->h_sh); std::swap(part, s->part); std::swap(part_sh, s->part_sh);
+    std::swap(moe_cap, s->moe_cap);
+}
 extern "C" {
 static void mtp_moved(pb_state* s, int64_t pos);
 static void mtp_forget(PbMtp* t, int64_t pos);
@@ -441,6 +466,7 @@ int pb_model_destroy(pb_model* m) {
     cudaStreamSynchronize(m->ctx->stream);
     for (auto& s : m->slots) { if (s.mat) pb_qmat_free(s.mat); if (s.vec) cudaFree(s.vec); }
     if (m->rope_inv) cudaFree(m->rope_inv);
+    if (m->ws.mem) cudaFree(m->ws.mem);
     delete m;
     return PB_OK;
 }
@@ -689,6 +715,16 @@ static int gemv_cols(pb_ctx* ctx, PbGemvQArgs a, int B, bool prefill = false) {
     return PB_OK;
 }
 
+// The same for the tokens of a prompt pass, chunk by chunk: a chunk's sums are the ones of a pass of its own
+static int gemv_chunks(pb_ctx* ctx, const PbGemvQArgs& a, int n, bool prefill) {
+    for (int t0 = 0; t0 < n; t0 += PB_PREFILL_CHUNK) {
+        PbGemvQArgs b = a;
+        b.x = a.x + (int64_t)t0 * a.ldx; b.y = a.y + (int64_t)t0 * a.ldy; b.z = a.z ? a.z + (int64_t)t0 * a.ldz : nullptr;
+        PB_TRY(gemv_cols(ctx, b, n - t0 < PB_PREFILL_CHUNK ? n - t0 : PB_PREFILL_CHUNK, prefill));
+    }
+    return PB_OK;
+}
+
 // Gated DeltaNet mixer: x_in (normalized when norm_w == null) -> y (stored or added)
 static int run_lin(pb_state* s, int il, const float* x_in, const float* norm_w, float* y, int64_t ldy, int accumulate) {
     pb_model* m = s->m; pb_ctx* ctx = m->ctx; const pb_cfg& c = m->cfg; const int B = s->batch, li = m->idx[il];
@@ -699,7 +735,7 @@ static int run_lin(pb_state* s, int il, const float* x_in, const float* norm_w, 
     a.x = x_in; a.ldx = c.d; a.y = s->proj; a.ldy = s->ldproj; a.mode = norm_w ? PB_ACT_NORM : PB_ACT_PLAIN; a.norm_w = norm_w; a.eps = c.eps;
     const int ncol = s->win_t > 0 ? s->win_t : B;   // window mode: the columns are consecutive tokens of sequence 0
     const bool prefill = s->win_t >= 16 && !s->win_ckpt;
-    PB_TRY(gemv_cols(ctx, a, ncol, prefill));
+    PB_TRY(gemv_chunks(ctx, a, ncol, prefill));
     PbDeltaParams d; memset(&d, 0, sizeof d);
     d.proj = s->proj; d.ldp = s->ldproj; d.conv_w = V(m, il, PB_R_LIN_CONV); d.a = V(m, il, PB_R_LIN_A); d.dt = V(m, il, PB_R_LIN_DT);
     d.conv = s->conv[li]; d.ssm = s->ssm[li]; d.pos = s->pos; d.out = s->olin; d.ldo = w;
@@ -726,7 +762,7 @@ static int run_lin(pb_state* s, int il, const float* x_in, const float* norm_w, 
     PbGemvQArgs o; memset(&o, 0, sizeof o);
     o.type = M(m, il, PB_R_LIN_OUT)->type; o.cols = w; o.nseg = 1; seg(o, 0, M(m, il, PB_R_LIN_OUT), 0);
     o.x = s->olin; o.ldx = w; o.y = y; o.ldy = ldy; o.mode = PB_ACT_GNORM; o.norm_w = V(m, il, PB_R_LIN_NORM); o.z = s->proj + ch; o.ldz = s->ldproj; o.head_dim = c.lin_dv; o.eps = c.eps; o.accumulate = accumulate;
-    return gemv_cols(ctx, o, ncol, prefill);
+    return gemv_chunks(ctx, o, ncol, prefill);
 }
 
 static void attn_params(pb_state* s, int il, PbAttnParams& p) {
@@ -759,7 +795,7 @@ static int run_attn(pb_state* s, int il, const float* x_in, const float* norm_w,
     a.x = x_in; a.ldx = c.d; a.y = s->proj; a.ldy = s->ldproj; a.mode = norm_w ? PB_ACT_NORM : PB_ACT_PLAIN; a.norm_w = norm_w; a.eps = c.eps;
     const int ncol = s->win_t > 0 ? s->win_t : B;
     const bool prefill = s->win_t >= 16 && !s->win_ckpt;
-    PB_TRY(gemv_cols(ctx, a, ncol, prefill));
+    PB_TRY(gemv_chunks(ctx, a, ncol, prefill));
     PbAttnParams p; attn_params(s, il, p);
     // QSA block-sparse attention (attn_core :1565-1599): two more projections of the same input give the raw index query
     // heads and the raw index key; after the KV append the indexer stores the key, pools the block the token completes,
@@ -779,17 +815,22 @@ static int run_attn(pb_state* s, int il, const float* x_in, const float* norm_w,
         // a prefill chunk or a verify window: all tokens are appended, the packed boundary moves once, then every token attends
         // to the positions <= its own in one launch (token j treats as packed what it would have found packed token by
         // token).  A verify window that is cut short afterwards gets its boundary back in pb_keep.
-        p.window = 1; p.pos = s->wpos; p.batch = s->win_t;
+        // (a pass over several chunks does this chunk by chunk: the ring holds the recent positions and one chunk)
+        p.window = 1;
+        for (int t0 = 0; t0 < s->win_t; t0 += PB_PREFILL_CHUNK) {
+        const int wt = s->win_t - t0 < PB_PREFILL_CHUNK ? s->win_t - t0 : PB_PREFILL_CHUNK;
+        p.proj = s->proj + (size_t)t0 * s->ldproj; p.pos = s->wpos + t0; p.att = s->att + (size_t)t0 * p.lda; p.batch = wt;
         const bool tiles = pb_attnw_supported(p);   // the model's head shape without a mask: 64 query rows share each cache tile
         const bool mma = s->nsplit_packed > 0;
         // splits per token: four for a chunk of hundreds of tokens, more for a window of a few, so that the grid fills the GPU
-        int ws = ctx->sm_count / (c.n_kv * s->win_t);
+        int ws = ctx->sm_count / (c.n_kv * wt);
         ws = ws < PB_WIN_SPLITS ? PB_WIN_SPLITS : (ws > 64 ? 64 : ws);
-        if ((size_t)ws * s->win_t > (size_t)PB_PREFILL_CHUNK * PB_WIN_SPLITS) ws = PB_WIN_SPLITS;
+        if ((size_t)ws * wt > (size_t)PB_PREFILL_CHUNK * PB_WIN_SPLITS) ws = PB_WIN_SPLITS;
         p.nsplit = tiles ? pb_attnw_splits(ctx, p, (int64_t)PB_PREFILL_CHUNK * PB_WIN_SPLITS) : mma ? ws : 1; p.nsplit_packed = mma ? ws - 1 : 0;
         PB_TRY(pb_launch_kv_append(ctx, p));
         PB_TRY(pb_launch_kv_pack(ctx, p));
         PB_TRY(tiles ? pb_launch_attn_window(ctx, p) : pb_launch_attn(ctx, p));
+        }
     } else if (s->win_t > 0) {
         // causal inside the window: token j is appended, then attends to positions <= its own
         // (models with an indexer take this form for prefill chunks too: every token makes its own selection)
@@ -807,7 +848,7 @@ static int run_attn(pb_state* s, int il, const float* x_in, const float* norm_w,
     PbGemvQArgs o; memset(&o, 0, sizeof o);
     o.type = M(m, il, PB_R_ATTN_O)->type; o.cols = c.n_head * c.hd; o.nseg = 1; seg(o, 0, M(m, il, PB_R_ATTN_O), 0);
     o.x = s->att; o.ldx = (int64_t)c.n_head * c.hd; o.y = y; o.ldy = ldy; o.mode = PB_ACT_PLAIN; o.accumulate = accumulate;
-    return gemv_cols(ctx, o, ncol, prefill);
+    return gemv_chunks(ctx, o, ncol, prefill);
 }
 
 // whether the expert kernels of layer il run on the tensor cores for t tokens (the type the kernels stream: re-coded copies where all have one)
@@ -1177,6 +1218,7 @@ static int run_window(pb_state* s, int t, bool ckpt, bool all_logits, bool logit
     pb_model* m = s->m; pb_ctx* ctx = m->ctx; const pb_cfg& c = m->cfg;
     struct Scope { pb_ctx* c; pb_state* s; Scope(pb_ctx* x, pb_state* y, int t, bool k) : c(x), s(y) { c->pdl_scope++; c->pdl_chain = false; s->win_t = t; s->win_ckpt = k; }
                    ~Scope() { c->pdl_scope--; c->pdl_chain = false; s->win_t = 0; s->win_ckpt = false; } } scope(ctx, s, t, ckpt);
+    struct Ws { pb_state* s; Ws(pb_state* x, int t) : s(t > PB_PREFILL_CHUNK ? x : nullptr) { if (s) s->m->ws.exchange(s); } ~Ws() { if (s) s->m->ws.exchange(s); } } ws(s, t);
     PB_TRY(pb_launch_window_pos(ctx, s->pos, s->wpos, t, 0));
     pb_qmat* embd = M(m, -1, PB_R_TOKEN_EMBD);
     if (c.hc > 0) { PB_TRY(run_layers_hc(s, t, all_logits ? 0 : t - 1, all_logits ? t : 1)); if (s->mtp) PB_TRY(pb_launch_mtp_keep(ctx, s->x, (int64_t)c.hc * c.d, s->wpos, t, s->mtp->ring, s->mtp->ring_cap, c.hc * c.d)); }
@@ -1305,6 +1347,41 @@ static void mtp_moved(pb_state* s, int64_t pos) {
     if (t->kv_c0 > t->kv_end) t->kv_c0 = t->kv_end;
 }
 
+// The model's prompt workspace, allocated by the first prompt that can use it; null where the model is outside what a pass over several chunks
+// is built for (pre-norm residual, dense attention, experts on the tensor cores of one GPU) or the memory cannot be had: prompts then go chunk by chunk
+static PbPromptWs* prompt_ws(pb_model* m) {
+    PbPromptWs& w = m->ws;
+    if (w.tried) return w.mem ? &w : nullptr;
+    w.tried = true;
+    pb_ctx* ctx = m->ctx; const pb_cfg& c = m->cfg;
+    if (c.hc > 0 || m->n_ple > 0 || m->qsa || m->mtp_window > 0 || m->ep_world > 1) return nullptr;
+    for (int il = 0; il < c.n_layers; il++) if (!expert_mma(m, il, 2)) return nullptr;
+    const size_t R = PB_PROMPT_ROWS, K = (size_t)c.top_k;
+    const size_t lin_w = (size_t)c.lin_nv * c.lin_dv, att_w = (size_t)c.n_head * c.hd, wide = lin_w > att_w ? lin_w : att_w;
+    const size_t lin_proj = 2 * (size_t)c.lin_nk * c.lin_dk + 2 * lin_w + 2 * (size_t)c.lin_nv, att_proj = 2 * att_w + 2 * (size_t)c.n_kv * c.hd;
+    const size_t ldproj = ((lin_proj > att_proj ? lin_proj : att_proj) + 3) & ~(size_t)3;   // as in state_create
+    PbDeltaParams dp; memset(&dp, 0, sizeof dp);
+    dp.nk = c.lin_nk; dp.nv = c.lin_nv; dp.dk = c.lin_dk; dp.dv = c.lin_dv;
+    size_t off = 0;
+    char* base = nullptr;
+    auto carve = [&](auto** p, size_t n) { *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(base + off); off = (off + n * sizeof(**p) + 511) & ~(size_t)255; };
+    for (int pass = 0; pass < 2; pass++) {
+        off = 0;
+        carve(&w.ids, R); carve(&w.wpos, R); carve(&w.ticket, 8 + (R + 7) / 8);
+        carve(&w.x, R * c.d); carve(&w.proj, R * ldproj); carve(&w.olin, R * wide); carve(&w.att, R * wide);
+        carve(&w.rlogits, R * (c.n_exp + 1)); carve(&w.dn_run, m->n_lin > 0 ? pb_deltanet_seq_scratch(dp, (int)R) : 1);
+        carve(&w.sel_e, R * K); carve(&w.sel_w, R * K); carve(&w.ent_tok, R * K); carve(&w.ent_slot, R * K); carve(&w.ent_w, R * K); carve(&w.tok_scale, R);
+        carve(&w.virt, (size_t)c.n_exp + R * K / PB_VGROUP + 1); carve(&w.h, R * K * c.ff_exp); carve(&w.h_sh, R * c.ff_sh);
+        carve(&w.part, R * K * c.d); carve(&w.part_sh, R * c.d);
+        if (pass == 0) {
+            if (cudaMalloc(&w.mem, off) != cudaSuccess) { cudaGetLastError(); w.mem = nullptr; return nullptr; }
+            base = (char*)w.mem;
+        }
+    }
+    if (cudaMemsetAsync(w.mem, 0, off, ctx->stream) != cudaSuccess) { cudaGetLastError(); cudaFree(w.mem); w.mem = nullptr; }
+    return w.mem ? &w : nullptr;
+}
+
 int pb_forward(pb_state* s, const uint32_t* ids_host, int t, float* logits_host) {
     if (!s) return PB_ERR_ARG;
     pb_ctx* ctx = s->m->ctx;
@@ -1318,13 +1395,23 @@ int pb_forward(pb_state* s, const uint32_t* ids_host, int t, float* logits_host)
         if (s->pos_host + t > s->m->cfg.max_ctx) PB_FAIL(ctx, PB_ERR_STATE, "context is full (%d positions)", s->m->cfg.max_ctx);
         mtp_note(s, s->pos_host, ids_host, t);
         timing_begin(s);
+        const int64_t pin_n = (s->trace_cap + 2) * B + PB_PREFILL_CHUNK;
+        int64_t pin = 0;
         for (int j0 = 0, n = 0; j0 < t; j0 += n) {
+            // from a multiple of the chunk on, several chunks share a pass: the experts' weights, of which 256 tokens need all and a pass
+            // decodes every one, serve four times the tokens.  All that a token's sums depend on -- the kernels, their cuts -- follows its chunk, so
+            // the results are those of a pass per chunk, bit for bit
             const int64_t to_grid = PB_PREFILL_CHUNK - s->pos_host % PB_PREFILL_CHUNK;
             n = t - j0 < to_grid ? t - j0 : (int)to_grid;
-            for (int j = 0; j < n; j++) s->pin_u32[j] = ids_host[j0 + j];
-            PB_CUDA(ctx, cudaMemcpyAsync(s->ids, s->pin_u32, (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
+            if (to_grid == PB_PREFILL_CHUNK && t - j0 >= PB_PREFILL_CHUNK + PB_PROMPT_TAIL && prompt_ws(s->m)) {
+                n = t - j0 < PB_PROMPT_ROWS ? t - j0 : PB_PROMPT_ROWS;
+                if (n % PB_PREFILL_CHUNK < PB_PROMPT_TAIL) n -= n % PB_PREFILL_CHUNK;
+            }
+            if (pin + n > pin_n) { PB_CUDA(ctx, cudaStreamSynchronize(ctx->stream)); pin = 0; }   // the pinned id buffer is reused
+            for (int j = 0; j < n; j++) s->pin_u32[pin + j] = ids_host[j0 + j];
+            PB_CUDA(ctx, cudaMemcpyAsync(n > PB_PREFILL_CHUNK ? s->m->ws.ids : s->ids, s->pin_u32 + pin, (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
+            pin += n;
             PB_TRY(window_once(s, n, false, false, j0 + n >= t));
-            if (j0 + n < t) PB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));   // the pinned id buffer is reused
         }
         s->verify_t = 0;
         timing_stop(s);

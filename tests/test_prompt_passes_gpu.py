@@ -45,3 +45,21 @@ def test_router_as_a_gemm(ctx, t):
     assert rel_err(y, yo) < 1e-5
     assert ctx.device_status() == 0
     st.destroy(); m.destroy()
+
+
+@pytest.mark.parametrize("n", [272, 1024, 1295, 1313])
+def test_several_chunks_in_one_pass(ctx, n):
+    """Whole chunks and a rest of 0, 15 (a pass of its own), 16 and 33 tokens: logits, states and the tokens that follow are those of a call per chunk, bit for bit."""
+    cfg = small_cfg(pb, max_ctx=1400, kv_bits=4)
+    m = synth.build_model(ctx, cfg, synth.model_spec(cfg, 12), 12)
+    a, b = m.new_state(1), m.new_state(1)
+    ids = np.random.default_rng(n).integers(0, cfg.vocab, n).astype(np.uint32)
+    la = a.forward(ids)
+    for i in range(0, n, 256):
+        lb = b.forward(ids[i:i + 256])
+    assert np.array_equal(la.view(np.uint32), lb.view(np.uint32))
+    for (ca, sa), (cb, sb) in zip((a.get_lin(0), a.get_lin(2)), (b.get_lin(0), b.get_lin(2))):
+        assert np.array_equal(ca.view(np.uint32), cb.view(np.uint32)) and np.array_equal(sa.view(np.uint32), sb.view(np.uint32))
+    assert a.decode_greedy([5], 8)[0].tolist() == b.decode_greedy([5], 8)[0].tolist()
+    assert ctx.device_status() == 0
+    a.destroy(); b.destroy(); m.destroy()
