@@ -715,12 +715,16 @@ static int gemv_cols(pb_ctx* ctx, PbGemvQArgs a, int B, bool prefill = false) {
     return PB_OK;
 }
 
-// The same for the tokens of a prompt pass, chunk by chunk: a chunk's sums are the ones of a pass of its own
+// The same for the tokens of a prompt pass: its whole chunks together, with the cuts of one chunk, then the rest, so that a token's sums are the
+// ones of a pass over its chunk alone
 static int gemv_chunks(pb_ctx* ctx, const PbGemvQArgs& a, int n, bool prefill) {
-    for (int t0 = 0; t0 < n; t0 += PB_PREFILL_CHUNK) {
+    const int whole = n / PB_PREFILL_CHUNK * PB_PREFILL_CHUNK;
+    for (int t0 = 0, k = 0; t0 < n; t0 += k) {
+        k = t0 < whole ? whole : n - t0;
         PbGemvQArgs b = a;
         b.x = a.x + (int64_t)t0 * a.ldx; b.y = a.y + (int64_t)t0 * a.ldy; b.z = a.z ? a.z + (int64_t)t0 * a.ldz : nullptr;
-        PB_TRY(gemv_cols(ctx, b, n - t0 < PB_PREFILL_CHUNK ? n - t0 : PB_PREFILL_CHUNK, prefill));
+        b.form_t = k > PB_PREFILL_CHUNK ? PB_PREFILL_CHUNK : 0;
+        PB_TRY(gemv_cols(ctx, b, k, prefill));
     }
     return PB_OK;
 }

@@ -25,7 +25,7 @@
 // Every wait is bounded; a wait that runs out records a status (the host call returns PB_ERR_DEVICE) and the CTA leaves
 // through the common exit, which frees its tensor memory.  A matrix of few tiles is cut along its columns over a cluster of up to eight CTAs, whose
 // sums meet through distributed shared memory; nothing is multicast, operands come only from this GPU.
-#include "pb_stream.cuh"
+#include "pb_tc.cuh"
 #include "pb_internal.h"
 
 #include <cuda_fp16.h>
@@ -46,54 +46,6 @@
 #define TC_THREADS ((TC_DECODERS + 2) * 32)
 #define TC_B_BYTES (2 * TC_NARROW * TC_KSTEP * 2)                 // high and low activation tiles of a stage: 32 KB, in the wide form twice that
 #define TC_XT_HEAD 4096             // bytes of per-token prescale inverses in front of the activation tiles
-
-enum : int { PB_DEV_TC_TIMEOUT = 6 };
-
-// ---------------------------------------------------------------- tcgen05 wrappers (cta_group::1)
-__device__ __forceinline__ void tc_alloc(uint32_t* smem_dst, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pb_smem_u32(smem_dst)), "r"(ncols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tc_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// D (tensor memory) (+)= A (tensor memory: lane = row, two f16 per cell along K) x B (shared memory, by descriptor)
-__device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// the mbarrier receives one arrival once every tcgen05.mma issued so far by this thread has completed
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(pb_smem_u32(bar)) : "memory");
-}
-// 32 lanes x 32 consecutive columns of 32-bit cells: thread l of the warp gets lane (base lane + l), columns c .. c+31
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-          "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-          "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// Shared-memory operand descriptor: K-major, 128-byte swizzle.  A row of the tile (one weight row or one token) is 128
-// contiguous bytes = the 64 columns of a step; its 16-byte chunk c sits at chunk position c ^ (row & 7); groups of 8
-// rows are 1024 bytes apart (the stride offset); the tile starts on a 1024-byte boundary.  A step of 16 columns along K
-// is 32 bytes further into the row: the start address moves, the swizzle is applied by the hardware on the address bits.
-__device__ __forceinline__ uint64_t tc_desc(uint32_t saddr) {
-    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-// Instruction descriptor of kind::f16: f32 accumulator, f16 A and B, both K-major, N >> 3 at bit 17, M >> 4 at bit 24.
-__device__ __forceinline__ uint32_t tc_idesc(int m, int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24); }
 
 // ---------------------------------------------------------------- activations -> operand tiles
 
@@ -188,25 +140,6 @@ __device__ __forceinline__ void tc_load_raw(TcRaw& r, uint32_t b, int row, int q
 #pragma unroll
     for (int i = 0; i < 2; i++) asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.c[2 * i].x), "=r"(r.c[2 * i].y), "=r"(r.c[2 * i + 1].x), "=r"(r.c[2 * i + 1].y) : "r"(b + 512 * i + (4 * row + qt) * 16) : "memory");
 }
-__device__ __forceinline__ void tc_cp_async16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-// the mbarrier (initialised with one count per issuing thread) gets this thread's arrival once its copies so far have landed
-__device__ __forceinline__ void tc_cp_async_arrive(uint64_t* bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(pb_smem_u32(bar)) : "memory");
-}
-// 32 cells of this thread's lane, consecutive columns from taddr on (taddr carries the warp's first lane in bits 16+)
-__device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
-          "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
-          "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-        : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
 // decode the 64 columns of step ks of this thread's row and store them as its lane of the weight tile at taddr
 // (tensor memory: lane = row, cell j = columns 2j, 2j + 1 of the step)
 __device__ __forceinline__ void tc_decode_store(const TcRaw& r, int ks, uint32_t taddr, float shift) {
@@ -253,10 +186,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
     constexpr int NB = WIDE ? TC_WIDE : TC_NARROW, NST = WIDE ? TC_STAGES / 2 : TC_STAGES;   // tokens of a CTA, stages of the ring
     constexpr size_t STB = WIDE ? 2 * TC_B_BYTES : TC_B_BYTES;                               // and their bytes
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem);             // [TC_STAGES] 128 decoder arrivals + the producer's, and the bulk-copy bytes
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem);             // [TC_STAGES] the arrivals of four decoder warps + the producer's, and the bulk-copy bytes
     uint64_t* empty = full + TC_STAGES;                             // [TC_STAGES] tcgen05.commit: the MMAs that read the stage are done
     uint64_t* raw_full = empty + TC_STAGES;                         // [TC_RAW_STAGES] 256 decoder threads (cp.async)
-    uint64_t* raw_empty = raw_full + TC_RAW_STAGES;                 // [TC_RAW_STAGES] 256 decoder threads
+    uint64_t* raw_empty = raw_full + TC_RAW_STAGES;                 // [TC_RAW_STAGES] 8 decoder warps
     uint64_t* acc_full = raw_empty + TC_RAW_STAGES;                 // accumulator complete
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 384);
     float* red = reinterpret_cast<float*>(smem + 416);              // [8] per-warp maxima of d
@@ -264,7 +197,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
     uint8_t* raw = b_ring + TC_STAGES * TC_B_BYTES;               // [TC_RAW_STAGES][128 rows][136 bytes]
     float* part = reinterpret_cast<float*>(b_ring);                 // [tokens][TC_ROWS] sums of this CTA's share of the contraction, once the MMAs are done
     static_assert((TC_STAGES * 2 + TC_RAW_STAGES * 2 + 1) * 8 <= 384 && TC_ACC_COLS + TC_STAGES * TC_A_COLS <= TC_TMEM_COLS, "barriers fit in front of the TMEM slot");
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tc_uniform_warp(), lane = tid & 31;
 
     const int ks = p.ks, rank = (int)blockIdx.x % ks, tile = (int)blockIdx.x / ks, tb = (int)blockIdx.y;   // (clusters are consecutive CTAs)
     int s = 0;
@@ -277,8 +210,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
     const uint32_t bbytes = 2u * (uint32_t)np * 128u;
 
     if (tid == 0) {
-        for (int i = 0; i < TC_STAGES; i++) { pb_mbar_init(&full[i], 128 + 1); pb_mbar_init(&empty[i], 1); }
-        for (int i = 0; i < TC_RAW_STAGES; i++) { pb_mbar_init(&raw_full[i], TC_DECODERS * 32); pb_mbar_init(&raw_empty[i], TC_DECODERS * 32); }
+        for (int i = 0; i < TC_STAGES; i++) { pb_mbar_init(&full[i], 4 + 1); pb_mbar_init(&empty[i], 1); }
+        for (int i = 0; i < TC_RAW_STAGES; i++) { pb_mbar_init(&raw_full[i], TC_DECODERS * 32); pb_mbar_init(&raw_empty[i], TC_DECODERS); }
         pb_mbar_init(acc_full, 1);
         pb_fence_barrier_init();
     }
@@ -312,26 +245,27 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
         // reads the weight tile once, and the epilogue adds the two halves of the accumulator
         pb_pdl_wait();
         const uint32_t idesc = tc_idesc(TC_ROWS, WIDE ? np : 2 * np);
+        const uint64_t bdesc = tc_desc(pb_smem_u32(b_ring));
+        const bool elected = tc_elect();
         bool ok = true;
         for (int k = 0; k < nk && ok; k++) {
             const int st = k % NST;
-            ok = pb_mbar_wait(&full[st], (k / NST) & 1, p.status, PB_DEV_TC_TIMEOUT);
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            ok = __all_sync(0xffffffffu, pb_mbar_wait(&full[st], (k / NST) & 1, p.status, PB_DEV_TC_TIMEOUT));
             if (!ok) break;
             tc_fence_after();
-            if (lane == 0) {
+            if (elected) {
                 const uint32_t a_t = tmem + TC_ACC_COLS + (uint32_t)st * TC_A_COLS;
-                const uint32_t b_s = pb_smem_u32(b_ring + (size_t)st * STB);
+                const uint64_t b = bdesc + (uint64_t)((uint32_t)st * (uint32_t)(STB >> 4));       // (addresses enter a descriptor in units of 16 bytes)
 #pragma unroll
                 for (int kk = 0; kk < TC_KSTEP / 16; kk++) {
-                    tc_mma_f16_ts(tmem, a_t + kk * 8, tc_desc(b_s + kk * 32), idesc, (k | kk) ? 1u : 0u);
-                    if (WIDE) tc_mma_f16_ts(tmem, a_t + kk * 8, tc_desc(b_s + (uint32_t)np * 128u + kk * 32), idesc, 1u);
+                    tc_mma_f16_ts(tmem, a_t + kk * 8, b + 2 * kk, idesc, kk ? 1u : (k ? 1u : 0u));
+                    if (WIDE) tc_mma_f16_ts(tmem, a_t + kk * 8, b + (uint64_t)((uint32_t)np * 8u) + 2 * kk, idesc, 1u);
                 }
                 tc_commit(&empty[st]);
             }
             __syncwarp();
         }
-        if (ok && lane == 0) tc_commit(acc_full);
+        if (ok && elected) tc_commit(acc_full);
         __syncwarp();
     } else {
         // ------------------------------------------------------------ decoders, then epilogue
@@ -378,7 +312,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
             TcRaw cur;
             tc_load_raw(cur, pb_smem_u32(raw + (size_t)rs * TC_RAW_BYTES) + (uint32_t)(row >> 3) * 1088u, row & 7, k & 3, live);
             if ((k & 3) == grp + 2) {
-                pb_mbar_arrive(&raw_empty[rs]);
+                tc_warp_arrive(&raw_empty[rs], lane);
                 if (kb + TC_RAW_STAGES < nkb) {
                     if (!pb_mbar_wait(&raw_empty[rs], (kb / TC_RAW_STAGES) & 1, p.status, PB_DEV_TC_TIMEOUT)) { ok = false; break; }
                     issue_raw(kb + TC_RAW_STAGES);
@@ -387,7 +321,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
             if (k >= NST && !pb_mbar_wait(&empty[st], ((k / NST) - 1) & 1, p.status, PB_DEV_TC_TIMEOUT)) { ok = false; break; }
             tc_decode_store(cur, k, tmem + ((uint32_t)((warp & 3) * 32) << 16) + TC_ACC_COLS + (uint32_t)st * TC_A_COLS, shift);
             tc_fence_before();                    // the stores are complete (wait::st); order them before the MMA warp's instructions
-            pb_mbar_arrive(&full[st]);
+            tc_warp_arrive(&full[st], lane);
         }
         // ---- epilogue: warp w reads lanes 32 (w % 4) .. + 31 (its rows); warps 0-3 take the first half of the tokens, 4-7 the rest; columns
         //      [0, np) hold the sums, or (narrow) the high parts' with the low parts' in [np, 2 np)
@@ -485,12 +419,13 @@ int pb_launch_gemmtc(pb_ctx* ctx, const PbGemvQArgs& a) {
     // Tokens per CTA and CTAs per tile, by the rounds the SMs need: a CTA walks its columns serially, a wide one takes half as long again per block
     // and twice as long around it (256 tokens of 12352 x 2048: two rounds of narrow ones 47 us, one of wide ones 39); a matrix with
     // fewer tiles than SMs is cut along its columns, and the parts' sums meet at the end (256 tokens of 2048 x 4096: 64 us uncut, 26 in four).
+    const int ft = a.form_t > 0 && a.t % a.form_t == 0 && a.form_t % TC_WIDE == 0 ? a.form_t : a.t;
     int nb = TC_NARROW, cut = 1, best = 0;
-    for (int w = TC_NARROW; w <= (a.t > TC_NARROW ? TC_WIDE : TC_NARROW); w *= 2)
+    for (int w = TC_NARROW; w <= (ft > TC_NARROW ? TC_WIDE : TC_NARROW); w *= 2)
         for (int ks = 1; ks <= 8 && a.cols / 256 % ks == 0 && (ks == 1 || a.cols / 256 / ks >= 2); ks *= 2) {
             const void* k = w == TC_WIDE ? reinterpret_cast<const void*>(pb_gemmtc_iq3s_kernel<true>) : reinterpret_cast<const void*>(pb_gemmtc_iq3s_kernel<false>);
             PB_TRY(pb_ensure_smem_fn(ctx, k, smem));
-            const int room = pb_max_clusters(ctx, k, TC_THREADS, smem, ks), rounds = (ntiles * ((a.t + w - 1) / w) + room - 1) / room;
+            const int room = pb_max_clusters(ctx, k, TC_THREADS, smem, ks), rounds = (ntiles * ((ft + w - 1) / w) + room - 1) / room;
             const int cost = rounds * ((w == TC_WIDE ? 12 : 6) + (ks > 1 ? 4 : 0) + a.cols / 256 / ks * (w == TC_WIDE ? 3 : 2));
             if (best == 0 || cost < best) { best = cost; nb = w; cut = ks; }
         }

@@ -193,6 +193,7 @@ struct PbGemvQArgs {
     int mode; const float* norm_w; const float* z; int64_t ldz; int head_dim; float eps;
     const uint32_t* xq_in;
     int accumulate;
+    int form_t;  // > 0: tokens by whose number the tcgen05 GEMM chooses its form (t is a multiple of it: several chunks of a prompt in one launch), else t
     int exact;   // keep the kernels whose weights enter the products exactly (decode steps feed recurrent state); 0 lets 16+ tokens use the tcgen05 GEMM, whose f16 weights carry one rounding
 };
 struct PbGemvQSeg { const uint8_t* w; int rows; int chunk0; int yoff; };
