@@ -865,6 +865,14 @@ static bool expert_mma(pb_model* m, int il, int t) {
     return c.ff_exp == c.ff_sh && pb_moeh_supported(type, c.d, c.ff_exp, t);
 }
 
+// whether they run on tcgen05 instead (same bits): from eight entries an expert on average, where a group's rows are decoded once for up to 24 (four
+// layers of a prompt with top 10 of 512 experts, warp level / tcgen05: 333 tokens 2.76 / 2.86 ms, 420 3.23 / 3.22, 512 3.61 / 3.48, 700 4.45 / 4.15)
+static bool expert_tc(pb_model* m, int il, int t) {
+    const pb_cfg& c = m->cfg;
+    const int type = M(m, il, PB_R_EXP_GATE)->type == PB_T_IQ3_S ? PB_T_IQ3S_N4 : M(m, il, PB_R_EXP_GATE)->type;
+    return m->ep_world == 1 && pb_moetc_supported(type, c.d, c.ff_exp) && (int64_t)t * c.top_k >= 8ll * c.n_exp;
+}
+
 // MoE block on t tokens: x_in [t][d] (normalized when norm_w == null) -> y (stored or added)
 static int run_moe(pb_state* s, int il, const float* x_in, const float* norm_w, int t, float* y, int64_t ldy, int accumulate) {
     pb_model* m = s->m; pb_ctx* ctx = m->ctx; const pb_cfg& c = m->cfg;
@@ -881,6 +889,8 @@ static int run_moe(pb_state* s, int il, const float* x_in, const float* norm_w, 
     q.ent_tok = s->ent_tok; q.ent_slot = s->ent_slot; q.ent_w = s->ent_w;
     // two and more tokens of the formats it covers: the expert kernels on the tensor cores, which read the token rows themselves
     const bool moeh = expert_mma(m, il, tt);
+    const bool moetc = moeh && expert_tc(m, il, tt);
+    q.tc = moetc;
     if (moeh) { r.scale_out = s->tok_scale; q.virt = s->virt; q.n_virt = s->n_used + 1; } else r.xq_out = s->xq;
     // prompts take the GEMM form at any length from 16 tokens on, so that a token's logits do not depend on the pass it is in; it is the shorter one
     // from about 128 tokens on (us, GEMM / the other: 34 / 26 at 32 tokens, 47 / 48 at 128, 187 / 232 at 1024)
@@ -916,7 +926,7 @@ static int run_moe(pb_state* s, int il, const float* x_in, const float* norm_w, 
     if (g->rdata && up->rdata && shg->rdata && shu->rdata) { e.w_a = g->rdata; e.w_b = up->rdata; e.sh_a = shg->rdata; e.sh_b = shu->rdata; gu_type = PB_T_IQ3S_N4; }   // re-coded copies
     e.rows_e = c.ff_exp; e.rows_sh = c.ff_sh;
     if (tt > s->moe_cap) PB_FAIL(ctx, PB_ERR_ARG, "MoE block on %d tokens, buffers hold %d", tt, s->moe_cap);
-    if (moeh) { e.virt = s->virt; e.n_virt = s->n_used + 1; e.x = r.x; e.ldx = r.ldx; e.norm_w = norm_w; e.tok_scale = s->tok_scale; PB_TRY(pb_launch_moeh_gu(ctx, e, gu_type, c.d)); }
+    if (moeh) { e.virt = s->virt; e.n_virt = s->n_used + 1; e.x = r.x; e.ldx = r.ldx; e.norm_w = norm_w; e.tok_scale = s->tok_scale; PB_TRY(moetc ? pb_launch_moetc_gu(ctx, e, c.d) : pb_launch_moeh_gu(ctx, e, gu_type, c.d)); }
     else PB_TRY(pb_launch_expert_gu(ctx, e, gu_type, c.d));
     pb_qmat* dn = M(m, il, PB_R_EXP_DOWN);
     e.e_base = dn->rows == (int64_t)c.d * c.n_exp ? 0 : m->e_lo;
@@ -932,7 +942,7 @@ static int run_moe(pb_state* s, int il, const float* x_in, const float* norm_w, 
     if (sh && s->p2p) e.part_tok = s->part_tok;            // finished rows go straight into the memory of the token's owner
     k.y = y; k.ldy = ldy; k.accumulate = accumulate;
     // few tokens on one GPU: the down kernel's last CTA also combines (one launch less per layer)
-    if (moeh) PB_TRY(pb_launch_moeh_down(ctx, e, dn_type, c.ff_exp));
+    if (moeh) PB_TRY(moetc ? pb_launch_moetc_down(ctx, e, c.ff_exp) : pb_launch_moeh_down(ctx, e, dn_type, c.ff_exp));
     else if (m->ep_world == 1 && (int64_t)t * c.d <= 8192) return pb_launch_expert_down(ctx, e, dn_type, c.ff_exp, &k, s->ticket + 1);
     else PB_TRY(pb_launch_expert_down(ctx, e, dn_type, c.ff_exp));
     // expert parallelism: every (token, slot) row was produced on exactly one rank and is zero elsewhere,

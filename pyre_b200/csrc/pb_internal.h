@@ -251,12 +251,15 @@ struct PbRouteParams {
     int* sel_e; float* sel_w;                 // [t][top_k], ascending expert id
     int* n_used; int* used_e; int* used_off;  // distinct local experts, entry offsets [n_used + 1]
     int* ent_tok; int* ent_slot; float* ent_w;
+    int tc;                                   // groups for the tcgen05 expert kernels (PB_VGROUP_TC entries)
     int4* virt; int* n_virt;                  // several tokens: distinct local experts in groups of up to PB_VGROUP entries {expert, first entry, entries, cost of the groups before}, and their number
 };
 #define PB_VGROUP 12
+#define PB_VGROUP_TC 24      // the same of the tcgen05 expert kernels (pb_moetc.cu)
 // Cost of a group of n entries in the expert kernels, in sixths of a group of up to four: five to eight entries take a second n-tile of mma and, as
-// fewer such groups share a phase, more preparation (measured: 1.3 of a small group), nine to twelve a third
-__host__ __device__ static inline int pb_vgroup_cost(int n) { return n <= 0 ? 0 : (n <= 4 ? 6 : (n <= 8 ? 8 : 11)); }
+// fewer such groups share a phase, more preparation (measured: 1.3 of a small group), nine to twelve a third.  tcgen05: decoding the rows, and draining
+// the columns of eight entries at a time
+__host__ __device__ static inline int pb_vgroup_cost(int n, bool tc = false) { return n <= 0 ? 0 : tc ? 8 + 3 * ((n + 7) / 8) : (n <= 4 ? 6 : (n <= 8 ? 8 : 11)); }
 struct PbExpertParams {
     const int* n_used; const int* used_e; const int* used_off;
     const int* ent_tok; const int* ent_slot; const float* ent_w;
@@ -294,6 +297,10 @@ int pb_launch_moe_combine(pb_ctx* ctx, const PbCombineParams& p);
 bool pb_moeh_supported(int type, int d, int ff, int t);
 int pb_launch_moeh_gu(pb_ctx* ctx, const PbExpertParams& p, int type, int cols);
 int pb_launch_moeh_down(pb_ctx* ctx, const PbExpertParams& p, int type, int cols);
+// pb_moetc.cu: the same for many tokens an expert, on tcgen05 (same bits)
+bool pb_moetc_supported(int type, int d, int ff);
+int pb_launch_moetc_gu(pb_ctx* ctx, const PbExpertParams& p, int cols);
+int pb_launch_moetc_down(pb_ctx* ctx, const PbExpertParams& p, int cols);
 
 // ---------------------------------------------------------------- pb_deltanet.cu
 struct PbDeltaParams {

@@ -116,9 +116,10 @@ __device__ __forceinline__ void pb_route_lists(const PbRouteParams& p, int* rsm)
     __syncthreads();
     // distinct local experts in ascending id with entry offsets: block-wide exclusive scans of
     // (used flag, entry count) over expert ids; thread t owns experts 4t .. 4t+3
-    int c4[4], f = 0, c = 0, v = 0, w = 0;   // distinct experts, entries, groups of PB_VGROUP entries, cost of the groups
+    const int vg = p.tc ? PB_VGROUP_TC : PB_VGROUP;
+    int c4[4], f = 0, c = 0, v = 0, w = 0;   // distinct experts, entries, groups of up to vg entries, cost of the groups
 #pragma unroll
-    for (int q = 0; q < 4; q++) { const int e = 4 * tid + q; c4[q] = e < p.n_exp ? cnt[e] : 0; f += c4[q] > 0; c += c4[q]; v += (c4[q] + PB_VGROUP - 1) / PB_VGROUP; w += c4[q] / PB_VGROUP * pb_vgroup_cost(PB_VGROUP) + pb_vgroup_cost(c4[q] % PB_VGROUP); }
+    for (int q = 0; q < 4; q++) { const int e = 4 * tid + q; c4[q] = e < p.n_exp ? cnt[e] : 0; f += c4[q] > 0; c += c4[q]; v += (c4[q] + vg - 1) / vg; w += c4[q] / vg * pb_vgroup_cost(vg, p.tc) + pb_vgroup_cost(c4[q] % vg, p.tc); }
     int fi = f, ci = c, vi = v, wi = w;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -142,7 +143,7 @@ __device__ __forceinline__ void pb_route_lists(const PbRouteParams& p, int* rsm)
         if (c4[q] > 0) {
             const int e = 4 * tid + q;
             p.used_e[n] = e; p.used_off[n] = off; cursor[e] = off;
-            if (p.virt) for (int k = 0; k < c4[q]; k += PB_VGROUP) { const int z = min(PB_VGROUP, c4[q] - k); p.virt[vn++] = make_int4(e, off + k, z, wn); wn += pb_vgroup_cost(z); }
+            if (p.virt) for (int k = 0; k < c4[q]; k += vg) { const int z = min(vg, c4[q] - k); p.virt[vn++] = make_int4(e, off + k, z, wn); wn += pb_vgroup_cost(z, p.tc); }
             n++; off += c4[q];
         }
     if (tid == NTHR - 1) { p.used_off[n] = off; *p.n_used = n; if (p.virt) *p.n_virt = vn; }

@@ -63,3 +63,25 @@ def test_several_chunks_in_one_pass(ctx, n):
     assert a.decode_greedy([5], 8)[0].tolist() == b.decode_greedy([5], 8)[0].tolist()
     assert ctx.device_status() == 0
     a.destroy(); b.destroy(); m.destroy()
+
+
+@pytest.mark.parametrize("t", [31, 32, 97, 161])
+def test_expert_groups_of_many_entries(ctx, t):
+    """16 experts, 4 per token: around the number of tokens from which the tcgen05 kernels take over, and groups of up to 24 entries with ragged ends; the
+    first tokens' results are those of a call of two tokens, bit for bit."""
+    import oracle
+    cfg = small_cfg(pb, n_layers=1, full_every=0)
+    spec = synth.model_spec(cfg, 8)
+    m = synth.build_model(ctx, cfg, spec, 8)
+    _, mats = oracle_model(cfg, spec, 8)
+    st = m.new_state(t)
+    x = np.random.default_rng(t).standard_normal((t, cfg.d)).astype(np.float32)
+    y, sel = st.moe_forward(0, x)
+    yo, selo, _ = oracle.moe(oracle_cfg(cfg), *(mats[(0, r)] for r in ("ROUTER", "EXP_GATE", "EXP_UP", "EXP_DOWN", "SH_GATE", "SH_UP", "SH_DOWN", "SH_GATE_INP")), x)
+    assert np.array_equal(np.sort(sel, axis=1), np.sort(selo, axis=1))
+    assert rel_err(y, yo) < 1e-5
+    for i in range(0, t - 1, 2):
+        y1, _ = st.moe_forward(0, x[i:i + 2])
+        assert np.array_equal(y1.view(np.uint32), y[i:i + 2].view(np.uint32)), i
+    assert ctx.device_status() == 0
+    st.destroy(); m.destroy()
