@@ -1907,6 +1907,7 @@ int pb_moe_forward(pb_state* s, int layer, const float* x_host, int t, float* y_
     if (t == 0) return PB_OK;
     const size_t xb = (size_t)t * c.d * 4, sb = (size_t)t * c.top_k * 4, yoff = xb + ((sb + 255) & ~(size_t)255);   // places in the staging buffer: x, sel, y
     bool ys = false, ss = false;
+    PbChain chain(ctx);
     PB_TRY(pb_h2d(ctx, s->xin, x_host, xb, 0));
     PB_TRY(run_moe(s, layer, s->xin, nullptr, t, s->yout, c.d, 0));
     if (sel_host) PB_TRY(pb_d2h(ctx, sel_host, s->sel_e, sb, xb, &ss));

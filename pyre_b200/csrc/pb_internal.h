@@ -125,6 +125,14 @@ static inline void pb_launch_kc(pb_ctx* ctx, K kern, dim3 grid, dim3 block, size
 template <typename K, typename... A>
 static inline void pb_launch_k(pb_ctx* ctx, K kern, dim3 grid, dim3 block, size_t smem, A... args) { pb_launch_kc(ctx, kern, grid, block, smem, 1, args...); }
 
+// The launches of one call are a chain of dependent launches: a kernel's set-up and first weights overlap the one before it.  The first is an ordinary launch,
+// and so is what the caller launches next.
+struct PbChain {
+    pb_ctx* c;
+    explicit PbChain(pb_ctx* x) : c(x) { if (c->pdl_scope++ == 0) c->pdl_chain = false; }
+    ~PbChain() { if (--c->pdl_scope == 0) c->pdl_chain = false; }
+};
+
 // Raise the kernel's dynamic shared-memory limit on this context's device when `smem` exceeds what was set before.  The limit belongs to
 // the device's copy of the function, which all contexts on that device share: it only ever grows (pb_api.cu).
 int pb_ensure_smem_fn(pb_ctx* ctx, const void* kern, size_t smem);
