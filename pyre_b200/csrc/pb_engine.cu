@@ -892,9 +892,6 @@ static int run_moe(pb_state* s, int il, const float* x_in, const float* norm_w, 
     const bool moetc = moeh && expert_tc(m, il, tt);
     q.tc = moetc;
     if (moeh) { r.scale_out = s->tok_scale; q.virt = s->virt; q.n_virt = s->n_used + 1; } else r.xq_out = s->xq;
-    // prompts take the GEMM form at any length from 16 tokens on, so that a token's logits do not depend on the pass it is in; it is the shorter one
-    // from about 128 tokens on (us, GEMM / the other: 34 / 26 at 32 tokens, 47 / 48 at 128, 187 / 232 at 1024)
-    r.gemm = (s->win_t >= 16 && !s->win_ckpt) || (s->win_t == 0 && tt >= 128);
     const float* logits; int64_t ldl;
     if (sh) {
         // router logits of the local tokens, written next to a copy of their residual rows; one all-gather

@@ -242,7 +242,6 @@ struct PbRouterParams {
     float* logits; int64_t ldl;               // [t][ldl >= n_exp + 1], entry n_exp = shared-gate logit
     uint32_t* xq_out;                         // [t][pb_xq_words(cols)] int8-split activations, or null
     float* scale_out;                         // [t] RMS scales for the tensor-core expert kernels, or null
-    int gemm;                                 // the tokens of a prompt, or many: the product as a GEMM (pb_router_gemm_kernel) where it takes the call
     // phase 0: everything.  Sharded tokens split it around the all-gather: phase 1 = logits of the local
     // tokens plus a raw copy of their rows into xcopy (row stride ldl); phase 2 = split + routing of all
     // gathered tokens (no GEMV)

@@ -95,21 +95,20 @@ __device__ __forceinline__ void pb_route_token_cta(const PbRouteParams& p, int b
     __syncthreads();
 }
 
-// Runs in ONE CTA of NTHR >= 256 threads (the last router CTA to finish) once every token is routed: the list of distinct local
+// Runs in ONE CTA of 256 threads (the last router CTA to finish) once every token is routed: the list of distinct local
 // experts with their (token, slot) entries.  rsm = 2048 ints of shared memory.
-template <int NTHR>
 __device__ __forceinline__ void pb_route_lists(const PbRouteParams& p, int* rsm) {
     int* cnt = rsm;                 // [1024] entries per expert (local experts only)
     int* cursor = rsm + 1024;       // [1024] start offset of the expert's entries, then a fill cursor
-    __shared__ int wsum[4][NTHR / 32];
+    __shared__ int wsum[4][8];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int e = tid; e < 1024; e += NTHR) { cnt[e] = 0; cursor[e] = 0; }
+    for (int e = tid; e < 1024; e += 256) { cnt[e] = 0; cursor[e] = 0; }
     __syncthreads();
     const int nsel = p.t * p.top_k;
-    for (int i0 = tid; i0 < nsel; i0 += NTHR * 8) {   // eight selections a thread are requested together
+    for (int i0 = tid; i0 < nsel; i0 += 256 * 8) {   // eight selections a thread are requested together
         int e[8];
 #pragma unroll
-        for (int u = 0; u < 8; u++) e[u] = i0 + NTHR * u < nsel ? __ldcg(p.sel_e + i0 + NTHR * u) : -1;
+        for (int u = 0; u < 8; u++) e[u] = i0 + 256 * u < nsel ? __ldcg(p.sel_e + i0 + 256 * u) : -1;
 #pragma unroll
         for (int u = 0; u < 8; u++) if (e[u] >= p.e_lo && e[u] < p.e_hi) atomicAdd(&cnt[e[u]], 1);
     }
@@ -146,15 +145,15 @@ __device__ __forceinline__ void pb_route_lists(const PbRouteParams& p, int* rsm)
             if (p.virt) for (int k = 0; k < c4[q]; k += vg) { const int z = min(vg, c4[q] - k); p.virt[vn++] = make_int4(e, off + k, z, wn); wn += pb_vgroup_cost(z, p.tc); }
             n++; off += c4[q];
         }
-    if (tid == NTHR - 1) { p.used_off[n] = off; *p.n_used = n; if (p.virt) *p.n_virt = vn; }
+    if (tid == 255) { p.used_off[n] = off; *p.n_used = n; if (p.virt) *p.n_virt = vn; }
     __syncthreads();
-    for (int i0 = tid; i0 < nsel; i0 += NTHR * 8) {
+    for (int i0 = tid; i0 < nsel; i0 += 256 * 8) {
         int e[8]; float w[8];
 #pragma unroll
-        for (int u = 0; u < 8; u++) { const int i = i0 + NTHR * u; e[u] = i < nsel ? __ldcg(p.sel_e + i) : -1; w[u] = i < nsel ? __ldcg(p.sel_w + i) : 0.f; }
+        for (int u = 0; u < 8; u++) { const int i = i0 + 256 * u; e[u] = i < nsel ? __ldcg(p.sel_e + i) : -1; w[u] = i < nsel ? __ldcg(p.sel_w + i) : 0.f; }
 #pragma unroll
         for (int u = 0; u < 8; u++)
-            if (e[u] >= p.e_lo && e[u] < p.e_hi) { const int i = i0 + NTHR * u, pos = atomicAdd(&cursor[e[u]], 1); p.ent_tok[pos] = i / p.top_k; p.ent_slot[pos] = i % p.top_k; p.ent_w[pos] = w[u]; }
+            if (e[u] >= p.e_lo && e[u] < p.e_hi) { const int i = i0 + 256 * u, pos = atomicAdd(&cursor[e[u]], 1); p.ent_tok[pos] = i / p.top_k; p.ent_slot[pos] = i % p.top_k; p.ent_w[pos] = w[u]; }
     }
 }
 
@@ -163,7 +162,7 @@ __device__ __forceinline__ void pb_route_lists(const PbRouteParams& p, int* rsm)
 // grid: ceil((n_exp + 1) / 8) CTAs of 256 threads; warp per router row (row n_exp = shared-gate vector).
 // CTA j additionally splits groups 4j..4j+3 of every token's normalized activations into int8
 // levels for the expert kernels, so that work is spread over the grid.
-#define PB_ROUTER_TPG 8   // tokens per router CTA (one warp each for the RMS scales)
+#define PB_ROUTER_TPG 8   // tokens per router CTA (one warp each for the RMS scales; 32 for many tokens: 1024 232 -> 221 us, but 333 88 -> 105 and 128 48 -> 59)
 #define PB_ROUTER_TICKETS 8   // ticket[0 .. 8): whole-launch counters (router, expert kernels); ticket[8 + g]: token group g of the router
 template <bool QUADS>
 __global__ void __launch_bounds__(256) pb_router_kernel(const PbRouterParams p, const PbRouteParams rp, unsigned int* ticket) {
@@ -334,144 +333,7 @@ __global__ void __launch_bounds__(256) pb_router_kernel(const PbRouterParams p, 
             if (local) { rp.used_e[n] = e; rp.used_off[n] = n; rp.ent_tok[n] = 0; rp.ent_slot[n] = lane; rp.ent_w[n] = __ldcg(rp.sel_w + lane); }
             if (lane == 0) { const int tot = __popc(m); rp.used_off[tot] = tot; *rp.n_used = tot; }
         }
-    } else pb_route_lists<256>(rp, reinterpret_cast<int*>(rs));
-    __syncthreads();
-    pb_stamp(p.stamps, 7, tid == 0);
-}
-
-template <int N> struct PbWidth { static constexpr int value = N; };
-
-// Router of the tokens of a prompt and of many tokens, at the model's width (2048): the product as an f32 GEMM, logits[t][e] = scale[t] * sum_c w[e][c] (x[t][c] n[c]).
-// A cluster of eight CTAs owns up to 128 tokens x 64 rows of the router (row n_exp = the shared-gate vector), each CTA 256 of the columns; its sixteen
-// warps take a quarter of the tokens (every fourth) x sixteen rows, a lane four tokens x four rows, and the CTAs' sums are added in column order through
-// distributed shared memory: a token's logits do not depend on how many tokens there are.  The last cluster of a token tile routes its tokens, a warp
-// each, the last of those builds the expert lists (as in pb_router_kernel).
-// Bound: f32 multiply-adds and the shared-memory reads that feed them (t = 1024: 1.08 G multiply-adds, 30 us at one per lane and cycle).  The
-// kernel above fetches the token rows from L2 for every eight router rows: 232 us at 1024 tokens, 48 at 128, 26 at 32; this one 187, 47 and 34.
-#define RG_TOK 128
-#define RG_EXP 64
-#define RG_LD 260            // floats of a row of 256 columns in shared memory: consecutive rows start 16 bytes apart modulo the banks
-#define RG_CL 8
-#define RG_THREADS 512
-__device__ __forceinline__ void rg_cluster_sync() { __syncwarp(); asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t rg_remote(uint32_t saddr, int rank) {
-    uint32_t a, v;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
-    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-    return v;
-}
-// grid (RG_CL * router tiles, token tiles)
-__global__ void __launch_bounds__(RG_THREADS, 1) pb_router_gemm_kernel(const PbRouterParams p, const PbRouteParams rp, unsigned int* ticket) {
-    extern __shared__ __align__(16) float rs[];
-    float* ws = rs;                              // [RG_EXP][RG_LD] router rows; then the routing pass
-    float* xs = rs + RG_EXP * RG_LD;             // [tokens][RG_LD] token rows times the norm weight; then the CTA's sums [RG_TOK][RG_EXP]
-    __shared__ float ssq[RG_TOK][2];             // sums of squares of the token rows' columns, by halves
-    __shared__ unsigned flag;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = (int)blockIdx.x % RG_CL, tile = (int)blockIdx.x / RG_CL;
-    const int e0 = tile * RG_EXP, t0 = (int)blockIdx.y * RG_TOK, c0 = rank * 256, nt = min(RG_TOK, p.t - t0);
-    const bool st_first = tid == 0 && blockIdx.x == 0 && blockIdx.y == 0;
-    pb_stamp(p.stamps, 0, st_first);
-    // router rows: model data, on their way before the previous kernel ends
-#pragma unroll
-    for (int j = 0; j < RG_EXP * 64 / RG_THREADS; j++) {
-        const int r = (tid >> 6) + RG_THREADS / 64 * j, c = (tid & 63) * 4, e = e0 + r;
-        if (e <= p.n_exp) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(pb_smem_u32(ws + r * RG_LD + c)), "l"((e < p.n_exp ? p.router + (size_t)e * p.cols : p.sh_gate_inp) + c0 + c) : "memory");
-        else *reinterpret_cast<float4*>(ws + r * RG_LD + c) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    float4 nw = make_float4(1.f, 1.f, 1.f, 1.f);
-    if (p.norm_w) nw = *reinterpret_cast<const float4*>(p.norm_w + c0 + (tid & 63) * 4);   // the thread's four columns, of every row it loads
-    pb_pdl_wait();
-    pb_pdl_trigger();
-    pb_stamp(p.stamps, 2, st_first);
-    // rows in rounds of 32, four requested together (a warp and a half of a row: no row is split inside a warp)
-    for (int r0 = tid >> 6; r0 < nt; r0 += 32) {
-        float4 v[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) v[j] = r0 + 8 * j < nt ? *reinterpret_cast<const float4*>(p.x + (size_t)(t0 + r0 + 8 * j) * p.ldx + c0 + (tid & 63) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int r = r0 + 8 * j;
-            const float q = pb_warp_sum(fmaf(v[j].x, v[j].x, fmaf(v[j].y, v[j].y, fmaf(v[j].z, v[j].z, __fmul_rn(v[j].w, v[j].w)))));
-            if (lane == 0) ssq[r][warp & 1] = q;
-            *reinterpret_cast<float4*>(xs + r * RG_LD + (tid & 63) * 4) = make_float4(v[j].x * nw.x, v[j].y * nw.y, v[j].z * nw.z, v[j].w * nw.w);
-        }
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-    // tokens tg + 4 (lr + 8 i), rows 16 eg + lc + 4 j
-    const int tg = warp & 3, eg = warp >> 2, lr = lane >> 2, lc = lane & 3, ni = (nt + 31) / 32;
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
-    const float *xa = xs + (tg + 4 * lr) * RG_LD, *wa = ws + (16 * eg + lc) * RG_LD;
-    auto product = [&](auto width) {
-        constexpr int NI = decltype(width)::value;
-#pragma unroll 2
-        for (int k = 0; k < 256; k += 4) {
-            float4 a[NI], b[4];
-#pragma unroll
-            for (int i = 0; i < NI; i++) a[i] = *reinterpret_cast<const float4*>(xa + 32 * i * RG_LD + k);
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = *reinterpret_cast<const float4*>(wa + 4 * j * RG_LD + k);
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-#pragma unroll
-                for (int i = 0; i < NI; i++) acc[i][j] = fmaf(b[j].w, a[i].w, fmaf(b[j].z, a[i].z, fmaf(b[j].y, a[i].y, fmaf(b[j].x, a[i].x, acc[i][j]))));
-        }
-    };
-    if (ni == 1) product(PbWidth<1>()); else if (ni == 2) product(PbWidth<2>()); else if (ni == 3) product(PbWidth<3>()); else product(PbWidth<4>());
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) if (i < ni) xs[(tg + 4 * (lr + 8 * i)) * RG_EXP + 16 * eg + lc + 4 * j] = acc[i][j];
-    rg_cluster_sync();
-    // this CTA adds up every eighth token
-    for (int o = tid; o < (nt + RG_CL - 1 - rank) / RG_CL * RG_EXP; o += RG_THREADS) {
-        const int r = o / RG_EXP * RG_CL + rank, e = e0 + o % RG_EXP, t = t0 + r;
-        float v = 0.f, s = 1.0f;
-#pragma unroll
-        for (int c = 0; c < RG_CL; c++) v += __uint_as_float(rg_remote(pb_smem_u32(xs + r * RG_EXP + o % RG_EXP), c));
-        if (p.norm_w) {
-            float q = 0.f;
-#pragma unroll
-            for (int c = 0; c < RG_CL; c++) q += __uint_as_float(rg_remote(pb_smem_u32(&ssq[r][0]), c)) + __uint_as_float(rg_remote(pb_smem_u32(&ssq[r][1]), c));
-            s = 1.0f / sqrtf(q / (float)p.cols + p.eps);
-        }
-        if (e <= p.n_exp) p.logits[(size_t)t * p.ldl + e] = v * s;
-        if (p.scale_out && tile == 0 && o % RG_EXP == 0) p.scale_out[t] = s;
-    }
-    __threadfence();
-    pb_stamp(p.stamps, 5, st_first);
-    rg_cluster_sync();                           // the cluster's logits are stored, and nobody reads its sums any more
-    const int ntiles = (int)gridDim.x / RG_CL;
-    if (rank == 0 && tid == 0) { __threadfence(); flag = atomicAdd(ticket + PB_ROUTER_TICKETS + blockIdx.y, 1u) == (unsigned)ntiles - 1; }
-    rg_cluster_sync();
-    const bool last = rg_remote(pb_smem_u32(&flag), 0) != 0;
-    if (last) {
-        __threadfence();
-        for (int r = rank + RG_CL * warp; r < nt; r += RG_TOK) {
-            const int b = t0 + r;
-            int my_e, rk; float w;
-            pb_route_token(rp.logits + (size_t)b * rp.ldl, rp.n_exp, rp.top_k, lane, my_e, w, rk);
-            if (lane < rp.top_k) { rp.sel_e[b * rp.top_k + rk] = my_e; rp.sel_w[b * rp.top_k + rk] = w; }
-        }
-        __threadfence();
-    }
-    rg_cluster_sync();                           // (rank 0 stays until its flag was read)
-    if (!last || rank != 0) return;
-    if (tid == 0) {
-        __threadfence();
-        ticket[PB_ROUTER_TICKETS + blockIdx.y] = 0;
-        flag = atomicAdd(ticket, 1u) == gridDim.y - 1;
-        if (flag) *ticket = 0;
-    }
-    __syncthreads();
-    if (!flag) return;
-    __threadfence();
-    pb_route_lists<RG_THREADS>(rp, reinterpret_cast<int*>(ws));
+    } else pb_route_lists(rp, reinterpret_cast<int*>(rs));
     __syncthreads();
     pb_stamp(p.stamps, 7, tid == 0);
 }
@@ -965,14 +827,6 @@ int pb_launch_router(pb_ctx* ctx, const PbRouterParams& p, const PbRouteParams& 
     PbRouterParams ps = p;
     ps.stamps = pb_stamp_slot(ctx, PB_K_ROUTER);
     const dim3 gd(grid, (p.t + PB_ROUTER_TPG - 1) / PB_ROUTER_TPG);
-    if (p.gemm && p.cols == 2048 && p.phase == 0 && !p.xq_out && !p.zero && !((uintptr_t)p.x & 15) && !(p.ldx & 3)) {
-        const size_t gsm = (size_t)(((p.t < RG_TOK ? (p.t + 31) & ~31 : RG_TOK)) + RG_EXP) * RG_LD * 4;   // (rows in rounds of 32)
-        PB_TRY(pb_ensure_smem(ctx, pb_router_gemm_kernel, gsm));
-        pb_launch_kc(ctx, pb_router_gemm_kernel, dim3(RG_CL * ((p.n_exp + 1 + RG_EXP - 1) / RG_EXP), (p.t + RG_TOK - 1) / RG_TOK), dim3(RG_THREADS), gsm, RG_CL, ps, rp, ticket);
-        ctx->kernels_launched++;
-        PB_CUDA(ctx, cudaGetLastError());
-        return PB_OK;
-    }
     // several tokens of the model's width: four rows x a quarter of the columns per warp
     if (p.cols == 2048 && p.phase != 2 && p.t > 1) pb_launch_k(ctx, pb_router_kernel<true>, gd, dim3(256), smem, ps, rp, ticket);
     else pb_launch_k(ctx, pb_router_kernel<false>, gd, dim3(256), smem, ps, rp, ticket);

@@ -1,4 +1,4 @@
-"""Prompt passes and the kernels that only they and large batches reach: runs of the DeltaNet recurrence in blocks of eight tokens, the router as a GEMM,
+"""Prompt passes and the kernels that only they and large batches reach: runs of the DeltaNet recurrence in blocks of eight tokens, the router and its lists for many tokens,
 several prompt chunks in one pass, expert groups of up to 24 entries."""
 import numpy as np
 import pytest
@@ -30,8 +30,9 @@ def test_deltanet_blocks_of_tokens(ctx, n):
 
 
 @pytest.mark.parametrize("t", [128, 131, 261])
-def test_router_as_a_gemm(ctx, t):
-    """70 experts (a ragged second tile of router rows), one, two and three token tiles, the last with a few tokens: selection and block against the oracle."""
+def test_router_of_many_tokens(ctx, t):
+    """70 experts (a ragged last group of router rows), the last group of tokens full and ragged: selection and block
+    against the oracle; the first tokens' results are those of a call of two tokens, bit for bit."""
     import oracle
     cfg = small_cfg(pb, n_layers=1, full_every=0, d=2048, n_exp=70)
     spec = synth.model_spec(cfg, 6)
@@ -43,6 +44,8 @@ def test_router_as_a_gemm(ctx, t):
     yo, selo, _ = oracle.moe(oracle_cfg(cfg), *(mats[(0, r)] for r in ("ROUTER", "EXP_GATE", "EXP_UP", "EXP_DOWN", "SH_GATE", "SH_UP", "SH_DOWN", "SH_GATE_INP")), x)
     assert np.array_equal(np.sort(sel, axis=1), np.sort(selo, axis=1))
     assert rel_err(y, yo) < 1e-5
+    y1, _ = st.moe_forward(0, x[:2])
+    assert np.array_equal(y1.view(np.uint32), y[:2].view(np.uint32))
     assert ctx.device_status() == 0
     st.destroy(); m.destroy()
 
