@@ -260,19 +260,20 @@ __global__ void __launch_bounds__(128) pb_deltanet_run_kernel(const PbDeltaParam
 //   g_t S_{t-1}^T k_t = G_t (S_0^T k_t) + sum_{s<t} (G_t / G_s) (k_s.k_t) delta_s,     G_t = g_0 .. g_t
 // so the sixteen products S_0^T k_t and S_0^T q_t of a block are formed from the state as the block found it, without waiting for one another,
 // then a triangular system of eight unknowns per column is solved by substitution, and the state takes its eight rank-one updates at once.  A
-// warp holds four columns, its lanes eight groups of sixteen rows x four columns; eight warps an SM.  What bounds it: issue slots (the token-by-token
-// walk is bound by the latency of one token).  1024 tokens of 32 heads of 128 x 128: 344 us token by token, 238 in blocks (four warps of eight
-// columns each: 245).  A token's values never enter an earlier token's: the sums run over s < t only.
+// warp holds eight columns, its lanes eight groups of sixteen rows x four pairs of columns; k of the block stays in registers from the products to the
+// update.  What bounds it: the instructions of one warp per scheduler and the reads of k and q from shared memory (the token-by-token walk: the
+// latency of one token).  1024 tokens of 32 heads of 128 x 128: 344 us token by token, 232 in blocks (eight warps of four columns, k read twice: 242).
+// A token's values never enter an earlier token's: the sums run over s < t only.
 #define DB_C 8               // tokens of a block
-__global__ void __launch_bounds__(256) pb_deltanet_block_kernel(const PbDeltaParams p, int T, const PbDeltaRun r) {
-    constexpr int DK = 128, C = DB_C, NT = 256;
+__global__ void __launch_bounds__(128, 1) pb_deltanet_block_kernel(const PbDeltaParams p, int T, const PbDeltaRun r) {
+    constexpr int DK = 128, C = DB_C, NT = 128;
     const int nk = p.nk, nv = p.nv, dv = p.dv;
     const int splits = dv / DN_COLS, h = blockIdx.x / splits, j0 = (blockIdx.x % splits) * DN_COLS, kh = h % nk;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = lane >> 2, col = lane & 3;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = lane >> 2, cp = lane & 3;
     struct __align__(16) In { float qk[C][2 * DK]; float v[C][DN_COLS]; float gram[2 * C * C]; float2 gb[C]; };
     __shared__ In in[2];
     __shared__ __align__(16) float mat[2][C][C], dec[2][C];            // decayed products (k.k, q.k); G_t and G_7 / G_s
-    __shared__ __align__(16) float ab[8][2][4][C], del[8][C][4];       // per warp: S^T k and S^T q of its columns, corrections
+    __shared__ __align__(16) float ab[4][2][8][C], del[4][C][8];       // per warp: S^T k and S^T q of its columns, corrections
     pb_pdl_wait();
     pb_pdl_trigger();
     auto fetch = [&](int t0, int buf) {
@@ -296,13 +297,14 @@ __global__ void __launch_bounds__(256) pb_deltanet_block_kernel(const PbDeltaPar
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     fetch(0, 0);
-    // the lane's rows 32 j + 4 rg + {0..3}, j = 0..3, of its column, as pairs of rows
-    float* S = p.ssm + ((size_t)h * DK) * dv + j0 + 4 * warp + col;
-    unsigned long long s[8];
+    // the lane's rows 32 j + 4 rg + {0..3}, j = 0..3, of its two columns, as pairs of rows
+    float* S = p.ssm + ((size_t)h * DK) * dv + j0 + 8 * warp + 2 * cp;
+    unsigned long long s[2][8];
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int row = 32 * (i >> 1) + 4 * rg + 2 * (i & 1);
-        s[i] = pb_f2(S[(size_t)row * dv], S[(size_t)(row + 1) * dv]);
+        const float2 a = *reinterpret_cast<const float2*>(S + (size_t)row * dv), b = *reinterpret_cast<const float2*>(S + (size_t)(row + 1) * dv);
+        s[0][i] = pb_f2(a.x, b.x); s[1][i] = pb_f2(a.y, b.y);
     }
     int buf = 0;
     for (int t0 = 0; t0 < T; t0 += C, buf ^= 1) {
@@ -311,47 +313,57 @@ __global__ void __launch_bounds__(256) pb_deltanet_block_kernel(const PbDeltaPar
         if (t0 + C < T) fetch(t0 + C, buf ^ 1);
         const In& d = in[buf];
         const int n = min(C, T - t0);
-        if (tid < 2 * C * C) {   // thread (t, which, s): the product decayed from s to t; then G_t and G_7 / G_s
+        {   // thread (t, which, s): the product decayed from s to t; then G_t and G_7 / G_s
             const int t = tid >> 4, which = (tid >> 3) & 1, q = tid & 7;
             float f = 1.f;
 #pragma unroll
             for (int i = 1; i < C; i++) if (i > q && i <= t) f *= d.gb[i].x;
             mat[which][t][q] = f * d.gram[which * C * C + t * C + q];   // (the entries that are read: s < t, or s <= t for q.k)
-        } else if (tid < 2 * C * C + 2 * C) {
-            const int which = (tid >> 3) & 1, q = tid & 7;
-            float e = 1.f;
+            if (tid < 2 * C) {
+                float e = 1.f;
 #pragma unroll
-            for (int i = 0; i < C; i++) if (which == 0 ? i <= q : i > q) e *= d.gb[i].x;
-            dec[which][q] = e;
+                for (int i = 0; i < C; i++) if (which == 0 ? i <= q : i > q) e *= d.gb[i].x;
+                dec[which][q] = e;
+            }
         }
         // S_0^T k_t and S_0^T q_t of the lane's rows, all of the block before anything is summed over the lanes
-        float v[2][C];
+        ulonglong2 k[C][4];
+        float v[2][C][2];
 #pragma unroll
         for (int t = 0; t < C; t++) {
-            unsigned long long a[2] = {0ull, 0ull}, b[2] = {0ull, 0ull};
+            ulonglong2 q[4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(&d.qk[t][32 * j + 4 * rg]), k = *reinterpret_cast<const ulonglong2*>(&d.qk[t][DK + 32 * j + 4 * rg]);
-                a[0] = j ? pb_fma2(s[2 * j], k.x, a[0]) : pb_mul2(s[0], k.x); a[1] = j ? pb_fma2(s[2 * j + 1], k.y, a[1]) : pb_mul2(s[1], k.y);
-                b[0] = j ? pb_fma2(s[2 * j], q.x, b[0]) : pb_mul2(s[0], q.x); b[1] = j ? pb_fma2(s[2 * j + 1], q.y, b[1]) : pb_mul2(s[1], q.y);
+            for (int j = 0; j < 4; j++) { q[j] = *reinterpret_cast<const ulonglong2*>(&d.qk[t][32 * j + 4 * rg]); k[t][j] = *reinterpret_cast<const ulonglong2*>(&d.qk[t][DK + 32 * j + 4 * rg]); }
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                unsigned long long a[2], b[2];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    a[0] = j ? pb_fma2(s[c][2 * j], k[t][j].x, a[0]) : pb_mul2(s[c][0], k[t][0].x); a[1] = j ? pb_fma2(s[c][2 * j + 1], k[t][j].y, a[1]) : pb_mul2(s[c][1], k[t][0].y);
+                    b[0] = j ? pb_fma2(s[c][2 * j], q[j].x, b[0]) : pb_mul2(s[c][0], q[0].x); b[1] = j ? pb_fma2(s[c][2 * j + 1], q[j].y, b[1]) : pb_mul2(s[c][1], q[0].y);
+                }
+                const float2 x = pb_f2_get(pb_add2(a[0], a[1])), y = pb_f2_get(pb_add2(b[0], b[1]));
+                v[0][t][c] = x.x + x.y; v[1][t][c] = y.x + y.y;
             }
-            const float2 x = pb_f2_get(pb_add2(a[0], a[1])), y = pb_f2_get(pb_add2(b[0], b[1]));
-            v[0][t] = x.x + x.y; v[1][t] = y.x + y.y;
         }
         {   // sums over the eight row groups (lane bits 2 .. 4): bit 4 keeps k or q, bit 3 half of the tokens, bit 2 a quarter
             const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
-            float w[C], u[C / 2], z[C / 4];
 #pragma unroll
-            for (int t = 0; t < C; t++) w[t] = (b4 ? v[1][t] : v[0][t]) + __shfl_xor_sync(0xffffffffu, b4 ? v[0][t] : v[1][t], 16);
+            for (int c = 0; c < 2; c++) {
+                float w[C], u[C / 2], z[C / 4];
 #pragma unroll
-            for (int t = 0; t < C / 2; t++) u[t] = (b3 ? w[t + 4] : w[t]) + __shfl_xor_sync(0xffffffffu, b3 ? w[t] : w[t + 4], 8);
+                for (int t = 0; t < C; t++) w[t] = (b4 ? v[1][t][c] : v[0][t][c]) + __shfl_xor_sync(0xffffffffu, b4 ? v[0][t][c] : v[1][t][c], 16);
 #pragma unroll
-            for (int t = 0; t < C / 4; t++) z[t] = (b2 ? u[t + 2] : u[t]) + __shfl_xor_sync(0xffffffffu, b2 ? u[t] : u[t + 2], 4);
-            *reinterpret_cast<float2*>(&ab[warp][lane >> 4][col][(b3 ? 4 : 0) + (b2 ? 2 : 0)]) = make_float2(z[0], z[1]);
+                for (int t = 0; t < C / 2; t++) u[t] = (b3 ? w[t + 4] : w[t]) + __shfl_xor_sync(0xffffffffu, b3 ? w[t] : w[t + 4], 8);
+#pragma unroll
+                for (int t = 0; t < C / 4; t++) z[t] = (b2 ? u[t + 2] : u[t]) + __shfl_xor_sync(0xffffffffu, b2 ? u[t] : u[t + 2], 4);
+                *reinterpret_cast<float2*>(&ab[warp][lane >> 4][2 * cp + c][(b3 ? 4 : 0) + (b2 ? 2 : 0)]) = make_float2(z[0], z[1]);
+            }
         }
         __syncthreads();                                    // the tables are complete (and the warp's sums)
-        // corrections of the lane's column, all of them by each of the column's eight lanes: delta_t = (v_t - g_t mem_t) beta_t (:1663); a correction
+        // corrections of column `col` of the warp, all of them by each of the column's four lanes: delta_t = (v_t - g_t mem_t) beta_t (:1663); a correction
         // is taken out of the later tokens as soon as it is known
+        const int col = lane & 7, rr = lane >> 3;
         float de[C], m[C][C];
         {
             const float4 x = *reinterpret_cast<const float4*>(&ab[warp][0][col][0]), y = *reinterpret_cast<const float4*>(&ab[warp][0][col][4]);
@@ -361,7 +373,7 @@ __global__ void __launch_bounds__(256) pb_deltanet_block_kernel(const PbDeltaPar
             for (int t = 0; t < C; t++) {
                 if (t > 0) { const float4 o = *reinterpret_cast<const float4*>(&mat[0][t][0]); m[t][0] = o.x; m[t][1] = o.y; m[t][2] = o.z; m[t][3] = o.w; }
                 if (t > 4) { const float4 o = *reinterpret_cast<const float4*>(&mat[0][t][4]); m[t][4] = o.x; m[t][5] = o.y; m[t][6] = o.z; m[t][7] = o.w; }
-                de[t] = fmaf(-gv[t], av[t], d.v[t][4 * warp + col]);
+                de[t] = fmaf(-gv[t], av[t], d.v[t][8 * warp + col]);
             }
         }
 #pragma unroll
@@ -370,36 +382,40 @@ __global__ void __launch_bounds__(256) pb_deltanet_block_kernel(const PbDeltaPar
 #pragma unroll
             for (int q = t + 1; q < C; q++) de[q] = fmaf(-m[q][t], de[t], de[q]);
         }
-        {   // each of the column's lanes forms one of the outputs: token rg
-            const float4 x = *reinterpret_cast<const float4*>(&mat[1][rg][0]), y = *reinterpret_cast<const float4*>(&mat[1][rg][4]);
-            const float w[C] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-            float o = dec[0][rg] * ab[warp][1][col][rg], own = de[0];
 #pragma unroll
-            for (int q = 0; q < C; q++) { if (q <= rg) o = fmaf(w[q], de[q], o); if (q == rg) own = de[q]; }
-            if (rg < n) p.out[(size_t)(t0 + rg) * p.ldo + h * dv + j0 + 4 * warp + col] = o;   // readout before the gated norm
-            del[warp][rg][col] = own * dec[1][rg];
+        for (int i = 0; i < 2; i++) {   // each of the column's lanes forms two of the outputs: tokens 2 rr and 2 rr + 1
+            const int t = 2 * rr + i;
+            const float4 x = *reinterpret_cast<const float4*>(&mat[1][t][0]), y = *reinterpret_cast<const float4*>(&mat[1][t][4]);
+            const float w[C] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+            float o = dec[0][t] * ab[warp][1][col][t], own = de[0];
+#pragma unroll
+            for (int q = 0; q < C; q++) { if (q <= t) o = fmaf(w[q], de[q], o); if (q == t) own = de[q]; }
+            if (t < n) p.out[(size_t)(t0 + t) * p.ldo + h * dv + j0 + 8 * warp + col] = o;   // readout before the gated norm
+            del[warp][t][col] = own * dec[1][t];
         }
         __syncwarp();
         const float g = dec[0][C - 1];
         const unsigned long long g2 = pb_f2(g, g);
 #pragma unroll
-        for (int i = 0; i < 8; i++) s[i] = pb_mul2(s[i], g2);
+        for (int c = 0; c < 2; c++)
+#pragma unroll
+            for (int i = 0; i < 8; i++) s[c][i] = pb_mul2(s[c][i], g2);
 #pragma unroll
         for (int t = 0; t < C; t++) {
-            const float e = del[warp][t][col];
-            const unsigned long long e2 = pb_f2(e, e);
+            const float2 e = *reinterpret_cast<const float2*>(&del[warp][t][2 * cp]);
+            const unsigned long long e2[2] = {pb_f2(e.x, e.x), pb_f2(e.y, e.y)};
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(&d.qk[t][DK + 32 * j + 4 * rg]);
-                s[2 * j] = pb_fma2(k.x, e2, s[2 * j]); s[2 * j + 1] = pb_fma2(k.y, e2, s[2 * j + 1]);
-            }
+            for (int c = 0; c < 2; c++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) { s[c][2 * j] = pb_fma2(k[t][j].x, e2[c], s[c][2 * j]); s[c][2 * j + 1] = pb_fma2(k[t][j].y, e2[c], s[c][2 * j + 1]); }
         }
     }
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int row = 32 * (i >> 1) + 4 * rg + 2 * (i & 1);
-        const float2 a = pb_f2_get(s[i]);
-        S[(size_t)row * dv] = a.x; S[(size_t)(row + 1) * dv] = a.y;
+        const float2 a = pb_f2_get(s[0][i]), b = pb_f2_get(s[1][i]);
+        *reinterpret_cast<float2*>(S + (size_t)row * dv) = make_float2(a.x, b.x);
+        *reinterpret_cast<float2*>(S + (size_t)(row + 1) * dv) = make_float2(a.y, b.y);
     }
     // the conv ring keeps the last K inputs.  Channels: this slice's v columns; q and k of a K head by the first slice of the first V head that reads it
     constexpr int K = 4;
@@ -431,7 +447,7 @@ int pb_launch_deltanet_seq(pb_ctx* ctx, const PbDeltaParams& p, int T, float* sc
     PB_CUDA(ctx, cudaGetLastError());
     const dim3 grid(p.nv * (p.dv / DN_COLS));
     if (blocks) {
-        pb_launch_k(ctx, pb_deltanet_block_kernel, grid, dim3(256), (size_t)0, p, T, r);
+        pb_launch_k(ctx, pb_deltanet_block_kernel, grid, dim3(128), (size_t)0, p, T, r);
         ctx->kernels_launched++;
         PB_CUDA(ctx, cudaGetLastError());
         return PB_OK;
