@@ -873,6 +873,11 @@ static bool expert_tc(pb_model* m, int il, int t) {
     return m->ep_world == 1 && pb_moetc_supported(type, c.d, c.ff_exp) && (int64_t)t * c.top_k >= 8ll * c.n_exp;
 }
 
+// whether the warp-level kernels take groups of twelve entries: from two entries an expert on average.  Below that few experts have more than eight, and the
+// third n-tile costs all groups registers (top 10 of 512 experts, groups of 8 / 12: 32 sequences a decode step 3.95 / 4.07 ms, 10 of Q4_K 606 / 656 us, 96
+// tokens of one layer 362 / 370, 128 430 / 426, four layers of 256 tokens of Q4_K 4.19 / 4.07 ms)
+static bool expert_many(pb_model* m, int t) { return (int64_t)t * m->cfg.top_k >= 2ll * m->cfg.n_exp; }
+
 // MoE block on t tokens: x_in [t][d] (normalized when norm_w == null) -> y (stored or added)
 static int run_moe(pb_state* s, int il, const float* x_in, const float* norm_w, int t, float* y, int64_t ldy, int accumulate) {
     pb_model* m = s->m; pb_ctx* ctx = m->ctx; const pb_cfg& c = m->cfg;
@@ -890,7 +895,7 @@ static int run_moe(pb_state* s, int il, const float* x_in, const float* norm_w, 
     // two and more tokens of the formats it covers: the expert kernels on the tensor cores, which read the token rows themselves
     const bool moeh = expert_mma(m, il, tt);
     const bool moetc = moeh && expert_tc(m, il, tt);
-    q.tc = moetc;
+    q.vgroup = moetc ? PB_VGROUP_TC : expert_many(m, tt) ? PB_VGROUP_MANY : PB_VGROUP;
     if (moeh) { r.scale_out = s->tok_scale; q.virt = s->virt; q.n_virt = s->n_used + 1; } else r.xq_out = s->xq;
     const float* logits; int64_t ldl;
     if (sh) {
@@ -913,7 +918,7 @@ static int run_moe(pb_state* s, int il, const float* x_in, const float* norm_w, 
     PbExpertParams e; memset(&e, 0, sizeof e);
     e.n_used = s->n_used; e.used_e = s->used_e; e.used_off = s->used_off; e.ent_tok = s->ent_tok; e.ent_slot = s->ent_slot; e.ent_w = s->ent_w;
     e.xq = s->xq; e.h = s->h; e.h_sh = s->h_sh; e.part = s->part; e.part_sh = s->part_sh;
-    e.has_shared = 1; e.t = tt; e.top_k = c.top_k; e.n_exp = c.n_exp;
+    e.has_shared = 1; e.t = tt; e.top_k = c.top_k; e.n_exp = c.n_exp; e.vgroup = q.vgroup;
     e.sh_tok0 = tok0; e.sh_ntok = t;   // the shared expert runs where the token lives
     pb_qmat* g = M(m, il, PB_R_EXP_GATE);
     e.e_base = g->rows == (int64_t)c.ff_exp * c.n_exp ? 0 : m->e_lo;

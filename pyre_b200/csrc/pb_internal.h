@@ -258,10 +258,11 @@ struct PbRouteParams {
     int* sel_e; float* sel_w;                 // [t][top_k], ascending expert id
     int* n_used; int* used_e; int* used_off;  // distinct local experts, entry offsets [n_used + 1]
     int* ent_tok; int* ent_slot; float* ent_w;
-    int tc;                                   // groups for the tcgen05 expert kernels (PB_VGROUP_TC entries)
-    int4* virt; int* n_virt;                  // several tokens: distinct local experts in groups of up to PB_VGROUP entries {expert, first entry, entries, cost of the groups before}, and their number
+    int vgroup;                               // entries of a group at most: PB_VGROUP, PB_VGROUP_MANY or, for the tcgen05 kernels, PB_VGROUP_TC
+    int4* virt; int* n_virt;                  // several tokens: distinct local experts in groups of up to vgroup entries {expert, first entry, entries, cost of the groups before}, and their number
 };
-#define PB_VGROUP 12
+#define PB_VGROUP 8
+#define PB_VGROUP_MANY 12    // many tokens: three n-tiles of mma (pb_moeh.cu)
 #define PB_VGROUP_TC 24      // the same of the tcgen05 expert kernels (pb_moetc.cu)
 // Cost of a group of n entries in the expert kernels, in sixths of a group of up to four: five to eight entries take a second n-tile of mma and, as
 // fewer such groups share a phase, more preparation (measured: 1.3 of a small group), nine to twelve a third.  tcgen05: decoding the rows, and draining
@@ -283,6 +284,7 @@ struct PbExpertParams {
     // tensor-core kernels (pb_moeh.cu): groups of entries, raw token rows with their RMS scales and the norm weight (null: x is normalized)
     const int4* virt; const int* n_virt;
     const float* x; int64_t ldx; const float* norm_w; const float* tok_scale;
+    int vgroup;                               // entries of a group at most, as the lists were made (PbRouteParams)
     int nslots;                               // token slots of a CTA
     int nx;                                   // activation-level vectors of a chunk's first nx entries ride along with its weights
     int* status;

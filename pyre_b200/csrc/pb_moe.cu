@@ -105,7 +105,14 @@ __device__ __forceinline__ void pb_route_lists(const PbRouteParams& p, int* rsm)
     for (int e = tid; e < 1024; e += 256) { cnt[e] = 0; cursor[e] = 0; }
     __syncthreads();
     const int nsel = p.t * p.top_k;
-    for (int i0 = tid; i0 < nsel; i0 += 256 * 8) {   // eight selections a thread are requested together
+    // a few tokens: one selection a thread (the code of eight costs more than it saves: its instructions are fetched for one use)
+    if (nsel <= 512) {
+#pragma unroll 1
+        for (int i = tid; i < nsel; i += 256) {
+            const int e = __ldcg(p.sel_e + i);
+            if (e >= p.e_lo && e < p.e_hi) atomicAdd(&cnt[e], 1);
+        }
+    } else for (int i0 = tid; i0 < nsel; i0 += 256 * 8) {   // eight selections a thread are requested together
         int e[8];
 #pragma unroll
         for (int u = 0; u < 8; u++) e[u] = i0 + 256 * u < nsel ? __ldcg(p.sel_e + i0 + 256 * u) : -1;
@@ -115,10 +122,12 @@ __device__ __forceinline__ void pb_route_lists(const PbRouteParams& p, int* rsm)
     __syncthreads();
     // distinct local experts in ascending id with entry offsets: block-wide exclusive scans of
     // (used flag, entry count) over expert ids; thread t owns experts 4t .. 4t+3
-    const int vg = p.tc ? PB_VGROUP_TC : PB_VGROUP;
+    const int vg = p.vgroup;
+    const bool tc = vg == PB_VGROUP_TC;
     int c4[4], f = 0, c = 0, v = 0, w = 0;   // distinct experts, entries, groups of up to vg entries, cost of the groups
 #pragma unroll
-    for (int q = 0; q < 4; q++) { const int e = 4 * tid + q; c4[q] = e < p.n_exp ? cnt[e] : 0; f += c4[q] > 0; c += c4[q]; v += (c4[q] + vg - 1) / vg; w += c4[q] / vg * pb_vgroup_cost(vg, p.tc) + pb_vgroup_cost(c4[q] % vg, p.tc); }
+    for (int q = 0; q < 4; q++) { const int e = 4 * tid + q; c4[q] = e < p.n_exp ? cnt[e] : 0; f += c4[q] > 0; c += c4[q]; }
+    if (p.virt) for (int q = 0; q < 4; q++) for (int k = c4[q]; k > 0; k -= vg) { v++; w += pb_vgroup_cost(min(vg, k), tc); }
     int fi = f, ci = c, vi = v, wi = w;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -142,12 +151,18 @@ __device__ __forceinline__ void pb_route_lists(const PbRouteParams& p, int* rsm)
         if (c4[q] > 0) {
             const int e = 4 * tid + q;
             p.used_e[n] = e; p.used_off[n] = off; cursor[e] = off;
-            if (p.virt) for (int k = 0; k < c4[q]; k += vg) { const int z = min(vg, c4[q] - k); p.virt[vn++] = make_int4(e, off + k, z, wn); wn += pb_vgroup_cost(z, p.tc); }
+            if (p.virt) for (int k = 0; k < c4[q]; k += vg) { const int z = min(vg, c4[q] - k); p.virt[vn++] = make_int4(e, off + k, z, wn); wn += pb_vgroup_cost(z, tc); }
             n++; off += c4[q];
         }
     if (tid == 255) { p.used_off[n] = off; *p.n_used = n; if (p.virt) *p.n_virt = vn; }
     __syncthreads();
-    for (int i0 = tid; i0 < nsel; i0 += 256 * 8) {
+    if (nsel <= 512) {
+#pragma unroll 1
+        for (int i = tid; i < nsel; i += 256) {
+            const int e = __ldcg(p.sel_e + i);
+            if (e >= p.e_lo && e < p.e_hi) { const int pos = atomicAdd(&cursor[e], 1); p.ent_tok[pos] = i / p.top_k; p.ent_slot[pos] = i % p.top_k; p.ent_w[pos] = __ldcg(p.sel_w + i); }
+        }
+    } else for (int i0 = tid; i0 < nsel; i0 += 256 * 8) {
         int e[8]; float w[8];
 #pragma unroll
         for (int u = 0; u < 8; u++) { const int i = i0 + 256 * u; e[u] = i < nsel ? __ldcg(p.sel_e + i) : -1; w[u] = i < nsel ? __ldcg(p.sel_w + i) : 0.f; }
