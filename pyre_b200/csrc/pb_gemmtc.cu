@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
         bool ok = true;
         for (int k = 0; k < nk && ok; k++) {
             const int st = k % NST;
-            ok = __all_sync(0xffffffffu, pb_mbar_wait(&full[st], (k / NST) & 1, p.status, PB_DEV_TC_TIMEOUT));
+            ok = tc_warp_wait(&full[st], (k / NST) & 1, p.status);
             if (!ok) break;
             tc_fence_after();
             if (elected) {
@@ -308,24 +308,24 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
             const int st = k % NST, kb = k >> 2, rs = kb % TC_RAW_STAGES;
             // this group's steps of a block are quarters grp and grp + 2: wait for the bytes at the first; after the second,
             // release the buffer and -- once all 256 threads have released it -- refill it
-            if ((k & 3) == grp && !pb_mbar_wait(&raw_full[rs], (kb / TC_RAW_STAGES) & 1, p.status, PB_DEV_TC_TIMEOUT)) { ok = false; break; }
+            if ((k & 3) == grp && !tc_warp_wait(&raw_full[rs], (kb / TC_RAW_STAGES) & 1, p.status)) { ok = false; break; }
             TcRaw cur;
             tc_load_raw(cur, pb_smem_u32(raw + (size_t)rs * TC_RAW_BYTES) + (uint32_t)(row >> 3) * 1088u, row & 7, k & 3, live);
             if ((k & 3) == grp + 2) {
                 tc_warp_arrive(&raw_empty[rs], lane);
                 if (kb + TC_RAW_STAGES < nkb) {
-                    if (!pb_mbar_wait(&raw_empty[rs], (kb / TC_RAW_STAGES) & 1, p.status, PB_DEV_TC_TIMEOUT)) { ok = false; break; }
+                    if (!tc_warp_wait(&raw_empty[rs], (kb / TC_RAW_STAGES) & 1, p.status)) { ok = false; break; }
                     issue_raw(kb + TC_RAW_STAGES);
                 }
             }
-            if (k >= NST && !pb_mbar_wait(&empty[st], ((k / NST) - 1) & 1, p.status, PB_DEV_TC_TIMEOUT)) { ok = false; break; }
+            if (k >= NST && !tc_warp_wait(&empty[st], ((k / NST) - 1) & 1, p.status)) { ok = false; break; }
             tc_decode_store(cur, k, tmem + ((uint32_t)((warp & 3) * 32) << 16) + TC_ACC_COLS + (uint32_t)st * TC_A_COLS, shift);
             tc_fence_before();                    // the stores are complete (wait::st); order them before the MMA warp's instructions
             tc_warp_arrive(&full[st], lane);
         }
         // ---- epilogue: warp w reads lanes 32 (w % 4) .. + 31 (its rows); warps 0-3 take the first half of the tokens, 4-7 the rest; columns
         //      [0, np) hold the sums, or (narrow) the high parts' with the low parts' in [np, 2 np)
-        if (ok && pb_mbar_wait(acc_full, 0, p.status, PB_DEV_TC_TIMEOUT)) {
+        if (ok && tc_warp_wait(acc_full, 0, p.status)) {
             tc_fence_after();
             const int half = ((np + 1) / 2 + 31) / 32 * 32;
             for (int c0 = grp * half; c0 < (grp + 1) * half && c0 < np; c0 += 32) {

@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) pb_moetc_kernel(const PbExpertP
         auto rows8 = [&](int j, int g) { return DOWN ? wa + (16 * (size_t)j + g) * rb8 : ((g & 2) ? wb : wa) + (8 * (size_t)j + 2 * (g >> 2) + (g & 1)) * rb8; };
         auto issue = [&](int i) {           // half block i of the group's units (a producer warp)
             const int slot = (H + i) % MT_RING, j = u00 + i / nh, h = i % nh;
-            if (!__all_sync(0xffffffffu, pb_mbar_wait(&hd.raw_empty[slot], (((H + i) / MT_RING) & 1) ^ 1, p.status, PB_DEV_TC_TIMEOUT))) return false;
+            if (!tc_warp_wait(&hd.raw_empty[slot], (((H + i) / MT_RING) & 1) ^ 1, p.status)) return false;
             const uint32_t dst = raw + (uint32_t)(slot * MT_RAW_BYTES);
             const size_t col = (size_t)(h >> 1) * 1088;
             const int r = lane >> 2, q = lane & 3;
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) pb_moetc_kernel(const PbExpertP
             uint64_t b = bdesc;
             for (int i = 0; i < nhb; i++) {
                 // (acc_empty of the first round of slots: the phase before the first counts as complete)
-                ok = __all_sync(0xffffffffu, pb_mbar_wait(&hd.acc_empty[slot], ph ^ 1, p.status, PB_DEV_TC_TIMEOUT) && pb_mbar_wait(&hd.a_full[slot], ph, p.status, PB_DEV_TC_TIMEOUT));
+                ok = tc_warp_wait(&hd.acc_empty[slot], ph ^ 1, p.status) && tc_warp_wait(&hd.a_full[slot], ph, p.status);
                 if (!ok) break;
                 tc_fence_after();
                 if (elected) {
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) pb_moetc_kernel(const PbExpertP
             const int grp = (warp - MT_DRAIN) >> 2, row = 32 * quad + lane, g = row >> 3, r = row & 7;
             for (int i = grp; i < nhb && ok; i += MT_RING) {   // (H and the half blocks of a row are even)
                 const int slot = (H + i) % MT_RING;
-                ok = __all_sync(0xffffffffu, pb_mbar_wait(&hd.raw_full[slot], ((H + i) / MT_RING) & 1, p.status, PB_DEV_TC_TIMEOUT));
+                ok = tc_warp_wait(&hd.raw_full[slot], ((H + i) / MT_RING) & 1, p.status);
                 if (!ok) break;
                 const uint32_t src = raw + (uint32_t)(slot * MT_RAW_BYTES);
                 const uint2 head = pb_ldsa64(src + 8192u + (uint32_t)(g * 64 + r * 8));
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) pb_moetc_kernel(const PbExpertP
                             cells[16 * uu + 8 + 2 * q + 1] = pb_as_u32(__hfma2(pb_as_h2(x8 & 0x00F000F0u), mhi[q], mof[q]));
                         }
                     if (s == 0) {   // the slot's tiles are free (its first use: the phase before the first counts as complete)
-                        ok = __all_sync(0xffffffffu, pb_mbar_wait(&hd.done[slot], (((H + i) / MT_RING) & 1) ^ 1, p.status, PB_DEV_TC_TIMEOUT));
+                        ok = tc_warp_wait(&hd.done[slot], (((H + i) / MT_RING) & 1) ^ 1, p.status);
                         if (!ok) break;
                         tc_fence_after();
                     }
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) pb_moetc_kernel(const PbExpertP
                         float acc[2 * NE];
 #pragma unroll
                         for (int hb = 0; hb < 2; hb++) {
-                            ok = ok && __all_sync(0xffffffffu, pb_mbar_wait(&hd.done[slot], ph, p.status, PB_DEV_TC_TIMEOUT));
+                            ok = ok && tc_warp_wait(&hd.done[slot], ph, p.status);
                             tc_fence_after();
                             float c[2][2 * NE];
 #pragma unroll

@@ -26,6 +26,9 @@ __device__ __forceinline__ bool tc_elect() {
 // One arrival for the whole warp, behind what all its lanes did.  (An arrival of every lane is 32 operations on one word of shared memory, one after the other:
 // with 128 or 256 arrivals a step they were what the pipelines of these kernels waited for.)
 __device__ __forceinline__ void tc_warp_arrive(uint64_t* bar, int lane) { __syncwarp(); if (lane == 0) pb_mbar_arrive(bar); }
+// A wait of the whole warp: it ends for all lanes alike.  (A lane that left alone, because only its wait ran out, would strand the others at the next
+// instruction that takes a converged warp -- tcgen05.ld / st, the arrival above -- and the kernel would never leave.)
+__device__ __forceinline__ bool tc_warp_wait(uint64_t* bar, uint32_t phase, int* status) { return __all_sync(0xffffffffu, pb_mbar_wait(bar, phase, status, PB_DEV_TC_TIMEOUT)) != 0; }
 __device__ __forceinline__ int tc_uniform_warp() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
 // D (tensor memory) (+)= A (tensor memory: lane = row, two f16 per cell along K) x B (shared memory, by descriptor)
 __device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
