@@ -2,6 +2,7 @@
 #include "pb_formats.cuh"
 #include "pb_common.cuh"
 #include "pb_internal.h"
+#include "pb_host_ranges.h"
 
 #include <stdio.h>
 #include <stdlib.h>
@@ -74,12 +75,7 @@ int pb_scratch(pb_ctx* ctx, size_t bytes, void** out) {
 }
 
 static int sync_status(pb_ctx* ctx, const char* who);
-// The device's address of page-locked host memory, or null for other memory
-static void* host_dev(const void* p) {
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-    return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
-}
+static PbHostRanges g_host;   // of the process: a buffer may outlive the context that made it (cudaMallocHost memory has one address for the host and all devices)
 bool pb_host_pinned(const void* p) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
@@ -98,7 +94,7 @@ __global__ void __launch_bounds__(256) pb_copy_kernel(uint4* __restrict__ dst, c
 #define PB_COPY_IN ((size_t)128 << 10)    // a copy engine moves more than this faster than a kernel's reads over the link
 #define PB_COPY_OUT ((size_t)256 << 10)
 static bool copy_fits(const void* dst, const void* src, size_t bytes, size_t most) {
-    return bytes <= most && bytes % 16 == 0 && (((uintptr_t)dst | (uintptr_t)src) & 15) == 0;
+    return bytes > 0 && bytes <= most && bytes % 16 == 0 && (((uintptr_t)dst | (uintptr_t)src) & 15) == 0;
 }
 static int copy_small(pb_ctx* ctx, void* dst, const void* src, size_t bytes, bool status) {
     const int n = (int)(bytes / 16);
@@ -122,7 +118,7 @@ static int pin_room(pb_ctx* ctx, size_t bytes, bool* ok) {
 int pb_h2d(pb_ctx* ctx, void* dst, const void* src, size_t bytes, size_t off) {
     bool stage = off + bytes <= PB_PIN_MAX && !pb_host_pinned(src);
     if (stage) PB_TRY(pin_room(ctx, off + bytes, &stage));
-    const void* dev = stage ? ctx->pin + off : (bytes <= PB_COPY_IN ? host_dev(src) : nullptr);   // (page-locked by this library: the same address on the device)
+    const void* dev = stage ? ctx->pin + off : (bytes <= PB_COPY_IN && g_host.inside(src, bytes) ? src : nullptr);   // (other page-locked memory: the copy engine)
     if (dev && copy_fits(dst, dev, bytes, PB_COPY_IN)) {
         if (stage) memcpy(ctx->pin + off, src, bytes);
         return copy_small(ctx, dst, dev, bytes, false);
@@ -141,8 +137,8 @@ int pb_h2d(pb_ctx* ctx, void* dst, const void* src, size_t bytes, size_t off) {
 static int finish_small(pb_ctx* ctx, void* dst, const void* src, size_t bytes, size_t off, const char* who, bool* done) {
     *done = false;
     if (bytes > PB_COPY_OUT) return PB_OK;
-    void* dev = host_dev(dst);
-    bool stage = !dev && off + bytes <= PB_PIN_MAX;
+    void* dev = g_host.inside(dst, bytes) ? dst : nullptr;
+    bool stage = !dev && off + bytes <= PB_PIN_MAX && !pb_host_pinned(dst);   // (other page-locked memory: the copy engine)
     if (stage) PB_TRY(pin_room(ctx, off + bytes, &stage));
     if (stage) dev = ctx->pin + off;
     if (!dev || !copy_fits(dev, src, bytes, PB_COPY_OUT)) return PB_OK;
@@ -249,10 +245,12 @@ int pb_host_alloc(pb_ctx* ctx, size_t nbytes, void** out) {
     *out = nullptr;
     PB_TRY(pb_enter(ctx));
     if (cudaMallocHost(out, nbytes ? nbytes : 1) != cudaSuccess) { cudaGetLastError(); *out = nullptr; PB_FAIL(ctx, PB_ERR_OOM, "page-locked allocation of %zu bytes failed", nbytes); }
+    g_host.add(*out, nbytes);
     return PB_OK;
 }
 int pb_host_free(pb_ctx* ctx, void* p) {
     if (!p) return PB_OK;
+    g_host.drop(p);
     if (!ctx) { if (cudaFreeHost(p) != cudaSuccess) { cudaGetLastError(); return PB_ERR_CUDA; } return PB_OK; }   // a buffer may outlive the context that made it
     PB_TRY(pb_enter(ctx));
     PB_CUDA(ctx, cudaFreeHost(p));
