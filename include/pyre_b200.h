@@ -205,6 +205,13 @@ int pb_model_set_ctx_train(pb_model* m, int ctx_train);
 int pb_model_finalize(pb_model* m, int ep_rank, int ep_world);
 int pb_model_cfg(const pb_model* m, pb_cfg* out);   /* the configuration the model was created with (Model.cfg) */
 int pb_model_destroy(pb_model* m);
+/* Prompts from a multiple of 256 tokens on may run up to 1024 tokens per pass over the layers (same bits as a pass per 256).  The row buffers of
+ * such a pass, 1024 x (d + projections + 2 mixer widths + experts per token x (d + expert width)) floats -- 245 MB at the benchmark's widths --
+ * belong to the model: the first batch-1 state of a context of 272 and more positions makes them, where the memory is to be had.  They are no
+ * claim on it: an allocation of this library that fails for want of memory takes them back first, and prompts then go 256 tokens at a time until a later
+ * prompt finds room.  on = 0 frees them and keeps prompts at 256 tokens per pass, for a process that shares the GPU's memory with allocators other
+ * than this library; on = 1 (the state of a new model) allows them again and makes them now.  No call of the model may be running. */
+int pb_model_prompt_passes(pb_model* m, int on);
 
 /* new_state :1345-1353; `batch` independent sequences decode together. */
 int pb_state_create(pb_model* m, int batch, pb_state** out);
@@ -233,7 +240,8 @@ int pb_state_pos(const pb_state* s, int64_t* pos);
 /* Model::forward(ids, st) -> logits, src/model/qwen4exp_gguf.rs:2050-2157 (= spec::Target::step,
  * src/spec.rs:106-120, QnTarget::step src/engine_qn.rs:247).  ids_host [batch][t]; the logits of
  * the last fed token of each sequence go to logits_host [batch][vocab].  A prompt (t >= 3) of a
- * batch-1 state runs in windows of up to 8 tokens that stream every weight matrix once per window. */
+ * batch-1 state runs in passes of up to 256 tokens, cut at the positions that are multiples of 256, or of up to 1024 from
+ * such a position on (pb_model_prompt_passes); a pass streams every weight matrix once. */
 int pb_forward(pb_state* s, const uint32_t* ids_host, int t, float* logits_host);
 /* forward + sampler::argmax (src/sampler.rs:142-148) on the device: next_host [batch]. */
 int pb_step_greedy(pb_state* s, const uint32_t* tok_host, uint32_t* next_host);

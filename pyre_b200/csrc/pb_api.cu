@@ -61,13 +61,56 @@ int pb_max_clusters(pb_ctx* ctx, const void* kern, int threads, size_t smem, int
     return n;
 }
 
+// ---- workspaces that give way (pb_internal.h)
+static std::mutex g_spare_mu;
+static std::vector<PbSpare*> g_spare;
+cudaError_t pb_malloc(pb_ctx* ctx, void** p, size_t bytes) {
+    *p = nullptr;
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        bool freed = false;
+        {
+            std::lock_guard<std::mutex> lock(g_spare_mu);
+            for (PbSpare* w : g_spare) if (w->device == ctx->device && w->mem && !w->held) { cudaFree(w->mem); w->mem = nullptr; freed = true; }
+        }
+        if (freed) e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) { cudaGetLastError(); *p = nullptr; }
+    return e;
+}
+void* pb_spare_hold(pb_ctx* ctx, PbSpare* w, size_t bytes) {
+    std::lock_guard<std::mutex> lock(g_spare_mu);
+    if (!w->mem) {
+        bool known = false;
+        for (PbSpare* o : g_spare) known = known || o == w;
+        try { if (!known) g_spare.push_back(w); } catch (...) { return nullptr; }
+        void* p = nullptr;
+        if (cudaMalloc(&p, bytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        if (cudaMemsetAsync(p, 0, bytes, ctx->stream) != cudaSuccess) { cudaGetLastError(); cudaFree(p); return nullptr; }
+        w->device = ctx->device; w->mem = p;
+    }
+    w->held++;
+    return w->mem;
+}
+void pb_spare_release(PbSpare* w) {
+    std::lock_guard<std::mutex> lock(g_spare_mu);
+    w->held--;
+}
+void pb_spare_free(PbSpare* w) {
+    std::lock_guard<std::mutex> lock(g_spare_mu);
+    for (size_t i = 0; i < g_spare.size(); i++) if (g_spare[i] == w) { g_spare.erase(g_spare.begin() + (long)i); break; }
+    if (w->mem) cudaFree(w->mem);
+    w->mem = nullptr;
+}
+
 int pb_scratch(pb_ctx* ctx, size_t bytes, void** out) {
     if (bytes > ctx->scratch_bytes) {
         PB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         if (ctx->scratch) cudaFree(ctx->scratch);
         ctx->scratch = nullptr; ctx->scratch_bytes = 0;
         const size_t want = (bytes + ((size_t)1 << 20)) & ~(((size_t)1 << 20) - 1);
-        PB_CUDA(ctx, cudaMalloc(&ctx->scratch, want));
+        PB_CUDA(ctx, pb_malloc(ctx, &ctx->scratch, want));
         ctx->scratch_bytes = want;
     }
     *out = ctx->scratch;
@@ -190,10 +233,10 @@ int pb_ctx_create(int device, pb_ctx** out) {
     c->max_smem_optin = (int)prop.sharedMemPerBlockOptin;
     if (cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess) { delete c; return PB_ERR_CUDA; }
     c->stream = c->own_stream;
-    if (cudaMalloc(&c->dev_status, 256) != cudaSuccess) { cudaStreamDestroy(c->own_stream); delete c; return PB_ERR_OOM; }
+    if (pb_malloc(c, (void**)&c->dev_status, 256) != cudaSuccess) { cudaStreamDestroy(c->own_stream); delete c; return PB_ERR_OOM; }
     cudaMemset(c->dev_status, 0, 256);
-    if (cudaMalloc(&c->xh_buf, PB_XH_BYTES) != cudaSuccess) { cudaFree(c->dev_status); cudaStreamDestroy(c->own_stream); delete c; return PB_ERR_OOM; }
-    if (cudaMalloc(&c->grid_sync, 256) != cudaSuccess) { cudaFree(c->xh_buf); cudaFree(c->dev_status); cudaStreamDestroy(c->own_stream); delete c; return PB_ERR_OOM; }
+    if (pb_malloc(c, (void**)&c->xh_buf, PB_XH_BYTES) != cudaSuccess) { cudaFree(c->dev_status); cudaStreamDestroy(c->own_stream); delete c; return PB_ERR_OOM; }
+    if (pb_malloc(c, (void**)&c->grid_sync, 256) != cudaSuccess) { cudaFree(c->xh_buf); cudaFree(c->dev_status); cudaStreamDestroy(c->own_stream); delete c; return PB_ERR_OOM; }
     cudaMemset(c->grid_sync, 0, 256);
     if (cudaMallocHost(&c->host_status, 256) != cudaSuccess) { cudaFree(c->dev_status); cudaStreamDestroy(c->own_stream); delete c; return PB_ERR_OOM; }
     *c->host_status = 0;
@@ -289,7 +332,7 @@ int pb_ctx_stamps_enable(pb_ctx* ctx, int slots) {
     if (ctx->stamps) { cudaFree(ctx->stamps); ctx->stamps = nullptr; }
     ctx->stamp_slots = 0; ctx->stamp_next = 0; ctx->stamp_ids.clear();
     if (slots == 0) return PB_OK;
-    PB_CUDA(ctx, cudaMalloc(&ctx->stamps, (size_t)slots * PB_STAMP_WORDS * 8));
+    PB_CUDA(ctx, pb_malloc(ctx, (void**)&ctx->stamps, (size_t)slots * PB_STAMP_WORDS * 8));
     PB_CUDA(ctx, cudaMemset(ctx->stamps, 0, (size_t)slots * PB_STAMP_WORDS * 8));
     ctx->stamp_slots = slots; ctx->stamp_ids.assign((size_t)slots, 0);
     return PB_OK;
@@ -321,7 +364,7 @@ static int qmat_alloc(pb_ctx* ctx, int type, int64_t rows, int64_t cols, pb_qmat
     m->nbytes = (size_t)rows * (size_t)m->row_bytes;
     { const int rc = pb_enter(ctx); if (rc != PB_OK) { delete m; return rc; } }
     // padded so that 16-byte-granular bulk copies of the last rows stay inside the allocation
-    cudaError_t e = cudaMalloc(&m->data, m->nbytes + 256);
+    cudaError_t e = pb_malloc(ctx, (void**)&m->data, m->nbytes + 256);
     if (e != cudaSuccess) { delete m; PB_FAIL(ctx, PB_ERR_OOM, "cudaMalloc(%zu): %s", m->nbytes + 256, cudaGetErrorString(e)); }
     cudaMemsetAsync(m->data + m->nbytes, 0, 256, ctx->stream);
     *out = m;
@@ -336,7 +379,7 @@ static int qmat_recode(pb_ctx* ctx, pb_qmat* m) {
     if (!on || m->type != PB_T_IQ3_S || m->cols % 256) return PB_OK;
     m->r_row_bytes = bpr * 136;
     const size_t nb = (size_t)((m->rows + 7) / 8 * 8) * (size_t)m->r_row_bytes;   // whole groups of eight rows
-    cudaError_t e = cudaMalloc(&m->rdata, nb + 256);
+    cudaError_t e = pb_malloc(ctx, (void**)&m->rdata, nb + 256);
     if (e != cudaSuccess) { m->rdata = nullptr; PB_FAIL(ctx, PB_ERR_OOM, "cudaMalloc(%zu) for the re-coded copy: %s", nb + 256, cudaGetErrorString(e)); }
     cudaMemsetAsync(m->rdata + nb, 0, 256, ctx->stream);
     return pb_launch_repack_iq3s(ctx, m->data, m->rdata, m->rows, (int)bpr);

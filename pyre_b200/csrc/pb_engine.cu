@@ -30,11 +30,13 @@ static size_t ssm_elems(const pb_cfg& c, int B) { return (size_t)B * c.lin_nv * 
 struct PbSlot { pb_qmat* mat = nullptr; float* vec = nullptr; int64_t nvec = 0; };
 
 struct pb_state;
-// Row buffers of a pass over more than one prompt chunk: one set per model, made by the first prompt that is long enough.  The states of a model
-// share their context's stream and its thread, so one pass at a time uses it; a pass exchanges the pointers with the state's own.
+// Row buffers of a pass over more than one prompt chunk: one set per model, made with its first batch-1 state that can hold such a prompt.  It gives way to
+// allocations that fail without its memory; a later prompt then tries to have it back.  The states of a model share their context's stream and its
+// thread, so one pass at a time uses it; a pass exchanges the pointers with the state's own.
 struct PbPromptWs {
-    bool tried = false;
-    void* mem = nullptr;
+    PbSpare spare;
+    bool off = false;        // pb_model_prompt_passes
+    int able = -1;           // whether the model is one that such a pass is built for; -1: not looked at yet
     uint32_t* ids = nullptr; int64_t* wpos = nullptr; unsigned int* ticket = nullptr;
     float *x = nullptr, *proj = nullptr, *olin = nullptr, *att = nullptr, *rlogits = nullptr, *dn_run = nullptr;
     int *sel_e = nullptr, *ent_tok = nullptr, *ent_slot = nullptr; float *sel_w = nullptr, *ent_w = nullptr, *tok_scale = nullptr; int4* virt = nullptr;
@@ -147,6 +149,7 @@ void PbPromptWs::exchange(pb_state* s) {
     std::swap(moe_cap, s->moe_cap);
 }
 extern "C" {
+static bool prompt_ws_hold(pb_model* m);
 static void mtp_moved(pb_state* s, int64_t pos);
 static void mtp_forget(PbMtp* t, int64_t pos);
 }
@@ -173,7 +176,7 @@ template <typename T>
 static int dalloc(pb_state* s, T** p, size_t n) {
     pb_ctx* ctx = s->m->ctx;
     void* q = nullptr;
-    PB_CUDA(ctx, cudaMalloc(&q, (n ? n : 1) * sizeof(T) + 256));
+    PB_CUDA(ctx, pb_malloc(ctx, &q, (n ? n : 1) * sizeof(T) + 256));
     PB_CUDA(ctx, cudaMemsetAsync(q, 0, (n ? n : 1) * sizeof(T) + 256, ctx->stream));
     s->allocs.push_back(q);
     *p = (T*)q;
@@ -279,7 +282,7 @@ int pb_model_set_vec(pb_model* m, int layer, int role, const float* v, int64_t n
     PbSlot& s = slot(m, layer, role);
     if (s.vec) cudaFree(s.vec);
     s.vec = nullptr;
-    PB_CUDA(ctx, cudaMalloc(&s.vec, (size_t)n * 4 + 256));
+    PB_CUDA(ctx, pb_malloc(ctx, (void**)&s.vec, (size_t)n * 4 + 256));
     PB_CUDA(ctx, cudaMemcpyAsync(s.vec, v, (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
     PB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     s.nvec = n;
@@ -452,7 +455,7 @@ int pb_model_finalize(pb_model* m, int ep_rank, int ep_world) {
         }
         inv[half] = 1.0f + 0.1f * logf(scale);
     }
-    PB_CUDA(ctx, cudaMalloc(&m->rope_inv, inv.size() * 4));
+    PB_CUDA(ctx, pb_malloc(ctx, (void**)&m->rope_inv, inv.size() * 4));
     PB_CUDA(ctx, cudaMemcpy(m->rope_inv, inv.data(), inv.size() * 4, cudaMemcpyHostToDevice));
     m->weight_bytes_step = wb;
     m->finalized = true;
@@ -466,7 +469,7 @@ int pb_model_destroy(pb_model* m) {
     cudaStreamSynchronize(m->ctx->stream);
     for (auto& s : m->slots) { if (s.mat) pb_qmat_free(s.mat); if (s.vec) cudaFree(s.vec); }
     if (m->rope_inv) cudaFree(m->rope_inv);
-    if (m->ws.mem) cudaFree(m->ws.mem);
+    pb_spare_free(&m->ws.spare);
     delete m;
     return PB_OK;
 }
@@ -622,6 +625,7 @@ static int state_create(pb_model* m, int batch, bool sharded, pb_state** out) {
     if (rc == PB_OK && cudaMallocHost(&s->pin_u32, (size_t)(s->trace_cap + 2) * B * 4 + PB_PREFILL_CHUNK * 4) != cudaSuccess) { ctx->err = "pinned allocation failed"; rc = PB_ERR_OOM; }
     if (rc == PB_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) { ctx->err = "stream sync failed"; rc = PB_ERR_CUDA; }
     if (rc != PB_OK) { pb_state_destroy(s); return rc; }
+    if (solo && c.max_ctx >= PB_PREFILL_CHUNK + PB_PROMPT_TAIL && prompt_ws_hold(m)) pb_spare_release(&m->ws.spare);   // (the stream orders its zeroing before any use)
     *out = s;
     return PB_OK;
 }
@@ -1363,15 +1367,16 @@ static void mtp_moved(pb_state* s, int64_t pos) {
     if (t->kv_c0 > t->kv_end) t->kv_c0 = t->kv_end;
 }
 
-// The model's prompt workspace, allocated by the first prompt that can use it; null where the model is outside what a pass over several chunks
-// is built for (pre-norm residual, dense attention, experts on the tensor cores of one GPU) or the memory cannot be had: prompts then go chunk by chunk
-static PbPromptWs* prompt_ws(pb_model* m) {
+// Holds the prompt workspace, made now where it is not there; false where the model is outside what a pass over several chunks is built for (pre-norm
+// residual, dense attention, experts on the tensor cores of one GPU), where it is switched off, or while the memory is not to be had: prompts then go chunk by chunk
+static bool prompt_ws_hold(pb_model* m) {
     PbPromptWs& w = m->ws;
-    if (w.tried) return w.mem ? &w : nullptr;
-    w.tried = true;
-    pb_ctx* ctx = m->ctx; const pb_cfg& c = m->cfg;
-    if (c.hc > 0 || m->n_ple > 0 || m->qsa || m->mtp_window > 0 || m->ep_world > 1) return nullptr;
-    for (int il = 0; il < c.n_layers; il++) if (!expert_mma(m, il, 2)) return nullptr;
+    const pb_cfg& c = m->cfg;
+    if (w.able < 0) {
+        w.able = !(c.hc > 0 || m->n_ple > 0 || m->qsa || m->mtp_window > 0 || m->ep_world > 1);
+        for (int il = 0; il < c.n_layers && w.able; il++) w.able = expert_mma(m, il, 2);
+    }
+    if (!w.able || w.off) return false;
     const size_t R = PB_PROMPT_ROWS, K = (size_t)c.top_k;
     const size_t lin_w = (size_t)c.lin_nv * c.lin_dv, att_w = (size_t)c.n_head * c.hd, wide = lin_w > att_w ? lin_w : att_w;
     const size_t lin_proj = 2 * (size_t)c.lin_nk * c.lin_dk + 2 * lin_w + 2 * (size_t)c.lin_nv, att_proj = 2 * att_w + 2 * (size_t)c.n_kv * c.hd;
@@ -1390,12 +1395,30 @@ static PbPromptWs* prompt_ws(pb_model* m) {
         carve(&w.virt, (size_t)c.n_exp + R * K / PB_VGROUP + 1); carve(&w.h, R * K * c.ff_exp); carve(&w.h_sh, R * c.ff_sh);
         carve(&w.part, R * K * c.d); carve(&w.part_sh, R * c.d);
         if (pass == 0) {
-            if (cudaMalloc(&w.mem, off) != cudaSuccess) { cudaGetLastError(); w.mem = nullptr; return nullptr; }
-            base = (char*)w.mem;
+            base = (char*)pb_spare_hold(m->ctx, &w.spare, off);
+            if (!base) return false;
         }
     }
-    if (cudaMemsetAsync(w.mem, 0, off, ctx->stream) != cudaSuccess) { cudaGetLastError(); cudaFree(w.mem); w.mem = nullptr; }
-    return w.mem ? &w : nullptr;
+    return true;
+}
+// A call's hold on it: from the first pass that wants it until the call's work is done
+struct PbPromptHold {
+    pb_model* m; bool has = false, asked = false;
+    explicit PbPromptHold(pb_model* x) : m(x) {}
+    bool get() {
+        if (!asked) { asked = true; has = prompt_ws_hold(m); }
+        return has;
+    }
+    ~PbPromptHold() { if (has) { cudaStreamSynchronize(m->ctx->stream); pb_spare_release(&m->ws.spare); } }
+};
+int pb_model_prompt_passes(pb_model* m, int on) {
+    if (!m) return PB_ERR_ARG;
+    pb_ctx* ctx = m->ctx;
+    PB_TRY(pb_enter(ctx));
+    if (!m->finalized) PB_FAIL(ctx, PB_ERR_STATE, "pb_model_prompt_passes: call pb_model_finalize first");
+    m->ws.off = !on;
+    if (!on) pb_spare_free(&m->ws.spare); else PbPromptHold(m).get();
+    return PB_OK;
 }
 
 int pb_forward(pb_state* s, const uint32_t* ids_host, int t, float* logits_host) {
@@ -1413,13 +1436,14 @@ int pb_forward(pb_state* s, const uint32_t* ids_host, int t, float* logits_host)
         timing_begin(s);
         const int64_t pin_n = (s->trace_cap + 2) * B + PB_PREFILL_CHUNK;
         int64_t pin = 0;
+        PbPromptHold ws(s->m);
         for (int j0 = 0, n = 0; j0 < t; j0 += n) {
             // from a multiple of the chunk on, several chunks share a pass: the experts' weights, of which 256 tokens need all and a pass
             // decodes every one, serve four times the tokens.  All that a token's sums depend on -- the kernels, their cuts -- follows its chunk, so
             // the results are those of a pass per chunk, bit for bit
             const int64_t to_grid = PB_PREFILL_CHUNK - s->pos_host % PB_PREFILL_CHUNK;
             n = t - j0 < to_grid ? t - j0 : (int)to_grid;
-            if (to_grid == PB_PREFILL_CHUNK && t - j0 >= PB_PREFILL_CHUNK + PB_PROMPT_TAIL && prompt_ws(s->m)) {
+            if (to_grid == PB_PREFILL_CHUNK && t - j0 >= PB_PREFILL_CHUNK + PB_PROMPT_TAIL && ws.get()) {
                 n = t - j0 < PB_PROMPT_ROWS ? t - j0 : PB_PROMPT_ROWS;
                 if (n % PB_PREFILL_CHUNK < PB_PROMPT_TAIL) n -= n % PB_PREFILL_CHUNK;
             }

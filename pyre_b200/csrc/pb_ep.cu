@@ -163,14 +163,14 @@ int pb_ep_symm_alloc(pb_ctx* ctx, size_t bytes, PbEpSymm* out) {
     if (!ctx->ep_comm) PB_FAIL(ctx, PB_ERR_STATE, "peer exchange without pb_ep_init");
     if (ctx->ep_world > PB_EP_MAX_WORLD) PB_FAIL(ctx, PB_UNSUPPORTED, "peer exchange over %d ranks (at most %d)", ctx->ep_world, PB_EP_MAX_WORLD);
     const int world = ctx->ep_world, rank = ctx->ep_rank;
-    PB_CUDA(ctx, cudaMalloc(&out->local, bytes));
+    PB_CUDA(ctx, pb_malloc(ctx, &out->local, bytes));
     PB_CUDA(ctx, cudaMemsetAsync(out->local, 0, bytes, ctx->stream));
     out->bytes = bytes;
     cudaIpcMemHandle_t mine;
     PB_CUDA(ctx, cudaIpcGetMemHandle(&mine, out->local));
     static_assert(sizeof(cudaIpcMemHandle_t) == 64, "handles travel as 16 floats");
     float* hbuf = nullptr;
-    PB_CUDA(ctx, cudaMalloc(&hbuf, (size_t)world * 64));
+    PB_CUDA(ctx, pb_malloc(ctx, (void**)&hbuf, (size_t)world * 64));
     PB_CUDA(ctx, cudaMemcpyAsync(reinterpret_cast<char*>(hbuf) + (size_t)rank * 64, &mine, 64, cudaMemcpyHostToDevice, ctx->stream));
     int rc = pb_ep_allgather(ctx, hbuf + (size_t)rank * 16, hbuf, 16);
     std::vector<cudaIpcMemHandle_t> all((size_t)world);
@@ -204,7 +204,7 @@ int pb_ep_probe_wait_timeout(pb_ctx* ctx, unsigned int spins) {
     if (!ctx) return PB_ERR_ARG;
     PB_TRY(pb_enter(ctx));
     unsigned long long* mem = nullptr;
-    PB_CUDA(ctx, cudaMalloc(&mem, 1024));
+    PB_CUDA(ctx, pb_malloc(ctx, (void**)&mem, 1024));
     PB_CUDA(ctx, cudaMemsetAsync(mem, 0, 1024, ctx->stream));
     PbEpExch x; memset(&x, 0, sizeof x);
     x.rank = 1; x.world = 2;                       // "rank 1 of 2": CTA 0 announces to rank 0 and waits for rank 0's flag

@@ -39,6 +39,17 @@ struct pb_ctx {
     unsigned long owner_thread = 0;   // pthread id of the creating thread (checked when PYRE_B200_CHECK_THREAD=1)
     bool check_thread = false;
 };
+// cudaMalloc for what a call cannot do without.  Where the memory is used up, idle workspaces that the library made for speed alone go first (of every
+// context of the process on this GPU), and the allocation is tried again.  A failure leaves no CUDA error behind for the next call to find.
+cudaError_t pb_malloc(pb_ctx* ctx, void** p, size_t bytes);
+// Such a workspace.  It may go whenever nobody holds it; a call holds it while its work on it is queued or running.
+struct PbSpare {
+    int device = 0, held = 0;
+    void* mem = nullptr;
+};
+void* pb_spare_hold(pb_ctx* ctx, PbSpare* w, size_t bytes);   // made (zeroed) where it is not there; null while the memory is not to be had
+void pb_spare_release(PbSpare* w);
+void pb_spare_free(PbSpare* w);
 // Every extern "C" entry point that touches the device calls this first: makes the context's GPU current
 // (a process may hold contexts on several GPUs) and, in the debug mode, verifies the calling thread.
 int pb_enter(pb_ctx* ctx);

@@ -63,6 +63,10 @@ class Model:
         batch of batch * world; see pb_state_create_sharded."""
         return State(self, batch, sharded)
 
+    def prompt_passes(self, on: bool):
+        """Whether prompts may run several 256-token chunks per pass (pb_model_prompt_passes); off frees the row buffers of such passes."""
+        self.ctx.check(lib().pb_model_prompt_passes(self.h, C.c_int(1 if on else 0)))
+
     def caps(self) -> Caps:
         c = Caps()
         self.ctx.check(lib().pb_caps_get(self.h, C.byref(c)))
