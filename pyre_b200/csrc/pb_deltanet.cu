@@ -69,8 +69,8 @@ __global__ void __launch_bounds__(256) pb_deltanet_inputs_kernel(const PbDeltaPa
     const bool isv = (int)blockIdx.y >= nk;
     const int head = isv ? (int)blockIdx.y - nk : (int)blockIdx.y;
     __shared__ float red[2][3][8];
-    constexpr int LD = 132;                                 // rows of a block's k and q, 4 banks apart
-    __shared__ __align__(16) float kqs[TB == 8 ? 2 : 1][TB == 8 ? 8 * LD : 1];
+    constexpr int LD = 130;                                 // rows of a block's k and q, 4 banks apart
+    __shared__ __align__(16) double kqs[TB == 8 ? 2 : 1][TB == 8 ? 8 * LD : 1];
     const int n = isv ? dv : dk;
     const bool live = tid < n;
     const int c0 = isv ? 2 * nk * dk + head * dv + tid : head * dk + tid, c1 = nk * dk + head * dk + tid;   // q and k channel, or the v channel
@@ -136,16 +136,20 @@ __global__ void __launch_bounds__(256) pb_deltanet_inputs_kernel(const PbDeltaPa
     if (TB == 8 && r.gram && !isv) {
         __syncthreads();
         const int which = tid >> 6, t = (tid >> 3) & 7, s = tid & 7;   // 128 threads: k_t.k_s and q_t.k_s
-        float d = 0.f;
+        // in 64 bits, rounded once: a product enters up to seven corrections and outputs, and its rounding with it (1024 tokens of 16 K heads: 66 us with
+        // sums in f32, 70 so)
+        double d = 0.0;
         if (s <= t && t0 + t < t1) {
-            float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+            double u[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
             for (int c = 0; c < 128; c += 4) {
-                const float4 x = *reinterpret_cast<const float4*>(&kqs[which][t * LD + c]), y = *reinterpret_cast<const float4*>(&kqs[0][s * LD + c]);
-                u.x = fmaf(x.x, y.x, u.x); u.y = fmaf(x.y, y.y, u.y); u.z = fmaf(x.z, y.z, u.z); u.w = fmaf(x.w, y.w, u.w);
+                const double2 x0 = *reinterpret_cast<const double2*>(&kqs[which][t * LD + c]), x1 = *reinterpret_cast<const double2*>(&kqs[which][t * LD + c + 2]);
+                const double2 y0 = *reinterpret_cast<const double2*>(&kqs[0][s * LD + c]), y1 = *reinterpret_cast<const double2*>(&kqs[0][s * LD + c + 2]);
+                u[0] = fma(x0.x, y0.x, u[0]); u[1] = fma(x0.y, y0.y, u[1]); u[2] = fma(x1.x, y1.x, u[2]); u[3] = fma(x1.y, y1.y, u[3]);
             }
-            d = (u.x + u.y) + (u.z + u.w);
+            d = (u[0] + u[1]) + (u[2] + u[3]);
         }
-        r.gram[((size_t)blockIdx.x * nk + head) * 128 + tid] = d;
+        r.gram[((size_t)blockIdx.x * nk + head) * 128 + tid] = (float)d;
     }
 }
 
@@ -262,7 +266,7 @@ __global__ void __launch_bounds__(128) pb_deltanet_run_kernel(const PbDeltaParam
 // then a triangular system of eight unknowns per column is solved by substitution, and the state takes its eight rank-one updates at once.  A
 // warp holds eight columns, its lanes eight groups of sixteen rows x four pairs of columns; k of the block stays in registers from the products to the
 // update.  What bounds it: the instructions of one warp per scheduler and the reads of k and q from shared memory (the token-by-token walk: the
-// latency of one token).  1024 tokens of 32 heads of 128 x 128: 344 us token by token, 232 in blocks (eight warps of four columns, k read twice: 242).
+// latency of one token).  1024 tokens of 32 heads of 128 x 128: 344 us token by token, 246 in blocks.
 // A token's values never enter an earlier token's: the sums run over s < t only.
 #define DB_C 8               // tokens of a block
 __global__ void __launch_bounds__(128, 1) pb_deltanet_block_kernel(const PbDeltaParams p, int T, const PbDeltaRun r) {
@@ -361,35 +365,40 @@ __global__ void __launch_bounds__(128, 1) pb_deltanet_block_kernel(const PbDelta
             }
         }
         __syncthreads();                                    // the tables are complete (and the warp's sums)
-        // corrections of column `col` of the warp, all of them by each of the column's four lanes: delta_t = (v_t - g_t mem_t) beta_t (:1663); a correction
-        // is taken out of the later tokens as soon as it is known
+        // corrections of column `col` of the warp, all of them by each of the column's four lanes: delta_t = (v_t - g_t mem_t) beta_t (:1663).  What the
+        // earlier corrections add to a token's memory is summed by itself: taken out of v_t one by one they would each round at
+        // v_t's magnitude (16 tokens with decays near 1, readout and state against 64 bits: 9.9e-8 and 10.4e-8 of the result that way, 8.6e-8 and 8.8e-8 so,
+        // token by token 9.5e-8 and 8.9e-8)
         const int col = lane & 7, rr = lane >> 3;
-        float de[C], m[C][C];
+        float de[C], m[C][C], av[C], gv[C], sum[C];
         {
             const float4 x = *reinterpret_cast<const float4*>(&ab[warp][0][col][0]), y = *reinterpret_cast<const float4*>(&ab[warp][0][col][4]);
             const float4 g = *reinterpret_cast<const float4*>(&dec[0][0]), e = *reinterpret_cast<const float4*>(&dec[0][4]);
-            const float av[C] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w}, gv[C] = {g.x, g.y, g.z, g.w, e.x, e.y, e.z, e.w};
+            const float xy[C] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w}, ge[C] = {g.x, g.y, g.z, g.w, e.x, e.y, e.z, e.w};
 #pragma unroll
             for (int t = 0; t < C; t++) {
+                av[t] = xy[t]; gv[t] = ge[t];
                 if (t > 0) { const float4 o = *reinterpret_cast<const float4*>(&mat[0][t][0]); m[t][0] = o.x; m[t][1] = o.y; m[t][2] = o.z; m[t][3] = o.w; }
                 if (t > 4) { const float4 o = *reinterpret_cast<const float4*>(&mat[0][t][4]); m[t][4] = o.x; m[t][5] = o.y; m[t][6] = o.z; m[t][7] = o.w; }
-                de[t] = fmaf(-gv[t], av[t], d.v[t][8 * warp + col]);
             }
         }
 #pragma unroll
         for (int t = 0; t < C; t++) {
-            de[t] = t < n ? de[t] * d.gb[t].y : 0.f;
+            float mem = t > 1 ? fmaf(gv[t], av[t], sum[t]) : gv[t] * av[t];
+            if (t) mem = fmaf(m[t][t - 1], de[t - 1], mem);        // (the token before is what the chain waits for)
+            de[t] = t < n ? (d.v[t][8 * warp + col] - mem) * d.gb[t].y : 0.f;
 #pragma unroll
-            for (int q = t + 1; q < C; q++) de[q] = fmaf(-m[q][t], de[t], de[q]);
+            for (int q = t + 2; q < C; q++) sum[q] = t ? fmaf(m[q][t], de[t], sum[q]) : m[q][0] * de[0];
         }
 #pragma unroll
         for (int i = 0; i < 2; i++) {   // each of the column's lanes forms two of the outputs: tokens 2 rr and 2 rr + 1
             const int t = 2 * rr + i;
             const float4 x = *reinterpret_cast<const float4*>(&mat[1][t][0]), y = *reinterpret_cast<const float4*>(&mat[1][t][4]);
             const float w[C] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-            float o = dec[0][t] * ab[warp][1][col][t], own = de[0];
+            float o = w[0] * de[0], own = de[0];
 #pragma unroll
-            for (int q = 0; q < C; q++) { if (q <= t) o = fmaf(w[q], de[q], o); if (q == t) own = de[q]; }
+            for (int q = 1; q < C; q++) { if (q <= t) o = fmaf(w[q], de[q], o); if (q == t) own = de[q]; }
+            o = fmaf(dec[0][t], ab[warp][1][col][t], o);     // (the state's part last)
             if (t < n) p.out[(size_t)(t0 + t) * p.ldo + h * dv + j0 + 8 * warp + col] = o;   // readout before the gated norm
             del[warp][t][col] = own * dec[1][t];
         }
