@@ -476,8 +476,9 @@ int pb_gemv_dev(pb_ctx* ctx, const pb_qmat* m, const float* x, int t, float* y) 
     PbChain chain(ctx);
     // many tokens of a re-coded IQ3_S matrix go to the tcgen05 GEMM in pieces as large as its operand buffer takes
     const bool tc = t >= pb_gemmtc_min_tokens() && m->rdata && pb_gemvq_supported(m->type, (int)m->cols) && pb_gemmtc_supported(m->type, (int)m->cols, t);   // what pb_launch_gemvq will pick
-    const int piece = tc ? pb_gemmtc_max_tokens((int)m->cols) : pb_gemmh_piece(m->type, (int)m->cols);
+    int piece = tc ? pb_gemmtc_max_tokens((int)m->cols) : 0;
     for (int t0 = 0; t0 < t; t0 += piece) {
+        if (!tc) PB_TRY(pb_gemmh_tokens(ctx, m->type, m->rdata != nullptr, m->rows, (int)m->cols, t - t0, &piece));
         PbGemvArgs a;
         a.w = m->data; a.wr = m->rdata; a.type = m->type; a.rows = m->rows; a.cols = (int)m->cols;
         a.x = x + (int64_t)t0 * m->cols; a.ldx = m->cols; a.t = t - t0 < piece ? t - t0 : piece;

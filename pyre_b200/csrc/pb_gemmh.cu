@@ -218,24 +218,65 @@ static bool gh_layout(pb_ctx* ctx, int cols, int t, int ks, int& nt, int& nw, Pb
 }
 
 template <int FMT>
+static const void* gh_kernel(int nt) {
+    const void* k[] = {(const void*)pb_gemmh_kernel<FMT, 1>, (const void*)pb_gemmh_kernel<FMT, 2>, (const void*)pb_gemmh_kernel<FMT, 3>, (const void*)pb_gemmh_kernel<FMT, 4>, (const void*)pb_gemmh_kernel<FMT, 6>, (const void*)pb_gemmh_kernel<FMT, 8>};
+    return k[nt <= 4 ? nt - 1 : nt / 2 + 1];
+}
+// Tiles of a round: one per warp of every cluster that is resident at a time (148 SMs hold 74 clusters of two CTAs, but 33 of four and 15 of eight)
+template <int FMT>
+static int gh_round(pb_ctx* ctx, int nt, int nw, size_t smem, int ks, int* tiles) {
+    PB_TRY(pb_ensure_smem_fn(ctx, gh_kernel<FMT>(nt), smem));
+    *tiles = nw * pb_max_clusters(ctx, gh_kernel<FMT>(nt), nw * 32, smem, ks);
+    return PB_OK;
+}
+
+// Whether r tokens, 17 to 32, go in one launch, on clusters of ks32 CTAs of 512 columns (32 tokens' activations fit beside the weights), or in launches of
+// sixteen.  One launch is the shorter one for every format, 17 to 31 tokens and 512 to 4096 columns while a CTA has at most one round of tiles (us, two launches /
+// one, 24 tokens: 2048 x 512 IQ3_S 12.3 / 9.9, 4096 x 2048 20.5 / 15.7, 8448 x 2048 24.2 / 18.5, Q6_K 39.0 / 27.1, 3584 x 4096 IQ2_XS 34.8 / 24.6;
+// 31 tokens: 8448 x 2048 IQ3_S 26.7 / 22.6, Q5_K 45.0 / 33.2), where the round counts the warps that fit: Q8_0 has eight with 25 and more tokens (31 tokens of
+// 4096 x 2048, 0.97 rounds, 28.7 / 24.6; of 4096 x 4096, 2.1 rounds, 41.0 / 51.2).  With more, the parts' sums are exchanged in every round.  A little more than a
+// round still pays where two launches have no second warp for a tile (4608 x 4096 24 tokens: Q4_K 32.9 / 28.9, Q6_K 51.2 / 38.7), for the formats of the
+// longest decodes (31 tokens of 4096 x 4096 IQ3_XXS 47.2 / 43.2, 9472 x 2048 IQ1_M 45.4 / 41.0), for 18 to 24 tokens (9472 x 2048 Q8_0 36.9 / 32.8) except
+// for short decodes in clusters of eight (4096 x 4096, 20 tokens: IQ3_S 23.8 / 24.6, Q4_K 26.9 / 28.7), and from 29 on but for the two shortest (31 tokens of
+// 9472 x 2048 Q6_K 45.1 / 42.9, IQ3_S 27.7 / 28.7); not for a single seventeenth token, which the dp4a kernel takes (9472 x 2048 Q4_0 28.7 / 30.8), nor
+// for 25 to 28 (25 tokens of 4096 x 4096 Q4_0 36.9 / 39.0).  Two rounds are left to two launches (24 tokens of 151936 x 2048 IQ3_S 138 / 221).
+template <int FMT>
+static int gh_one_launch(pb_ctx* ctx, int cols, int all, int r, int ks16, int ks32, bool* one) {
+    *one = false;
+    if (all > GH_WARPS * (ctx->sm_count / ks32)) return PB_OK;
+    PbGemmHParams h;
+    int nt, nw, nt16, nw16, round, round16; size_t smem, smem16;
+    memset(&h, 0, sizeof h);
+    if (!gh_layout<FMT>(ctx, cols, r, ks32, nt, nw, h, smem) || nt <= 4) return PB_OK;
+    PB_TRY((gh_round<FMT>(ctx, nt, nw, smem, ks32, &round)));
+    if (all <= round) { *one = true; return PB_OK; }
+    if (4 * all > 5 * round || !gh_layout<FMT>(ctx, cols, 16, ks16, nt16, nw16, h, smem16)) return PB_OK;
+    PB_TRY((gh_round<FMT>(ctx, nt16, nw16, smem16, ks16, &round16)));
+    constexpr bool longest = FMT == PB_T_IQ3_XXS || FMT == PB_T_IQ2_XXS || FMT == PB_T_IQ1_M || FMT == PB_T_IQ2_XS;
+    constexpr bool brief = FMT == PB_T_IQ3S_N4 || FMT == PB_T_Q4_K || FMT == PB_T_IQ2_S;
+    *one = 2 * all > round16 || longest || (nt <= 6 ? r > 17 && !(brief && ks32 == 8) : r > 28 && nw == GH_WARPS && (!brief || FMT == PB_T_Q4_K));
+    return PB_OK;
+}
+
+// CTAs of a cluster.  Launches of up to sixteen tokens: 1024 columns each above 2048; half a row each where a CTA has at most a round of tiles and the
+// activations of several tokens would take as long to prepare as the product
+static int gh_ks16(pb_ctx* ctx, int cols, int all, int t) { return cols > 2048 ? cols / 1024 : (cols == 2048 && all <= 16 * ctx->sm_count && t > 4 ? 2 : 1); }
+static int gh_ks32(int cols) { return cols > 512 ? cols / 512 : 1; }
+
+template <int FMT>
 static int launch_fmt(pb_ctx* ctx, const PbGemvQArgs& a, bool recoded) {
     int el, bs;
     pb_geom(FMT, &el, &bs);
     int all = 0;
     for (int s = 0; s < a.nseg; s++) all += (int)((a.seg[s].rows + 15) / 16);
-    // CTAs of a cluster: 1024 columns each above 2048; half a row each where a CTA has at most a round of tiles and the activations of several
-    // tokens would take as long to prepare as the product
-    const int ks16 = a.cols > 2048 ? a.cols / 1024 : (a.cols == 2048 && all <= 16 * ctx->sm_count && a.t > 4 ? 2 : 1);
-    // More than 16 tokens in one launch: 512 columns per CTA (32 tokens' activations fit beside the weights), worth it where every CTA of a cluster has at
-    // most one round of tiles; with more, the exchange of the parts' sums in every round costs more than the second launch (us for 24 tokens of IQ3_S, two
-    // launches / one: 2048 x 512 15.5 / 10.4, 4096 x 2048 22.7 / 16.5, 2048 x 4096 23.5 / 16.5, 12351 x 2048 31 / 28, 151936 x 2048 138 / 221).
-    const int ks32 = a.cols > 512 ? a.cols / 512 : 1;
-    const int most = all <= 16 * (ctx->sm_count / ks32) ? 4 * GH_MAXNT : 16;
+    const int ks16 = gh_ks16(ctx, a.cols, all, a.t), ks32 = gh_ks32(a.cols);
     for (int t0 = 0, n = 0; t0 < a.t; t0 += n) {
         PbGemmHParams h;
         memset(&h, 0, sizeof h);
-        int nt, nw; size_t smem;
-        const int r = a.t - t0 < most ? a.t - t0 : most, ks = r > 16 ? ks32 : ks16;
+        int nt, nw, r = a.t - t0 < 4 * GH_MAXNT ? a.t - t0 : 4 * GH_MAXNT; size_t smem;
+        bool one = true;
+        if (r > 16) { PB_TRY((gh_one_launch<FMT>(ctx, a.cols, all, r, ks16, ks32, &one))); if (!one) r = 16; }
+        const int ks = r > 16 ? ks32 : ks16;
         h.ks = ks;
         if (!gh_layout<FMT>(ctx, a.cols, r, ks, nt, nw, h, smem)) PB_FAIL(ctx, PB_UNSUPPORTED, "gemm: %d columns do not fit shared memory", a.cols);
         n = r < 4 * nt ? r : 4 * nt;
@@ -259,9 +300,26 @@ static int launch_fmt(pb_ctx* ctx, const PbGemvQArgs& a, bool recoded) {
     return PB_OK;
 }
 
-int pb_gemmh_piece(int type, int cols) {
+template <int FMT>
+static int tokens_fmt(pb_ctx* ctx, int64_t rows, int cols, int t, int* n) {
+    const int all = (int)((rows + 15) / 16), r = t < 4 * GH_MAXNT ? t : 4 * GH_MAXNT;
+    bool one = false;
+    PB_TRY((gh_one_launch<FMT>(ctx, cols, all, r, gh_ks16(ctx, cols, all, t), gh_ks32(cols), &one)));
+    *n = one ? r : 16;
+    return PB_OK;
+}
+int pb_gemmh_tokens(pb_ctx* ctx, int type, bool recoded, int64_t rows, int cols, int t, int* n) {
     static const bool use_mma = !(getenv("PYRE_B200_MMA") && atoi(getenv("PYRE_B200_MMA")) == 0);
-    return use_mma && pb_gemvq_supported(type, cols) ? 32 : 16;
+    *n = t < 16 ? t : 16;
+    if (t <= 16 || !use_mma || !pb_gemvq_supported(type, cols)) return PB_OK;
+#define GO(F) case F: return tokens_fmt<F>(ctx, rows, cols, t, n)
+    switch (type) {
+        case PB_T_IQ3_S: return recoded ? tokens_fmt<PB_T_IQ3S_N4>(ctx, rows, cols, t, n) : tokens_fmt<PB_T_IQ3_S>(ctx, rows, cols, t, n);
+        GO(PB_T_IQ3S_N4); GO(PB_T_IQ2_XS); GO(PB_T_Q4_K); GO(PB_T_Q8_0); GO(PB_T_IQ3_XXS); GO(PB_T_IQ2_S); GO(PB_T_IQ4_NL); GO(PB_T_IQ4_XS);
+        GO(PB_T_Q2_0); GO(PB_T_IQ2_XXS); GO(PB_T_Q6_K); GO(PB_T_IQ1_M); GO(PB_T_Q4_0); GO(PB_T_Q5_0); GO(PB_T_Q3_K); GO(PB_T_Q5_K);
+        default: return PB_OK;
+    }
+#undef GO
 }
 bool pb_gemmh_supported(int type, int cols, int t) { return t >= 2 && pb_gemvq_supported(type, cols); }
 

@@ -234,7 +234,7 @@ bool pb_gemvq_supported(int type, int cols);
 int pb_launch_gemvq(pb_ctx* ctx, const PbGemvQArgs& a);
 // pb_gemmh.cu: warp-level tensor-core path from two columns on, every quantized format
 bool pb_gemmh_supported(int type, int cols, int t);
-int pb_gemmh_piece(int type, int cols);   // tokens of one call: 32 where this kernel takes them, else the 16 of the other GEMV kernels
+int pb_gemmh_tokens(pb_ctx* ctx, int type, bool recoded, int64_t rows, int cols, int t, int* n);   // tokens of the next launch for t of one matrix: up to 32 where one launch of this kernel is the shorter way, else up to 16
 int pb_launch_gemmh(pb_ctx* ctx, const PbGemvQArgs& a);
 // pb_gemmtc.cu: tcgen05 path for 16 and more columns of IQ3_S weights that have a re-coded copy
 bool pb_gemmtc_supported(int type, int cols, int t);
