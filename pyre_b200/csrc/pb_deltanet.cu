@@ -446,11 +446,13 @@ int pb_launch_deltanet_seq(pb_ctx* ctx, const PbDeltaParams& p, int T, float* sc
     if (ckp) ck = *ckp;
     PbDeltaRun r;
     r.qk = scratch; r.v = r.qk + (size_t)T * 2 * p.nk * p.dk; r.gb = reinterpret_cast<float2*>(r.v + (size_t)T * p.nv * p.dv); r.kq = reinterpret_cast<float*>(r.gb + (size_t)T * p.nv);
-    // blocks of eight tokens from two full blocks on, for the one head size they are built for; verify windows need the state after every token
-    const bool blocks = !ckp && T >= 16 && p.dk == 128 && p.dv <= 128;
+    // blocks of eight tokens for the one head size they are built for; verify windows need the state after every token.  From 32 tokens on, where the inputs
+    // are made eight tokens at a time anyway: below, making them one by one on many CTAs and walking takes 9 to 10 us less per layer (a pass over three layers,
+    // blocks / token by token: 16 tokens 387 / 355 us, 24 465 / 438, 31 516 / 489), from there on as long, and from 64 tokens on blocks are shorter
+    const bool blocks = !ckp && T >= PB_DELTA_BLOCKS && p.dk == 128 && p.dv <= 128;
     r.gram = blocks ? reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(r.kq + (size_t)T * p.nk) + 15) & ~(uintptr_t)15) : nullptr;
     const int wide = p.dk > p.dv ? p.dk : p.dv;
-    if (T >= 32 || blocks) pb_launch_k(ctx, pb_deltanet_inputs_kernel<8>, dim3((T + 7) / 8, p.nk + p.nv), dim3((wide + 31) & ~31), (size_t)0, p, T, r);
+    if (T >= PB_DELTA_BLOCKS) pb_launch_k(ctx, pb_deltanet_inputs_kernel<8>, dim3((T + 7) / 8, p.nk + p.nv), dim3((wide + 31) & ~31), (size_t)0, p, T, r);
     else pb_launch_k(ctx, pb_deltanet_inputs_kernel<1>, dim3(T, p.nk + p.nv), dim3((wide + 31) & ~31), (size_t)0, p, T, r);
     ctx->kernels_launched++;
     PB_CUDA(ctx, cudaGetLastError());

@@ -754,7 +754,13 @@ static int run_lin(pb_state* s, int il, const float* x_in, const float* norm_w, 
         d.pos = s->wpos; d.batch = 1;
         PbDeltaCk ck; memset(&ck, 0, sizeof ck);
         if (s->win_ckpt) for (int j = 0; j + 1 < s->win_t; j++) { ck.conv[j] = s->ck_conv[(size_t)li * PB_MAX_WINDOW + j]; ck.ssm[j] = s->ck_ssm[(size_t)li * PB_MAX_WINDOW + j]; }
-        PB_TRY(pb_launch_deltanet_seq(ctx, d, s->win_t, s->dn_run, s->win_ckpt ? &ck : nullptr));
+        // a pass over several chunks: the chunks in one run, and a rest too short for blocks of tokens in a run of its own, as a pass over it alone makes it
+        const int rest = s->win_t > PB_PREFILL_CHUNK ? s->win_t % PB_PREFILL_CHUNK : 0, n = rest < PB_DELTA_BLOCKS ? s->win_t - rest : s->win_t;
+        PB_TRY(pb_launch_deltanet_seq(ctx, d, n, s->dn_run, s->win_ckpt ? &ck : nullptr));
+        if (n < s->win_t) {
+            d.proj += (size_t)n * s->ldproj; d.out += (size_t)n * w; d.pos += n;
+            PB_TRY(pb_launch_deltanet_seq(ctx, d, s->win_t - n, s->dn_run));
+        }
     } else if (s->win_t > 0) {
         // the recurrence is sequential: one launch per token, with a rollback checkpoint after each but the last
         for (int j = 0; j < s->win_t; j++) {

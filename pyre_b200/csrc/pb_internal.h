@@ -337,6 +337,7 @@ int pb_launch_deltanet(pb_ctx* ctx, const PbDeltaParams& p);
 bool pb_deltanet_seq_supported(const PbDeltaParams& p);
 // rollback checkpoints of a window: the state as it is after token j (conv ring and ssm of one sequence), or null
 struct PbDeltaCk { float* conv[8]; float* ssm[8]; };
+#define PB_DELTA_BLOCKS 32   // tokens from which a run goes in blocks of eight
 size_t pb_deltanet_seq_scratch(const PbDeltaParams& p, int T);   // floats of scratch that a run of T tokens needs
 int pb_launch_deltanet_seq(pb_ctx* ctx, const PbDeltaParams& p, int T, float* scratch, const PbDeltaCk* ck = nullptr);   // T consecutive tokens of sequence 0, state kept in registers
 

@@ -1,4 +1,4 @@
-"""Runs of the DeltaNet recurrence against 64 bits, from their own f32 projections: the blocks of eight tokens that prompts of 16 and more tokens take must be no
+"""Runs of the DeltaNet recurrence against 64 bits, from their own f32 projections: the blocks of eight tokens that prompts of 32 and more tokens take must be no
 farther off than the walk token by token, which the same tokens take in pieces of eight; and a token that is not finite must not reach the tokens before it."""
 import numpy as np
 import pytest
@@ -44,7 +44,7 @@ def _f64(cfg, spec, proj):
 
 
 @pytest.mark.parametrize("decay", [1.0, 1e-3, 30.0])          # as synthesised; near 1, where the state of hundreds of tokens ago counts; near 0
-@pytest.mark.parametrize("n", [16, 31, 256])
+@pytest.mark.parametrize("n", [32, 39, 256])
 def test_blocks_are_as_close_to_64_bits_as_single_tokens(ctx, n, decay):
     """The bound: the walk's own error in the mean of three models; 3 % for the state, whose rounding differs in order only."""
     cfg = _cfg()
@@ -73,7 +73,7 @@ def test_blocks_are_as_close_to_64_bits_as_single_tokens(ctx, n, decay):
     assert ctx.device_status() == 0
 
 
-@pytest.mark.parametrize("bad_at", [0, 7, 8, 13, 23])
+@pytest.mark.parametrize("bad_at", [0, 7, 8, 13, 38])
 def test_a_token_that_is_not_finite_leaves_the_readout_before_it_alone(ctx, bad_at):
     cfg = _cfg()
     spec, bad = synth.model_spec(cfg, 13), 77
@@ -92,10 +92,10 @@ def test_a_token_that_is_not_finite_leaves_the_readout_before_it_alone(ctx, bad_
     out = []
     for tok in (bad, 5):
         st.reset()
-        ids = np.arange(100, 124, dtype=np.uint32)
+        ids = np.arange(100, 139, dtype=np.uint32)
         ids[bad_at] = tok
         st.forward(ids)
-        out.append(st.peek(2, 24 * cfg.lin_nv * cfg.lin_dv).reshape(24, -1))
+        out.append(st.peek(2, 39 * cfg.lin_nv * cfg.lin_dv).reshape(39, -1))
     assert np.array_equal(out[0][:bad_at].view(np.uint32), out[1][:bad_at].view(np.uint32))
     assert np.isnan(out[0][bad_at:]).all() and np.isfinite(out[1]).all()
     assert ctx.device_status() == 0

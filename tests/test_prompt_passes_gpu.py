@@ -11,12 +11,12 @@ from helpers import oracle_cfg, oracle_model, small_cfg
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [16, 23, 24])
+@pytest.mark.parametrize("n", [16, 23, 24, 31, 32, 39, 40])
 def test_deltanet_blocks_of_tokens(ctx, n):
-    """Two full blocks, and a last block of seven tokens: the state that n single steps leave (below 32 tokens the projections' weights are exact;
-    two layers and the gates amplify the last bits of f32 sums)."""
+    """The longest run token by token, full blocks of eight (from 32 tokens on) and a last block of seven: the state that n single steps leave (Q4_K: exact
+    weights in the projections; two layers and the gates amplify the last bits of f32 sums)."""
     cfg = small_cfg(pb, n_layers=2, full_every=0)
-    m = synth.build_model(ctx, cfg, synth.model_spec(cfg, 9), 9)
+    m = synth.build_model(ctx, cfg, synth.model_spec(cfg, 9, pb.Q4_K), 9)
     a, b = m.new_state(1), m.new_state(1)
     ids = np.random.default_rng(n).integers(0, cfg.vocab, n).astype(np.uint32)
     la = a.forward(ids)
