@@ -458,7 +458,10 @@ int pb_launch_deltanet_seq(pb_ctx* ctx, const PbDeltaParams& p, int T, float* sc
     PB_CUDA(ctx, cudaGetLastError());
     const dim3 grid(p.nv * (p.dv / DN_COLS));
     if (blocks) {
-        pb_launch_k(ctx, pb_deltanet_block_kernel, grid, dim3(128), (size_t)0, p, T, r);
+        // one CTA per SM, by shared memory that it does not use: started while the inputs' CTAs leave, two often met on one SM and took half as long again
+        const size_t apart = (size_t)96 << 10;
+        PB_TRY(pb_ensure_smem(ctx, pb_deltanet_block_kernel, apart));
+        pb_launch_k(ctx, pb_deltanet_block_kernel, grid, dim3(128), apart, p, T, r);
         ctx->kernels_launched++;
         PB_CUDA(ctx, cudaGetLastError());
         return PB_OK;
