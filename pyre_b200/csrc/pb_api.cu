@@ -126,7 +126,7 @@ bool pb_host_pinned(const void* p) {
 }
 // Small copies between device and page-locked host memory by a kernel, 16 bytes a thread: a copy through the copy engine is handed over twice, and the status
 // word takes one more (st_dst, null or the host's copy of it).  Latency of the host link bounds it.  Four tokens of 4096 x 2048 through host buffers:
-// 44.7 us by the copy engine, 41.3 so, 37.1 with the call's launches as a chain.
+// 43 us by the copy engine with ordinary launches, 35 so.
 __global__ void __launch_bounds__(256) pb_copy_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, int n, int* st_dst, const int* st_src) {
     const int i = (int)(blockIdx.x * 256 + threadIdx.x);
     pb_pdl_trigger();
@@ -134,7 +134,12 @@ __global__ void __launch_bounds__(256) pb_copy_kernel(uint4* __restrict__ dst, c
     if (i < n) dst[i] = src[i];
     if (i == 0 && st_dst) *st_dst = *st_src;
 }
-#define PB_COPY_IN ((size_t)128 << 10)    // a copy engine moves more than this faster than a kernel's reads over the link
+// Sizes, us a call by kernel / engine.  Inputs of up to 24 KB are the engine's: the driver sends them along with the command (2 KB to 512 x 512 24.0 / 22.8,
+// 8 KB to 4096 x 2048 32.4 / 30.5, to 151936 x 2048 of IQ3_S 81.5 / 78.5; 24 KB to 12352 x 2048 40.5 / 39.5, 32 KB 42.5 / 43.5).  From there the kernel's
+// advantage grows (64 KB 37 / 42, 128 KB 44 / 49) and is gone at half a megabyte (256 KB 56 / 57, 512 KB 84 / 83).  Results gain at every size (16 KB 29 / 34,
+// 256 KB 37 / 46, 1.5 MB 71 / 73).  Both limits stand where they gain most of what there is.
+#define PB_COPY_IN_OVER ((size_t)24 << 10)
+#define PB_COPY_IN ((size_t)128 << 10)
 #define PB_COPY_OUT ((size_t)256 << 10)
 static bool copy_fits(const void* dst, const void* src, size_t bytes, size_t most) {
     return bytes > 0 && bytes <= most && bytes % 16 == 0 && (((uintptr_t)dst | (uintptr_t)src) & 15) == 0;
@@ -162,11 +167,11 @@ int pb_h2d(pb_ctx* ctx, void* dst, const void* src, size_t bytes, size_t off) {
     bool stage = off + bytes <= PB_PIN_MAX && !pb_host_pinned(src);
     if (stage) PB_TRY(pin_room(ctx, off + bytes, &stage));
     const void* dev = stage ? ctx->pin + off : (bytes <= PB_COPY_IN && g_host.inside(src, bytes) ? src : nullptr);   // (other page-locked memory: the copy engine)
-    if (dev && copy_fits(dst, dev, bytes, PB_COPY_IN)) {
+    if (dev && bytes > PB_COPY_IN_OVER && copy_fits(dst, dev, bytes, PB_COPY_IN)) {
         if (stage) memcpy(ctx->pin + off, src, bytes);
         return copy_small(ctx, dst, dev, bytes, false);
     }
-    // staged in pieces: the link moves one while the next is written
+    // staged in pieces: the link moves one while the next is written (512 KB 83 us a call in pieces of 256 KB, 87 of 128 KB, 103 of 64 KB, 84 in one)
     const size_t piece = stage ? (size_t)256 << 10 : bytes;
     for (size_t i = 0, n; i < bytes; i += n) {
         n = bytes - i < piece ? bytes - i : piece;
