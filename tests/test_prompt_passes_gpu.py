@@ -68,6 +68,40 @@ def test_several_chunks_in_one_pass(ctx, n):
     a.destroy(); b.destroy(); m.destroy()
 
 
+@pytest.mark.parametrize("name,start,kw", [
+    ("Q4_K", 0, dict(kv_bits=4)),                              # projections in launches of 32, experts at the warp level
+    ("IQ3_S", 0, dict(kv_bits=0)),                             # f32 cache
+    ("IQ3_S", 40, dict(kv_bits=4)),                            # off the grid: a piece up to the next multiple of 256 goes first
+    ("IQ3_S", 256, dict(kv_bits=4)),                           # on it
+    ("IQ3_S", 0, dict(kv_bits=4, full_every=2, n_rot=32)),     # attention without the shared tiles, two layers of it
+    ("IQ3_S", 0, dict(kv_bits=4, lin_dk=64)),                  # no blocks of tokens in the recurrence
+])
+@pytest.mark.parametrize("n", [560, 600, 1060])
+def test_several_chunks_in_one_pass_of_other_models_and_starts(ctx, name, start, kw, n):
+    """Two to four chunks and a rest of 36 to 88 tokens: one call with passes over several chunks against one with a pass per chunk.  That the first call
+    has such passes shows in the memory of their row buffers, which turning them off gives back."""
+    import torch
+    cfg = small_cfg(pb, max_ctx=1400, **kw)
+    m = synth.build_model(ctx, cfg, synth.model_spec(cfg, 12, getattr(pb, name)), 12)
+    rng = np.random.default_rng(n)
+    before, ids = rng.integers(0, cfg.vocab, 256).astype(np.uint32)[:start], rng.integers(0, cfg.vocab, n).astype(np.uint32)
+    got = []
+    a, b = m.new_state(1), m.new_state(1)
+    for st in (a, b):
+        if start:
+            st.forward(before)
+        if st is b:
+            ctx.sync(); free = torch.cuda.mem_get_info(0)[0]
+            m.prompt_passes(False)
+            assert torch.cuda.mem_get_info(0)[0] >= free + (16 << 20)
+        lg = st.forward(ids)
+        got.append((lg, *[x for il in range(cfg.n_layers) if (il + 1) % cfg.full_every for x in st.get_lin(il)], st.decode_greedy([5], 8)))
+    for u, v in zip(*got):
+        assert np.array_equal(np.asarray(u).view(np.uint32), np.asarray(v).view(np.uint32))
+    assert ctx.device_status() == 0
+    a.destroy(); b.destroy(); m.destroy()
+
+
 @pytest.mark.parametrize("t", [31, 32, 97, 161])
 def test_expert_groups_of_many_entries(ctx, t):
     """16 experts, 4 per token: around the number of tokens from which the tcgen05 kernels take over, and groups of up to 24 entries with ragged ends; the
