@@ -389,11 +389,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) pb_gemmtc_iq3s_kernel(const TcP
 
 bool pb_gemmtc_supported(int type, int cols, int t) { return type == PB_T_IQ3_S && t >= 16 && cols % 256 == 0 && cols >= 256; }
 
-// Fewest tokens the dispatchers send here.  The kernel works from 16 tokens on; there the warp-level kernel, which takes 16 tokens a launch, is the
-// shorter one on every matrix (us, this kernel / that one: 4096 x 2048 17.6 / 12.5, 12351 x 2048 25.5 / 17.4, 151936 x 2048 181 / 82).  From its second
-// launch on it is not (17 tokens 18.0 / 19.6, 25.7 / 27.2, 181 / 119; 31 tokens 18.6 / 24.9, 26.8 / 33.9, 185 / 163; 33 tokens 18.6 / 33.0, 26.8 / 45.4,
-// 188 / 211), but its weights are exact, and here they are rounded to f16 (2e-4 of the result against 1e-7): the line stays where two launches
-// end.  PYRE_B200_TC_MIN overrides (tests run the kernel at 16).
+// Fewest tokens the dispatchers send here.  The kernel works from 16 tokens on; there the warp-level kernel is as short or shorter (us, this kernel / that
+// one: 4096 x 2048 12.4 / 12.4, 12351 x 2048 20.5 / 16.7, 151936 x 2048 153 / 82).  From 17 tokens on that one is longer on the layers' matrices, in one launch
+// (4096 x 2048, 17 tokens 13.3 / 14.4, 31 14.4 / 17.6) and in two (12351 x 2048, 20.6 / 24.7 and 20.6 / 31.8), and from 32 on the lm-head (31 tokens
+// 158 / 158, 33 162 / 195); but its weights are exact, and here they are rounded to f16 (2e-4 of the result against 1e-7): up to 31 tokens, the longest call
+// that the warp-level kernel takes in two launches at most, results keep their exact weights.  PYRE_B200_TC_MIN overrides (tests run the kernel at 16).
 int pb_gemmtc_min_tokens() {
     const char* e = getenv("PYRE_B200_TC_MIN");
     const int v = e ? atoi(e) : 32;

@@ -24,13 +24,12 @@ struct pb_ctx {
     void* scratch = nullptr;
     size_t scratch_bytes = 0;
     uint64_t kernels_launched = 0;
-    // expert-parallel group (pb_ep.cu); ep_comm is an ncclComm_t
-    // programmatic dependent launch is used only inside the token step, where every stream op is ours
+    // programmatic dependent launch is used only inside a token step, a window or one call's launches (PbChain), where every stream op is ours
     bool use_pdl = true;
     bool step_pdl = true;    // the fused step kernel takes part in the dependent-launch chain (PYRE_B200_STEP_PDL=0: it does not)
-    int pdl_scope = 0;       // > 0 while run_step is issuing launches
+    int pdl_scope = 0;       // > 0 while a step, a window or a call is issuing its launches
     bool pdl_chain = false;  // the previous op on the stream was one of our kernels
-    void* ep_comm = nullptr;
+    void* ep_comm = nullptr; // expert-parallel group (pb_ep.cu): an ncclComm_t
     int ep_rank = 0, ep_world = 1;
     // tracing: stamp slots handed to the launches of the streaming kernels while enabled (pb_ctx_stamps_enable)
     unsigned long long* stamps = nullptr; int stamp_slots = 0, stamp_next = 0;

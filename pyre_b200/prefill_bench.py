@@ -4,9 +4,9 @@
 
 Builds the synthetic model (`--layers` of the 48 layers of the benchmark shapes, 4-bit KV cache), feeds a seeded
 random prompt from an empty context and prints wall-clock milliseconds and tokens per second per repetition.  The
-prompt runs in 256-token chunks on the absolute grid; the first repetition includes the eager chunk and the capture of
-the chunk graph.  With a small `--layers` and `--tokens 256` this is the command to put under a profiler for the launch
-list of one chunk.
+prompt runs in passes of up to four 256-token chunks on the absolute grid; the first repetition includes the loading of the
+kernels.  With a small `--layers` this is the command to put under a profiler for the launch list of a pass (`--tokens 1024`)
+or of one chunk (`--tokens 256`).
 """
 from __future__ import annotations
 
