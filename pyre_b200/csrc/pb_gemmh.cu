@@ -239,7 +239,9 @@ static int gh_round(pb_ctx* ctx, int nt, int nw, size_t smem, int ks, int* tiles
 // longest decodes (31 tokens of 4096 x 4096 IQ3_XXS 47.2 / 43.2, 9472 x 2048 IQ1_M 45.4 / 41.0), for 18 to 24 tokens (9472 x 2048 Q8_0 36.9 / 32.8) except
 // for short decodes in clusters of eight (4096 x 4096, 20 tokens: IQ3_S 23.8 / 24.6, Q4_K 26.9 / 28.7), and from 29 on but for the two shortest (31 tokens of
 // 9472 x 2048 Q6_K 45.1 / 42.9, IQ3_S 27.7 / 28.7); not for a single seventeenth token, which the dp4a kernel takes (9472 x 2048 Q4_0 28.7 / 30.8), nor
-// for 25 to 28 (25 tokens of 4096 x 4096 Q4_0 36.9 / 39.0).  Two rounds are left to two launches (24 tokens of 151936 x 2048 IQ3_S 138 / 221).
+// for 25 to 28 (25 tokens of 4096 x 4096 Q4_0 36.9 / 39.0).  Several rounds are shorter in two launches (24 tokens of 151936 x 2048 IQ3_S 138 / 221); at one and a
+// half the formats differ (12351 x 2048, 17 tokens IQ3_S 24.6 / 26.7, Q4_K 30.8 / 30.7; 24 tokens IQ3_S 26.9 / 26.7, IQ2_XS 41.0 / 32.8, Q8_0 47.2 / 38.9; 25
+// tokens IQ3_S 28.7 / 32.7, Q8_0 49.2 / 57.4, IQ3_XXS 55.3 / 49.2) and two launches are kept for all.
 template <int FMT>
 static int gh_one_launch(pb_ctx* ctx, int cols, int all, int r, int ks16, int ks32, bool* one) {
     *one = false;

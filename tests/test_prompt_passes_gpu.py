@@ -1,5 +1,7 @@
 """Prompt passes and the kernels that only they and large batches reach: runs of the DeltaNet recurrence in blocks of eight tokens, the router and its lists for many tokens,
 several prompt chunks in one pass, expert groups of up to 24 entries."""
+import os
+
 import numpy as np
 import pytest
 
@@ -93,7 +95,8 @@ def test_several_chunks_in_one_pass_of_other_models_and_starts(ctx, name, start,
         if st is b:
             ctx.sync(); free = torch.cuda.mem_get_info(0)[0]
             m.prompt_passes(False)
-            assert torch.cuda.mem_get_info(0)[0] >= free + (16 << 20)
+            if name != "IQ3_S" or os.environ.get("PYRE_B200_REPACK") != "0":       # (without re-coded copies IQ3_S has no experts on the tensor cores, and no such passes)
+                assert torch.cuda.mem_get_info(0)[0] >= free + (16 << 20)
         lg = st.forward(ids)
         got.append((lg, *[x for il in range(cfg.n_layers) if (il + 1) % cfg.full_every for x in st.get_lin(il)], st.decode_greedy([5], 8)))
     for u, v in zip(*got):
